@@ -768,7 +768,7 @@ __device__ __forceinline__ uint32_t pack_rgba8(const GaussRec& R, float a)
 // [54:0] value.  Epoch 0 means "not yet written in this use".  Values are
 // kept mod 2^55: the sort's digit counts, the run counts and the u32 scans
 // (whose sums are wanted mod 2^32) stay far below that; the u64 scan, whose
-// prefixes may use all 64 bits, uses lookback_exclusive_wide.
+// prefixes may use all 64 bits, uses lookback_exclusive_warp.
 // ------------------------------------------------------------------------
 constexpr uint64_t LB_VALUE_MASK = (1ull << 55) - 1ull;
 constexpr uint64_t LB_INCL = 1ull << 55;
@@ -866,55 +866,80 @@ __device__ __forceinline__ uint64_t lookback_exclusive(uint64_t* status, uint64_
     return lookback_walk(status, tile, aggregate, epoch, err, stride, max_op);
 }
 
-// The same walk for sums that may use all 64 bits (the prefix is exact mod
-// 2^64, as uint64 addition is).  Per tile four words: the aggregate's low and
-// high halves, then the inclusive prefix's, each word (epoch << 32) | half.
-// Every word is written once per use, so two halves that both carry the
-// current epoch belong to the same value: a reader can never combine halves
-// of different values.
-__device__ __forceinline__ uint64_t lookback_exclusive_wide(uint64_t* status, uint64_t tile, uint64_t aggregate,
+// The same for sums that may use all 64 bits (the prefix is exact mod 2^64, as
+// uint64 addition is), walked by a whole warp: every lane of it must call, and
+// gets the exclusive prefix.  Per tile four words: the aggregate's low and high
+// halves, then the inclusive prefix's, each word (epoch << 32) | half.  Every
+// word is written once per use and carries its own tag, so two halves that both
+// carry the current epoch belong to the same value, and no order among the
+// words matters (relaxed accesses).
+// A launch's tiles start together, so a tile's nearest inclusive prefix may be
+// hundreds of tiles back, and a walk of one thread is a chain of that many L2
+// round trips; here a round trip covers 32 tiles (lane i reads the predecessor
+// p - i): the scans of a 2M-Gaussian call 1.31 -> 0.30 ms.
+__device__ __forceinline__ void st_relaxed_u64(uint64_t* p, uint64_t v)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p)
+{
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ uint64_t lookback_exclusive_warp(uint64_t* status, uint64_t tile, uint64_t aggregate,
                                                             uint32_t epoch, int* err)
 {
+    const int lane = threadIdx.x & 31;
     const LbControl ctl = lb_control(err);
     const uint64_t tag = (uint64_t)epoch << 32;
     uint64_t* mine = status + 4 * tile;
-    if (tile > 0 && !ctl.withhold)
-    {
-        st_release_u64(mine + 0, tag | (aggregate & 0xffffffffull));
-        st_release_u64(mine + 1, tag | (aggregate >> 32));
-    }
+    if (tile > 0 && !ctl.withhold && lane < 2)
+        st_relaxed_u64(mine + lane, tag | (lane ? aggregate >> 32 : aggregate & 0xffffffffull));
     uint64_t excl = 0;
     int64_t p = (int64_t)tile - 1;
     uint32_t spins = 0;
     while (p >= 0)
     {
-        const uint64_t* w = status + 4 * (uint64_t)p;
-        const uint64_t il = ld_acquire_u64(w + 2), ih = ld_acquire_u64(w + 3);
-        if ((il >> 32) == epoch && (ih >> 32) == epoch)
+        const int64_t q = p - lane;
+        bool incl = q < 0, ready = incl; // before the first tile: an inclusive prefix of 0
+        uint64_t v = 0;
+        if (q >= 0)
         {
-            excl += (ih << 32) | (il & 0xffffffffull);
-            break;
+            const uint64_t* w = status + 4 * (uint64_t)q;
+            const uint64_t al = ld_relaxed_u64(w + 0), ah = ld_relaxed_u64(w + 1);
+            const uint64_t il = ld_relaxed_u64(w + 2), ih = ld_relaxed_u64(w + 3);
+            incl = (il >> 32) == epoch && (ih >> 32) == epoch;
+            ready = incl || ((al >> 32) == epoch && (ah >> 32) == epoch);
+            v = incl ? (ih << 32) | (il & 0xffffffffull) : (ah << 32) | (al & 0xffffffffull);
         }
-        const uint64_t al = ld_acquire_u64(w + 0), ah = ld_acquire_u64(w + 1);
-        if ((al >> 32) == epoch && (ah >> 32) == epoch)
+        const uint32_t mi = __ballot_sync(0xffffffffu, incl), mr = __ballot_sync(0xffffffffu, ready);
+        const int first_incl = mi ? __ffs(mi) - 1 : 32, first_gap = ~mr ? __ffs(~mr) - 1 : 32;
+        const int take = first_incl < first_gap ? first_incl + 1 : first_gap; // lanes [0, take) are added
+        if (take == 0)
         {
-            excl += (ah << 32) | (al & 0xffffffffull);
-            p--;
+            if (++spins > ctl.limit)
+            {
+                if (lane == 0)
+                    atomicOr(err, 1); // ERR_LOOKBACK
+                break;
+            }
+            __nanosleep(32);
             continue;
         }
-        if (++spins > ctl.limit)
-        {
-            atomicOr(err, 1); // ERR_LOOKBACK
+        uint64_t c = lane < take ? v : 0;
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+            c += __shfl_xor_sync(0xffffffffu, c, o);
+        excl += c;
+        if (first_incl < first_gap)
             break;
-        }
-        __nanosleep(32);
+        p -= take;
     }
     const uint64_t incl = excl + aggregate;
-    if (!ctl.withhold)
-    {
-        st_release_u64(mine + 2, tag | (incl & 0xffffffffull));
-        st_release_u64(mine + 3, tag | (incl >> 32));
-    }
+    if (!ctl.withhold && lane < 2)
+        st_relaxed_u64(mine + 2 + lane, tag | (lane ? incl >> 32 : incl & 0xffffffffull));
     return excl;
 }
 

@@ -38,6 +38,8 @@ size_t scan_status_words(int64_t n)
     return 4 * ((size_t)((n + SCAN_TILE - 1) / SCAN_TILE) + 1);
 }
 
+// VEC: in and out are 16-byte aligned (full tiles move as 16-byte words)
+template <bool VEC>
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_excl(const uint64_t* in, uint64_t* out, int64_t n, int mode,
                                                             uint64_t* total, uint64_t* status, uint32_t epoch,
                                                             uint32_t* counter, int* err)
@@ -46,40 +48,66 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_excl(const uint64_t* in, ui
     __shared__ uint64_t s_excl;
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0)
-        s_tile = atomicAdd(counter, 1u);
+        s_tile = counter ? atomicAdd(counter, 1u) : 0u; // no counter: a single tile
     __syncthreads();
     const uint64_t tile = s_tile;
     const int64_t base = (int64_t)tile * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+    const bool full = VEC && ((int64_t)tile + 1) * SCAN_TILE <= n;
     uint64_t v[SCAN_ITEMS];
+    if (full)
+    {
+        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(in + base);
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS / 2; i++)
+        {
+            const ulonglong2 x = src[i];
+            v[2 * i] = x.x;
+            v[2 * i + 1] = x.y;
+        }
+    }
+    else
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; i++)
+            v[i] = base + i < n ? in[base + i] : 0ull;
     uint64_t sum = 0;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++)
     {
-        int64_t idx = base + i;
-        uint64_t x = idx < n ? in[idx] : 0ull;
         if (mode & 1)
-            x = (uint64_t)__popcll(x);
-        v[i] = x;
-        sum += x;
+            v[i] = (uint64_t)__popcll(v[i]);
+        sum += v[i];
     }
     uint64_t block_total;
-    uint64_t texcl = block_excl_scan_u64(sum, s_warp, block_total);
-    if (threadIdx.x == 0)
-        s_excl = lookback_exclusive_wide(status, tile, block_total, epoch, err);
+    const uint64_t texcl = block_excl_scan_u64(sum, s_warp, block_total);
+    if (threadIdx.x < 32)
+    {
+        const uint64_t e = lookback_exclusive_warp(status, tile, block_total, epoch, err);
+        if (threadIdx.x == 0)
+            s_excl = e;
+    }
     __syncthreads();
     uint64_t run = s_excl + texcl;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++)
     {
-        int64_t idx = base + i;
-        if (idx < n)
-        {
-            out[idx] = (mode & 2) ? run + v[i] : run;
-            run += v[i];
-            if (idx == n - 1)
-                *total = run;
-        }
+        const uint64_t next = run + v[i];
+        if (base + i == n - 1)
+            *total = next;
+        v[i] = (mode & 2) ? next : run;
+        run = next;
     }
+    if (full)
+    {
+        ulonglong2* dst = reinterpret_cast<ulonglong2*>(out + base);
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS / 2; i++)
+            dst[i] = make_ulonglong2(v[2 * i], v[2 * i + 1]);
+    }
+    else
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; i++)
+            if (base + i < n)
+                out[base + i] = v[i];
 }
 
 void scan_exclusive_u64(const uint64_t* in, uint64_t* out, int64_t n, int mode, uint64_t* total, uint64_t* status,
@@ -91,9 +119,15 @@ void scan_exclusive_u64(const uint64_t* in, uint64_t* out, int64_t n, int mode, 
         cudaMemsetAsync(total, 0, sizeof(uint64_t), s);
         return;
     }
-    cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    { k_scan_excl<<<(unsigned)tiles, SCAN_BLOCK, 0, s>>>(in, out, n, mode, total, status, epoch, counter, err); count_launch(); }
+    const int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+    if (tiles == 1)
+        counter = nullptr;
+    else
+        cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
+    const bool vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0;
+    auto kern = vec ? k_scan_excl<true> : k_scan_excl<false>;
+    kern<<<(unsigned)tiles, SCAN_BLOCK, 0, s>>>(in, out, n, mode, total, status, epoch, counter, err);
+    count_launch();
 }
 
 // u32 scans: the reference's global_scan (sum, wrapping mod 2^32) and
