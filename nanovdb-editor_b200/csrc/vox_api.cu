@@ -68,13 +68,12 @@ struct vox_context_t
     DevBuf recs, footprints, frag_off, root_bits, root_prefix, root_of_rank, lower_bits, lower_prefix, lower_cell;
     DevBuf scan_status, run_status;
     DevBuf keys, ids, keys_alt, ids_alt, sort_ws;
-    DevBuf vox_start, leaf_vstart, lower_lstart, lower_rank;
-    DevBuf lower_origin, lower_upper_n, upper_head, upper_scan, lower_parent, upper_root_n, upper_lostart;
-    DevBuf leaf_lower, leaf_lower_n, leaf_mask, leaf_origin;
-    DevBuf vox_leaf, vox_n, rank_to_lower;
+    DevBuf leaf_vstart, lower_lstart;
+    DevBuf lower_upper_n, lower_parent, upper_root_n, upper_lostart;
+    DevBuf leaf_cand, leaf_lower, leaf_lower_n, leaf_origin;
     // leaf-granular pipeline
     DevBuf cand_org, tile_g0, lcols, lcol_off, lc_count, lc_mask, lc_off, emit_gid, emit_flag, lflags, lpos, cand_key, cand_start, cand_mask, pair_gid;
-    DevBuf s_rgba, s_dens, s_col, s_pairs, cand_cnt, cand_voff, vkeys, vslot, vpairs, pair_off, cand_vbase, cloud_pairs;
+    DevBuf s_rgba, s_dens, s_col, s_pairs, cand_voff, vpairs, pair_off, cand_vbase, cloud_pairs;
     DevBuf partials, exp_keys, exp_ids;
     // reference node order
     DevBuf nwin, win_before, cand_wkey, wkey_u, wkey_lo, wkey_leaf, wcnt, wbase, okeys, okeys_alt, ovals, ovals_alt;
@@ -282,7 +281,7 @@ static int window_order(vox_context_t* ctx, NodeParams& N, int64_t U, int64_t Lo
     uint64_t* cnt = (uint64_t*)ctx->wcnt.p; // [3][W]
     uint64_t* base = (uint64_t*)ctx->wbase.p; // [4][W + 1]
     cudaMemsetAsync(cnt, 0, 8 * 3 * (size_t)W, s);
-    launch_leaf_wkey(L, N.leaf_vstart, (const uint32_t*)ctx->vslot.p, (const uint64_t*)ctx->cand_wkey.p, wk_leaf, s);
+    launch_leaf_wkey(L, N.leaf_cand, (const uint64_t*)ctx->cand_wkey.p, wk_leaf, s);
     launch_run_min(Lo, N.lower_lstart, wk_leaf, wk_lo, s);
     launch_run_min(U, N.upper_lostart, wk_lo, wk_u, s);
     const int key_bits = 40 + bits_for((uint64_t)W + 1);
@@ -502,7 +501,6 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
 
     // ---------------------------------------------------------- leaf pairs
     RankTables T{ root_bits, root_prefix, lower_bits, lower_prefix };
-    const size_t kb = key64 ? 8 : 4;
     const int leaf_key_bits = 12 + bits_for(NL > 1 ? NL : 2);
     if (leaf_key_bits > 32)
     {
@@ -623,12 +621,8 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     const size_t slots = 512 * (size_t)(NCL + 1);
     if (!ensure(ctx, ctx->cand_mask, 64 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->s_rgba, 4 * slots) ||
         !ensure(ctx, ctx->s_dens, 4 * slots) || !ensure(ctx, ctx->s_col, 12 * slots) || !ensure(ctx, ctx->s_pairs, 4 * slots) ||
-        !ensure(ctx, ctx->cand_cnt, 8 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->cand_voff, 8 * (size_t)(NCL + 1)) ||
-        !ensure(ctx, ctx->cand_vbase, 8 * (size_t)(NCL + 1)) ||
-        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * scan_status_words(NCL + 1) * 2))
+        !ensure(ctx, ctx->cand_voff, 8 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->cand_vbase, 8 * (size_t)(NCL + 1)))
         return VOX_ERR_MEMORY;
-    scan_status = (uint64_t*)ctx->scan_status.p;
-    scan_words = ctx->scan_status.cap / sizeof(uint64_t);
     uint64_t* win_before = nullptr;
     if (window)
     {
@@ -676,103 +670,34 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     ctx->walk_variant = ctx->walk_choice[ctx->walk_mode].pick((int64_t)Q);
     ctx->stats.walk_ctas_per_sm = launch_leaf_pass(LP, d_counter, ctx->num_sms, s, ctx->walk_variant);
     cudaEventRecord(ctx->timers.ev[4], s);
-    launch_leaf_popc(LP.cand_mask, NCL, (uint64_t*)ctx->cand_cnt.p, s);
-    scan_exclusive_u64((const uint64_t*)ctx->cand_cnt.p, (uint64_t*)ctx->cand_voff.p, NCL, 0, sc + SC_NVOX, scan_status,
-                       ctx->scan_epochs.next(scan_status, scan_words, s), d_counter, d_err, ctx->num_sms, s);
-    rc = sync_scalars(ctx, "leaf walk");
-    if (rc)
-        return rc;
-    const int64_t VX = (int64_t)ctx->hscal[SC_NVOX];
-    const int64_t P_pairs = (int64_t)ctx->hscal[SC_P];
-    ctx->stats.pairs = P_pairs;
-    ctx->last_P = P_pairs;
-    if (!ensure(ctx, ctx->vkeys, kb * (size_t)(VX + 1)) || !ensure(ctx, ctx->vslot, 4 * (size_t)(VX + 1)))
-        return VOX_ERR_MEMORY;
-    launch_voxel_keys(LP.cand_mask, LP.cand_key, LP.cand_voff, NCL, ctx->vkeys.p, key64, (uint32_t*)ctx->vslot.p, s);
-    const void* skeys = ctx->vkeys.p;
 
-    // ------------------------------------------- runs over the voxel keys
-    const int64_t rtiles = runs_tile_count(VX);
-    if (!ensure(ctx, ctx->vox_start, 4 * (size_t)(VX + 2)) || !ensure(ctx, ctx->leaf_vstart, 4 * (size_t)(VX + 2)) ||
-        !ensure(ctx, ctx->lower_lstart, 4 * (size_t)(NL + 2)) || !ensure(ctx, ctx->lower_rank, 4 * (size_t)(NL + 2)) ||
-        !ensure(ctx, ctx->run_status, sizeof(uint64_t) * 3 * (size_t)(rtiles + 1)) ||
-        !ensure(ctx, ctx->vox_leaf, 4 * (size_t)(VX + 2)) || !ensure(ctx, ctx->vox_n, 2 * (size_t)(VX + 2)))
-        return VOX_ERR_MEMORY;
-    RunParams Rp;
-    Rp.P = VX;
-    Rp.vox_start = (uint32_t*)ctx->vox_start.p;
-    Rp.vox_leaf = (uint32_t*)ctx->vox_leaf.p;
-    Rp.vox_n = (uint16_t*)ctx->vox_n.p;
-    Rp.leaf_vstart = (uint32_t*)ctx->leaf_vstart.p;
-    Rp.lower_lstart = (uint32_t*)ctx->lower_lstart.p;
-    Rp.lower_rank = (uint32_t*)ctx->lower_rank.p;
-    Rp.counts = sc + SC_V;
-    Rp.status = (uint64_t*)ctx->run_status.p;
-    Rp.epoch = ctx->run_epochs.next(Rp.status, ctx->run_status.cap / sizeof(uint64_t), s);
-    Rp.counter = d_counter;
-    Rp.err = d_err;
-    Rp.lower_cap = NL + 2;
-    if (VX == 0)
-    {
-        cudaMemsetAsync(Rp.vox_start, 0, 4, s);
-        cudaMemsetAsync(Rp.leaf_vstart, 0, 4, s);
-        cudaMemsetAsync(Rp.lower_lstart, 0, 4, s);
-    }
-    launch_runs(Rp, skeys, key64, s);
-    rc = sync_scalars(ctx, "runs");
-    if (rc)
-        return rc;
-    const int64_t V = (int64_t)ctx->hscal[SC_V], L = (int64_t)ctx->hscal[SC_L], Lo = (int64_t)ctx->hscal[SC_LO];
-
-    // ---------------------------------------------------------- node tables
-    if (!ensure(ctx, ctx->lower_origin, 12 * (size_t)(Lo + 1)) || !ensure(ctx, ctx->lower_upper_n, 4 * (size_t)(Lo + 1)) ||
-        !ensure(ctx, ctx->upper_head, 8 * (size_t)(Lo + 1)) || !ensure(ctx, ctx->upper_scan, 8 * (size_t)(Lo + 1)) ||
-        !ensure(ctx, ctx->lower_parent, 4 * (size_t)(Lo + 1)) || !ensure(ctx, ctx->upper_root_n, 4 * (size_t)(Lo + 1)) ||
-        !ensure(ctx, ctx->upper_lostart, 4 * (size_t)(Lo + 2)) || !ensure(ctx, ctx->leaf_lower, 4 * (size_t)(L + 1)) ||
-        !ensure(ctx, ctx->leaf_lower_n, 4 * (size_t)(L + 1)) || !ensure(ctx, ctx->leaf_mask, 64 * (size_t)(L + 1)) ||
-        !ensure(ctx, ctx->leaf_origin, 12 * (size_t)(L + 1)) || !ensure(ctx, ctx->rank_to_lower, 4 * (size_t)(NL + 1)) ||
-        !ensure(ctx, ctx->order, 8 * 3 * (size_t)((Lo + 1) * 2 + (L + 1))) ||
-        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * scan_status_words(Lo + 1) * 2))
-        return VOX_ERR_MEMORY;
-    // per-cloud tables: 3 x (B + 1) u32 starts, L u32 leaf clouds, 9 x (B + 1) u64 layout words, 6 B i32 bbox
+    // ------------------------------------------------ tree: tables and layout
+    // leaves <= candidates, lowers <= min(touched lower cells, candidates), uppers <= lowers
+    const size_t lcap = (size_t)std::min<uint64_t>(NL, (uint64_t)NCL) + 2;
+    // per-cloud tables: 3 x (B + 1) u32 starts, NCL u32 leaf clouds, 9 x (B + 1) u64 layout words, 6 B i32 bbox
     const size_t cl_u32 = 3 * (size_t)(B + 1), cl_u64 = 9 * (size_t)(B + 1);
-    const size_t cl_bytes = 8 * cl_u64 + 4 * (cl_u32 + (size_t)L + 6 * (size_t)B) + 64;
-    if (!ensure(ctx, ctx->clouds, cl_bytes))
+    const size_t cl_bytes = 8 * cl_u64 + 4 * (cl_u32 + (size_t)NCL + 6 * (size_t)B) + 64;
+    if (!ensure(ctx, ctx->leaf_vstart, 4 * (size_t)(NCL + 2)) || !ensure(ctx, ctx->leaf_cand, 4 * (size_t)(NCL + 1)) ||
+        !ensure(ctx, ctx->leaf_lower, 4 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->leaf_lower_n, 4 * (size_t)(NCL + 1)) ||
+        !ensure(ctx, ctx->leaf_origin, 12 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->lower_lstart, 4 * lcap) ||
+        !ensure(ctx, ctx->lower_upper_n, 4 * lcap) || !ensure(ctx, ctx->lower_parent, 4 * lcap) ||
+        !ensure(ctx, ctx->upper_root_n, 4 * lcap) || !ensure(ctx, ctx->upper_lostart, 4 * lcap) ||
+        !ensure(ctx, ctx->run_status, sizeof(uint64_t) * tree_status_words(NCL)) || !ensure(ctx, ctx->clouds, cl_bytes))
         return VOX_ERR_MEMORY;
-    scan_status = (uint64_t*)ctx->scan_status.p;
-    scan_words = ctx->scan_status.cap / sizeof(uint64_t);
-    NodeParams N;
-    N.Lo = Lo;
-    N.L = L;
-    N.lower_rank = (const uint32_t*)ctx->lower_rank.p;
+    NodeParams N{};
     N.lower_cell = (const uint32_t*)ctx->lower_cell.p;
     N.root_of_rank = (const uint32_t*)ctx->root_of_rank.p;
-    N.lower_lstart = (const uint32_t*)ctx->lower_lstart.p;
-    N.leaf_vstart = (const uint32_t*)ctx->leaf_vstart.p;
-    N.vox_start = (const uint32_t*)ctx->vox_start.p;
-    N.lower_origin = (int32_t*)ctx->lower_origin.p;
+    N.cand_mask = LP.cand_mask;
+    N.lower_lstart = (uint32_t*)ctx->lower_lstart.p;
     N.lower_upper_n = (uint32_t*)ctx->lower_upper_n.p;
-    N.rank_to_lower = (uint32_t*)ctx->rank_to_lower.p;
-    N.upper_head = (uint64_t*)ctx->upper_head.p;
-    N.upper_scan = (uint64_t*)ctx->upper_scan.p;
     N.lower_parent = (uint32_t*)ctx->lower_parent.p;
     N.upper_root_n = (uint32_t*)ctx->upper_root_n.p;
     N.upper_lostart = (uint32_t*)ctx->upper_lostart.p;
-    N.upper_count = sc + SC_U;
+    N.leaf_vstart = (uint32_t*)ctx->leaf_vstart.p;
+    N.leaf_cand = (uint32_t*)ctx->leaf_cand.p;
     N.leaf_lower = (uint32_t*)ctx->leaf_lower.p;
     N.leaf_lower_n = (uint32_t*)ctx->leaf_lower_n.p;
-    N.leaf_mask = (uint64_t*)ctx->leaf_mask.p;
     N.leaf_origin = (int32_t*)ctx->leaf_origin.p;
-    uint64_t* ord = (uint64_t*)ctx->order.p;
-    N.upper_idx = ord;
-    N.upper_addr = ord + (Lo + 1);
-    N.upper_vidx = ord + 2 * (Lo + 1);
-    N.lower_idx = ord + 3 * (Lo + 1);
-    N.lower_addr = ord + 4 * (Lo + 1);
-    N.lower_vidx = ord + 5 * (Lo + 1);
-    N.leaf_idx = ord + 6 * (Lo + 1);
-    N.leaf_addr = ord + 6 * (Lo + 1) + (L + 1);
-    N.leaf_vidx = ord + 6 * (Lo + 1) + 2 * (L + 1);
     {
         CloudParams& C = N.C;
         uint64_t* w64 = (uint64_t*)ctx->clouds.p;
@@ -790,28 +715,58 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         C.lower_start = w32 + (B + 1);
         C.leaf_start = w32 + 2 * (B + 1);
         C.leaf_cloud = w32 + cl_u32;
-        C.bbox = (int32_t*)(w32 + cl_u32 + L);
+        C.bbox = (int32_t*)(w32 + cl_u32 + NCL);
         C.cloud_vs = d_cloud_vs;
         C.voxel_size = voxel_size;
         C.cloud_start = d_cloud_start;
         C.frag_off = frag_off;
         C.F_total = sc + SC_F;
         C.G = G;
-        C.P = P_pairs;
-        C.V = V;
         C.node_order = (flags & VOX_FLAG_WINDOW_ORDER) ? 1u : 0u;
-        cudaMemsetAsync(C.upper_start, 0, 4 * cl_u32, s); // clouds without nodes start at 0
+        if (NCL == 0) // no candidate, no tables: every cloud starts (and ends) at 0
+        {
+            cudaMemsetAsync(C.vstart, 0, 8 * (size_t)(B + 1), s);
+            cudaMemsetAsync(C.upper_start, 0, 4 * cl_u32, s);
+        }
     }
-    launch_lower_info(N, s);
-    scan_exclusive_u64(N.upper_head, N.upper_scan, Lo, 0, sc + SC_SCRATCH + 1, scan_status,
-                       ctx->scan_epochs.next(scan_status, scan_words, s), d_counter, d_err, ctx->num_sms, s);
-    launch_upper_info(N, s);
-    launch_leaf_tables(N, skeys, key64, s);
+    TreeParams TP;
+    TP.NCL = NCL;
+    TP.cand_mask = LP.cand_mask;
+    TP.cand_key = LP.cand_key;
+    TP.cand_org = LP.cand_org;
+    TP.cand_voff = (uint64_t*)ctx->cand_voff.p;
+    TP.counts = sc + SC_V;
+    TP.status = (uint64_t*)ctx->run_status.p;
+    TP.epoch = ctx->run_epochs.next(TP.status, ctx->run_status.cap / sizeof(uint64_t), s);
+    TP.counter = d_counter;
+    TP.err = d_err;
+    TP.lower_cap = lcap;
+    launch_tree(TP, N, s);
     launch_cloud_layout(N, s);
     cudaMemcpyAsync(sc + SC_GRID_BYTES, N.C.grid_off + B, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
-    rc = sync_scalars(ctx, "node tables");
+    rc = sync_scalars(ctx, "tree");
     if (rc)
         return rc;
+    const int64_t P_pairs = (int64_t)ctx->hscal[SC_P];
+    const int64_t V = (int64_t)ctx->hscal[SC_V], L = (int64_t)ctx->hscal[SC_L], Lo = (int64_t)ctx->hscal[SC_LO];
+    ctx->stats.pairs = P_pairs;
+    ctx->last_P = P_pairs;
+    N.C.P = P_pairs;
+    N.C.V = V;
+    N.Lo = Lo;
+    N.L = L;
+    if (!ensure(ctx, ctx->order, 8 * 3 * (size_t)((Lo + 1) * 2 + (L + 1))))
+        return VOX_ERR_MEMORY;
+    uint64_t* ord = (uint64_t*)ctx->order.p;
+    N.upper_idx = ord;
+    N.upper_addr = ord + (Lo + 1);
+    N.upper_vidx = ord + 2 * (Lo + 1);
+    N.lower_idx = ord + 3 * (Lo + 1);
+    N.lower_addr = ord + 4 * (Lo + 1);
+    N.lower_vidx = ord + 5 * (Lo + 1);
+    N.leaf_idx = ord + 6 * (Lo + 1);
+    N.leaf_addr = ord + 6 * (Lo + 1) + (L + 1);
+    N.leaf_vidx = ord + 6 * (Lo + 1) + 2 * (L + 1);
     const uint64_t U = Lo > 0 ? ctx->hscal[SC_U] : 0;
     const uint64_t grid_bytes = ctx->hscal[SC_GRID_BYTES];
     if (window)
@@ -829,7 +784,6 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         return VOX_ERR_MEMORY;
     uint8_t* grid = (uint8_t*)ctx->grid.p;
     launch_zero_gaps(N, grid, grid_bytes, s);
-    launch_leaf_masks(N, LP.cand_mask, (const uint32_t*)ctx->vslot.p, s);
     uint64_t* cloud_pairs = nullptr;
     if (B > 1)
     {
@@ -839,22 +793,16 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         cudaMemsetAsync(cloud_pairs, 0, 8 * (size_t)B, s);
     }
     ValueParams VA;
-    VA.V = V;
-    VA.vslot = (const uint32_t*)ctx->vslot.p;
     VA.s_rgba = LP.s_rgba;
     VA.s_dens = LP.s_dens;
     VA.s_col = LP.s_col;
     VA.s_pairs = LP.s_pairs;
     VA.cloud_pairs = cloud_pairs;
     VA.cand_vbase = (uint64_t*)ctx->cand_vbase.p;
-    VA.vox_leaf = (const uint32_t*)ctx->vox_leaf.p;
-    VA.vox_n = (const uint16_t*)ctx->vox_n.p;
     VA.out = grid;
-    launch_values(VA, N, s);
+    launch_write_leaves(VA, N, ctx->num_sms, s);
     N.C.cloud_pairs = cloud_pairs;
-    N.C.P = P_pairs;
     cudaEventRecord(ctx->timers.ev[5], s);
-    launch_leaf_bbox(N, s);
     launch_write_nodes(N, U, grid, s);
     launch_write_headers(N, grid, s);
     ctx->h_grid_off.resize((size_t)B + 1);
@@ -982,21 +930,6 @@ static int run_backward(vox_context_t* ctx, const vox_gaussians_t* gs, const flo
     return VOX_OK;
 }
 
-// coordinates of the active voxels by value index (clouds back to back)
-__global__ void k_voxel_coords(int64_t V, const uint32_t* vox_leaf, const uint16_t* vox_n, const int32_t* leaf_origin,
-                               const uint32_t* leaf_vstart, const uint64_t* leaf_vidx, const uint32_t* leaf_cloud,
-                               const uint64_t* value_base, int32_t* out)
-{
-    int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V)
-        return;
-    const uint32_t l = vox_leaf[v], n = vox_n[v];
-    const uint64_t slot = value_base[leaf_cloud[l]] + leaf_vidx[l] + (uint64_t)(v - leaf_vstart[l]);
-    out[3 * slot + 0] = leaf_origin[3 * l + 0] + (int32_t)(n >> 6);
-    out[3 * slot + 1] = leaf_origin[3 * l + 1] + (int32_t)((n >> 3) & 7);
-    out[3 * slot + 2] = leaf_origin[3 * l + 2] + (int32_t)(n & 7);
-}
-
 // hierarchical key of a compact key: rank -> cell -> (root_n, upper_n)
 __global__ void k_export_keys(const void* keys, int key64, const uint32_t* lower_cell, const uint32_t* root_of_rank,
                               int64_t n, uint64_t* out)
@@ -1063,16 +996,14 @@ void vox_context_destroy(vox_context_t* ctx)
     DevBuf* all[] = { &ctx->recs, &ctx->footprints, &ctx->frag_off, &ctx->root_bits, &ctx->root_prefix,
                       &ctx->root_of_rank, &ctx->lower_bits, &ctx->lower_prefix, &ctx->lower_cell, &ctx->scan_status,
                       &ctx->run_status, &ctx->keys, &ctx->ids, &ctx->keys_alt, &ctx->ids_alt,
-                      &ctx->sort_ws, &ctx->vox_start, &ctx->leaf_vstart, &ctx->lower_lstart, &ctx->lower_rank,
-                      &ctx->lower_origin, &ctx->lower_upper_n, &ctx->upper_head, &ctx->upper_scan,
-                      &ctx->lower_parent, &ctx->upper_root_n, &ctx->upper_lostart, &ctx->leaf_lower,
-                      &ctx->leaf_lower_n, &ctx->leaf_mask, &ctx->leaf_origin, &ctx->order, &ctx->grid, &ctx->scal,
-                      &ctx->vox_leaf, &ctx->vox_n, &ctx->rank_to_lower,
+                      &ctx->sort_ws, &ctx->leaf_vstart, &ctx->lower_lstart, &ctx->lower_upper_n,
+                      &ctx->lower_parent, &ctx->upper_root_n, &ctx->upper_lostart, &ctx->leaf_cand, &ctx->leaf_lower,
+                      &ctx->leaf_lower_n, &ctx->leaf_origin, &ctx->order, &ctx->grid, &ctx->scal,
                       &ctx->hier_keys, &ctx->prim_keys_alt, &ctx->prim_vals_alt, &ctx->vb_work, &ctx->vb_keys, &ctx->vb_ids_c, &ctx->vb_used, &ctx->dual_idx, &ctx->vb_rec, &ctx->cloud_start,
                       &ctx->cloud_vs, &ctx->clouds, &ctx->lcols, &ctx->lcol_off, &ctx->lc_count, &ctx->lc_mask, &ctx->lc_off,
                       &ctx->cand_org, &ctx->tile_g0, &ctx->emit_gid, &ctx->emit_flag, &ctx->lflags, &ctx->lpos, &ctx->cand_key, &ctx->cand_start,
-                      &ctx->cand_mask, &ctx->pair_gid, &ctx->s_rgba, &ctx->s_dens, &ctx->s_col, &ctx->s_pairs, &ctx->cand_cnt,
-                      &ctx->cand_voff, &ctx->vkeys, &ctx->vslot, &ctx->vpairs, &ctx->pair_off, &ctx->cand_vbase, &ctx->cloud_pairs,
+                      &ctx->cand_mask, &ctx->pair_gid, &ctx->s_rgba, &ctx->s_dens, &ctx->s_col, &ctx->s_pairs,
+                      &ctx->cand_voff, &ctx->vpairs, &ctx->pair_off, &ctx->cand_vbase, &ctx->cloud_pairs,
                       &ctx->partials, &ctx->exp_keys, &ctx->exp_ids, &ctx->nwin, &ctx->win_before,
                       &ctx->cand_wkey, &ctx->wkey_u, &ctx->wkey_lo, &ctx->wkey_leaf, &ctx->wcnt, &ctx->wbase,
                       &ctx->okeys, &ctx->okeys_alt, &ctx->ovals, &ctx->ovals_alt, &ctx->rank_u, &ctx->rank_lo,
@@ -1275,8 +1206,7 @@ int vox_voxel_coords(vox_context_t* ctx, int32_t* d_ijk, int64_t capacity)
     if (V == 0)
         return VOX_OK;
     cudaSetDevice(ctx->device);
-    const NodeParams& N = ctx->last_N;
-    { k_voxel_coords<<<(unsigned)((V + 255) / 256), 256, 0, ctx->stream>>>(V, (const uint32_t*)ctx->vox_leaf.p, (const uint16_t*)ctx->vox_n.p, N.leaf_origin, N.leaf_vstart, N.leaf_vidx, N.C.leaf_cloud, N.C.value_base, d_ijk); count_launch(); }
+    launch_voxel_coords(ctx->last_N, d_ijk, ctx->stream);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
         return check_cuda(ctx, "vox_voxel_coords");
     return VOX_OK;
@@ -1308,8 +1238,7 @@ int vox_copy_pairs(vox_context_t* ctx, uint64_t* keys, uint32_t* ids, int64_t ca
         return VOX_ERR_MEMORY;
     uint64_t* scan_status = (uint64_t*)ctx->scan_status.p;
     const size_t scan_words = ctx->scan_status.cap / sizeof(uint64_t);
-    launch_voxel_pairs(V, (const uint32_t*)ctx->vslot.p, (const uint32_t*)ctx->s_pairs.p, (uint64_t*)ctx->vpairs.p,
-                       ctx->stream);
+    launch_voxel_pairs(ctx->last_N, (const uint32_t*)ctx->s_pairs.p, (uint64_t*)ctx->vpairs.p, ctx->stream);
     scan_exclusive_u64((const uint64_t*)ctx->vpairs.p, (uint64_t*)ctx->pair_off.p, V, 0, sc + SC_SCRATCH + 3,
                        scan_status, ctx->scan_epochs.next(scan_status, scan_words, ctx->stream),
                        (uint32_t*)(sc + SC_SCRATCH), (int*)(sc + SC_ERR), ctx->num_sms, ctx->stream);

@@ -18,9 +18,8 @@
 //       its voxels, keeps the RGBA8 maximum (gaussian_frag_color.slang:239-246)
 //       and sums the float channels in (voxel key, Gaussian id) order; the
 //       leaf's value mask comes from ballots;
-//   k_leaf_popc / k_voxel_keys   active voxels as sorted compact keys, which
-//       the run / node-table / node2-writer stage turns into the tree;
-//   k_values      staged values to their value index.
+//   k_write_leaves   once the tree's tables stand (k_tree): staged values to
+//       their value index, leaf nodes, bbox.
 // The adjoint (k_leaf_backward) and the sorted pair list (k_leaf_export)
 // replay the same walk.
 #include <cstdio>
@@ -1383,99 +1382,192 @@ __global__ void __launch_bounds__(LP_THREADS) k_leaf_export(LeafPassParams P, ui
     }
 }
 
-__global__ void k_leaf_popc(const uint64_t* cand_mask, int64_t NCL, uint64_t* counts)
+// ------------------------------------------------------------ leaf output ----
+// lane r of a warp (r < 16): word r of a leaf's value mask as 32-bit words and
+// the active voxels in the words before it
+__device__ __forceinline__ uint32_t leaf_mask_word(const NodeParams& N, int64_t l, int lane, uint32_t& before)
 {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= NCL)
-        return;
-    uint64_t n = 0;
-    for (int w = 0; w < 8; w++)
-        n += (uint64_t)__popcll(cand_mask[8 * c + w]);
-    counts[c] = n;
+    const uint32_t* m32 = reinterpret_cast<const uint32_t*>(N.cand_mask + 8 * (uint64_t)N.leaf_cand[l]);
+    const uint32_t m = lane < 16 ? m32[lane] : 0u;
+    uint32_t incl = __popc(m);
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+            incl += y;
+    }
+    before = incl - __popc(m);
+    return m;
 }
 
-// one warp per candidate leaf, 32 voxels per round: each active voxel's rank is
-// the popcount of the mask bits below it, so the writes are contiguous
-template <class K>
-__global__ void k_voxel_keys(const uint64_t* cand_mask, const uint32_t* cand_key, const uint64_t* cand_voff,
-                             int64_t NCL, K* vkeys, uint32_t* vslot)
+// One warp per leaf (a CTA's warps take consecutive leaves): the leaf's staged
+// values to its value indices, its node2 node (grid_build_finalize.slang) and
+// its share of the cloud's bbox (grid_build_compute_bbox.slang).  A round takes
+// 32 slots of the leaf: staged reads and value writes are runs of consecutive
+// words.  HBM-bound: 24 B read and 20 B written per voxel, 1.04 ms for 106M
+// voxels (4.5 TB/s; the loads of 2 / 4 / 8 rounds in flight: 1.11 / 1.04 / 1.12 ms,
+// of one 1.76 ms).
+constexpr int WL_THREADS = 256;
+constexpr int WL_ROUNDS = 4; // rounds whose loads are in flight together
+
+__global__ void __launch_bounds__(WL_THREADS) k_write_leaves(ValueParams A, NodeParams N, int per_warp)
 {
-    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (c >= NCL)
-        return;
-    const uint32_t* m32 = reinterpret_cast<const uint32_t*>(cand_mask + 8 * c);
-    const uint32_t mine = m32[lane & 15];
-    uint64_t base = cand_voff[c];
-    const uint64_t lk = (uint64_t)cand_key[c] << 9;
+    __shared__ int32_t s_bb[6];
+    __shared__ unsigned long long s_pairs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
+    const CloudParams& C = N.C;
+    const int64_t l0 = (int64_t)blockIdx.x * (WL_THREADS / 32) * per_warp;
+    const uint32_t cb = C.leaf_cloud[l0]; // the CTA's first leaf's cloud: its sums stay in shared memory
+    if (threadIdx.x < 6)
+        s_bb[threadIdx.x] = threadIdx.x < 3 ? 0x7FFFFFFF : (int32_t)0x80000000;
+    if (threadIdx.x == 0)
+        s_pairs = 0;
+    __syncthreads();
+    for (int k = 0; k < per_warp; k++)
+    {
+        const int64_t l = l0 + (int64_t)warp * per_warp + k;
+        if (l >= N.L)
+            break;
+        const uint32_t b = C.leaf_cloud[l], c = N.leaf_cand[l];
+        uint32_t before;
+        const uint32_t mine = leaf_mask_word(N, l, lane, before);
+        const uint64_t vidx = N.leaf_vidx[l];
+        uint32_t* rgba = (uint32_t*)(A.out + C.rgba_off[b]) + vidx;
+        float* dens = (float*)(A.out + C.dens_off[b]) + vidx;
+        float* col = (float*)(A.out + C.col_off[b]) + 3 * vidx;
+        uint32_t pairs = 0;
+#pragma unroll 1
+        for (int r0 = 0; r0 < 16; r0 += WL_ROUNDS)
+        {
+            uint32_t at[WL_ROUNDS], vr[WL_ROUNDS], vp[WL_ROUNDS];
+            float vd[WL_ROUNDS], vc[WL_ROUNDS][3];
+#pragma unroll
+            for (int i = 0; i < WL_ROUNDS; i++)
+            {
+                const uint32_t bits = __shfl_sync(0xffffffffu, mine, r0 + i);
+                const uint32_t base = __shfl_sync(0xffffffffu, before, r0 + i);
+                at[i] = (bits >> lane) & 1u ? base + __popc(bits & lt) : ~0u;
+                const uint64_t slot = (uint64_t)c * 512u + (uint32_t)(32 * (r0 + i) + lane);
+                if (at[i] != ~0u)
+                {
+                    vr[i] = __ldcs(A.s_rgba + slot);
+                    vd[i] = __ldcs(A.s_dens + slot);
+#pragma unroll
+                    for (int k2 = 0; k2 < 3; k2++)
+                        vc[i][k2] = __ldcs(A.s_col + 3 * slot + k2);
+                    if (A.cloud_pairs)
+                        vp[i] = __ldcs(A.s_pairs + slot);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < WL_ROUNDS; i++)
+                if (at[i] != ~0u)
+                {
+                    __stcs(rgba + at[i], vr[i]);
+                    __stcs(dens + at[i], vd[i]);
+#pragma unroll
+                    for (int k2 = 0; k2 < 3; k2++)
+                        __stcs(col + 3 * at[i] + k2, vc[i][k2]);
+                    if (A.cloud_pairs)
+                        pairs += vp[i];
+                }
+        }
+        // the node: index, value index, prefix words, mask (128 B)
+        const uint32_t total = __shfl_sync(0xffffffffu, before + __popc(mine), 15);
+        uint64_t word = 0;
+        const uint64_t m_lo = __shfl_sync(0xffffffffu, mine, (2 * (lane - 8)) & 31);
+        const uint64_t m_hi = __shfl_sync(0xffffffffu, mine, (2 * (lane - 8) + 1) & 31);
+        uint64_t prefix[2] = { total & 0xFFFFu, 0 };
+#pragma unroll
+        for (int q = 1; q < 8; q++)
+            prefix[q >> 2] |= (uint64_t)(__shfl_sync(0xffffffffu, before, 2 * q) & 0xFFFFu) << (16 * (q & 3));
+        if (lane == 0)
+        {
+            word = N.leaf_idx[l];
+            A.cand_vbase[c] = C.value_base[b] + vidx;
+        }
+        else if (lane == 1)
+            word = vidx;
+        else if (lane == 6 || lane == 7)
+            word = prefix[lane - 6];
+        else if (lane >= 8)
+            word = m_lo | (m_hi << 32);
+        if (lane < 16)
+            ((uint64_t*)(A.out + N.leaf_addr[l]))[lane] = word;
+        // bbox: x from the mask words with a voxel, y and z from their union
+        const uint32_t even = __reduce_or_sync(0xffffffffu, (lane & 1) ? 0u : mine),
+                       odd = __reduce_or_sync(0xffffffffu, (lane & 1) ? mine : 0u);
+        const uint32_t nz = __ballot_sync(0xffffffffu, mine != 0u);
+        uint32_t ym = 0, zm = even | odd;
+        zm |= zm >> 16;
+        zm = (zm | (zm >> 8)) & 0xffu;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            ym |= ((even >> (8 * q)) & 0xffu ? 1u : 0u) << q | ((odd >> (8 * q)) & 0xffu ? 1u : 0u) << (q + 4);
+        if (lane < 6)
+        {
+            const int a = lane % 3;
+            const int32_t lo = a == 0 ? (__ffs(nz) - 1) >> 1 : __ffs(a == 1 ? ym : zm) - 1;
+            const int32_t hi = a == 0 ? (31 - __clz(nz)) >> 1 : 31 - __clz(a == 1 ? ym : zm);
+            int32_t* bb = b == cb ? s_bb : C.bbox + 6 * (uint64_t)b;
+            const int32_t o = N.leaf_origin[3 * l + a];
+            if (lane < 3)
+                atomicMin(&bb[a], o + lo);
+            else
+                atomicMax(&bb[3 + a], o + hi);
+        }
+        if (A.cloud_pairs)
+        {
+            pairs = __reduce_add_sync(0xffffffffu, pairs);
+            if (lane == 0)
+                atomicAdd(b == cb ? &s_pairs : (unsigned long long*)&A.cloud_pairs[b], (unsigned long long)pairs);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3)
+        atomicMin(&C.bbox[6 * (uint64_t)cb + threadIdx.x], s_bb[threadIdx.x]);
+    else if (threadIdx.x < 6)
+        atomicMax(&C.bbox[6 * (uint64_t)cb + threadIdx.x], s_bb[threadIdx.x]);
+    if (threadIdx.x == 0 && A.cloud_pairs && s_pairs)
+        atomicAdd((unsigned long long*)&A.cloud_pairs[cb], s_pairs);
+}
+
+// f(voxel in canonical order, leaf, leaf_n) for every active voxel, a warp per leaf
+template <class F>
+__device__ __forceinline__ void each_voxel(const NodeParams& N, F f)
+{
+    const int64_t l = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (l >= N.L)
+        return;
+    uint32_t before;
+    const uint32_t mine = leaf_mask_word(N, l, lane, before);
+    const uint64_t v0 = N.leaf_vstart[l];
     for (int r = 0; r < 16; r++)
     {
-        const uint32_t bits = __shfl_sync(0xffffffffu, mine, r);
+        const uint32_t bits = __shfl_sync(0xffffffffu, mine, r), base = __shfl_sync(0xffffffffu, before, r);
         if ((bits >> lane) & 1u)
-        {
-            const uint64_t at = base + (uint64_t)__popc(bits & lt);
-            const uint32_t n = (uint32_t)(32 * r + lane);
-            vkeys[at] = (K)(lk | n);
-            vslot[at] = (uint32_t)(c * 512 + n);
-        }
-        base += (uint64_t)__popc(bits);
+            f(v0 + base + __popc(bits & ((1u << lane) - 1u)), l, (uint32_t)(32 * r + lane));
     }
 }
 
-// staged values -> value index of every active voxel; leaf masks
-__global__ void k_values(ValueParams A, NodeParams N)
+// pairs per voxel (canonical order) from the staged counts
+__global__ void k_voxel_pairs(NodeParams N, const uint32_t* s_pairs, uint64_t* vpairs)
 {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= A.V)
-        return;
-    const uint32_t slot = A.vslot[v];
-    const uint32_t l = A.vox_leaf[v];
-    const uint32_t n = A.vox_n[v];
-    const uint64_t vi = N.leaf_vidx[l] + (uint64_t)(v - N.leaf_vstart[l]);
-    const uint32_t b = N.C.leaf_cloud[l];
-    ((uint32_t*)(A.out + N.C.rgba_off[b]))[vi] = A.s_rgba[slot];
-    ((float*)(A.out + N.C.dens_off[b]))[vi] = A.s_dens[slot];
-    float* col = (float*)(A.out + N.C.col_off[b]);
-    col[3 * vi + 0] = A.s_col[3 * (uint64_t)slot + 0];
-    col[3 * vi + 1] = A.s_col[3 * (uint64_t)slot + 1];
-    col[3 * vi + 2] = A.s_col[3 * (uint64_t)slot + 2];
-    if ((uint64_t)v == N.leaf_vstart[l])
-        A.cand_vbase[slot >> 9] = N.C.value_base[b] + N.leaf_vidx[l];
-    (void)n;
-    if (A.cloud_pairs)
-    {
-        // pairs per cloud: a warp whose voxels share a cloud adds once
-        uint64_t pc = A.s_pairs[slot];
-        const uint32_t peers = __match_any_sync(__activemask(), b);
-        for (int off = 16; off; off >>= 1)
-        {
-            const uint64_t o = __shfl_down_sync(__activemask(), pc, off);
-            pc += ((threadIdx.x & 31) + off < 32 && ((peers >> ((threadIdx.x & 31) + off)) & 1u)) ? o : 0ull;
-        }
-        if ((threadIdx.x & 31) == __ffs(peers) - 1)
-            atomicAdd((unsigned long long*)&A.cloud_pairs[b], (unsigned long long)pc);
-    }
+    each_voxel(N, [&](uint64_t v, int64_t l, uint32_t n) { vpairs[v] = s_pairs[(uint64_t)N.leaf_cand[l] * 512u + n]; });
 }
 
-// every leaf's value mask is its candidate leaf's mask
-__global__ void k_leaf_masks(int64_t L, const uint32_t* leaf_vstart, const uint32_t* vslot, const uint64_t* cand_mask,
-                             uint64_t* leaf_mask)
+// coordinates of the active voxels by value index (clouds back to back)
+__global__ void k_voxel_coords(NodeParams N, int32_t* out)
 {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= L * 8)
-        return;
-    const int64_t l = t >> 3;
-    const uint32_t c = vslot[leaf_vstart[l]] >> 9;
-    leaf_mask[t] = cand_mask[8 * (uint64_t)c + (t & 7)];
-}
-
-// pairs per voxel (run order) from the staged counts
-__global__ void k_voxel_pairs(int64_t V, const uint32_t* vslot, const uint32_t* s_pairs, uint64_t* vpairs)
-{
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < V)
-        vpairs[v] = s_pairs[vslot[v]];
+    each_voxel(N, [&](uint64_t v, int64_t l, uint32_t n) {
+        const uint64_t at = N.C.value_base[N.C.leaf_cloud[l]] + N.leaf_vidx[l] + (v - N.leaf_vstart[l]);
+        out[3 * at + 0] = N.leaf_origin[3 * l + 0] + (int32_t)(n >> 6);
+        out[3 * at + 1] = N.leaf_origin[3 * l + 1] + (int32_t)((n >> 3) & 7);
+        out[3 * at + 2] = N.leaf_origin[3 * l + 2] + (int32_t)(n & 7);
+    });
 }
 
 // ---------------------------------------------------------------- launch ----
@@ -1572,44 +1664,31 @@ void launch_leaf_export(const LeafPassParams& P, uint32_t* counter, int num_sms,
     { k_leaf_export<<<walk_grid(P.NCL, num_sms), LP_THREADS, 0, s>>>(P, counter); count_launch(); }
 }
 
-void launch_leaf_popc(const uint64_t* cand_mask, int64_t NCL, uint64_t* counts, cudaStream_t s)
-{
-    if (NCL <= 0)
-        return;
-    { k_leaf_popc<<<(unsigned)((NCL + 255) / 256), 256, 0, s>>>(cand_mask, NCL, counts); count_launch(); }
-}
-
-void launch_voxel_keys(const uint64_t* cand_mask, const uint32_t* cand_key, const uint64_t* cand_voff, int64_t NCL,
-                       void* vkeys, int key64, uint32_t* vslot, cudaStream_t s)
-{
-    if (NCL <= 0)
-        return;
-    const unsigned blocks = (unsigned)((NCL * 32 + 255) / 256);
-    if (key64)
-        { k_voxel_keys<uint64_t><<<blocks, 256, 0, s>>>(cand_mask, cand_key, cand_voff, NCL, (uint64_t*)vkeys, vslot); count_launch(); }
-    else
-        { k_voxel_keys<uint32_t><<<blocks, 256, 0, s>>>(cand_mask, cand_key, cand_voff, NCL, (uint32_t*)vkeys, vslot); count_launch(); }
-}
-
-void launch_values(const ValueParams& A, const NodeParams& N, cudaStream_t s)
-{
-    if (A.V <= 0)
-        return;
-    { k_values<<<(unsigned)((A.V + 255) / 256), 256, 0, s>>>(A, N); count_launch(); }
-}
-
-void launch_leaf_masks(const NodeParams& N, const uint64_t* cand_mask, const uint32_t* vslot, cudaStream_t s)
+void launch_write_leaves(const ValueParams& A, const NodeParams& N, int num_sms, cudaStream_t s)
 {
     if (N.L <= 0)
         return;
-    { k_leaf_masks<<<(unsigned)((N.L * 8 + 255) / 256), 256, 0, s>>>(N.L, N.leaf_vstart, vslot, cand_mask, N.leaf_mask); count_launch(); }
+    // up to 8 leaves per warp (its CTA adds 64 leaves to the bbox at once), but no
+    // more than leave every SM its 8 CTAs
+    const int64_t per_cta = WL_THREADS / 32;
+    int64_t per_warp = N.L / (per_cta * 8 * num_sms);
+    per_warp = per_warp < 1 ? 1 : per_warp > 8 ? 8 : per_warp;
+    const int64_t grid = (N.L + per_cta * per_warp - 1) / (per_cta * per_warp);
+    { k_write_leaves<<<(unsigned)grid, WL_THREADS, 0, s>>>(A, N, (int)per_warp); count_launch(); }
 }
 
-void launch_voxel_pairs(int64_t V, const uint32_t* vslot, const uint32_t* s_pairs, uint64_t* vpairs, cudaStream_t s)
+void launch_voxel_pairs(const NodeParams& N, const uint32_t* s_pairs, uint64_t* vpairs, cudaStream_t s)
 {
-    if (V <= 0)
+    if (N.L <= 0)
         return;
-    { k_voxel_pairs<<<(unsigned)((V + 255) / 256), 256, 0, s>>>(V, vslot, s_pairs, vpairs); count_launch(); }
+    { k_voxel_pairs<<<(unsigned)((N.L + 7) / 8), 256, 0, s>>>(N, s_pairs, vpairs); count_launch(); }
+}
+
+void launch_voxel_coords(const NodeParams& N, int32_t* out, cudaStream_t s)
+{
+    if (N.L <= 0)
+        return;
+    { k_voxel_coords<<<(unsigned)((N.L + 7) / 8), 256, 0, s>>>(N, out); count_launch(); }
 }
 
 } // namespace vox

@@ -39,12 +39,11 @@ __global__ void k_batch_windows(const uint64_t* frag_off, const uint64_t* F_tota
     nwin[b] = (f1 - f0 + REF_WINDOW - 1) / REF_WINDOW;
 }
 
-__global__ void k_leaf_wkey(int64_t L, const uint32_t* leaf_vstart, const uint32_t* vslot, const uint64_t* cand_wkey,
-                            uint64_t* leaf_wkey)
+__global__ void k_leaf_wkey(int64_t L, const uint32_t* leaf_cand, const uint64_t* cand_wkey, uint64_t* leaf_wkey)
 {
     const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (l < L)
-        leaf_wkey[l] = cand_wkey[vslot[leaf_vstart[l]] >> 9];
+        leaf_wkey[l] = cand_wkey[leaf_cand[l]];
 }
 
 // minimum over the children runs [start[i], start[i + 1])
@@ -161,12 +160,12 @@ void launch_batch_windows(const uint64_t* frag_off, const uint64_t* F_total, int
     { k_batch_windows<<<blocks_for(nbatch), 256, 0, s>>>(frag_off, F_total, G, nbatch, nwin); count_launch(); }
 }
 
-void launch_leaf_wkey(int64_t L, const uint32_t* leaf_vstart, const uint32_t* vslot, const uint64_t* cand_wkey,
-                      uint64_t* leaf_wkey, cudaStream_t s)
+void launch_leaf_wkey(int64_t L, const uint32_t* leaf_cand, const uint64_t* cand_wkey, uint64_t* leaf_wkey,
+                      cudaStream_t s)
 {
     if (L <= 0)
         return;
-    { k_leaf_wkey<<<blocks_for(L), 256, 0, s>>>(L, leaf_vstart, vslot, cand_wkey, leaf_wkey); count_launch(); }
+    { k_leaf_wkey<<<blocks_for(L), 256, 0, s>>>(L, leaf_cand, cand_wkey, leaf_wkey); count_launch(); }
 }
 
 void launch_run_min(int64_t n, const uint32_t* start, const uint64_t* child, uint64_t* out, cudaStream_t s)

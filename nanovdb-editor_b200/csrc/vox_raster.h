@@ -17,21 +17,20 @@ struct RankTables
     const uint64_t* lower_prefix;
 };
 
-struct RunParams
+// the tree from the candidate leaves' masks (k_tree)
+struct TreeParams
 {
-    int64_t P;
-    uint32_t* vox_start;    // [V + 1]
-    uint32_t* leaf_vstart;  // [L + 1]
-    uint32_t* lower_lstart; // [Lo + 1]
-    uint32_t* lower_rank;   // [Lo]
-    uint64_t* counts;       // V, L, Lo
-    uint64_t* status;       // 3 per tile
+    int64_t NCL;
+    const uint64_t* cand_mask; // [NCL][8]
+    const uint32_t* cand_key;  // [NCL] ascending: lower rank << 12 | lower_n
+    const int4* cand_org;      // [NCL] origins
+    uint64_t* cand_voff;       // [NCL] first voxel (canonical order) of each candidate
+    uint64_t* counts;          // V, L, Lo, U
+    uint64_t* status;          // look-back words of the four counts, tree_status_words(NCL)
     uint32_t epoch;
     uint32_t* counter;
     int* err;
-    uint64_t lower_cap;     // entries of lower_lstart / lower_rank (heads beyond it are an error)
-    uint32_t* vox_leaf;     // [V] leaf index of each voxel
-    uint16_t* vox_n;        // [V] leaf_n (position in the leaf) of each voxel
+    uint64_t lower_cap;        // entries of the lower and upper tables (heads beyond it are an error)
 };
 
 // per-cloud layout: every cloud gets its own self-contained grid (header,
@@ -62,25 +61,19 @@ struct NodeParams
 {
     int64_t Lo, L;
     CloudParams C;
-    const uint32_t* lower_rank;
     const uint32_t* lower_cell;   // lower rank -> cell (root rank << 15 | upper_n)
     const uint32_t* root_of_rank; // root rank -> root_n
-    const uint32_t* lower_lstart;
-    const uint32_t* leaf_vstart;
-    const uint32_t* vox_start;
-    int32_t* lower_origin;
+    const uint64_t* cand_mask;    // [candidate][8] value masks
+    uint32_t* lower_lstart;       // [Lo + 1] first leaf
     uint32_t* lower_upper_n;
-    uint32_t* rank_to_lower; // [touched lower cells] lower rank -> lower node index
-    uint64_t* upper_head;
-    uint64_t* upper_scan;
     uint32_t* lower_parent;
-    uint32_t* upper_root_n;
-    uint32_t* upper_lostart;
-    uint64_t* upper_count;
+    uint32_t* upper_root_n;       // cloud << 15 | root_n
+    uint32_t* upper_lostart;      // [U + 1] first lower
+    uint32_t* leaf_vstart;        // [L + 1] first voxel
+    uint32_t* leaf_cand;          // candidate of each leaf
     uint32_t* leaf_lower;
     uint32_t* leaf_lower_n;
-    uint64_t* leaf_mask;
-    int32_t* leaf_origin;
+    int32_t* leaf_origin;         // [L][3]
     uint64_t *upper_idx, *upper_addr, *upper_vidx;
     uint64_t *lower_idx, *lower_addr, *lower_vidx;
     uint64_t *leaf_idx, *leaf_addr, *leaf_vidx;
@@ -183,27 +176,20 @@ void launch_leaf_compact(const uint32_t* keys, const uint32_t* vals, const uint3
 int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant = 0);
 void launch_leaf_backward(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s);
 void launch_leaf_export(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s);
-void launch_leaf_popc(const uint64_t* cand_mask, int64_t NCL, uint64_t* counts, cudaStream_t s);
-void launch_voxel_keys(const uint64_t* cand_mask, const uint32_t* cand_key, const uint64_t* cand_voff, int64_t NCL,
-                       void* vkeys, int key64, uint32_t* vslot, cudaStream_t s);
 
 struct ValueParams
 {
-    int64_t V;
-    const uint32_t* vslot;     // [V] staging slot (candidate * 512 + leaf_n)
     const uint32_t* s_rgba;
     const float* s_dens;
     const float* s_col;
     const uint32_t* s_pairs;
     uint64_t* cloud_pairs;     // [B] passing pairs per cloud, summed here (null: one cloud)
     uint64_t* cand_vbase;      // [NCL]
-    const uint32_t* vox_leaf;
-    const uint16_t* vox_n;
     uint8_t* out;
 };
-void launch_values(const ValueParams& A, const NodeParams& N, cudaStream_t s);
-void launch_leaf_masks(const NodeParams& N, const uint64_t* cand_mask, const uint32_t* vslot, cudaStream_t s);
-void launch_voxel_pairs(int64_t V, const uint32_t* vslot, const uint32_t* s_pairs, uint64_t* vpairs, cudaStream_t s);
+void launch_write_leaves(const ValueParams& A, const NodeParams& N, int num_sms, cudaStream_t s);
+void launch_voxel_pairs(const NodeParams& N, const uint32_t* s_pairs, uint64_t* vpairs, cudaStream_t s);
+void launch_voxel_coords(const NodeParams& N, int32_t* out, cudaStream_t s);
 void launch_zero_gaps(const NodeParams& N, uint8_t* out, uint64_t grid_bytes, cudaStream_t s);
 
 // the reference's fragment batches and windows (raster/Raster.cpp:443-444)
@@ -221,8 +207,8 @@ struct WindowOrderParams
 };
 void launch_batch_windows(const uint64_t* frag_off, const uint64_t* F_total, int64_t G, int64_t nbatch,
                           uint64_t* nwin, cudaStream_t s);
-void launch_leaf_wkey(int64_t L, const uint32_t* leaf_vstart, const uint32_t* vslot, const uint64_t* cand_wkey,
-                      uint64_t* leaf_wkey, cudaStream_t s);
+void launch_leaf_wkey(int64_t L, const uint32_t* leaf_cand, const uint64_t* cand_wkey, uint64_t* leaf_wkey,
+                      cudaStream_t s);
 void launch_run_min(int64_t n, const uint32_t* start, const uint64_t* child, uint64_t* out, cudaStream_t s);
 void launch_level_keys(int64_t n, const uint64_t* wkey, const uint32_t* parent, const uint32_t* parent_rank,
                        const uint32_t* nval, uint32_t nmask, uint64_t* keys, uint32_t* vals, uint64_t* wcount,
@@ -241,12 +227,8 @@ void launch_prep(const PrepParams& P, GaussRec* recs, uint64_t* footprints, uint
 void launch_mark_lower(const GaussRec* recs, int64_t G, const uint64_t* root_bits, const uint64_t* root_prefix,
                        uint64_t* lower_bits, cudaStream_t s);
 void launch_invert_bits(const uint64_t* bits, const uint64_t* prefix, int64_t words, uint32_t* out, cudaStream_t s);
-void launch_runs(const RunParams& Rp, const void* keys, int key64, cudaStream_t s);
-int64_t runs_tile_count(int64_t P);
-void launch_lower_info(const NodeParams& N, cudaStream_t s);
-void launch_upper_info(const NodeParams& N, cudaStream_t s);
-void launch_leaf_tables(const NodeParams& N, const void* keys, int key64, cudaStream_t s);
-void launch_leaf_bbox(const NodeParams& N, cudaStream_t s);
+size_t tree_status_words(int64_t NCL);
+void launch_tree(const TreeParams& T, const NodeParams& N, cudaStream_t s);
 void launch_cloud_layout(const NodeParams& N, cudaStream_t s);
 void launch_canonical_order(const NodeParams& N, uint64_t U, cudaStream_t s);
 void launch_write_nodes(const NodeParams& N, uint64_t U, uint8_t* out, cudaStream_t s);
