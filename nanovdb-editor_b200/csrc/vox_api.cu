@@ -783,7 +783,6 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     if (!ensure(ctx, ctx->grid, grid_bytes))
         return VOX_ERR_MEMORY;
     uint8_t* grid = (uint8_t*)ctx->grid.p;
-    launch_zero_gaps(N, grid, grid_bytes, s);
     uint64_t* cloud_pairs = nullptr;
     if (B > 1)
     {
@@ -804,7 +803,6 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     N.C.cloud_pairs = cloud_pairs;
     cudaEventRecord(ctx->timers.ev[5], s);
     launch_write_nodes(N, U, grid, s);
-    launch_write_headers(N, grid, s);
     ctx->h_grid_off.resize((size_t)B + 1);
     ctx->h_value_base.resize((size_t)B + 1);
     cudaMemcpyAsync(ctx->h_grid_off.data(), N.C.grid_off, sizeof(uint64_t) * (B + 1), cudaMemcpyDeviceToHost, s);

@@ -13,7 +13,7 @@
 //                 first nodes
 //   k_cloud_layout   per-cloud grid layout
 //   [vox_leaf.cu] k_write_leaves: leaf nodes, values, bbox
-//   k_write_*     the other node2 nodes, per-cloud headers, written exactly
+//   k_write_nodes the other node2 nodes, headers and gaps
 #include <cstdio>
 #include <cuda_runtime.h>
 
@@ -450,193 +450,205 @@ __global__ void k_canonical_order(NodeParams N, uint64_t U)
 }
 
 // per cloud: the grid header (vox_grid_header_t) and the bbox blind data
-__global__ void k_write_headers(NodeParams N, uint8_t* out)
-{
-    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const CloudParams& C = N.C;
-    if (b >= C.B)
-        return;
-    const uint64_t g = C.grid_off[b];
-    vox_grid_header_t h;
-    memset(&h, 0, sizeof(h));
-    const uint64_t vc = 2 + (C.vstart[b + 1] - C.vstart[b]);
-    h.magic = VOX_GRID_MAGIC;
-    h.version = 1;
-    h.header_bytes = VOX_GRID_HEADER_BYTES;
-    h.grid_bytes = C.grid_off[b + 1] - g;
-    h.node2_offset = VOX_GRID_HEADER_BYTES;
-    h.node2_bytes = C.node2_bytes[b];
-    h.upper_count = C.upper_start[b + 1] - C.upper_start[b];
-    h.lower_count = C.lower_start[b + 1] - C.lower_start[b];
-    h.leaf_count = C.leaf_start[b + 1] - C.leaf_start[b];
-    h.node_order = C.node_order;
-    h.value_count = vc;
-    h.bbox_offset = C.bbox_off[b] - g;
-    h.rgba8_offset = C.rgba_off[b] - g;
-    h.density_offset = C.dens_off[b] - g;
-    h.color_offset = C.col_off[b] - g;
-    h.voxel_size = C.cloud_vs ? C.cloud_vs[b] : C.voxel_size;
-    if (vc > 2)
-        for (int a = 0; a < 6; a++)
-            h.bbox[a] = C.bbox[6 * b + a];
-    h.pair_count = C.cloud_pairs ? C.cloud_pairs[b] : (uint64_t)C.P;
-    const int64_t g0 = C.cloud_start ? C.cloud_start[b] : 0, g1 = C.cloud_start ? C.cloud_start[b + 1] : C.G;
-    const uint64_t f0 = g0 < C.G ? C.frag_off[g0] : *C.F_total, f1 = g1 < C.G ? C.frag_off[g1] : *C.F_total;
-    h.candidate_count = f1 - f0;
-    const uint32_t* src = (const uint32_t*)&h;
-    uint32_t* dst = (uint32_t*)(out + g);
-    for (int w = 0; w < (int)(sizeof(h) / 4); w++)
-        dst[w] = src[w];
-    int32_t* bb = (int32_t*)(out + C.bbox_off[b]);
-    for (int a = 0; a < 6; a++)
-        bb[a] = h.bbox[a];
-}
-
 // ------------------------------------------------------------ node2 write ----
-// prefix words of a mask (grid_build_count_new.slang:49-88): field (w & 3) of
-// word (w >> 2) = popcount(mask[0 .. w-1]); field 0 of word 0 = total.
-// One CTA, mask of nw words in shared memory.
-__device__ void write_prefix_block(uint64_t* dst, const uint64_t* s_mask, uint32_t nw, uint32_t* s_scan)
+// Node2 roots, uppers and lowers, headers and the gaps between a grid's parts,
+// in one launch.  A CTA writes a stretch of NODE_PART words of one node (a root
+// is 542 KB, an upper 274 KB: one CTA each would run for as long as all the rest)
+// and every word of it once, so nothing is cleared first.  A node's first
+// stretch holds its indices, masks and prefix words
+// (grid_build_count_new.slang:49-88), the others children only.  Bound by the
+// latency of a lower's up to 4096 child loads; 11 us for 8 uppers, 8 full lowers
+// (separate kernels that cleared the region and summed prefixes in one thread: 62 us).
+constexpr int NODE_THREADS = 256;
+constexpr uint32_t NODE_PART = 4352; // words: a whole lower node (4292)
+__host__ __device__ constexpr uint32_t node_words(int t)
 {
-    // exclusive scan of popcounts into s_scan[0..nw], serial per 32-word chunk
-    for (uint32_t w = threadIdx.x; w < nw; w += blockDim.x)
-        s_scan[w] = __popcll(s_mask[w]);
+    return (uint32_t)(n2_node_bytes(t) / 8);
+}
+__host__ __device__ constexpr uint32_t node_parts(int t)
+{
+    return (node_words(t) + NODE_PART - 1) / NODE_PART;
+}
+
+// word w of the prefix of a mask with exclusive popcounts ex[0 .. nw) and total ex[nw]
+__device__ __forceinline__ uint64_t prefix_word(const uint16_t* ex, uint32_t nw, uint32_t q)
+{
+    uint64_t v = q == 0 ? (uint64_t)ex[nw] : (uint64_t)ex[4 * q];
+    for (uint32_t f = 1; f < 4; f++)
+        v |= (uint64_t)ex[4 * q + f] << (16 * f);
+    return v;
+}
+
+// the CTA's stretch of node type T; child(i) is the i-th of its `children` child words
+template <int T, class Child>
+__device__ __forceinline__ void write_node_part(uint64_t* W, uint32_t part, uint64_t idx, uint64_t vidx,
+                                                uint32_t children, const uint64_t* s_mask, const uint16_t* s_ex,
+                                                Child child)
+{
+    constexpr uint32_t nw = T == 2 ? 64u : 512u;
+    const uint32_t w0 = part * NODE_PART, w1 = min(node_words(T), w0 + NODE_PART);
+    if (part == 0)
+        for (uint32_t w = threadIdx.x; w < n2_off_children(T); w += NODE_THREADS)
+        {
+            uint64_t v = 0;
+            if (w == N2_OFF_NODE_IDX)
+                v = idx;
+            else if (w == N2_OFF_VALUE_IDX)
+                v = vidx;
+            else if (w - n2_off_child_mask(T) < nw)
+                v = s_mask[w - n2_off_child_mask(T)];
+            else if (w - n2_off_child_prefix(T) < nw / 4)
+                v = prefix_word(s_ex, nw, w - n2_off_child_prefix(T));
+            else if (T == 0 && w - N2_OFF_KEY_MASK_ROOT < nw)
+                v = s_mask[w - N2_OFF_KEY_MASK_ROOT];
+            else if (T == 0 && w - N2_OFF_KEY_PREFIX_ROOT < nw / 4)
+                v = prefix_word(s_ex, nw, w - N2_OFF_KEY_PREFIX_ROOT);
+            W[w] = v;
+        }
+    const uint32_t c0 = max(w0, n2_off_children(T));
+#pragma unroll 4
+    for (uint32_t w = c0 + threadIdx.x; w < w1; w += NODE_THREADS)
+    {
+        const uint32_t i = w - n2_off_children(T);
+        W[w] = i < children ? child(i) : (T == 0 && i < 65536u ? N2_END_KEY : 0ull);
+    }
+}
+
+// the first stretch's mask and its exclusive popcounts: slot(i) is child i's bit
+template <int T, class Slot>
+__device__ __forceinline__ void node_mask(uint64_t* s_mask, uint16_t* s_ex, uint64_t* s_warp, uint32_t children, Slot slot)
+{
+    constexpr uint32_t nw = T == 2 ? 64u : 512u;
+    for (uint32_t i = threadIdx.x; i < nw; i += NODE_THREADS)
+        s_mask[i] = 0;
     __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < children; i += NODE_THREADS)
+    {
+        const uint32_t n = slot(i);
+        // 32-bit words: a 64-bit OR in shared memory is a compare-and-swap loop
+        atomicOr(reinterpret_cast<uint32_t*>(s_mask) + (n >> 5), 1u << (n & 31));
+    }
+    __syncthreads();
+    const uint32_t w = 2 * threadIdx.x;
+    const uint32_t a = w < nw ? __popcll(s_mask[w]) : 0, b = w < nw ? __popcll(s_mask[w + 1]) : 0;
+    uint64_t total;
+    const uint64_t ex = block_excl_scan_u64(a + b, s_warp, total);
+    if (w < nw)
+    {
+        s_ex[w] = (uint16_t)ex;
+        s_ex[w + 1] = (uint16_t)(ex + a);
+    }
     if (threadIdx.x == 0)
-    {
-        uint32_t run = 0;
-        for (uint32_t w = 0; w < nw; w++)
-        {
-            uint32_t c = s_scan[w];
-            s_scan[w] = run;
-            run += c;
-        }
-        s_scan[nw] = run;
-    }
-    __syncthreads();
-    for (uint32_t q = threadIdx.x; q < nw / 4; q += blockDim.x)
-    {
-        uint64_t word = 0;
-        for (uint32_t f = 0; f < 4; f++)
-        {
-            uint32_t w = 4 * q + f;
-            uint32_t v = (w == 0) ? s_scan[nw] : s_scan[w];
-            word |= ((uint64_t)(v & 0xFFFFu)) << (16 * f);
-        }
-        dst[q] = word;
-    }
+        s_ex[nw] = (uint16_t)total;
     __syncthreads();
 }
 
-// one CTA per cloud: the root of that cloud's grid
-__global__ void __launch_bounds__(1024) k_write_root(NodeParams N, uint8_t* out)
+// bytes [a, b) of the output zeroed by the CTA (multiples of 4, a few hundred)
+__device__ __forceinline__ void zero_words(uint8_t* out, uint64_t a, uint64_t b)
+{
+    for (uint64_t o = a + 4 * threadIdx.x; o < b; o += 4 * NODE_THREADS)
+        *reinterpret_cast<uint32_t*>(out + o) = 0u;
+}
+
+// cloud b's header, bbox, background values (the two slots before each channel's
+// first voxel) and alignment gaps
+__device__ __forceinline__ void write_grid_header(const NodeParams& N, uint64_t b, uint8_t* out, vox_grid_header_t& h)
+{
+    const CloudParams& C = N.C;
+    const uint64_t g = C.grid_off[b];
+    const uint64_t vc = 2 + (C.vstart[b + 1] - C.vstart[b]);
+    if (threadIdx.x == 0)
+    {
+        memset(&h, 0, sizeof(h));
+        h.magic = VOX_GRID_MAGIC;
+        h.version = 1;
+        h.header_bytes = VOX_GRID_HEADER_BYTES;
+        h.grid_bytes = C.grid_off[b + 1] - g;
+        h.node2_offset = VOX_GRID_HEADER_BYTES;
+        h.node2_bytes = C.node2_bytes[b];
+        h.upper_count = C.upper_start[b + 1] - C.upper_start[b];
+        h.lower_count = C.lower_start[b + 1] - C.lower_start[b];
+        h.leaf_count = C.leaf_start[b + 1] - C.leaf_start[b];
+        h.node_order = C.node_order;
+        h.value_count = vc;
+        h.bbox_offset = C.bbox_off[b] - g;
+        h.rgba8_offset = C.rgba_off[b] - g;
+        h.density_offset = C.dens_off[b] - g;
+        h.color_offset = C.col_off[b] - g;
+        h.voxel_size = C.cloud_vs ? C.cloud_vs[b] : C.voxel_size;
+        if (vc > 2)
+            for (int a = 0; a < 6; a++)
+                h.bbox[a] = C.bbox[6 * b + a];
+        h.pair_count = C.cloud_pairs ? C.cloud_pairs[b] : (uint64_t)C.P;
+        const int64_t g0 = C.cloud_start ? C.cloud_start[b] : 0, g1 = C.cloud_start ? C.cloud_start[b + 1] : C.G;
+        const uint64_t f0 = g0 < C.G ? C.frag_off[g0] : *C.F_total, f1 = g1 < C.G ? C.frag_off[g1] : *C.F_total;
+        h.candidate_count = f1 - f0;
+    }
+    __syncthreads();
+    if (threadIdx.x < sizeof(h) / 4)
+        ((uint32_t*)(out + g))[threadIdx.x] = reinterpret_cast<const uint32_t*>(&h)[threadIdx.x];
+    if (threadIdx.x < 6)
+        ((int32_t*)(out + C.bbox_off[b]))[threadIdx.x] = h.bbox[threadIdx.x];
+    zero_words(out, g + VOX_GRID_HEADER_BYTES + C.node2_bytes[b], C.bbox_off[b]);
+    zero_words(out, C.bbox_off[b] + 24, C.rgba_off[b] + 8);
+    zero_words(out, C.rgba_off[b] + 4 * vc, C.dens_off[b] + 8);
+    zero_words(out, C.dens_off[b] + 4 * vc, C.col_off[b] + 24);
+    zero_words(out, C.col_off[b] + 12 * vc, C.grid_off[b + 1]);
+}
+static_assert(sizeof(vox_grid_header_t) == VOX_GRID_HEADER_BYTES && VOX_GRID_HEADER_BYTES / 4 <= NODE_THREADS,
+              "the header is written by one word per thread");
+
+__global__ void __launch_bounds__(NODE_THREADS) k_write_nodes(NodeParams N, uint64_t U, uint8_t* out)
 {
     __shared__ uint64_t s_mask[512];
-    __shared__ uint32_t s_scan[513];
-    const uint64_t b = blockIdx.x;
-    const uint64_t root_addr = N.C.grid_off[b] + VOX_GRID_HEADER_BYTES;
-    uint64_t* W = (uint64_t*)(out + root_addr);
-    const uint32_t u0 = N.C.upper_start[b];
-    const uint64_t U = N.C.upper_start[b + 1] - u0;
-    for (int i = threadIdx.x; i < 512; i += blockDim.x)
-        s_mask[i] = 0;
-    __syncthreads();
-    for (uint64_t u = threadIdx.x; u < U; u += blockDim.x)
+    __shared__ uint16_t s_ex[513];
+    __shared__ uint64_t s_warp[33];
+    __shared__ vox_grid_header_t s_head;
+    uint64_t k = blockIdx.x;
+    if (k < (uint64_t)N.C.B * node_parts(0)) // roots, headers
     {
-        uint32_t rn = N.upper_root_n[u0 + u] & 32767u;
-        atomicOr((unsigned long long*)&s_mask[rn >> 6], 1ull << (rn & 63));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        W[N2_OFF_NODE_IDX] = 0;
-        W[N2_OFF_VALUE_IDX] = 2;
-    }
-    for (int i = threadIdx.x; i < 512; i += blockDim.x)
-    {
-        W[n2_off_child_mask(0) + i] = s_mask[i];
-        W[N2_OFF_KEY_MASK_ROOT + i] = s_mask[i];
-    }
-    write_prefix_block(W + n2_off_child_prefix(0), s_mask, 512, s_scan);
-    write_prefix_block(W + N2_OFF_KEY_PREFIX_ROOT, s_mask, 512, s_scan);
-    uint64_t* ch = W + n2_off_children(0);
-    for (uint32_t e = threadIdx.x; e < 65536u; e += blockDim.x)
-    {
-        uint64_t val = N2_END_KEY;
-        if (e < U)
-            val = N.upper_addr[u0 + e] - root_addr;
-        else if (e < 2 * U)
+        const uint64_t b = k / node_parts(0);
+        const uint32_t part = (uint32_t)(k % node_parts(0));
+        const uint64_t addr = N.C.grid_off[b] + VOX_GRID_HEADER_BYTES;
+        const uint32_t u0 = N.C.upper_start[b], nu = N.C.upper_start[b + 1] - u0;
+        if (part == 0)
         {
-            uint32_t rn = N.upper_root_n[u0 + e - U] & 32767u;
-            int32_t x = (int32_t)(((rn >> 10) & 31) << 12), y = (int32_t)(((rn >> 5) & 31) << 12),
-                    z = (int32_t)((rn & 31) << 12);
-            x = x >= 65536 ? x - 131072 : x;
-            y = y >= 65536 ? y - 131072 : y;
-            z = z >= 65536 ? z - 131072 : z;
-            val = (uint64_t)((uint32_t)z >> 12) | ((uint64_t)((uint32_t)y >> 12) << 21) |
-                  ((uint64_t)((uint32_t)x >> 12) << 42);
+            write_grid_header(N, b, out, s_head);
+            node_mask<0>(s_mask, s_ex, s_warp, nu, [&](uint32_t i) { return N.upper_root_n[u0 + i] & 32767u; });
         }
-        ch[e] = val;
+        // per child its offset, then per child its key
+        write_node_part<0>((uint64_t*)(out + addr), part, 0, 2, 2 * nu, s_mask, s_ex, [&](uint32_t i) -> uint64_t {
+            if (i < nu)
+                return N.upper_addr[u0 + i] - addr;
+            int32_t o[3];
+            root_tile_origin(N.upper_root_n[u0 + i - nu] & 32767u, o);
+            return (uint64_t)((uint32_t)o[2] >> 12) | ((uint64_t)((uint32_t)o[1] >> 12) << 21) |
+                   ((uint64_t)((uint32_t)o[0] >> 12) << 42);
+        });
+        return;
     }
+    k -= (uint64_t)N.C.B * node_parts(0);
+    if (k < U * node_parts(1)) // uppers
+    {
+        const uint64_t u = k / node_parts(1);
+        const uint32_t part = (uint32_t)(k % node_parts(1));
+        const uint64_t addr = N.upper_addr[u];
+        const uint32_t lo0 = N.upper_lostart[u], n = N.upper_lostart[u + 1] - lo0;
+        if (part == 0)
+            node_mask<1>(s_mask, s_ex, s_warp, n, [&](uint32_t i) { return N.lower_upper_n[lo0 + i]; });
+        write_node_part<1>((uint64_t*)(out + addr), part, N.upper_idx[u], N.upper_vidx[u], n, s_mask, s_ex,
+                           [&](uint32_t i) { return N.lower_addr[lo0 + i] - addr; });
+        return;
+    }
+    k -= U * node_parts(1); // lowers
+    const uint64_t addr = N.lower_addr[k];
+    const uint32_t l0 = N.lower_lstart[k], n = N.lower_lstart[k + 1] - l0;
+    node_mask<2>(s_mask, s_ex, s_warp, n, [&](uint32_t i) { return N.leaf_lower_n[l0 + i]; });
+    write_node_part<2>((uint64_t*)(out + addr), 0, N.lower_idx[k], N.lower_vidx[k], n, s_mask, s_ex,
+                       [&](uint32_t i) { return N.leaf_addr[l0 + i] - addr; });
 }
-
-__global__ void __launch_bounds__(512) k_write_upper(NodeParams N, uint8_t* node2)
-{
-    __shared__ uint64_t s_mask[512];
-    __shared__ uint32_t s_scan[513];
-    const uint64_t u = blockIdx.x;
-    uint64_t* W = (uint64_t*)(node2 + N.upper_addr[u]);
-    for (int i = threadIdx.x; i < 512; i += blockDim.x)
-        s_mask[i] = 0;
-    __syncthreads();
-    const uint32_t lo0 = N.upper_lostart[u], lo1 = N.upper_lostart[u + 1];
-    for (uint32_t lo = lo0 + threadIdx.x; lo < lo1; lo += blockDim.x)
-    {
-        uint32_t un = N.lower_upper_n[lo];
-        atomicOr((unsigned long long*)&s_mask[un >> 6], 1ull << (un & 63));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        W[N2_OFF_NODE_IDX] = N.upper_idx[u];
-        W[N2_OFF_VALUE_IDX] = N.upper_vidx[u];
-    }
-    for (int i = threadIdx.x; i < 512; i += blockDim.x)
-        W[n2_off_child_mask(1) + i] = s_mask[i];
-    write_prefix_block(W + n2_off_child_prefix(1), s_mask, 512, s_scan);
-    uint64_t* ch = W + n2_off_children(1);
-    for (uint32_t lo = lo0 + threadIdx.x; lo < lo1; lo += blockDim.x)
-        ch[lo - lo0] = N.lower_addr[lo] - N.upper_addr[u];
-}
-
-__global__ void __launch_bounds__(256) k_write_lower(NodeParams N, uint8_t* node2)
-{
-    __shared__ uint64_t s_mask[64];
-    __shared__ uint32_t s_scan[65];
-    const uint64_t lo = blockIdx.x;
-    uint64_t* W = (uint64_t*)(node2 + N.lower_addr[lo]);
-    for (int i = threadIdx.x; i < 64; i += blockDim.x)
-        s_mask[i] = 0;
-    __syncthreads();
-    const uint32_t l0 = N.lower_lstart[lo], l1 = N.lower_lstart[lo + 1];
-    for (uint32_t l = l0 + threadIdx.x; l < l1; l += blockDim.x)
-    {
-        uint32_t ln = N.leaf_lower_n[l];
-        atomicOr((unsigned long long*)&s_mask[ln >> 6], 1ull << (ln & 63));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        W[N2_OFF_NODE_IDX] = N.lower_idx[lo];
-        W[N2_OFF_VALUE_IDX] = N.lower_vidx[lo];
-    }
-    for (int i = threadIdx.x; i < 64; i += blockDim.x)
-        W[n2_off_child_mask(2) + i] = s_mask[i];
-    write_prefix_block(W + n2_off_child_prefix(2), s_mask, 64, s_scan);
-    uint64_t* ch = W + n2_off_children(2);
-    for (uint32_t l = l0 + threadIdx.x; l < l1; l += blockDim.x)
-        ch[l - l0] = N.leaf_addr[l] - N.lower_addr[lo];
-}
+static_assert(node_parts(2) == 1, "a lower node is one stretch");
 
 // =================================================================== launch
 void launch_prep(const PrepParams& P, GaussRec* recs, uint64_t* footprints, uint64_t* root_bits, int* err,
@@ -690,60 +702,11 @@ void launch_canonical_order(const NodeParams& N, uint64_t U, cudaStream_t s)
 }
 void launch_write_nodes(const NodeParams& N, uint64_t U, uint8_t* out, cudaStream_t s)
 {
-    { k_write_root<<<(unsigned)N.C.B, 1024, 0, s>>>(N, out); count_launch(); }
-    if (U)
-        { k_write_upper<<<(unsigned)U, 512, 0, s>>>(N, out); count_launch(); }
-    if (N.Lo)
-        { k_write_lower<<<(unsigned)N.Lo, 256, 0, s>>>(N, out); count_launch(); }
+    const uint64_t grid = (uint64_t)N.C.B * node_parts(0) + U * node_parts(1) + (uint64_t)N.Lo;
+    { k_write_nodes<<<(unsigned)grid, NODE_THREADS, 0, s>>>(N, U, out); count_launch(); }
 }
 void launch_cloud_layout(const NodeParams& N, cudaStream_t s)
 {
     { k_cloud_layout<<<1, 1024, 0, s>>>(N); count_launch(); }
-}
-// Zero every byte of each cloud's grid that the node / value writers leave
-// alone: header, node2 region, bbox, the two background values of each value
-// array and the alignment gaps (the values 2 .. vc - 1 are all written).
-__device__ __forceinline__ void zero_range(uint8_t* out, uint64_t a, uint64_t b, uint64_t i, uint64_t n)
-{
-    // a, b multiples of 4
-    const uint64_t a16 = (a + 15) & ~15ull, b16 = b & ~15ull;
-    if (a16 >= b16)
-    {
-        for (uint64_t o = a + 4 * i; o < b; o += 4 * n)
-            *reinterpret_cast<uint32_t*>(out + o) = 0u;
-        return;
-    }
-    for (uint64_t o = a + 4 * i; o < a16; o += 4 * n)
-        *reinterpret_cast<uint32_t*>(out + o) = 0u;
-    for (uint64_t o = a16 + 16 * i; o < b16; o += 16 * n)
-        *reinterpret_cast<uint4*>(out + o) = make_uint4(0u, 0u, 0u, 0u);
-    for (uint64_t o = b16 + 4 * i; o < b; o += 4 * n)
-        *reinterpret_cast<uint32_t*>(out + o) = 0u;
-}
-
-__global__ void k_zero_gaps(NodeParams N, uint8_t* out)
-{
-    const CloudParams& C = N.C;
-    const int64_t b = blockIdx.y;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, n = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t vc = 2 + (C.vstart[b + 1] - C.vstart[b]);
-    zero_range(out, C.grid_off[b], C.rgba_off[b] + 8, i, n);
-    zero_range(out, C.rgba_off[b] + 4 * vc, C.dens_off[b] + 8, i, n);
-    zero_range(out, C.dens_off[b] + 4 * vc, C.col_off[b] + 24, i, n);
-    zero_range(out, C.col_off[b] + 12 * vc, C.grid_off[b + 1], i, n);
-}
-
-void launch_zero_gaps(const NodeParams& N, uint8_t* out, uint64_t grid_bytes, cudaStream_t s)
-{
-    if (N.C.B <= 0)
-        return;
-    uint64_t bx = grid_bytes / (uint64_t)N.C.B / (1ull << 19);
-    bx = bx < 1 ? 1 : (bx > 1024 ? 1024 : bx);
-    { k_zero_gaps<<<dim3((unsigned)bx, (unsigned)N.C.B), 256, 0, s>>>(N, out); count_launch(); }
-}
-
-void launch_write_headers(const NodeParams& N, uint8_t* out, cudaStream_t s)
-{
-    { k_write_headers<<<(unsigned)((N.C.B + 127) / 128), 128, 0, s>>>(N, out); count_launch(); }
 }
 } // namespace vox

@@ -190,7 +190,6 @@ struct ValueParams
 void launch_write_leaves(const ValueParams& A, const NodeParams& N, int num_sms, cudaStream_t s);
 void launch_voxel_pairs(const NodeParams& N, const uint32_t* s_pairs, uint64_t* vpairs, cudaStream_t s);
 void launch_voxel_coords(const NodeParams& N, int32_t* out, cudaStream_t s);
-void launch_zero_gaps(const NodeParams& N, uint8_t* out, uint64_t grid_bytes, cudaStream_t s);
 
 // the reference's fragment batches and windows (raster/Raster.cpp:443-444)
 constexpr int64_t REF_PRIM_BATCH = 262144; // Gaussians per batch (2^18)
@@ -232,7 +231,6 @@ void launch_tree(const TreeParams& T, const NodeParams& N, cudaStream_t s);
 void launch_cloud_layout(const NodeParams& N, cudaStream_t s);
 void launch_canonical_order(const NodeParams& N, uint64_t U, cudaStream_t s);
 void launch_write_nodes(const NodeParams& N, uint64_t U, uint8_t* out, cudaStream_t s);
-void launch_write_headers(const NodeParams& N, uint8_t* out, cudaStream_t s);
 
 // VoxelBVH Gaussian ingestion (raster/VoxelBVH.cpp:1225-1435)
 struct VoxelBvhParams
