@@ -284,35 +284,45 @@ static int window_order(vox_context_t* ctx, NodeParams& N, int64_t U, int64_t Lo
     launch_leaf_wkey(L, N.leaf_cand, (const uint64_t*)ctx->cand_wkey.p, wk_leaf, s);
     launch_run_min(Lo, N.lower_lstart, wk_leaf, wk_lo, s);
     launch_run_min(U, N.upper_lostart, wk_lo, wk_u, s);
-    const int key_bits = 40 + bits_for((uint64_t)W + 1);
     struct Level
     {
-        int64_t n;
+        int64_t n, parents;
         const uint64_t* wkey;
         const uint32_t* parent;
         const uint32_t* parent_rank;
         const uint32_t* nval;
-        uint32_t nmask;
+        int nbits;
         uint32_t* rank;
-    } lv[3] = { { U, wk_u, nullptr, nullptr, N.upper_root_n, 32767u, (uint32_t*)ctx->rank_u.p },
-                { Lo, wk_lo, N.lower_parent, (const uint32_t*)ctx->rank_u.p, N.lower_upper_n, 32767u,
+    } lv[3] = { { U, 1, wk_u, nullptr, nullptr, N.upper_root_n, 15, (uint32_t*)ctx->rank_u.p },
+                { Lo, U, wk_lo, N.lower_parent, (const uint32_t*)ctx->rank_u.p, N.lower_upper_n, 15,
                   (uint32_t*)ctx->rank_lo.p },
-                { L, wk_leaf, N.leaf_lower, (const uint32_t*)ctx->rank_lo.p, N.leaf_lower_n, 4095u,
+                { L, Lo, wk_leaf, N.leaf_lower, (const uint32_t*)ctx->rank_lo.p, N.leaf_lower_n, 12,
                   (uint32_t*)ctx->rank_leaf.p } };
     for (int l = 0; l < 3; l++)
     {
-        if (lv[l].n <= 0)
+        const Level& v = lv[l];
+        if (v.n <= 0)
             continue;
-        launch_level_keys(lv[l].n, lv[l].wkey, lv[l].parent, lv[l].parent_rank, lv[l].nval, lv[l].nmask,
-                          (uint64_t*)ctx->okeys.p, (uint32_t*)ctx->ovals.p, cnt + (size_t)l * W, s);
-        const int in_alt = sort_pairs_u64((uint64_t*)ctx->okeys.p, (uint32_t*)ctx->ovals.p, (uint64_t*)ctx->okeys_alt.p,
-                                          (uint32_t*)ctx->ovals_alt.p, lv[l].n, key_bits, ctx->sort_ws.p,
-                                          &ctx->sort_epochs, d_err, ctx->num_sms, s, ctx->tuning);
-        const uint32_t* sv = (const uint32_t*)(in_alt ? ctx->ovals_alt.p : ctx->ovals.p);
-        launch_level_rank(lv[l].n, sv, lv[l].rank, s);
-        if (l == 2)
-            launch_leaf_popc_sorted(L, sv, N.leaf_vstart, (uint64_t*)ctx->leaf_popc.p, s);
+        const int pbits = bits_for((uint64_t)v.parents), bits = v.nbits + pbits + bits_for((uint64_t)W);
+        const bool small = v.n <= LEVEL_RANK_SMALL_MAX;
+        const int key64 = small || bits > 32;
+        launch_level_keys(v.n, v.wkey, v.parent, v.parent_rank, v.nval, v.nbits, pbits, ctx->okeys.p, key64,
+                          (uint32_t*)ctx->ovals.p, cnt + (size_t)l * W, s);
+        if (small)
+        {
+            launch_level_rank_small(v.n, (const uint64_t*)ctx->okeys.p, v.rank, s);
+            continue;
+        }
+        const int in_alt =
+            key64 ? sort_pairs_u64((uint64_t*)ctx->okeys.p, (uint32_t*)ctx->ovals.p, (uint64_t*)ctx->okeys_alt.p,
+                                   (uint32_t*)ctx->ovals_alt.p, v.n, bits, ctx->sort_ws.p, &ctx->sort_epochs, d_err,
+                                   ctx->num_sms, s, ctx->tuning)
+                  : sort_pairs_u32((uint32_t*)ctx->okeys.p, (uint32_t*)ctx->ovals.p, (uint32_t*)ctx->okeys_alt.p,
+                                   (uint32_t*)ctx->ovals_alt.p, v.n, bits, ctx->sort_ws.p, &ctx->sort_epochs, d_err,
+                                   ctx->num_sms, s, ctx->tuning);
+        launch_level_rank(v.n, (const uint32_t*)(in_alt ? ctx->ovals_alt.p : ctx->ovals.p), v.rank, s);
     }
+    launch_leaf_popc_ranked(L, lv[2].rank, N.leaf_vstart, (uint64_t*)ctx->leaf_popc.p, s);
     uint64_t* scan_status = (uint64_t*)ctx->scan_status.p;
     const size_t scan_words = ctx->scan_status.cap / sizeof(uint64_t);
     scan_exclusive_u64((const uint64_t*)ctx->leaf_popc.p, (uint64_t*)ctx->leaf_voff.p, L, 0, sc + SC_SCRATCH + 4,
@@ -363,7 +373,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         set_error(ctx, "vox_voxelize: missing attribute array");
         return VOX_ERR_ARGS;
     }
-    const bool window = (flags & VOX_FLAG_WINDOW_ORDER) != 0;
+    bool window = (flags & VOX_FLAG_WINDOW_ORDER) != 0; // the reference's windows matter to the node order
     if (window && B > 1)
     {
         set_error(ctx, "vox_voxelize_batch: the reference window node order is for one cloud per call");
@@ -471,6 +481,10 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         return VOX_ERR_MEMORY;
     launch_invert_bits(root_bits, root_prefix, 512 * B, (uint32_t*)ctx->root_of_rank.p, s);
     ctx->stats.candidates = (int64_t)F;
+    // one batch and at most one window: every node is created in window 0, and
+    // the order by (window, parent rank, n) is the canonical one
+    if (G <= REF_PRIM_BATCH && F <= REF_WINDOW)
+        window = false;
 
     // ------------------------------------------------------- lower ranks
     const int64_t lwords = (int64_t)(NR > 0 ? NR : 1) * 512;

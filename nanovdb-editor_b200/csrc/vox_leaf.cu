@@ -901,7 +901,11 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         // (gaussian_frag_alloc.slang:55-58) after the Gaussian's batch offset
                         const uint64_t r = (uint64_t)(x - R.q4.x) * (uint64_t)R.q5.y * (uint64_t)R.q5.z +
                                            (uint64_t)(yy - R.q4.y) * (uint64_t)R.q5.z + (uint64_t)(zz - R.q4.z);
-                        atomicMin(&A.wmin, (unsigned long long)(C.wbase[j] + (C.wf0[j] + r) / REF_WINDOW));
+                        const unsigned long long wk = C.wbase[j] + (C.wf0[j] + r) / REF_WINDOW;
+                        // read first: a 64-bit minimum in shared memory is a compare-and-swap loop,
+                        // and nearly every pair's window is no earlier than the one there
+                        if (wk < *(volatile unsigned long long*)&A.wmin)
+                            atomicMin(&A.wmin, wk);
                     }
                 }
                 const uint32_t bal = __ballot_sync(0xffffffffu, defer);

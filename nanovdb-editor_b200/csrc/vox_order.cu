@@ -13,9 +13,11 @@
 // A node is created in the first window holding a passing fragment of one of
 // its voxels.  The leaf walk records that window per candidate leaf (the
 // minimum over its passing pairs); lowers and uppers take the minimum over
-// their children.  Per level, a sort by (window, parent rank, n) gives each
+// their children.  Per level, the order by (window, parent rank, n) gives each
 // node's rank; per-window counts place the levels of a window after the
-// nodes of every earlier window.
+// nodes of every earlier window.  A call whose fragments fit one window has the
+// canonical order (every node in window 0, so ranks go by parent and n) and
+// takes none of this (vox_api.cu).
 #include <cstdio>
 #include <cuda_runtime.h>
 
@@ -46,29 +48,47 @@ __global__ void k_leaf_wkey(int64_t L, const uint32_t* leaf_cand, const uint64_t
         leaf_wkey[l] = cand_wkey[leaf_cand[l]];
 }
 
-// minimum over the children runs [start[i], start[i + 1])
+// minimum over the children runs [start[i], start[i + 1]), a warp per run
+// (a lower has up to 4096 leaves: one thread per run took 61 us for 8 lowers)
 __global__ void k_run_min(int64_t n, const uint32_t* start, const uint64_t* child, uint64_t* out)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (i >= n)
         return;
     uint64_t m = ~0ull;
-    for (uint32_t c = start[i]; c < start[i + 1]; c++)
-        m = child[c] < m ? child[c] : m;
-    out[i] = m;
+    const uint32_t c1 = start[i + 1];
+#pragma unroll 4
+    for (uint32_t c = start[i] + lane; c < c1; c += 32)
+    {
+        const uint64_t v = child[c];
+        m = v < m ? v : m;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+    {
+        const uint64_t v = __shfl_xor_sync(0xffffffffu, m, o);
+        m = v < m ? v : m;
+    }
+    if (lane == 0)
+        out[i] = m;
 }
 
-// sort key of a level: window << 40 | parent rank << 15 | n
+// sort key of a level: window, parent rank, n (nbits bits; pbits for the rank);
+// nodes per window (lanes of one window add once)
+template <class K>
 __global__ void k_level_keys(int64_t n, const uint64_t* wkey, const uint32_t* parent, const uint32_t* parent_rank,
-                             const uint32_t* nval, uint32_t nmask, uint64_t* keys, uint32_t* vals, uint64_t* wcount)
+                             const uint32_t* nval, int nbits, int pbits, K* keys, uint32_t* vals, uint64_t* wcount)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const uint64_t pr = parent ? (uint64_t)parent_rank[parent[i]] : 0ull;
-    keys[i] = (wkey[i] << 40) | (pr << 15) | (uint64_t)(nval[i] & nmask);
+    const uint64_t pr = parent ? (uint64_t)parent_rank[parent[i]] : 0ull, w = wkey[i];
+    keys[i] = (K)((w << (pbits + nbits)) | (pr << nbits) | (uint64_t)(nval[i] & ((1u << nbits) - 1u)));
     vals[i] = (uint32_t)i;
-    atomicAdd((unsigned long long*)&wcount[wkey[i]], 1ull);
+    const uint32_t peers = __match_any_sync(__activemask(), w);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1)
+        atomicAdd((unsigned long long*)&wcount[w], (unsigned long long)__popc(peers));
 }
 
 __global__ void k_level_rank(int64_t n, const uint32_t* sorted_vals, uint32_t* rank)
@@ -78,14 +98,33 @@ __global__ void k_level_rank(int64_t n, const uint32_t* sorted_vals, uint32_t* r
         rank[sorted_vals[p]] = (uint32_t)p;
 }
 
-__global__ void k_leaf_popc_sorted(int64_t L, const uint32_t* sorted_vals, const uint32_t* leaf_vstart,
-                                   uint64_t* out)
+// A level of at most LEVEL_RANK_SMALL_MAX nodes: a node's rank is the number of smaller
+// keys (the keys are distinct).  One launch of n^2 comparisons in shared memory
+// (2048 nodes: 16k per thread, 10 us) for the histogram, the passes and the
+// inversion of a radix sort.
+__global__ void __launch_bounds__(256) k_level_rank_small(int n, const uint64_t* keys, uint32_t* rank)
 {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= L)
+    __shared__ uint64_t s_key[LEVEL_RANK_SMALL_MAX];
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        s_key[i] = keys[i];
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
         return;
-    const uint32_t l = sorted_vals[p];
-    out[p] = (uint64_t)(leaf_vstart[l + 1] - leaf_vstart[l]);
+    const uint64_t k = s_key[i];
+    uint32_t r = 0;
+#pragma unroll 8
+    for (int j = 0; j < n; j++)
+        r += s_key[j] < k ? 1u : 0u;
+    rank[i] = r;
+}
+
+// voxels of every leaf, in the level's order
+__global__ void k_leaf_popc_ranked(int64_t L, const uint32_t* rank, const uint32_t* leaf_vstart, uint64_t* out)
+{
+    const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (l < L)
+        out[rank[l]] = (uint64_t)(leaf_vstart[l + 1] - leaf_vstart[l]);
 }
 
 // node_idx, byte address and value index of every node from its level rank and
@@ -124,27 +163,31 @@ __global__ void k_window_place(WindowOrderParams W, NodeParams N)
     }
 }
 
-__global__ void k_window_bases(int64_t nw, const uint64_t* cu, const uint64_t* clo, const uint64_t* cleaf,
-                               uint64_t* base_u, uint64_t* base_lo, uint64_t* base_leaf, uint64_t* base_all)
+// nodes of each level in earlier windows: one CTA, 1024 windows at a time
+__global__ void __launch_bounds__(1024) k_window_bases(int64_t nw, const uint64_t* cu, const uint64_t* clo,
+                                                       const uint64_t* cleaf, uint64_t* base_u, uint64_t* base_lo,
+                                                       uint64_t* base_leaf, uint64_t* base_all)
 {
-    // one thread: the number of windows is small (total fragments / 8M)
-    if (blockIdx.x != 0 || threadIdx.x != 0)
-        return;
-    uint64_t su = 0, slo = 0, sl = 0;
-    for (int64_t w = 0; w < nw; w++)
+    __shared__ uint64_t s_warp[33];
+    const uint64_t* cnt[3] = { cu, clo, cleaf };
+    uint64_t* base[3] = { base_u, base_lo, base_leaf };
+    uint64_t run[3] = { 0, 0, 0 };
+    for (int64_t w0 = 0; w0 <= nw; w0 += blockDim.x)
     {
-        base_u[w] = su;
-        base_lo[w] = slo;
-        base_leaf[w] = sl;
-        base_all[w] = su + slo + sl;
-        su += cu[w];
-        slo += clo[w];
-        sl += cleaf[w];
+        const int64_t w = w0 + threadIdx.x;
+        uint64_t all = 0;
+        for (int k = 0; k < 3; k++)
+        {
+            uint64_t total;
+            const uint64_t ex = run[k] + block_excl_scan_u64(w < nw ? cnt[k][w] : 0ull, s_warp, total);
+            run[k] += total;
+            all += ex;
+            if (w <= nw)
+                base[k][w] = ex;
+        }
+        if (w <= nw)
+            base_all[w] = all;
     }
-    base_u[nw] = su;
-    base_lo[nw] = slo;
-    base_leaf[nw] = sl;
-    base_all[nw] = su + slo + sl;
 }
 
 static unsigned blocks_for(int64_t n)
@@ -172,16 +215,26 @@ void launch_run_min(int64_t n, const uint32_t* start, const uint64_t* child, uin
 {
     if (n <= 0)
         return;
-    { k_run_min<<<blocks_for(n), 256, 0, s>>>(n, start, child, out); count_launch(); }
+    { k_run_min<<<blocks_for(32 * n), 256, 0, s>>>(n, start, child, out); count_launch(); }
 }
 
 void launch_level_keys(int64_t n, const uint64_t* wkey, const uint32_t* parent, const uint32_t* parent_rank,
-                       const uint32_t* nval, uint32_t nmask, uint64_t* keys, uint32_t* vals, uint64_t* wcount,
-                       cudaStream_t s)
+                       const uint32_t* nval, int nbits, int pbits, void* keys, int key64, uint32_t* vals,
+                       uint64_t* wcount, cudaStream_t s)
 {
     if (n <= 0)
         return;
-    { k_level_keys<<<blocks_for(n), 256, 0, s>>>(n, wkey, parent, parent_rank, nval, nmask, keys, vals, wcount); count_launch(); }
+    if (key64)
+        { k_level_keys<uint64_t><<<blocks_for(n), 256, 0, s>>>(n, wkey, parent, parent_rank, nval, nbits, pbits, (uint64_t*)keys, vals, wcount); count_launch(); }
+    else
+        { k_level_keys<uint32_t><<<blocks_for(n), 256, 0, s>>>(n, wkey, parent, parent_rank, nval, nbits, pbits, (uint32_t*)keys, vals, wcount); count_launch(); }
+}
+
+void launch_level_rank_small(int64_t n, const uint64_t* keys, uint32_t* rank, cudaStream_t s)
+{
+    if (n <= 0)
+        return;
+    { k_level_rank_small<<<blocks_for(n), 256, 0, s>>>((int)n, keys, rank); count_launch(); }
 }
 
 void launch_level_rank(int64_t n, const uint32_t* sorted_vals, uint32_t* rank, cudaStream_t s)
@@ -191,18 +244,18 @@ void launch_level_rank(int64_t n, const uint32_t* sorted_vals, uint32_t* rank, c
     { k_level_rank<<<blocks_for(n), 256, 0, s>>>(n, sorted_vals, rank); count_launch(); }
 }
 
-void launch_leaf_popc_sorted(int64_t L, const uint32_t* sorted_vals, const uint32_t* leaf_vstart, uint64_t* out,
+void launch_leaf_popc_ranked(int64_t L, const uint32_t* rank, const uint32_t* leaf_vstart, uint64_t* out,
                              cudaStream_t s)
 {
     if (L <= 0)
         return;
-    { k_leaf_popc_sorted<<<blocks_for(L), 256, 0, s>>>(L, sorted_vals, leaf_vstart, out); count_launch(); }
+    { k_leaf_popc_ranked<<<blocks_for(L), 256, 0, s>>>(L, rank, leaf_vstart, out); count_launch(); }
 }
 
 void launch_window_bases(int64_t nw, const uint64_t* cu, const uint64_t* clo, const uint64_t* cleaf, uint64_t* base_u,
                          uint64_t* base_lo, uint64_t* base_leaf, uint64_t* base_all, cudaStream_t s)
 {
-    { k_window_bases<<<1, 1, 0, s>>>(nw, cu, clo, cleaf, base_u, base_lo, base_leaf, base_all); count_launch(); }
+    { k_window_bases<<<1, 1024, 0, s>>>(nw, cu, clo, cleaf, base_u, base_lo, base_leaf, base_all); count_launch(); }
 }
 
 void launch_window_place(const WindowOrderParams& W, const NodeParams& N, cudaStream_t s)

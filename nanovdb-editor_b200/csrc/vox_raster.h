@@ -209,11 +209,15 @@ void launch_batch_windows(const uint64_t* frag_off, const uint64_t* F_total, int
 void launch_leaf_wkey(int64_t L, const uint32_t* leaf_cand, const uint64_t* cand_wkey, uint64_t* leaf_wkey,
                       cudaStream_t s);
 void launch_run_min(int64_t n, const uint32_t* start, const uint64_t* child, uint64_t* out, cudaStream_t s);
+// keys of (window, parent rank, n) in pbits + nbits low bits, 64- or 32-bit
 void launch_level_keys(int64_t n, const uint64_t* wkey, const uint32_t* parent, const uint32_t* parent_rank,
-                       const uint32_t* nval, uint32_t nmask, uint64_t* keys, uint32_t* vals, uint64_t* wcount,
-                       cudaStream_t s);
+                       const uint32_t* nval, int nbits, int pbits, void* keys, int key64, uint32_t* vals,
+                       uint64_t* wcount, cudaStream_t s);
+// ranks of at most LEVEL_RANK_SMALL_MAX distinct 64-bit keys by counting
+constexpr int64_t LEVEL_RANK_SMALL_MAX = 2048;
+void launch_level_rank_small(int64_t n, const uint64_t* keys, uint32_t* rank, cudaStream_t s);
 void launch_level_rank(int64_t n, const uint32_t* sorted_vals, uint32_t* rank, cudaStream_t s);
-void launch_leaf_popc_sorted(int64_t L, const uint32_t* sorted_vals, const uint32_t* leaf_vstart, uint64_t* out,
+void launch_leaf_popc_ranked(int64_t L, const uint32_t* rank, const uint32_t* leaf_vstart, uint64_t* out,
                              cudaStream_t s);
 void launch_window_bases(int64_t nw, const uint64_t* cu, const uint64_t* clo, const uint64_t* cleaf, uint64_t* base_u,
                          uint64_t* base_lo, uint64_t* base_leaf, uint64_t* base_all, cudaStream_t s);
