@@ -73,7 +73,7 @@ struct vox_context_t
     DevBuf leaf_cand, leaf_lower, leaf_lower_n, leaf_origin;
     // leaf-granular pipeline
     DevBuf cand_org, tile_g0, lcols, lcol_off, lc_count, lc_mask, lc_off, emit_gid, emit_flag, lflags, lpos, cand_key, cand_start, cand_mask, pair_gid;
-    DevBuf s_rgba, s_dens, s_col, s_pairs, cand_voff, vpairs, pair_off, cand_vbase, cloud_pairs;
+    DevBuf s_rgba, s_dens, s_col, cand_pairs, cand_voff, vpairs, pair_off, cand_vbase, cloud_pairs;
     DevBuf partials, exp_keys, exp_ids;
     // reference node order
     DevBuf nwin, win_before, cand_wkey, wkey_u, wkey_lo, wkey_leaf, wcnt, wbase, okeys, okeys_alt, ovals, ovals_alt;
@@ -634,7 +634,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     // ------------------------------------------------------------ leaf walk
     const size_t slots = 512 * (size_t)(NCL + 1);
     if (!ensure(ctx, ctx->cand_mask, 64 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->s_rgba, 4 * slots) ||
-        !ensure(ctx, ctx->s_dens, 4 * slots) || !ensure(ctx, ctx->s_col, 12 * slots) || !ensure(ctx, ctx->s_pairs, 4 * slots) ||
+        !ensure(ctx, ctx->s_dens, 4 * slots) || !ensure(ctx, ctx->s_col, 12 * slots) || !ensure(ctx, ctx->cand_pairs, 8 * (size_t)(NCL + 1)) ||
         !ensure(ctx, ctx->cand_voff, 8 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->cand_vbase, 8 * (size_t)(NCL + 1)))
         return VOX_ERR_MEMORY;
     uint64_t* win_before = nullptr;
@@ -674,7 +674,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LP.s_rgba = (uint32_t*)ctx->s_rgba.p;
     LP.s_dens = (float*)ctx->s_dens.p;
     LP.s_col = (float*)ctx->s_col.p;
-    LP.s_pairs = (uint32_t*)ctx->s_pairs.p;
+    LP.cand_pairs = (uint64_t*)ctx->cand_pairs.p;
     LP.total_pairs = sc + SC_P;
     LP.err = d_err;
     LP.cand_vbase = (const uint64_t*)ctx->cand_vbase.p;
@@ -809,7 +809,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     VA.s_rgba = LP.s_rgba;
     VA.s_dens = LP.s_dens;
     VA.s_col = LP.s_col;
-    VA.s_pairs = LP.s_pairs;
+    VA.cand_pairs = LP.cand_pairs;
     VA.cloud_pairs = cloud_pairs;
     VA.cand_vbase = (uint64_t*)ctx->cand_vbase.p;
     VA.out = grid;
@@ -1014,7 +1014,7 @@ void vox_context_destroy(vox_context_t* ctx)
                       &ctx->hier_keys, &ctx->prim_keys_alt, &ctx->prim_vals_alt, &ctx->vb_work, &ctx->vb_keys, &ctx->vb_ids_c, &ctx->vb_used, &ctx->dual_idx, &ctx->vb_rec, &ctx->cloud_start,
                       &ctx->cloud_vs, &ctx->clouds, &ctx->lcols, &ctx->lcol_off, &ctx->lc_count, &ctx->lc_mask, &ctx->lc_off,
                       &ctx->cand_org, &ctx->tile_g0, &ctx->emit_gid, &ctx->emit_flag, &ctx->lflags, &ctx->lpos, &ctx->cand_key, &ctx->cand_start,
-                      &ctx->cand_mask, &ctx->pair_gid, &ctx->s_rgba, &ctx->s_dens, &ctx->s_col, &ctx->s_pairs,
+                      &ctx->cand_mask, &ctx->pair_gid, &ctx->s_rgba, &ctx->s_dens, &ctx->s_col, &ctx->cand_pairs,
                       &ctx->cand_voff, &ctx->vpairs, &ctx->pair_off, &ctx->cand_vbase, &ctx->cloud_pairs,
                       &ctx->partials, &ctx->exp_keys, &ctx->exp_ids, &ctx->nwin, &ctx->win_before,
                       &ctx->cand_wkey, &ctx->wkey_u, &ctx->wkey_lo, &ctx->wkey_leaf, &ctx->wcnt, &ctx->wbase,
@@ -1242,7 +1242,7 @@ int vox_copy_pairs(vox_context_t* ctx, uint64_t* keys, uint32_t* ids, int64_t ca
     const size_t kb = ctx->key64 ? 8 : 4;
     if (!ensure(ctx, ctx->exp_keys, kb * (size_t)P) || !ensure(ctx, ctx->exp_ids, 4 * (size_t)P))
         return VOX_ERR_MEMORY;
-    // pairs before each voxel: the staged per-voxel counts in run order, scanned
+    // pairs before each voxel: counted by a first replay of the leaf walk, scanned
     const int64_t V = ctx->last_V;
     uint64_t* sc = (uint64_t*)ctx->scal.p;
     if (!ensure(ctx, ctx->vpairs, 8 * (size_t)(V + 1)) || !ensure(ctx, ctx->pair_off, 8 * (size_t)(V + 1)) ||
@@ -1250,7 +1250,7 @@ int vox_copy_pairs(vox_context_t* ctx, uint64_t* keys, uint32_t* ids, int64_t ca
         return VOX_ERR_MEMORY;
     uint64_t* scan_status = (uint64_t*)ctx->scan_status.p;
     const size_t scan_words = ctx->scan_status.cap / sizeof(uint64_t);
-    launch_voxel_pairs(ctx->last_N, (const uint32_t*)ctx->s_pairs.p, (uint64_t*)ctx->vpairs.p, ctx->stream);
+    launch_leaf_export(ctx->last_LP, (uint64_t*)ctx->vpairs.p, (uint32_t*)(sc + SC_SCRATCH), ctx->num_sms, ctx->stream);
     scan_exclusive_u64((const uint64_t*)ctx->vpairs.p, (uint64_t*)ctx->pair_off.p, V, 0, sc + SC_SCRATCH + 3,
                        scan_status, ctx->scan_epochs.next(scan_status, scan_words, ctx->stream),
                        (uint32_t*)(sc + SC_SCRATCH), (int*)(sc + SC_ERR), ctx->num_sms, ctx->stream);
@@ -1259,7 +1259,7 @@ int vox_copy_pairs(vox_context_t* ctx, uint64_t* keys, uint32_t* ids, int64_t ca
     LP.pair_off = (const uint64_t*)ctx->pair_off.p;
     LP.out_keys = ctx->exp_keys.p;
     LP.out_ids = (uint32_t*)ctx->exp_ids.p;
-    launch_leaf_export(LP, (uint32_t*)((uint64_t*)ctx->scal.p + SC_SCRATCH), ctx->num_sms, ctx->stream);
+    launch_leaf_export(LP, nullptr, (uint32_t*)(sc + SC_SCRATCH), ctx->num_sms, ctx->stream);
     DevBuf tmp;
     if (!ensure(ctx, tmp, 8 * (size_t)P))
         return VOX_ERR_MEMORY;

@@ -486,15 +486,25 @@ __device__ __forceinline__ float pair_alpha(const GaussRec& R, const Aabb& b)
 // reference, the lattice points): 2^-20 2 Bl_r, Bl_r = il is_r sum_a |m_ra|
 // Cm_a bounding every bound's magnitude in the leaf.  So per row this AABB,
 // and its four lattice points, are within dab_r of the reference's for every
-// voxel of the leaf.  The leaf test (leaf_test_chunk) classifies voxels from
-// it, Delta = sum_r dab_r giving its thresholds lo_t / hi_t.
+// voxel of the leaf.
+//
+// The leaf test (leaf_test_columns) classifies voxels from the same AABB as
+// centre and half width, both halved (exactly): row r of the box origin's voxel
+// is c_r = 0.5 base_r + 0.25 ((A_r0 + A_r1) + A_r2), carried from the anchor to
+// the box origin by three fma, then two per column and one per voxel; the half
+// width is h_r = 0.25 W_r.  In units of 2^-24 il is_r sum_a |m_ra| E_a the
+// roundings are the chain's 3, k and base 2, the steps' 3 times |t| <= 7 with
+// 8 vs <= E (2.6), c 1.5, the way to the box origin 3, column and voxel 3, the
+// final difference and h 1.5: 16.6 where dab_r covers 16 (2^-20), so the test
+// takes 1.5 dab_r: Delta = 1.5 sum_r dab_r gives its thresholds lo_t / hi_t.
 struct LeafPairConst
 {
     float lo0[3], W[3]; // per row: the scaled lower bound of the anchor voxel, the scaled voxel width
     float A[3][3];      // A[r][a]: the scaled step of one voxel along axis a
     float dab[3];       // per row: the reference / float-channel AABB difference bound
-    float lo_t, hi_t;   // the linear z classification: certain pass below lo_t, certain fail above hi_t
-    uint32_t r0;        // the anchor voxel in the leaf: r0_x | r0_y << 8 | r0_z << 16
+    float c[3];         // per row: half the centre of the anchor voxel
+    float lo_t, hi_t;   // a quarter of the squared distances below which a voxel surely passes / above which it fails
+    int32_t r0[3];      // the anchor voxel in the leaf
 };
 
 // the anchor of the float channels' AABB along one axis (leaf origin o)
@@ -519,12 +529,11 @@ __device__ __forceinline__ LeafPairConst leaf_pair_consts(const GaussRec& R, flo
     const float is[3] = { R.q3.y, R.q3.z, R.q3.w };
     const RInv M = rinv_of(R);
     float d0[3], Gr[3], G[3], Cm[3];
-    c.r0 = 0;
 #pragma unroll
     for (int a = 0; a < 3; a++)
     {
         const int32_t r0 = anchor_of((&R.q4.x)[a], (&R.q5.x)[a], o[a]);
-        c.r0 |= (uint32_t)r0 << (8 * a);
+        c.r0[a] = r0;
         d0[a] = VOX_FFMA((float)(o[a] + r0), vs, -mu[a]);
         const float w0 = (float)o[a] * vs, w1 = (float)(o[a] + 8) * vs;
         const float W = fmaxf(fabsf(w0), fabsf(w1)) * (1.f + 0x1p-20f);
@@ -546,6 +555,7 @@ __device__ __forceinline__ LeafPairConst leaf_pair_consts(const GaussRec& R, flo
         c.lo0[r] = VOX_FADD(VOX_FADD(VOX_FADD(base, fminf(c.A[r][0], 0.f)), fminf(c.A[r][1], 0.f)),
                             fminf(c.A[r][2], 0.f));
         c.W[r] = VOX_FADD(VOX_FADD(fabsf(c.A[r][0]), fabsf(c.A[r][1])), fabsf(c.A[r][2]));
+        c.c[r] = 0.5f * base + 0.25f * ((c.A[r][0] + c.A[r][1]) + c.A[r][2]);
         const float s = (1.f + 0x1p-20f) * il * is[r];
         const float m0 = fabsf(M.m[r][0]), m1 = fabsf(M.m[r][1]), m2 = fabsf(M.m[r][2]);
         const float Bl = s * (m0 * Cm[0] + m1 * Cm[1] + m2 * Cm[2]);
@@ -553,11 +563,11 @@ __device__ __forceinline__ LeafPairConst leaf_pair_consts(const GaussRec& R, flo
         c.dab[r] = s * (m0 * G[0] + m1 * G[1] + m2 * G[2]) + 0x1p-20f * 2.f * Bl;
         Dl += c.dab[r];
     }
-    Dl *= 1.f + 0x1p-20f;
+    Dl *= 1.5f * (1.f + 0x1p-20f);
     if (Dl <= 0.0625f) // false for NaN
     {
-        c.lo_t = 1.f - (2.f * Dl + 0x1p-19f);
-        c.hi_t = 1.f + (2.f * Dl + Dl * Dl + 0x1p-18f);
+        c.lo_t = 0.25f * (1.f - (2.f * Dl + 0x1p-19f));
+        c.hi_t = 0.25f * (1.f + (2.f * Dl + Dl * Dl + 0x1p-18f));
     }
     else
     {
@@ -567,12 +577,10 @@ __device__ __forceinline__ LeafPairConst leaf_pair_consts(const GaussRec& R, flo
     return c;
 }
 
-// the float channels' local AABB of voxel o + (rx, ry, rz) from the leaf's constants (r0: the packed anchor)
-__device__ __forceinline__ Aabb stable_leaf_aabb(const float lo0[3], const float W[3], const float A[3][3], uint32_t r0,
-                                                 int32_t rx, int32_t ry, int32_t rz)
+// the float channels' local AABB of the voxel (fx, fy, fz) voxels from the anchor
+__device__ __forceinline__ Aabb stable_leaf_aabb(const float lo0[3], const float W[3], const float A[3][3], float fx,
+                                                 float fy, float fz)
 {
-    const float fx = (float)(rx - (int32_t)(r0 & 255u)), fy = (float)(ry - (int32_t)((r0 >> 8) & 255u)),
-                fz = (float)(rz - (int32_t)(r0 >> 16));
     Aabb b;
 #pragma unroll
     for (int r = 0; r < 3; r++)
@@ -583,20 +591,66 @@ __device__ __forceinline__ Aabb stable_leaf_aabb(const float lo0[3], const float
     return b;
 }
 
+// vox_expf_ch and vox_powf_ch (x <= 0; b in [0, 1], e > 0), the same results from
+// cheaper instructions: floor as an addition rounded down to the integers'
+// binade (|x / ln2| < 2^22) instead of the conversion unit's floor and
+// float-to-int, 2^k from that sum's low bits, the exponent split with one
+// integer add (mantissas above sqrt(2)'s carry into the exponent).  The cases
+// b = 0 and b = 1 fold: log(1) = 0 and exp(0) = 1 come out exactly.
+__device__ __forceinline__ float expf_ch_dev(float x)
+{
+    const float xc = fmaxf(x, -87.3f);
+    const float t = __fadd_rd(VOX_FADD(VOX_FMUL(xc, VOX_INV_LN2_F), 0.5f), 12582912.f);
+    const float kf = VOX_FSUB(t, 12582912.f);
+    const float r = VOX_FSUB(VOX_FSUB(xc, VOX_FMUL(kf, VOX_LN2_HI_F)), VOX_FMUL(kf, VOX_LN2_LO_F));
+    float p = 0.001384272240102291f;
+    p = VOX_FFMA(p, r, 0.008374955505132675f);
+    p = VOX_FFMA(p, r, 0.041668057441711426f);
+    p = VOX_FFMA(p, r, 0.1666642129421234f);
+    p = VOX_FFMA(p, r, 0.4999999403953552f);
+    p = VOX_FFMA(p, r, 1.0f);
+    p = VOX_FFMA(p, r, 1.0f);
+    const float y = VOX_FMUL(p, __uint_as_float((__float_as_uint(t) << 23) + 0x3f800000u));
+    return x < -87.3f ? 0.0f : y;
+}
+
+__device__ __forceinline__ float powf_ch_dev(float b, float e)
+{
+    const uint32_t ix = __float_as_uint(b) + (0x3f800000u - 0x3f3504f4u); // 0x3fb504f3: VOX_SQRT2_F
+    const float m = __uint_as_float((ix & 0x007fffffu) + 0x3f3504f4u);
+    const float ef = VOX_FSUB(__uint_as_float(0x4b400000u - 127u + (ix >> 23)), 12582912.f);
+    const float f = VOX_FSUB(m, 1.0f);
+    float q = -0.07633855938911438f;
+    q = VOX_FFMA(q, f, 0.1292378008365631f);
+    q = VOX_FFMA(q, f, -0.1324782371520996f);
+    q = VOX_FFMA(q, f, 0.1417929232120514f);
+    q = VOX_FFMA(q, f, -0.16608239710330963f);
+    q = VOX_FFMA(q, f, 0.2000207006931305f);
+    q = VOX_FFMA(q, f, -0.2500161826610565f);
+    q = VOX_FFMA(q, f, 0.33333325386047363f);
+    q = VOX_FFMA(q, f, -0.49999988079071045f);
+    q = VOX_FFMA(q, f, 1.0f);
+    const float lg = VOX_FADD(VOX_FMUL(ef, VOX_LN2_HI_F), VOX_FADD(VOX_FMUL(ef, VOX_LN2_LO_F), VOX_FMUL(f, q)));
+    const float y = expf_ch_dev(VOX_FMUL(e, lg));
+    return b == 0.0f ? 0.0f : y;
+}
+
 // Alpha of the float density / colour channels from their local AABB
 // (stable_leaf_aabb): the lattice points lo + w (hi - lo), float exp / pow
 // (vox_expf_ch / vox_powf_ch: about 2 ulp, no division).  The oracle's
-// frag_alpha_f evaluates the same operations in the same order.  Also keeps
-// what alpha_byte_bound needs: the lattice minimum d, op exp(-ls d) and the
-// smallest lattice square per axis.
+// frag_alpha_f evaluates the same operations in the same order (rounded
+// squares are monotone in |p|, so the smallest square is the square of the
+// smallest |p|).  Also keeps what alpha_byte_bound needs: the lattice minimum
+// d, op exp(-ls d) and the lattice point nearest to zero per axis.  q6: the
+// record's opacity, ls and e.
 struct AlphaF
 {
-    float a1;   // the channel's alpha
+    float a1;   // the channel's alpha, before the cull
     float d;    // smallest lattice |p|^2
     float a;    // op exp(-ls d), before the opacity transform
-    float m[3]; // the smallest lattice square per axis
+    float p[3]; // the smallest lattice |p| per axis
 };
-__device__ __forceinline__ AlphaF pair_alpha_f_ex(const GaussRec& R, const Aabb& b)
+__device__ __forceinline__ AlphaF pair_alpha_f_ex(const float4& q6, const Aabb& b)
 {
     AlphaF f;
     float m[3];
@@ -605,24 +659,15 @@ __device__ __forceinline__ AlphaF pair_alpha_f_ex(const GaussRec& R, const Aabb&
     {
         const float dd = VOX_FSUB(b.hi[a], b.lo[a]);
         const float p1 = VOX_FFMA(dd, 0x1.555556p-2f, b.lo[a]), p2 = VOX_FFMA(dd, 0x1.555556p-1f, b.lo[a]);
-        const float s0 = VOX_FMUL(b.lo[a], b.lo[a]), s1 = VOX_FMUL(p1, p1), s2 = VOX_FMUL(p2, p2),
-                    s3 = VOX_FMUL(b.hi[a], b.hi[a]);
-        m[a] = fminf(fminf(s0, s1), fminf(s2, s3)); // squares: no NaN, no signed zero
-        f.m[a] = m[a];
+        f.p[a] = fminf(fminf(fabsf(b.lo[a]), fabsf(p1)), fminf(fabsf(p2), fabsf(b.hi[a])));
+        m[a] = VOX_FMUL(f.p[a], f.p[a]);
     }
     f.d = VOX_FADD(VOX_FADD(m[0], m[1]), m[2]);
-    float a = VOX_FMUL(R.q6.x, vox_expf_ch(-VOX_FMUL(R.q6.y, f.d)));
-    a = a > 0.f ? a : 0.f;
+    float a = VOX_FMUL(q6.x, expf_ch_dev(-VOX_FMUL(q6.y, f.d)));
+    a = fmaxf(a, 0.f);
     f.a = a;
-    a = VOX_FSUB(1.f, vox_powf_ch(VOX_FSUB(1.f, a), R.q6.z));
-    if (R.q7.w != 0.f)
-        a = 0.f;
-    f.a1 = a;
+    f.a1 = VOX_FSUB(1.f, powf_ch_dev(VOX_FSUB(1.f, a), q6.z));
     return f;
-}
-__device__ __forceinline__ float pair_alpha_f(const GaussRec& R, const Aabb& b)
-{
-    return pair_alpha_f_ex(R, b).a1;
 }
 
 
@@ -631,12 +676,11 @@ __device__ __forceinline__ float pair_alpha_f(const GaussRec& R, const Aabb& b)
 // channel's alpha f (same formula, evaluated from stable_leaf_aabb).
 // Per row the two AABBs' bounds, and so their four lattice points, differ by at
 // most D_r = dab_r (leaf_pair_consts: the scalings' and lattice points'
-// roundings included).  With m_r
-// the float evaluation's smallest lattice square, either evaluation's
-// minimizing point is within u_r = sqrt(m_r) + D_r of zero, so the row minima
-// differ by at most 2 sqrt(m_r) D_r + D_r^2 + 2^-22 u_r^2 (rounded squares) and
-// the lattice minima d by md = sum_r of that (times 1 + 2^-20) + 2^-21 d (the
-// two rounded sums); and the
+// roundings included).  With p_r the float evaluation's lattice point nearest to
+// zero, either evaluation's minimizing point is within u_r = |p_r| + D_r of zero,
+// so the row minima differ by at most 2 |p_r| D_r + D_r^2 + 2^-22 u_r^2 (rounded
+// squares) and the lattice minima d by md = sum_r of that (times 1 + 2^-20) +
+// 2^-21 d (the two rounded sums); and the
 // alpha a' = 1 - (1 - op e^-ls d)^e, whose slope in d is at most
 // e ls a_hi (times 1 / (1 - a_hi) when e < 1) for a_hi >= op e^-ls (d - md),
 // by at most that slope times md, plus both evaluations' own error: the exps
@@ -650,16 +694,16 @@ __device__ __forceinline__ float pair_alpha_f(const GaussRec& R, const Aabb& b)
 // decided is set; otherwise the caller runs the reference's evaluation
 // (ref_alpha_byte).  VOX_CHECK_EMIT=1 compares every decided byte with the
 // reference's evaluation.
-// an upper bound of sqrt(x) for x >= 0: the hardware approximation (relative
-// error far below 2^-20) raised by 2^-18, plus 2^-60 for subnormal inputs
-__device__ __forceinline__ float sqrt_upper(float x)
+
+// the byte as the low bits of a float in [2^23, 2^23 + 256): clamped to [0, 1]
+// (a NaN to 0: its pair is never decided), the truncation an addition rounded down
+__device__ __forceinline__ uint32_t alpha_byte_bits(float v)
 {
-    float y;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y * (1.f + 0x1p-18f) + 0x1p-60f;
+    return __float_as_uint(__fadd_rd(VOX_FMUL(255.f, __saturatef(v)), 8388608.f));
 }
 
-__device__ __forceinline__ uint32_t alpha_byte_bound(const GaussRec& R, const AlphaF& f, const float dab[3],
+// the byte in bits 24-31, the rest 0
+__device__ __forceinline__ uint32_t alpha_byte_bound(const float4& q6, float cull, const AlphaF& f, const float dab[3],
                                                      bool& decided)
 {
     // branch-free (the pairs of a warp take different cases): every quantity is
@@ -668,12 +712,12 @@ __device__ __forceinline__ uint32_t alpha_byte_bound(const GaussRec& R, const Al
 #pragma unroll
     for (int r = 0; r < 3; r++)
     {
-        const float D = dab[r]; // dab_r + 2^-20 B_r, folded per leaf (leaf_pair_consts)
-        const float u = sqrt_upper(f.m[r]) + D; // bounds both evaluations' minimizing lattice point
+        const float D = dab[r];
+        const float u = f.p[r] + D; // bounds both evaluations' minimizing lattice point
         md += (2.f * u - D) * D + 0x1p-22f * u * u;
     }
     md = md * (1.f + 0x1p-20f) + 0x1p-21f * f.d;
-    const float ls = R.q6.y, e = R.q6.z;
+    const float ls = q6.y, e = q6.z;
     const float x = ls * md;
     const float a_hi = f.a * (1.f + 2.f * x) * (1.f + 1e-6f); // e^x <= 1 + 2x for x <= 1
     // 1 / (1 - a_hi) from the fast reciprocal (within 2 ulp for 1 - a_hi >= 2^-24,
@@ -682,10 +726,10 @@ __device__ __forceinline__ uint32_t alpha_byte_bound(const GaussRec& R, const Al
     const float slope_e = e < 1.f ? e * inv : e; // the pow's slope bound
     const float slope = slope_e * ls * a_hi;
     const float delta = 1.25f * slope * md + slope_e * (1.1e-6f * a_hi + 1.8e-7f) + 9.3e-7f;
-    const uint32_t lo = rgba8_byte(f.a1 - delta), hi = rgba8_byte(f.a1 + delta);
-    const bool culled = R.q7.w != 0.f; // culled by scale: both alphas are 0
+    const uint32_t lo = alpha_byte_bits(f.a1 - delta), hi = alpha_byte_bits(f.a1 + delta);
+    const bool culled = cull != 0.f; // culled by scale: both alphas are 0
     decided = culled || (x < 0.25f && a_hi < 1.f && lo == hi);
-    return culled ? 0u : lo;
+    return culled ? 0u : lo << 24;
 }
 
 // the reference's RGBA8 alpha byte of voxel (i, j, k) and the record's Gaussian

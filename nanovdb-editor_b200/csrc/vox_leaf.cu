@@ -325,37 +325,35 @@ struct RecSlot
 
 struct LeafChunk
 {
-    RecSlot rec[LQ_CHUNK];                               // first member: 16-byte aligned for cp.async
-    int32_t bx0[LQ_CHUNK], by0[LQ_CHUNK], bz0[LQ_CHUNK]; // box origin, leaf-relative
-    uint32_t bny[LQ_CHUNK], bnz[LQ_CHUNK];               // box extents in y and z
-    uint32_t bdiv_y[LQ_CHUNK];                           // 65536 / ny, rounded up (exact division below 64)
-    uint32_t bcol[LQ_CHUNK];                             // box columns, nx * ny (0: empty box)
-    uint32_t rgb24[LQ_CHUNK];                            // the colour bytes of the packed RGBA8 value
-    float vs[LQ_CHUNK];
-    // leaf_pair_consts of each (leaf, Gaussian), by row
-    float lo0[3][LQ_CHUNK], wid[3][LQ_CHUNK]; // the float channels' AABB of the leaf's voxel (0, 0, 0)
-    float stp[3][3][LQ_CHUNK];                 // [r][a]: the scaled voxel steps ([r][2]: the z step of the test)
-    float dab[3][LQ_CHUNK];                    // reference / float-channel AABB difference bound
-    float lo_t[LQ_CHUNK], hi_t[LQ_CHUNK];      // the linear z classification's thresholds
-    uint32_t anchor[LQ_CHUNK];                 // the float channels' anchor voxel (packed)
-    uint32_t cstart[16];    // first column of box j (boxes past the chunk's count: empty); [LQ_CHUNK]: all
+    RecSlot rec[LQ_CHUNK]; // first member: 16-byte aligned for cp.async
+    // Constants of each (leaf, Gaussian) as 16-byte words, one load each:
+    // the test's (leaf_pair_consts, halved; c at the box origin's voxel)
+    //   [0] c 0..2, lo_t   [1] x steps 0..2, hi_t   [2] y steps 0..2, h 0   [3] z steps 0..2, h 1
+    //   [4] h 2, 65536 / ny rounded up (exact division below 64), ny | nz << 8, j << 9 | box origin's leaf_n
+    float4 tq[5][LQ_CHUNK];
+    // the float channels'
+    //   [r] lo0 r, W r, x step r, y step r   [3] z steps 0..2, colour bytes of the RGBA8 value
+    //   [4] dab 0..2, voxel size   [5] 2^23 + anchor x, y, z
+    float4 aq[6][LQ_CHUNK];
+    uint32_t cstart[16];    // first column of box j (boxes past the chunk's count: none left); [LQ_CHUNK]: all
     uint8_t flag[LQ_CHUNK];
     uint64_t wf0[LQ_CHUNK], wbase[LQ_CHUNK]; // reference windows: fragment offset in its batch, windows before
 };
 
+// Per-voxel sums as two 32-bit words (acc_add)
 struct LeafAcc
 {
-    unsigned long long dens[512];   // fixed-point sums
-    unsigned long long col[3][512];
-    uint32_t cnt[512];              // passing pairs
-    uint32_t rgba[512];             // packed RGBA8 maximum
-    unsigned long long wmin;        // creation window (reference node order)
+    uint32_t dens[2][512];
+    uint32_t col[3][2][512];
+    uint32_t rgba[512];       // packed RGBA8 maximum
+    unsigned long long wmin;  // creation window (reference node order)
 };
 
 struct LeafQSmem
 {
     LeafChunk ch[3];
-    LeafAcc acc[1];
+    LeafAcc acc;
+    uint32_t mask[3][16]; // value masks of the leaf being tested and of the two before it
     uint16_t queue[2][LQ_CHUNK * 512];
     uint16_t defer[LP_THREADS / 32][64]; // per warp: queued pairs whose RGBA8 byte the bound left open
     uint32_t dcount[LP_THREADS / 32];     // per warp: the open pairs left at the end of its alpha
@@ -365,199 +363,166 @@ struct LeafQSmem
     uint32_t nxt_q0[2], nxt_p1[2];
     uint32_t cand_next[2];
     uint32_t cand;
-    unsigned long long pairs;
 };
 
-// The reference test on the boxes of a chunk, one box column per thread, its
-// passing (Gaussian, voxel) pairs appended to queue (entry j << 9 | leaf_n).
-// Bit-identical to voxel_local_aabb + aabb_hits_unit_sphere per voxel: the z
-// corner c1 of voxel z is c0 of voxel z + 1 (integer-valued floats), and "lo >
-// 0: subtract lo^2, else hi < 0: subtract hi^2" selects the pre-scale bound
-// with the same sign (inv_ls, inv_s > 0; an underflow to zero subtracts zero).
-// Every thread of the CTA calls it (warp-synchronous queue slots).  PER_WARP:
-// warp w appends to its own region queue[w * 512, ...) at warp-local
-// positions and stores its count in qcount[w] - a deterministic order (a warp
-// tests at most 2 x 32 columns of 8 voxels).  Otherwise one shared queue, a
-// shared atomic per warp and round.
-//
-// APPROX (a LeafChunk, carrying the leaf_pair_consts of each Gaussian): each
-// voxel of the column is first classified from the float channels' local AABB
-// (stable_leaf_aabb: per column the x / y terms once, then one fma per row
-// and voxel), and only voxels near the sphere run the reference test.  Per
-// row that AABB is within delta_r = dab_r of the reference's
-// (leaf_pair_consts), so the selected values (max(lo, min(hi, 0)),
-// 1-Lipschitz in both bounds) differ by at most delta_r and the vectors of the
-// three by eta <= Delta = sum delta_r in norm.  The reference passes a voxel
-// when its fl-evaluated 1 - S > 0: surely if S < 1 - 2^-22 (three subtractions
-// and squares of values below 1) and surely not if S > 1 + 2^-20.  With D the
-// fma-summed squares of the float values (relative error <= 3 2^-24) and
-// Delta <= 1/16, (sqrt(D) + eta)^2 < 1 - 2^-22 holds when D < lo_t = 1 -
-// (2 Delta + 2^-19), and (sqrt(D) - eta)^2 > 1 + 2^-20 when D > hi_t = 1 +
-// (2 Delta + Delta^2 + 2^-18) (the slack covers the roundings of the
-// thresholds themselves).  Voxels with D in [lo_t, hi_t] (or NaN), and every
-// voxel of a (leaf, Gaussian) with Delta > 1/16 (lo_t = -1, hi_t = inf), take
-// the reference test.  In CHECK mode every voxel also takes it and a
-// difference sets ERR_BOUNDS.
-template <bool CHECK, bool PER_WARP = false, bool APPROX = false, class Chunk>
-__device__ __forceinline__ void leaf_test_chunk(const LeafPassParams& P, const Chunk& C, uint32_t cnt,
-                                                const int32_t o[3], uint16_t* queue, uint32_t* qcount, int t, int lane,
-                                                uint32_t rot = 0)
+// One term of an exact fixed-point sum, (hi, lo) += (xh, xl) with the carry from
+// the low word's old value: the total is the same integer in any order.  A
+// 64-bit add in shared memory is a compare-and-swap loop (several round trips
+// where lanes meet on a voxel); 32-bit adds are single instructions, and the
+// high word is touched only when something reaches it (about once in 1 / alpha
+// terms).
+__device__ __forceinline__ void acc_add(uint32_t* lo, uint32_t* hi, uint32_t xl, uint32_t xh)
 {
-    uint32_t wbase = 0; // PER_WARP: entries this warp has written
-    if (PER_WARP)
-        queue += (t >> 5) * (LQ_CHUNK * 64);
-    uint32_t start[LQ_CHUNK + 1];
-    uint32_t T;
-    if constexpr (APPROX)
-        T = C.cstart[LQ_CHUNK]; // the staged prefix (no registers held across the rounds)
-    else
-    {
-        start[0] = 0;
-#pragma unroll
-        for (int j = 0; j < LQ_CHUNK; j++)
-            start[j + 1] = start[j] + (j < (int)cnt ? C.bcol[j] : 0u);
-        T = start[LQ_CHUNK];
-    }
+    const uint32_t old = atomicAdd(lo, xl);
+    const uint32_t up = xh + (old + xl < old ? 1u : 0u);
+    if (up)
+        atomicAdd(hi, up);
+}
+__device__ __forceinline__ void acc_add(uint32_t* lo, uint32_t* hi, unsigned long long x)
+{
+    acc_add(lo, hi, (uint32_t)x, (uint32_t)(x >> 32));
+}
+
+// Two floats in one register pair; add and fma round each half as the scalar
+// instruction does and take one issue slot for both.
+struct F2
+{
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi)
+{
+    F2 o;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(o.v) : "f"(lo), "f"(hi));
+    return o;
+}
+__device__ __forceinline__ float2 f2_get(F2 a)
+{
+    float2 o;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(a.v));
+    return o;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
+{
+    F2 o;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(o.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return o;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b)
+{
+    F2 o;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(o.v) : "l"(a.v), "l"(b.v));
+    return o;
+}
+
+// The forward walk's test: the boxes of a chunk, one box column per lane; the
+// passing (Gaussian, voxel) pairs are appended to queue (entry j << 9 | leaf_n)
+// and their voxels set in mask (the leaf's value mask as 32-bit words).  The
+// results are voxel_local_aabb + aabb_hits_unit_sphere per voxel, decided where
+// possible from the float channels' local AABB as centre and half width
+// (leaf_pair_consts; per row x = max(|c| - h, 0) is the AABB's point nearest to
+// zero, 1-Lipschitz in c and h).  Per row that is within delta_r = 1.5 dab_r of
+// the reference's, so the vectors of the three differ by eta <= Delta = sum
+// delta_r in norm.  The reference passes a voxel when its fl-evaluated 1 - S >
+// 0: surely if S < 1 - 2^-22 (three subtractions and squares of values below 1)
+// and surely not if S > 1 + 2^-20.  With D the fma-summed squares of the float
+// values (relative error <= 3 2^-24) and Delta <= 1/16, (sqrt(D) + eta)^2 <
+// 1 - 2^-22 holds when D < 1 - (2 Delta + 2^-19), and (sqrt(D) - eta)^2 > 1 +
+// 2^-20 when D > 1 + (2 Delta + Delta^2 + 2^-18) (the slack covers the
+// roundings of the thresholds themselves).  The kernel holds c, h and the steps
+// halved, D and the thresholds quartered: a halved x saturates at 1 (a quarter
+// of D at least 1: far above the fail threshold).  Voxels between the
+// thresholds, and every voxel of a (leaf, Gaussian) with Delta > 1/16 (lo_t =
+// -1, hi_t = inf; also NaN), take the reference test.  In CHECK mode every
+// voxel also takes it and a difference sets ERR_BOUNDS.
+//
+// The walk is bound by instruction issue, and integer and min / max instructions
+// run at half the rate of FP32 ones, so the z loop has two voxels per step in
+// packed FP32 arithmetic, |c| - h clamped by the addition itself (.sat), and the
+// comparisons as sign bits of differences shifted into the masks (highest z
+// first): 11 instructions per voxel for 24.  With acc_add, the constants as
+// 16-byte words and the value masks set here instead of counted per pair, the
+// walk of 2M Gaussians (1.6e9 pairs) 42.9 -> 34.1 ms.
+template <bool CHECK>
+__device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const LeafChunk& C, const int32_t o[3],
+                                                  uint16_t* queue, uint32_t* qcount, uint32_t* mask, int t, int lane,
+                                                  uint32_t rot)
+{
+    const uint32_t T = C.cstart[LQ_CHUNK];
+    const uint32_t cs = lane < LQ_CHUNK ? C.cstart[lane] : 0x7fffffffu;
+    const uint32_t le = 0xffffffffu >> (31 - lane);
     // rounds of 32 columns dealt to the warps in turn, starting at warp rot (mod 8):
-    // the forward continues the deal where the alpha's rounds of 32 pairs stopped,
-    // so the warps' loads in a phase differ by at most one round
+    // the deal continues where the alpha's rounds of 32 pairs stopped, so the warps'
+    // loads in a phase differ by at most one round
     const uint32_t first = (uint32_t)(((t >> 5) - (int)(rot & 7u)) & 7);
-    for (uint32_t tu = first; tu * 32u < T; tu += LP_THREADS / 32)
+    for (uint32_t e0 = first * 32u; e0 < T; e0 += LP_THREADS)
     {
-        const uint32_t e = tu * 32u + (uint32_t)lane;
+        // j: the last box whose first column is <= e (a box with columns: every
+        // emitted leaf meets its Gaussian's bbox); sj its first column
+        const uint32_t rel = cs - e0;
+        const uint32_t heads = __reduce_or_sync(0xffffffffu, rel - 1u < 31u ? 1u << rel : 0u);
+        const uint32_t j = (uint32_t)(__popc(__ballot_sync(0xffffffffu, cs <= e0)) - 1 + __popc(heads & le)) & 15u;
+        const uint32_t sj = __shfl_sync(0xffffffffu, cs, (int)j);
+        const uint32_t e = e0 + (uint32_t)lane;
         uint32_t zmask = 0, ebase = 0;
         if (e < T)
         {
-            // j: the last box whose first column is <= e (empty boxes skipped); sj its first column
-            int j = 0;
-            uint32_t sj = 0;
-            if constexpr (APPROX)
-            {
-#pragma unroll
-                for (int s = 8; s; s >>= 1)
-                    if (j + s < LQ_CHUNK && C.cstart[j + s] <= e)
-                        j += s;
-                sj = C.cstart[j];
-            }
-            else
-            {
-#pragma unroll
-                for (int q = 1; q < LQ_CHUNK; q++) // without a dynamically indexed (local memory) array
-                {
-                    const bool ge = e >= start[q];
-                    j += ge ? 1 : 0;
-                    sj = ge ? start[q] : sj;
-                }
-            }
+            const float4 q0 = C.tq[0][j], q1 = C.tq[1][j], q2 = C.tq[2][j], q3 = C.tq[3][j], q4 = C.tq[4][j];
+            const uint32_t ext = __float_as_uint(q4.z), ny = ext & 255u, nz = ext >> 8;
             const uint32_t local = e - sj;
-            const uint32_t dx = (local * C.bdiv_y[j]) >> 16;
-            const uint32_t dy = local - dx * C.bny[j];
-            const int32_t rx = C.bx0[j] + (int32_t)dx, ry = C.by0[j] + (int32_t)dy, rz0 = C.bz0[j];
-            const GaussRec& R = C.rec[j].r;
-            const float vsf = C.vs[j];
-            const uint32_t nz = C.bnz[j];
-            if constexpr (APPROX)
+            const uint32_t dx = (local * __float_as_uint(q4.y)) >> 16;
+            const uint32_t dy = local - dx * ny;
+            ebase = __float_as_uint(q4.w) + (dx << 6) + (dy << 3);
+            const float fx = (float)dx, fy = (float)dy;
+            const float b0 = VOX_FFMA(fy, q2.x, VOX_FFMA(fx, q1.x, q0.x)), b1 = VOX_FFMA(fy, q2.y, VOX_FFMA(fx, q1.y, q0.y)),
+                        b2 = VOX_FFMA(fy, q2.z, VOX_FFMA(fx, q1.z, q0.z));
+            const F2 B0 = f2(b0, b0), B1 = f2(b1, b1), B2 = f2(b2, b2);
+            const F2 S0 = f2(q3.x, q3.x), S1 = f2(q3.y, q3.y), S2 = f2(q3.z, q3.z);
+            const F2 nlo = f2(-q0.w, -q0.w), hi2 = f2(q1.w, q1.w), m1 = f2(-1.f, -1.f), m2 = f2(-2.f, -2.f),
+                     zero = f2(0.f, 0.f);
+            const float h0 = q2.w, h1 = q3.w, h2 = q4.x;
+            const uint32_t steps = (nz + 1u) >> 1; // voxels (2 k - 2, 2 k - 1) for k = steps .. 1
+            const float ft = (float)(2u * steps);
+            F2 K = f2(ft - 2.f, ft - 1.f);
+            uint32_t pass = 0, fail = 0;
+#pragma unroll 1
+            for (uint32_t k = steps; k; k--)
             {
-                // the float channels' AABB of the run's voxels (stable_leaf_aabb: the
-                // column's x / y terms once, then one fma per row and voxel), within
-                // delta_r of the reference's for every voxel of the leaf
-                const uint32_t anc = C.anchor[j];
-                const float tx = (float)(rx - (int32_t)(anc & 255u)), ty = (float)(ry - (int32_t)((anc >> 8) & 255u)),
-                            tz0 = (float)(rz0 - (int32_t)(anc >> 16));
-                float base[3], wid[3], st[3];
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-                {
-                    base[r] = VOX_FFMA(ty, C.stp[r][1][j], VOX_FFMA(tx, C.stp[r][0][j], C.lo0[r][j]));
-                    wid[r] = C.wid[r][j];
-                    st[r] = C.stp[r][2][j];
-                }
-                const float lo_t = C.lo_t[j], hi_t = C.hi_t[j];
-                uint32_t unc = 0;
-                {
-                    float kf = tz0;
-#pragma unroll 1 // measured: unrolling by 2, 4 or 8 is slower
-                    for (uint32_t k = 0; k < nz; k++, kf += 1.f)
-                    {
-                        float D = 0.f;
-#pragma unroll
-                        for (int r = 0; r < 3; r++)
-                        {
-                            const float a = VOX_FFMA(kf, st[r], base[r]), b = VOX_FADD(a, wid[r]);
-                            const float xs = fmaxf(a, fminf(b, 0.f));
-                            D = __fmaf_rn(xs, xs, D);
-                        }
-                        zmask |= (D < lo_t ? 1u : 0u) << k;
-                        unc |= (D > hi_t ? 0u : 1u) << k; // not surely failing (NaN included)
-                    }
-                    unc &= ~zmask; // neither surely passing nor surely failing
-                }
-                // the reference test of one voxel, from the record (nothing of the column kept live)
-                auto exact_voxel = [&](uint32_t k) -> uint32_t {
-                    const Aabb b = voxel_local_aabb(R, rinv_of(R), vsf, o[0] + rx, o[1] + ry, o[2] + rz0 + (int32_t)k);
-                    return aabb_hits_unit_sphere(b) ? 1u << k : 0u;
-                };
-                for (uint32_t m = unc; m; m &= m - 1u)
-                    zmask |= exact_voxel((uint32_t)(__ffs(m) - 1));
-                if (CHECK)
-                {
-                    uint32_t ex = 0;
-                    for (uint32_t k = 0; k < nz; k++)
-                        ex |= exact_voxel(k);
-                    if (ex != zmask)
-                        atomicOr(P.err, ERR_BOUNDS); // a linear classification differs from the reference test
-                }
+                const float2 c0 = f2_get(f2_fma(K, S0, B0)), c1 = f2_get(f2_fma(K, S1, B1)), c2 = f2_get(f2_fma(K, S2, B2));
+                const F2 x0 = f2(__saturatef(VOX_FSUB(fabsf(c0.x), h0)), __saturatef(VOX_FSUB(fabsf(c0.y), h0)));
+                const F2 x1 = f2(__saturatef(VOX_FSUB(fabsf(c1.x), h1)), __saturatef(VOX_FSUB(fabsf(c1.y), h1)));
+                const F2 x2 = f2(__saturatef(VOX_FSUB(fabsf(c2.x), h2)), __saturatef(VOX_FSUB(fabsf(c2.y), h2)));
+                const F2 D = f2_fma(x2, x2, f2_fma(x1, x1, f2_fma(x0, x0, zero)));
+                const float2 dl = f2_get(f2_add(D, nlo)), dh = f2_get(f2_fma(D, m1, hi2));
+                pass = __funnelshift_l(__float_as_uint(dl.y), pass, 1);
+                pass = __funnelshift_l(__float_as_uint(dl.x), pass, 1);
+                fail = __funnelshift_l(__float_as_uint(dh.y), fail, 1);
+                fail = __funnelshift_l(__float_as_uint(dh.x), fail, 1);
+                K = f2_add(K, m2);
             }
-            else
+            const uint32_t valid = (1u << nz) - 1u;
+            zmask = pass & valid;
+            // the reference test of one voxel, from the record (nothing of the column kept live)
+            auto exact_voxel = [&](uint32_t k) -> uint32_t {
+                const GaussRec& R = C.rec[j].r;
+                const uint32_t n = (ebase & 511u) + k;
+                const Aabb b = voxel_local_aabb(R, rinv_of(R), C.aq[4][j].w, o[0] + (int32_t)(n >> 6),
+                                                o[1] + (int32_t)((n >> 3) & 7u), o[2] + (int32_t)(n & 7u));
+                return aabb_hits_unit_sphere(b) ? 1u << k : 0u;
+            };
+            for (uint32_t m = ~(pass | fail) & valid; m; m &= m - 1u)
+                zmask |= exact_voxel((uint32_t)(__ffs(m) - 1));
+            if (CHECK)
             {
-                const RInv M = rinv_of(R);
-                const float il = R.q0.w, pz = R.q0.z;
-                const float is[3] = { R.q3.y, R.q3.z, R.q3.w };
-                float cx0, cx1, cy0, cy1;
-                axis_corners(vsf, R.q0.x, o[0] + rx, cx0, cx1);
-                axis_corners(vsf, R.q0.y, o[1] + ry, cy0, cy1);
-                float slo[3], shi[3], pa[3];
-                float v = (float)(o[2] + rz0);
-                float cz = VOX_FSUB(VOX_FMUL(v, vsf), pz);
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-                {
-                    float xn, xx, yn, yx;
-                    minmax_prod(cx0, cx1, M.m[r][0], xn, xx);
-                    minmax_prod(cy0, cy1, M.m[r][1], yn, yx);
-                    slo[r] = VOX_FADD(xn, yn);
-                    shi[r] = VOX_FADD(xx, yx);
-                    pa[r] = VOX_FMUL(cz, M.m[r][2]);
-                }
-                // the reference test along the z run
-#pragma unroll 2
+                uint32_t ex = 0;
                 for (uint32_t k = 0; k < nz; k++)
-                {
-                    v = VOX_FADD(v, 1.f);
-                    cz = VOX_FSUB(VOX_FMUL(v, vsf), pz);
-                    float d2 = 1.f;
-#pragma unroll
-                    for (int r = 0; r < 3; r++)
-                    {
-                        // the corner offsets grow with z: per row the smaller product is the
-                        // lower corner's when the matrix entry is >= 0 (fl(c m) is monotone
-                        // in c; a tie differs at most in the sign of a zero, which is squared)
-                        const float pb = VOX_FMUL(cz, M.m[r][2]);
-                        const bool up = M.m[r][2] >= 0.f;
-                        const float zn = up ? pa[r] : pb, zx = up ? pb : pa[r];
-                        pa[r] = pb;
-                        const float xl = VOX_FADD(slo[r], zn), xh = VOX_FADD(shi[r], zx);
-                        // xl <= xh: the bound of the row's interval nearest to zero, or zero
-                        const float xs = VOX_FADD(fmaxf(xl, 0.f), fminf(xh, 0.f));
-                        const float sv = VOX_FMUL(VOX_FMUL(xs, il), is[r]);
-                        d2 = VOX_FSUB(d2, VOX_FMUL(sv, sv));
-                    }
-                    zmask |= (d2 > 0.f ? 1u : 0u) << k;
-                }
+                    ex |= exact_voxel(k);
+                if (ex != zmask)
+                    atomicOr(P.err, ERR_BOUNDS); // a classification differs from the reference test
+                if (zmask && C.flag[j])
+                    atomicOr(P.err, ERR_BOUNDS); // the leaf test would have dropped a passing voxel
             }
-            ebase = ((uint32_t)j << 9) | (uint32_t)((rx << 6) | (ry << 3) | rz0);
-            if (CHECK && zmask && C.flag[j])
-                atomicOr(P.err, ERR_BOUNDS); // the leaf test would have dropped a passing voxel
+            if (zmask)
+                atomicOr(&mask[(ebase & 511u) >> 5], zmask << (ebase & 31u));
         }
         // queue slots: warp inclusive scan of the pass counts, one shared atomic per warp
         const uint32_t np = (uint32_t)__popc(zmask);
@@ -570,47 +535,150 @@ __device__ __forceinline__ void leaf_test_chunk(const LeafPassParams& P, const C
                 incl += y;
         }
         uint32_t qb = 0;
-        if (PER_WARP)
-        {
-            qb = wbase + incl - np;
-            wbase += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        else
-        {
-            if (lane == 31 && incl)
-                qb = atomicAdd(qcount, incl);
-            qb = __shfl_sync(0xffffffffu, qb, 31) + incl - np;
-        }
+        if (lane == 31 && incl)
+            qb = atomicAdd(qcount, incl);
+        qb = __shfl_sync(0xffffffffu, qb, 31) + incl - np;
         for (uint32_t m = zmask; m; m &= m - 1)
             queue[qb++] = (uint16_t)(ebase + (uint32_t)(__ffs(m) - 1));
     }
-    if (PER_WARP && lane == 0)
+}
+
+// The adjoint walk's test, the reference's own on every voxel: one box column
+// per thread, the passing (Gaussian, voxel) pairs appended to queue (entry j <<
+// 9 | leaf_n), warp w to its own region queue[w * 512, ...) at warp-local
+// positions, its count in qcount[w] - a deterministic order (a warp tests at
+// most 2 x 32 columns of 8 voxels).
+// Bit-identical to voxel_local_aabb + aabb_hits_unit_sphere per voxel: the z
+// corner c1 of voxel z is c0 of voxel z + 1 (integer-valued floats), and "lo >
+// 0: subtract lo^2, else hi < 0: subtract hi^2" selects the pre-scale bound
+// with the same sign (inv_ls, inv_s > 0; an underflow to zero subtracts zero).
+// Every thread of the CTA calls it (warp-synchronous queue slots).
+template <class Chunk>
+__device__ __forceinline__ void leaf_test_chunk(const Chunk& C, uint32_t cnt, const int32_t o[3], uint16_t* queue,
+                                                uint32_t* qcount, int t, int lane)
+{
+    uint32_t wbase = 0; // entries this warp has written
+    queue += (t >> 5) * (LQ_CHUNK * 64);
+    uint32_t start[LQ_CHUNK + 1];
+    start[0] = 0;
+#pragma unroll
+    for (int j = 0; j < LQ_CHUNK; j++)
+        start[j + 1] = start[j] + (j < (int)cnt ? C.bcol[j] : 0u);
+    const uint32_t T = start[LQ_CHUNK];
+    for (uint32_t tu = (uint32_t)(t >> 5); tu * 32u < T; tu += LP_THREADS / 32)
+    {
+        const uint32_t e = tu * 32u + (uint32_t)lane;
+        uint32_t zmask = 0, ebase = 0;
+        if (e < T)
+        {
+            // j: the last box whose first column is <= e (empty boxes skipped); sj its first column
+            int j = 0;
+            uint32_t sj = 0;
+#pragma unroll
+            for (int q = 1; q < LQ_CHUNK; q++) // without a dynamically indexed (local memory) array
+            {
+                const bool ge = e >= start[q];
+                j += ge ? 1 : 0;
+                sj = ge ? start[q] : sj;
+            }
+            const uint32_t local = e - sj;
+            const uint32_t dx = (local * C.bdiv_y[j]) >> 16;
+            const uint32_t dy = local - dx * C.bny[j];
+            const int32_t rx = C.bx0[j] + (int32_t)dx, ry = C.by0[j] + (int32_t)dy, rz0 = C.bz0[j];
+            const GaussRec& R = C.rec[j].r;
+            const float vsf = C.vs[j];
+            const uint32_t nz = C.bnz[j];
+            const RInv M = rinv_of(R);
+            const float il = R.q0.w, pz = R.q0.z;
+            const float is[3] = { R.q3.y, R.q3.z, R.q3.w };
+            float cx0, cx1, cy0, cy1;
+            axis_corners(vsf, R.q0.x, o[0] + rx, cx0, cx1);
+            axis_corners(vsf, R.q0.y, o[1] + ry, cy0, cy1);
+            float slo[3], shi[3], pa[3];
+            float v = (float)(o[2] + rz0);
+            float cz = VOX_FSUB(VOX_FMUL(v, vsf), pz);
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+            {
+                float xn, xx, yn, yx;
+                minmax_prod(cx0, cx1, M.m[r][0], xn, xx);
+                minmax_prod(cy0, cy1, M.m[r][1], yn, yx);
+                slo[r] = VOX_FADD(xn, yn);
+                shi[r] = VOX_FADD(xx, yx);
+                pa[r] = VOX_FMUL(cz, M.m[r][2]);
+            }
+            // the reference test along the z run
+#pragma unroll 2
+            for (uint32_t k = 0; k < nz; k++)
+            {
+                v = VOX_FADD(v, 1.f);
+                cz = VOX_FSUB(VOX_FMUL(v, vsf), pz);
+                float d2 = 1.f;
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+                {
+                    // the corner offsets grow with z: per row the smaller product is the
+                    // lower corner's when the matrix entry is >= 0 (fl(c m) is monotone
+                    // in c; a tie differs at most in the sign of a zero, which is squared)
+                    const float pb = VOX_FMUL(cz, M.m[r][2]);
+                    const bool up = M.m[r][2] >= 0.f;
+                    const float zn = up ? pa[r] : pb, zx = up ? pb : pa[r];
+                    pa[r] = pb;
+                    const float xl = VOX_FADD(slo[r], zn), xh = VOX_FADD(shi[r], zx);
+                    // xl <= xh: the bound of the row's interval nearest to zero, or zero
+                    const float xs = VOX_FADD(fmaxf(xl, 0.f), fminf(xh, 0.f));
+                    const float sv = VOX_FMUL(VOX_FMUL(xs, il), is[r]);
+                    d2 = VOX_FSUB(d2, VOX_FMUL(sv, sv));
+                }
+                zmask |= (d2 > 0.f ? 1u : 0u) << k;
+            }
+            ebase = ((uint32_t)j << 9) | (uint32_t)((rx << 6) | (ry << 3) | rz0);
+        }
+        // queue slots: warp inclusive scan of the pass counts
+        const uint32_t np = (uint32_t)__popc(zmask);
+        uint32_t incl = np;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off)
+                incl += y;
+        }
+        uint32_t qb = wbase + incl - np;
+        wbase += __shfl_sync(0xffffffffu, incl, 31);
+        for (uint32_t m = zmask; m; m &= m - 1)
+            queue[qb++] = (uint16_t)(ebase + (uint32_t)(__ffs(m) - 1));
+    }
+    if (lane == 0)
         qcount[t >> 5] = wbase;
 }
 
-// the part of a Gaussian's bbox inside the leaf at o
-template <class Chunk>
-__device__ __forceinline__ void leaf_box_fields(Chunk& C, int j, const GaussRec& R, const int32_t o[3])
+// the part of a Gaussian's bbox inside the leaf at o, leaf-relative
+struct LeafBox
 {
+    int32_t lo[3];
+    uint32_t nx, ny, nz; // nx = 0: empty
+};
+__device__ __forceinline__ LeafBox leaf_box(const GaussRec& R, const int32_t o[3])
+{
+    LeafBox b;
     const int32_t x0 = max(R.q4.x, o[0]) - o[0], x1 = min(R.q4.x + R.q5.x - 1, o[0] + 7) - o[0];
     const int32_t y0 = max(R.q4.y, o[1]) - o[1], y1 = min(R.q4.y + R.q5.y - 1, o[1] + 7) - o[1];
     const int32_t z0 = max(R.q4.z, o[2]) - o[2], z1 = min(R.q4.z + R.q5.z - 1, o[2] + 7) - o[2];
     const bool empty = x1 < x0 || y1 < y0 || z1 < z0;
-    const uint32_t ny = empty ? 1u : (uint32_t)(y1 - y0 + 1), nz = empty ? 1u : (uint32_t)(z1 - z0 + 1);
-    C.bx0[j] = x0;
-    C.by0[j] = y0;
-    C.bz0[j] = z0;
-    C.bny[j] = ny;
-    C.bnz[j] = nz;
-    C.bdiv_y[j] = (65536u + ny - 1u) / ny;
-    C.bcol[j] = empty ? 0u : (uint32_t)(x1 - x0 + 1) * ny;
+    b.lo[0] = x0;
+    b.lo[1] = y0;
+    b.lo[2] = z0;
+    b.nx = empty ? 0u : (uint32_t)(x1 - x0 + 1);
+    b.ny = empty ? 1u : (uint32_t)(y1 - y0 + 1);
+    b.nz = empty ? 1u : (uint32_t)(z1 - z0 + 1);
+    return b;
 }
 
-// all stagers (lanes 0 .. LQ_CHUNK - 1 of the last warp), once the boxes of the
-// chunk's cnt Gaussians are placed: the chunk's column prefix
-__device__ __forceinline__ void leaf_stage_prefix(LeafChunk& C, int js, uint32_t cnt)
+// all stagers (lanes 0 .. LQ_CHUNK - 1 of the last warp): the chunk's column
+// prefix from each stager's own box columns (0 past the chunk's count)
+__device__ __forceinline__ void leaf_stage_prefix(LeafChunk& C, int js, uint32_t b)
 {
-    uint32_t b = js < (int)cnt ? C.bcol[js] : 0u;
 #pragma unroll
     for (int off = 1; off < LQ_CHUNK; off <<= 1)
     {
@@ -645,36 +713,43 @@ __device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, Ga
     return g;
 }
 
-// once the record landed: the part of the Gaussian's bbox inside the leaf at o
+// once the record landed: the chunk's constants of Gaussian j; returns its box columns
 template <bool CHECK, bool WINDOW>
-__device__ __forceinline__ void leaf_stage_box(const LeafPassParams& P, LeafChunk& C, int j, uint32_t q, uint32_t g,
-                                               const int32_t o[3])
+__device__ __forceinline__ uint32_t leaf_stage_box(const LeafPassParams& P, LeafChunk& C, int j, uint32_t q, uint32_t g,
+                                                   const int32_t o[3])
 {
     const GaussRec& R = C.rec[j].r;
-    leaf_box_fields(C, j, R, o);
-    C.rgb24[j] = rgba8_byte(R.q7.x) | (rgba8_byte(R.q7.y) << 8) | (rgba8_byte(R.q7.z) << 16);
-    C.vs[j] = rec_vs(R, P.voxel_size, P.cloud_vs);
-    const LeafPairConst K = leaf_pair_consts(R, C.vs[j], o);
+    const LeafBox b = leaf_box(R, o);
+    const float vs = rec_vs(R, P.voxel_size, P.cloud_vs);
+    const LeafPairConst K = leaf_pair_consts(R, vs, o);
+    const uint32_t rgb24 = rgba8_byte(R.q7.x) | (rgba8_byte(R.q7.y) << 8) | (rgba8_byte(R.q7.z) << 16);
+    const float bx = (float)(b.lo[0] - K.r0[0]), by = (float)(b.lo[1] - K.r0[1]), bz = (float)(b.lo[2] - K.r0[2]);
+    float c[3];
 #pragma unroll
     for (int r = 0; r < 3; r++)
-    {
-        C.lo0[r][j] = K.lo0[r];
-        C.wid[r][j] = K.W[r];
-        C.dab[r][j] = K.dab[r];
+        c[r] = VOX_FFMA(bz, 0.5f * K.A[r][2], VOX_FFMA(by, 0.5f * K.A[r][1], VOX_FFMA(bx, 0.5f * K.A[r][0], K.c[r])));
+    C.tq[0][j] = make_float4(c[0], c[1], c[2], K.lo_t);
+    C.tq[1][j] = make_float4(0.5f * K.A[0][0], 0.5f * K.A[1][0], 0.5f * K.A[2][0], K.hi_t);
+    C.tq[2][j] = make_float4(0.5f * K.A[0][1], 0.5f * K.A[1][1], 0.5f * K.A[2][1], 0.25f * K.W[0]);
+    C.tq[3][j] = make_float4(0.5f * K.A[0][2], 0.5f * K.A[1][2], 0.5f * K.A[2][2], 0.25f * K.W[1]);
+    C.tq[4][j] = make_float4(0.25f * K.W[2], __uint_as_float((65536u + b.ny - 1u) / b.ny),
+                             __uint_as_float(b.ny | b.nz << 8),
+                             __uint_as_float((uint32_t)j << 9 | (uint32_t)(b.lo[0] << 6 | b.lo[1] << 3 | b.lo[2])));
 #pragma unroll
-        for (int a = 0; a < 3; a++)
-            C.stp[r][a][j] = K.A[r][a];
-    }
-    C.lo_t[j] = K.lo_t;
-    C.hi_t[j] = K.hi_t;
-    C.anchor[j] = K.r0;
-    C.flag[j] = CHECK ? P.emit_flag[P.vals[q]] : 0;
+    for (int r = 0; r < 3; r++)
+        C.aq[r][j] = make_float4(K.lo0[r], K.W[r], K.A[r][0], K.A[r][1]);
+    C.aq[3][j] = make_float4(K.A[0][2], K.A[1][2], K.A[2][2], __uint_as_float(rgb24));
+    C.aq[4][j] = make_float4(K.dab[0], K.dab[1], K.dab[2], vs);
+    C.aq[5][j] = make_float4(8388608.f + (float)K.r0[0], 8388608.f + (float)K.r0[1], 8388608.f + (float)K.r0[2], 0.f);
+    if (CHECK)
+        C.flag[j] = P.emit_flag[P.vals[q]];
     if (WINDOW)
     {
         const int64_t batch = (int64_t)g / REF_PRIM_BATCH;
         C.wf0[j] = P.frag_off[g] - P.frag_off[batch * REF_PRIM_BATCH];
         C.wbase[j] = P.win_before[batch];
     }
+    return b.nx * b.ny;
 }
 
 template <bool CHECK, bool WINDOW, int MINB = 4>
@@ -689,22 +764,14 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
     {
         S.cand = atomicAdd(counter, 1u);
         S.cand_next[0] = atomicAdd(counter, 1u);
-        S.pairs = 0;
         S.qn[0] = S.qn[1] = S.qn[2] = 0;
         S.dfin = 0;
-        S.acc[0].wmin = ~0ull;
+        S.acc.wmin = ~0ull;
     }
-#pragma unroll
-    for (int b = 0; b < 1; b++)
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-        {
-            const int n = t + 256 * h;
-            S.acc[b].dens[n] = 0;
-            S.acc[b].col[0][n] = S.acc[b].col[1][n] = S.acc[b].col[2][n] = 0;
-            S.acc[b].cnt[n] = 0;
-            S.acc[b].rgba[n] = 0;
-        }
+    for (int i = t; i < 9 * 512; i += LP_THREADS) // the sums and the RGBA8 maxima
+        (&S.acc.dens[0][0])[i] = 0;
+    if (t < 48)
+        S.mask[0][t] = 0;
     __syncthreads();
     // the chunk being tested (t*), the chunk whose alpha runs (a*), the leaf being flushed (f*)
     int64_t tc = S.cand;
@@ -727,20 +794,21 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
     uint32_t tq0 = P.cand_start[tc], tp1 = P.cand_start[tc + 1];
     if (stager)
     {
-        const uint32_t c0 = min((uint32_t)LQ_CHUNK, tp1 - tq0);
-        if (js < (int)c0)
+        uint32_t cols = 0;
+        if (js < (int)min((uint32_t)LQ_CHUNK, tp1 - tq0))
         {
             const uint32_t g = leaf_stage_issue(P, &S.ch[0].rec[js].r, tq0 + (uint32_t)js);
             cp_async_wait_all();
-            leaf_stage_box<CHECK, WINDOW>(P, S.ch[0], js, tq0 + (uint32_t)js, g, to);
+            cols = leaf_stage_box<CHECK, WINDOW>(P, S.ch[0], js, tq0 + (uint32_t)js, g, to);
         }
-        leaf_stage_prefix(S.ch[0], js, c0);
+        leaf_stage_prefix(S.ch[0], js, cols);
     }
     __syncthreads();
     bool t_valid = true, a_valid = false, f_valid = false, a_leaf_end = false;
-    int tpar = 0, apar = 0, fpar = 0;
+    int tm = 0, am = 0, fm = 0; // value mask buffers, one per leaf in turn
     int64_t ac = 0, fc = 0;
     int32_t ao[3] = { 0, 0, 0 };
+    unsigned long long leaf_pairs = 0, all_pairs = 0; // thread 0's
     uint32_t i = 0; // phase
     while (t_valid || a_valid || f_valid)
     {
@@ -773,22 +841,21 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         // ---- flush of the leaf whose last alpha ran in the previous phase
         if (f_valid)
         {
-            LeafAcc& A = S.acc[0];
-            uint32_t cnt[2];
+            LeafAcc& A = S.acc;
+            const uint32_t* mask = S.mask[fm];
 #pragma unroll
             for (int h = 0; h < 2; h++)
             {
                 const uint32_t n = (uint32_t)(t + 256 * h);
-                cnt[h] = A.cnt[n];
-                if (cnt[h])
+                if ((mask[warp + 8 * h] >> lane) & 1u)
                 {
                     const uint64_t slot = (uint64_t)fc * 512u + n;
-                    const float ds = fx_to_float(A.dens[n]);
+                    const float ds = fx_to_float((unsigned long long)A.dens[1][n] << 32 | A.dens[0][n]);
                     float col[3];
 #pragma unroll
                     for (int k = 0; k < 3; k++)
                     {
-                        col[k] = fx_to_float(A.col[k][n]);
+                        col[k] = fx_to_float((unsigned long long)A.col[k][1][n] << 32 | A.col[k][0][n]);
                         if (!P.smooth)
                             col[k] = ds > 0.f ? VOX_FDIV(col[k], ds) : 0.f;
                     }
@@ -797,33 +864,27 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                     P.s_col[3 * slot + 0] = col[0];
                     P.s_col[3 * slot + 1] = col[1];
                     P.s_col[3 * slot + 2] = col[2];
-                    P.s_pairs[slot] = cnt[h];
-                    A.dens[n] = 0;
-                    A.col[0][n] = A.col[1][n] = A.col[2][n] = 0;
-                    A.cnt[n] = 0;
-                    A.rgba[n] = 0;
+#pragma unroll
+                    for (int k = 0; k < 9; k++)
+                        (&A.dens[0][0])[512 * k + n] = 0;
                 }
             }
-            // value mask: voxel t of warp w is bit lane of 32-bit word w (w + 8 for voxel t + 256)
-            const uint32_t ba = __ballot_sync(0xffffffffu, cnt[0] > 0), bb = __ballot_sync(0xffffffffu, cnt[1] > 0);
-            unsigned long long wp = cnt[0] + cnt[1];
-#pragma unroll
-            for (int off = 16; off; off >>= 1)
-                wp += __shfl_xor_sync(0xffffffffu, wp, off);
-            if (lane == 0)
+            if (t < 16)
+                reinterpret_cast<uint32_t*>(P.cand_mask + 8 * (uint64_t)fc)[t] = mask[t];
+            if (t == 0)
             {
-                uint32_t* m32 = reinterpret_cast<uint32_t*>(P.cand_mask + 8 * (uint64_t)fc);
-                m32[warp] = ba;
-                m32[8 + warp] = bb;
-                if (wp)
-                    atomicAdd(&S.pairs, wp);
-            }
-            if (WINDOW && t == 0)
-            {
-                P.cand_wkey[fc] = A.wmin;
-                A.wmin = ~0ull;
+                P.cand_pairs[fc] = leaf_pairs;
+                all_pairs += leaf_pairs;
+                leaf_pairs = 0;
+                if (WINDOW)
+                {
+                    P.cand_wkey[fc] = A.wmin;
+                    A.wmin = ~0ull;
+                }
             }
             __syncthreads(); // the next leaf's alpha reuses the accumulators
+            if (t < 16)
+                S.mask[fm][t] = 0; // filled again by the leaf after next, from the next phase on
         }
         const uint32_t a_rounds = a_valid ? (S.qn[ab] + 31u) / 32u : 0u; // the alpha's rounds of 32 pairs
         // ---- alpha of the previous chunk, one queued pair per thread.  A pair
@@ -833,17 +894,18 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         if (a_valid)
         {
             const LeafChunk& C = S.ch[ab];
-            LeafAcc& A = S.acc[0];
+            LeafAcc& A = S.acc;
             const uint16_t* queue = S.queue[(i + 1u) & 1u];
             const uint32_t qn = S.qn[ab];
+            if (t == 0)
+                leaf_pairs += qn;
             uint16_t* dq = S.defer[warp];
             uint32_t dn = 0; // this warp's deferred pairs (warp-uniform)
             auto ref_byte = [&](uint32_t q) {
                 const uint32_t j = q >> 9, n = q & 511u;
-                const GaussRec& R = C.rec[j].r;
-                const uint32_t a8 = ref_alpha_byte(R, C.vs[j], ao[0] + (int32_t)(n >> 6),
+                const uint32_t a8 = ref_alpha_byte(C.rec[j].r, C.aq[4][j].w, ao[0] + (int32_t)(n >> 6),
                                                    ao[1] + (int32_t)((n >> 3) & 7u), ao[2] + (int32_t)(n & 7u));
-                atomicMax(&A.rgba[n], (a8 << 24) | C.rgb24[j]);
+                atomicMax(&A.rgba[n], (a8 << 24) | __float_as_uint(C.aq[3][j].w));
             };
             for (uint32_t e0 = (uint32_t)(t & ~31); e0 < qn; e0 += LP_THREADS) // warp-uniform trip count
             {
@@ -855,50 +917,63 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                     q = queue[e];
                     const uint32_t j = q >> 9, n = q & 511u;
                     const GaussRec& R = C.rec[j].r;
-                    const float vsf = C.vs[j];
-                    const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
-                                  zz = ao[2] + (int32_t)(n & 7);
+                    const float4 a3 = C.aq[3][j], q7 = R.q7;
                     float a;
                     uint32_t a8;
                     if (P.smooth)
                     {
+                        const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
+                                      zz = ao[2] + (int32_t)(n & 7);
+                        const float vsf = C.aq[4][j].w;
                         SmoothTerms st;
                         a = smooth_kernel(R, rinv_of(R), vsf, x, yy, zz, st);
-                        a8 = ref_alpha_byte(R, vsf, x, yy, zz);
+                        a8 = ref_alpha_byte(R, vsf, x, yy, zz) << 24;
                     }
                     else
                     {
-                        float lo0[3], wid[3], stp[3][3];
-#pragma unroll
-                        for (int r = 0; r < 3; r++)
-                        {
-                            lo0[r] = C.lo0[r][j];
-                            wid[r] = C.wid[r][j];
-#pragma unroll
-                            for (int a = 0; a < 3; a++)
-                                stp[r][a] = C.stp[r][a][j];
-                        }
-                        const AlphaF af = pair_alpha_f_ex(R, stable_leaf_aabb(lo0, wid, stp, C.anchor[j], (int32_t)(n >> 6),
-                                                                              (int32_t)((n >> 3) & 7u), (int32_t)(n & 7u)));
-                        a = af.a1;
+                        const float4 r0 = C.aq[0][j], r1 = C.aq[1][j], r2 = C.aq[2][j], anc = C.aq[5][j], q6 = R.q6;
+                        const float lo0[3] = { r0.x, r1.x, r2.x }, wid[3] = { r0.y, r1.y, r2.y };
+                        const float stp[3][3] = { { r0.z, r0.w, a3.x }, { r1.z, r1.w, a3.y }, { r2.z, r2.w, a3.z } };
+                        // voxels from the anchor, exactly (2^23 + n is a float's last place)
+                        const float fx = VOX_FSUB(__uint_as_float(0x4b000000u | (n >> 6)), anc.x),
+                                    fy = VOX_FSUB(__uint_as_float(0x4b000000u | ((n >> 3) & 7u)), anc.y),
+                                    fz = VOX_FSUB(__uint_as_float(0x4b000000u | (n & 7u)), anc.z);
+                        const AlphaF af = pair_alpha_f_ex(q6, stable_leaf_aabb(lo0, wid, stp, fx, fy, fz));
+                        a = q7.w != 0.f ? 0.f : af.a1;
                         bool decided;
-                        const float dab[3] = { C.dab[0][j], C.dab[1][j], C.dab[2][j] };
-                        a8 = alpha_byte_bound(R, af, dab, decided);
+                        const float4 db = C.aq[4][j];
+                        const float dab[3] = { db.x, db.y, db.z };
+                        a8 = alpha_byte_bound(q6, q7.w, af, dab, decided);
                         defer = !decided;
-                        if (CHECK && decided && a8 != ref_alpha_byte(R, vsf, x, yy, zz))
+                        if (CHECK && decided &&
+                            a8 >> 24 != ref_alpha_byte(R, db.w, ao[0] + (int32_t)(n >> 6), ao[1] + (int32_t)((n >> 3) & 7),
+                                                       ao[2] + (int32_t)(n & 7)))
                             atomicOr(P.err, ERR_BOUNDS); // the margin failed to cover the reference's byte
                     }
-                    atomicAdd(&A.cnt[n], 1u);
                     if (!defer)
-                        atomicMax(&A.rgba[n], (a8 << 24) | C.rgb24[j]);
-                    atomicAdd(&A.dens[n], fx_of_unit(a));
-                    atomicAdd(&A.col[0][n], fx_of(VOX_FMUL(a, R.q7.x)));
-                    atomicAdd(&A.col[1][n], fx_of(VOX_FMUL(a, R.q7.y)));
-                    atomicAdd(&A.col[2][n], fx_of(VOX_FMUL(a, R.q7.z)));
+                        atomicMax(&A.rgba[n], a8 | __float_as_uint(a3.w));
+                    const float c0 = VOX_FMUL(a, q7.x), c1 = VOX_FMUL(a, q7.y), c2 = VOX_FMUL(a, q7.z);
+                    if (a < 1.f && c0 >= 0.f && c0 < 1.f && c1 >= 0.f && c1 < 1.f && c2 >= 0.f && c2 < 1.f)
+                    {
+                        // terms in [0, 1): below 2^32 units (a is never negative)
+                        acc_add(&A.dens[0][n], &A.dens[1][n], __float2uint_rn(VOX_FMUL(a, FX_SCALE)), 0u);
+                        acc_add(&A.col[0][0][n], &A.col[0][1][n], __float2uint_rn(VOX_FMUL(c0, FX_SCALE)), 0u);
+                        acc_add(&A.col[1][0][n], &A.col[1][1][n], __float2uint_rn(VOX_FMUL(c1, FX_SCALE)), 0u);
+                        acc_add(&A.col[2][0][n], &A.col[2][1][n], __float2uint_rn(VOX_FMUL(c2, FX_SCALE)), 0u);
+                    }
+                    else
+                    {
+                        acc_add(&A.dens[0][n], &A.dens[1][n], fx_of_unit(a));
+                        acc_add(&A.col[0][0][n], &A.col[0][1][n], fx_of(c0));
+                        acc_add(&A.col[1][0][n], &A.col[1][1][n], fx_of(c1));
+                        acc_add(&A.col[2][0][n], &A.col[2][1][n], fx_of(c2));
+                    }
                     if (WINDOW)
                     {
                         // the reference's window of this fragment: x-major index in the bbox
                         // (gaussian_frag_alloc.slang:55-58) after the Gaussian's batch offset
+                        const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
+                                      zz = ao[2] + (int32_t)(n & 7);
                         const uint64_t r = (uint64_t)(x - R.q4.x) * (uint64_t)R.q5.y * (uint64_t)R.q5.z +
                                            (uint64_t)(yy - R.q4.y) * (uint64_t)R.q5.z + (uint64_t)(zz - R.q4.z);
                         const unsigned long long wk = C.wbase[j] + (C.wf0[j] + r) / REF_WINDOW;
@@ -974,8 +1049,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         }
         // ---- test of this chunk
         if (t_valid)
-            leaf_test_chunk<CHECK, false, true>(P, S.ch[tb], min((uint32_t)LQ_CHUNK, tp1 - tq0), to, S.queue[i & 1u],
-                                                &S.qn[tb], t, lane, a_rounds);
+            leaf_test_columns<CHECK>(P, S.ch[tb], to, S.queue[i & 1u], &S.qn[tb], S.mask[tm], t, lane, a_rounds);
         // the counter the test of phase i + 1 fills: last read by the alpha of phase i - 1
         if (t == 0)
             S.qn[nb] = 0;
@@ -989,12 +1063,13 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 no[1] = pre_org.y;
                 no[2] = pre_org.z;
             }
+            uint32_t cols = 0;
             if (js < (int)ncnt)
             {
                 cp_async_wait_all();
-                leaf_stage_box<CHECK, WINDOW>(P, S.ch[nb], js, nq0 + (uint32_t)js, ng, no);
+                cols = leaf_stage_box<CHECK, WINDOW>(P, S.ch[nb], js, nq0 + (uint32_t)js, ng, no);
             }
-            leaf_stage_prefix(S.ch[nb], js, ncnt);
+            leaf_stage_prefix(S.ch[nb], js, cols);
             if (js == 0)
             {
                 const int pp = (int)(i & 1u);
@@ -1011,11 +1086,11 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         // ---- advance: flush <- alpha (at a leaf end), alpha <- test, test <- next
         f_valid = a_valid && a_leaf_end;
         fc = ac;
-        fpar = apar;
+        fm = am;
         a_valid = t_valid;
         a_leaf_end = t_leaf_end;
         ac = tc;
-        apar = tpar;
+        am = tm;
         ao[0] = to[0];
         ao[1] = to[1];
         ao[2] = to[2];
@@ -1026,7 +1101,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
             {
                 cn = S.cand_next[pp];
                 cn_fresh = true;
-                tpar ^= 1;
+                tm = tm == 2 ? 0 : tm + 1;
             }
             tc = nc;
             tq0 = S.nxt_q0[pp];
@@ -1038,8 +1113,8 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         t_valid = n_valid;
         i++;
     }
-    if (t == 0 && S.pairs)
-        atomicAdd((unsigned long long*)P.total_pairs, S.pairs);
+    if (t == 0 && all_pairs)
+        atomicAdd((unsigned long long*)P.total_pairs, all_pairs);
 }
 
 __device__ __forceinline__ uint32_t mask_rank(const uint64_t* m, uint32_t n)
@@ -1064,7 +1139,6 @@ struct LeafBChunk
     int32_t bx0[LQ_CHUNK], by0[LQ_CHUNK], bz0[LQ_CHUNK];
     uint32_t bny[LQ_CHUNK], bnz[LQ_CHUNK], bdiv_y[LQ_CHUNK], bcol[LQ_CHUNK];
     float vs[LQ_CHUNK];
-    uint8_t flag[LQ_CHUNK];
     uint32_t eidx[LQ_CHUNK]; // emission index of each leaf pair
     uint64_t mask[8];        // the leaf's value mask
     uint64_t vbase;          // value index of the leaf's first voxel
@@ -1106,9 +1180,15 @@ __device__ __forceinline__ void leaf_bstage(const LeafPassParams& P, LeafBChunk&
     if (js < (int)cnt)
     {
         cp_async_wait_all();
-        leaf_box_fields(C, js, C.rec[js].r, o);
+        const LeafBox b = leaf_box(C.rec[js].r, o);
+        C.bx0[js] = b.lo[0];
+        C.by0[js] = b.lo[1];
+        C.bz0[js] = b.lo[2];
+        C.bny[js] = b.ny;
+        C.bnz[js] = b.nz;
+        C.bdiv_y[js] = (65536u + b.ny - 1u) / b.ny;
+        C.bcol[js] = b.nx * b.ny;
         C.vs[js] = rec_vs(C.rec[js].r, P.voxel_size, P.cloud_vs);
-        C.flag[js] = 0;
         C.eidx[js] = P.vals[q0 + (uint32_t)js];
     }
 }
@@ -1277,8 +1357,7 @@ __global__ void __launch_bounds__(LP_THREADS, 3) k_leaf_backward(LeafPassParams 
         }
         // ---- test of chunk p
         if (t_valid)
-            leaf_test_chunk<false, true>(P, S.ch[tb], min((uint32_t)LQ_CHUNK, tp1 - tq0), to, S.queue[p & 1u],
-                                         S.wqn[p & 1u], t, lane);
+            leaf_test_chunk(S.ch[tb], min((uint32_t)LQ_CHUNK, tp1 - tq0), to, S.queue[p & 1u], S.wqn[p & 1u], t, lane);
         // ---- stagers: chunk p + 1's mask words and boxes
         if (stager && n_valid)
         {
@@ -1323,8 +1402,9 @@ __global__ void __launch_bounds__(LP_THREADS, 3) k_leaf_backward(LeafPassParams 
 }
 
 // the sorted (voxel key, Gaussian id) pair list: per voxel, its Gaussians in
-// ascending id, at the voxel's pair offset
-__global__ void __launch_bounds__(LP_THREADS) k_leaf_export(LeafPassParams P, uint32_t* counter)
+// ascending id, at the voxel's pair offset (COUNT: only the pairs per voxel)
+template <bool COUNT>
+__global__ void __launch_bounds__(LP_THREADS) k_leaf_export(LeafPassParams P, uint64_t* vpairs, uint32_t* counter)
 {
     __shared__ LeafSmem S;
     const int t = threadIdx.x;
@@ -1350,7 +1430,7 @@ __global__ void __launch_bounds__(LP_THREADS) k_leaf_export(LeafPassParams P, ui
         {
             const uint32_t n = (uint32_t)(t + 256 * h);
             act[h] = (S.mask[n >> 6] >> (n & 63)) & 1ull;
-            if (act[h])
+            if (act[h] && !COUNT)
                 dst[h] = P.pair_off[P.cand_voff[c] + mask_rank(S.mask, n)];
         }
         const uint32_t p0 = P.cand_start[c], p1 = P.cand_start[c + 1];
@@ -1372,16 +1452,27 @@ __global__ void __launch_bounds__(LP_THREADS) k_leaf_export(LeafPassParams P, ui
                         continue;
                     if (!aabb_hits_unit_sphere(voxel_local_aabb(R, M, vsf, x, y, z)))
                         continue;
-                    const uint64_t k = ((uint64_t)key << 9) | (uint32_t)(t + 256 * h);
-                    if (P.key64)
-                        ((uint64_t*)P.out_keys)[dst[h]] = k;
-                    else
-                        ((uint32_t*)P.out_keys)[dst[h]] = (uint32_t)k;
-                    P.out_ids[dst[h]] = S.gid[j];
+                    if (!COUNT)
+                    {
+                        const uint64_t k = ((uint64_t)key << 9) | (uint32_t)(t + 256 * h);
+                        if (P.key64)
+                            ((uint64_t*)P.out_keys)[dst[h]] = k;
+                        else
+                            ((uint32_t*)P.out_keys)[dst[h]] = (uint32_t)k;
+                        P.out_ids[dst[h]] = S.gid[j];
+                    }
                     dst[h]++;
                 }
             }
             __syncthreads();
+        }
+        if (COUNT)
+        {
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                if (act[h])
+                    vpairs[P.cand_voff[c] + mask_rank(S.mask, (uint32_t)(t + 256 * h))] = dst[h];
+            __syncthreads(); // the mask is reloaded for the next candidate
         }
     }
 }
@@ -1409,7 +1500,7 @@ __device__ __forceinline__ uint32_t leaf_mask_word(const NodeParams& N, int64_t 
 // values to its value indices, its node2 node (grid_build_finalize.slang) and
 // its share of the cloud's bbox (grid_build_compute_bbox.slang).  A round takes
 // 32 slots of the leaf: staged reads and value writes are runs of consecutive
-// words.  HBM-bound: 24 B read and 20 B written per voxel, 1.04 ms for 106M
+// words.  HBM-bound: 20 B read and 20 B written per voxel, 1.04 ms for 106M
 // voxels (4.5 TB/s; the loads of 2 / 4 / 8 rounds in flight: 1.11 / 1.04 / 1.12 ms,
 // of one 1.76 ms).
 constexpr int WL_THREADS = 256;
@@ -1441,11 +1532,10 @@ __global__ void __launch_bounds__(WL_THREADS) k_write_leaves(ValueParams A, Node
         uint32_t* rgba = (uint32_t*)(A.out + C.rgba_off[b]) + vidx;
         float* dens = (float*)(A.out + C.dens_off[b]) + vidx;
         float* col = (float*)(A.out + C.col_off[b]) + 3 * vidx;
-        uint32_t pairs = 0;
 #pragma unroll 1
         for (int r0 = 0; r0 < 16; r0 += WL_ROUNDS)
         {
-            uint32_t at[WL_ROUNDS], vr[WL_ROUNDS], vp[WL_ROUNDS];
+            uint32_t at[WL_ROUNDS], vr[WL_ROUNDS];
             float vd[WL_ROUNDS], vc[WL_ROUNDS][3];
 #pragma unroll
             for (int i = 0; i < WL_ROUNDS; i++)
@@ -1461,8 +1551,6 @@ __global__ void __launch_bounds__(WL_THREADS) k_write_leaves(ValueParams A, Node
 #pragma unroll
                     for (int k2 = 0; k2 < 3; k2++)
                         vc[i][k2] = __ldcs(A.s_col + 3 * slot + k2);
-                    if (A.cloud_pairs)
-                        vp[i] = __ldcs(A.s_pairs + slot);
                 }
             }
 #pragma unroll
@@ -1474,8 +1562,6 @@ __global__ void __launch_bounds__(WL_THREADS) k_write_leaves(ValueParams A, Node
 #pragma unroll
                     for (int k2 = 0; k2 < 3; k2++)
                         __stcs(col + 3 * at[i] + k2, vc[i][k2]);
-                    if (A.cloud_pairs)
-                        pairs += vp[i];
                 }
         }
         // the node: index, value index, prefix words, mask (128 B)
@@ -1522,12 +1608,8 @@ __global__ void __launch_bounds__(WL_THREADS) k_write_leaves(ValueParams A, Node
             else
                 atomicMax(&bb[3 + a], o + hi);
         }
-        if (A.cloud_pairs)
-        {
-            pairs = __reduce_add_sync(0xffffffffu, pairs);
-            if (lane == 0)
-                atomicAdd(b == cb ? &s_pairs : (unsigned long long*)&A.cloud_pairs[b], (unsigned long long)pairs);
-        }
+        if (A.cloud_pairs && lane == 0)
+            atomicAdd(b == cb ? &s_pairs : (unsigned long long*)&A.cloud_pairs[b], (unsigned long long)A.cand_pairs[c]);
     }
     __syncthreads();
     if (threadIdx.x < 3)
@@ -1555,12 +1637,6 @@ __device__ __forceinline__ void each_voxel(const NodeParams& N, F f)
         if ((bits >> lane) & 1u)
             f(v0 + base + __popc(bits & ((1u << lane) - 1u)), l, (uint32_t)(32 * r + lane));
     }
-}
-
-// pairs per voxel (canonical order) from the staged counts
-__global__ void k_voxel_pairs(NodeParams N, const uint32_t* s_pairs, uint64_t* vpairs)
-{
-    each_voxel(N, [&](uint64_t v, int64_t l, uint32_t n) { vpairs[v] = s_pairs[(uint64_t)N.leaf_cand[l] * 512u + n]; });
 }
 
 // coordinates of the active voxels by value index (clouds back to back)
@@ -1660,12 +1736,15 @@ void launch_leaf_backward(const LeafPassParams& P, uint32_t* counter, int num_sm
     { k_leaf_backward<<<(unsigned)grid, LP_THREADS, smem, s>>>(P, counter); count_launch(); }
 }
 
-void launch_leaf_export(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s)
+void launch_leaf_export(const LeafPassParams& P, uint64_t* vpairs, uint32_t* counter, int num_sms, cudaStream_t s)
 {
     if (P.NCL <= 0)
         return;
     cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    { k_leaf_export<<<walk_grid(P.NCL, num_sms), LP_THREADS, 0, s>>>(P, counter); count_launch(); }
+    if (vpairs)
+        { k_leaf_export<true><<<walk_grid(P.NCL, num_sms), LP_THREADS, 0, s>>>(P, vpairs, counter); count_launch(); }
+    else
+        { k_leaf_export<false><<<walk_grid(P.NCL, num_sms), LP_THREADS, 0, s>>>(P, nullptr, counter); count_launch(); }
 }
 
 void launch_write_leaves(const ValueParams& A, const NodeParams& N, int num_sms, cudaStream_t s)
@@ -1679,13 +1758,6 @@ void launch_write_leaves(const ValueParams& A, const NodeParams& N, int num_sms,
     per_warp = per_warp < 1 ? 1 : per_warp > 8 ? 8 : per_warp;
     const int64_t grid = (N.L + per_cta * per_warp - 1) / (per_cta * per_warp);
     { k_write_leaves<<<(unsigned)grid, WL_THREADS, 0, s>>>(A, N, (int)per_warp); count_launch(); }
-}
-
-void launch_voxel_pairs(const NodeParams& N, const uint32_t* s_pairs, uint64_t* vpairs, cudaStream_t s)
-{
-    if (N.L <= 0)
-        return;
-    { k_voxel_pairs<<<(unsigned)((N.L + 7) / 8), 256, 0, s>>>(N, s_pairs, vpairs); count_launch(); }
 }
 
 void launch_voxel_coords(const NodeParams& N, int32_t* out, cudaStream_t s)

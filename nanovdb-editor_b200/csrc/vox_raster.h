@@ -142,7 +142,7 @@ struct LeafPassParams
     uint32_t* s_rgba;          // staging [NCL * 512]
     float* s_dens;
     float* s_col;              // [NCL * 512][3]
-    uint32_t* s_pairs;
+    uint64_t* cand_pairs;      // [NCL] passing pairs
     uint64_t* total_pairs;
     int* err;
     // adjoint
@@ -175,20 +175,20 @@ void launch_leaf_compact(const uint32_t* keys, const uint32_t* vals, const uint3
 // returns the CTAs per SM it ran with
 int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant = 0);
 void launch_leaf_backward(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s);
-void launch_leaf_export(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s);
+// vpairs non-null: only the pairs per voxel (canonical order), into it
+void launch_leaf_export(const LeafPassParams& P, uint64_t* vpairs, uint32_t* counter, int num_sms, cudaStream_t s);
 
 struct ValueParams
 {
     const uint32_t* s_rgba;
     const float* s_dens;
     const float* s_col;
-    const uint32_t* s_pairs;
+    const uint64_t* cand_pairs;
     uint64_t* cloud_pairs;     // [B] passing pairs per cloud, summed here (null: one cloud)
     uint64_t* cand_vbase;      // [NCL]
     uint8_t* out;
 };
 void launch_write_leaves(const ValueParams& A, const NodeParams& N, int num_sms, cudaStream_t s);
-void launch_voxel_pairs(const NodeParams& N, const uint32_t* s_pairs, uint64_t* vpairs, cudaStream_t s);
 void launch_voxel_coords(const NodeParams& N, int32_t* out, cudaStream_t s);
 
 // the reference's fragment batches and windows (raster/Raster.cpp:443-444)
