@@ -65,7 +65,7 @@ struct vox_context_t
     std::string last_error;
     std::vector<DevBuf*> bufs;
     // device buffers
-    DevBuf recs, footprints, frag_off, root_bits, root_prefix, root_of_rank, lower_bits, lower_prefix, lower_cell;
+    DevBuf recs, walk, footprints, frag_off, root_bits, root_prefix, root_of_rank, lower_bits, lower_prefix, lower_cell;
     DevBuf scan_status, run_status;
     DevBuf keys, ids, keys_alt, ids_alt, sort_ws;
     DevBuf leaf_vstart, lower_lstart;
@@ -398,7 +398,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
 
     // ---------------------------------------------------------------- prep
     const float cull = cull_scale > 0.f ? cull_scale : 0.05f;
-    if (!ensure(ctx, ctx->recs, sizeof(GaussRec) * (size_t)(G + 1)) ||
+    if (!ensure(ctx, ctx->recs, sizeof(GaussRec) * (size_t)(G + 1)) || !ensure(ctx, ctx->walk, sizeof(WalkRec) * (size_t)(G + 1)) ||
         !ensure(ctx, ctx->footprints, sizeof(uint64_t) * (size_t)(G + 1)) ||
         !ensure(ctx, ctx->frag_off, sizeof(uint64_t) * (size_t)(G + 1)) ||
         !ensure(ctx, ctx->root_bits, sizeof(uint64_t) * 512 * B) || !ensure(ctx, ctx->root_prefix, sizeof(uint64_t) * 512 * B) ||
@@ -416,6 +416,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         d_cloud_vs = (const float*)ctx->cloud_vs.p;
     }
     GaussRec* recs = (GaussRec*)ctx->recs.p;
+    WalkRec* walk = (WalkRec*)ctx->walk.p;
     uint64_t* footprints = (uint64_t*)ctx->footprints.p;
     uint64_t* frag_off = (uint64_t*)ctx->frag_off.p;
     uint64_t* root_bits = (uint64_t*)ctx->root_bits.p;
@@ -454,7 +455,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
             cudaStreamWaitEvent(s, ctx->up_ev[1 + c], 0);
             P.g0 = g0;
             P.g1 = g1;
-            launch_prep(P, recs, footprints, root_bits, d_err, s);
+            launch_prep(P, recs, walk, footprints, root_bits, d_err, s);
         }
     }
     else
@@ -463,7 +464,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
             for (int a = 0; a < 5; a++)
                 cudaMemcpyAsync(ctx->upload.dev[a], ctx->upload.host[a],
                                 (size_t)ctx->upload.width[a] * ctx->upload.es * (size_t)G, cudaMemcpyHostToDevice, s);
-        launch_prep(P, recs, footprints, root_bits, d_err, s);
+        launch_prep(P, recs, walk, footprints, root_bits, d_err, s);
     }
     ctx->upload.active = false;
     uint64_t* scan_status = (uint64_t*)ctx->scan_status.p;
@@ -657,6 +658,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LP.win_before = win_before;
     LP.cand_wkey = window ? (uint64_t*)ctx->cand_wkey.p : nullptr;
     LP.recs = recs;
+    LP.walk = walk;
     LP.vals = lvals;
     LP.emit_gid = (const uint32_t*)ctx->emit_gid.p;
     LP.pair_gid = (const uint32_t*)ctx->pair_gid.p;
@@ -1005,7 +1007,7 @@ void vox_context_destroy(vox_context_t* ctx)
         return;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    DevBuf* all[] = { &ctx->recs, &ctx->footprints, &ctx->frag_off, &ctx->root_bits, &ctx->root_prefix,
+    DevBuf* all[] = { &ctx->recs, &ctx->walk, &ctx->footprints, &ctx->frag_off, &ctx->root_bits, &ctx->root_prefix,
                       &ctx->root_of_rank, &ctx->lower_bits, &ctx->lower_prefix, &ctx->lower_cell, &ctx->scan_status,
                       &ctx->run_status, &ctx->keys, &ctx->ids, &ctx->keys_alt, &ctx->ids_alt,
                       &ctx->sort_ws, &ctx->leaf_vstart, &ctx->lower_lstart, &ctx->lower_upper_n,

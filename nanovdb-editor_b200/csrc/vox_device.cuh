@@ -452,8 +452,8 @@ __device__ __forceinline__ float pair_alpha(const GaussRec& R, const Aabb& b)
     return alpha_of_d2(R, lattice_min_d2(b));
 }
 
-// Per (leaf, Gaussian) constants of the leaf walk, computed once when a chunk
-// is staged (leaf_pair_consts).
+// Constants of the leaf walk per Gaussian (WalkRec, written with the record) and
+// per (leaf, Gaussian) (leaf_consts, computed when a chunk is staged).
 //
 // The float channels' local AABB is anchored at one voxel of the leaf: c =
 // o + r0, r0_a = clamp(bmin_a + (range_a >> 1) - o_a, 0, 7) (the leaf voxel
@@ -466,46 +466,45 @@ __device__ __forceinline__ float pair_alpha(const GaussRec& R, const Aabb& b)
 //   W_r    = fl(fl(|A_r0| + |A_r1|) + |A_r2|)
 //   lo_r   = fma(t_z, A_r2, fma(t_y, A_r1, fma(t_x, A_r0, lo0_r))),  hi_r = fl(lo_r + W_r)
 // (the lower corner of each axis is the one picked by the sign of the step).
-// Every rounding is relative to the local magnitudes E_a = |d0_a| + 8 vs
-// (|t| <= 7), and near the centre the anchor's offsets are about a voxel, so
-// the form is about as accurate as one rounding of each corner offset; a pair
-// costs three fma and one add per row.  The oracle's frag_alpha_f evaluates the same operations in
-// the same order.
+// The oracle's frag_alpha_f evaluates the same operations in the same order.
+// The record holds A halved and W quartered (exact); a pair multiplies the
+// halved steps by 2 t.
 //
 // dab_r bounds how far the reference's local AABB (voxel_local_aabb) and this
-// one can differ in the leaf, apart from the per-pair 2^-20 B_r term added in
-// alpha_byte_bound: per axis the reference's corner offset fl(fl(v vs) -
-// mu) is within 0.5 ulp(W) + 0.5 ulp(Cm) of exact (W, Cm: the largest |v vs|
-// and |v vs - mu| over the leaf's corners), its products and two sums add at
-// most 3 2^-24 sum_a |m_ra| Cm_a <= 2^-21 sum_a |m_ra| Cm_a; this form's d0
-// rounding adds 0.5 ulp(E_a), its other roundings (the chain 3, k and base 2,
-// the steps' 3 times |t| <= 7 with 8 vs <= E, lo0 3, the per-voxel fma 3, W and
-// the hi sum about 1.3, in units of 2^-24 sum_a |m_ra| E_a) at most
-// 2^-20 sum_a |m_ra| E_a; all scaled by il is_r.  dab_r also carries the
-// roundings proportional to the bound magnitude (the sum and scalings of the
-// reference, the lattice points): 2^-20 2 Bl_r, Bl_r = il is_r sum_a |m_ra|
-// Cm_a bounding every bound's magnitude in the leaf.  So per row this AABB,
-// and its four lattice points, are within dab_r of the reference's for every
-// voxel of the leaf.
+// one can differ for any voxel of the Gaussian's bbox, every leaf included: all
+// the walk's positions (anchor, box origin, voxels) are voxels of the bbox,
+// whose corner offsets from mu are at most Cm_a per axis (W_a: the largest
+// |v vs|).  The reference's corner offset fl(fl(v vs) - mu) is within
+// 0.5 ulp(W_a) + 0.5 ulp(Cm_a) of exact, its products and two sums add at most
+// 3 2^-24 sum_a |m_ra| Cm_a <= 2^-21 sum_a |m_ra| Cm_a.  This form's d0
+// rounding adds 0.5 ulp(E_a), E_a = Cm_a + vs, and its other roundings, in
+// units of 2^-24 sum_a |m_ra| E_a: the chain 3, k and base 2, the steps' 3
+// times |t| vs <= 2 Cm (6), lo0 3, the per-voxel fma 3, W (4.3 times vs <= 2 E /
+// 3: 2.9) and the hi sum 1: 20.9, taken as 24; all scaled by il is_r.  dab_r
+// also carries the roundings proportional to the bound magnitude (the sum and
+// scalings of the reference, the lattice points): 2^-20 2 Bl_r, Bl_r = il is_r
+// sum_a |m_ra| Cm_a bounding every bound's magnitude in the bbox.  So per row
+// this AABB, and its four lattice points, are within dab_r of the reference's
+// for every voxel of the bbox.
 //
 // The leaf test (leaf_test_columns) classifies voxels from the same AABB as
 // centre and half width, both halved (exactly): row r of the box origin's voxel
 // is c_r = 0.5 base_r + 0.25 ((A_r0 + A_r1) + A_r2), carried from the anchor to
 // the box origin by three fma, then two per column and one per voxel; the half
-// width is h_r = 0.25 W_r.  In units of 2^-24 il is_r sum_a |m_ra| E_a the
-// roundings are the chain's 3, k and base 2, the steps' 3 times |t| <= 7 with
-// 8 vs <= E (2.6), c 1.5, the way to the box origin 3, column and voxel 3, the
-// final difference and h 1.5: 16.6 where dab_r covers 16 (2^-20), so the test
-// takes 1.5 dab_r: Delta = 1.5 sum_r dab_r gives its thresholds lo_t / hi_t.
-struct LeafPairConst
+// width is h_r = 0.25 W_r.  In the same units: the chain, k and base 5, the
+// steps 6, c 2.3, the way to the box origin 3, column and voxel 3, the final
+// difference 1, h 1.7: 22 of the 24 in dab_r.  Delta = sum_r dab_r gives its
+// thresholds lo_t / hi_t.
+struct __align__(16) WalkRec
 {
-    float lo0[3], W[3]; // per row: the scaled lower bound of the anchor voxel, the scaled voxel width
-    float A[3][3];      // A[r][a]: the scaled step of one voxel along axis a
-    float dab[3];       // per row: the reference / float-channel AABB difference bound
-    float c[3];         // per row: half the centre of the anchor voxel
-    float lo_t, hi_t;   // a quarter of the squared distances below which a voxel surely passes / above which it fails
-    int32_t r0[3];      // the anchor voxel in the leaf
+    float4 w0; // half x steps A_00 A_10 A_20, hi_t
+    float4 w1; // half y steps, h_0
+    float4 w2; // half z steps, h_1
+    float4 w3; // dab_0..2, voxel size
+    float4 w4; // k_0..2, h_2
+    float4 w5; // lo_t, the colour bytes of the RGBA8 value
 };
+constexpr int WALK_WORDS = 6; // 16-byte words of a WalkRec
 
 // the anchor of the float channels' AABB along one axis (leaf origin o)
 // (bbox minimum bmin, extent range = max + 1 - min)
@@ -521,72 +520,99 @@ __device__ __forceinline__ float ulp_of(float x)
     return __uint_as_float(__float_as_uint(fabsf(x)) & 0x7f800000u) * 0x1p-23f;
 }
 
-__device__ __forceinline__ LeafPairConst leaf_pair_consts(const GaussRec& R, float vs, const int32_t o[3])
+__device__ __forceinline__ WalkRec walk_record(const GaussRec& R, float vs)
 {
-    LeafPairConst c;
     const float mu[3] = { R.q0.x, R.q0.y, R.q0.z };
     const float il = R.q0.w;
     const float is[3] = { R.q3.y, R.q3.z, R.q3.w };
     const RInv M = rinv_of(R);
-    float d0[3], Gr[3], G[3], Cm[3];
+    float G[3], Cm[3];
 #pragma unroll
     for (int a = 0; a < 3; a++)
     {
-        const int32_t r0 = anchor_of((&R.q4.x)[a], (&R.q5.x)[a], o[a]);
-        c.r0[a] = r0;
-        d0[a] = VOX_FFMA((float)(o[a] + r0), vs, -mu[a]);
-        const float w0 = (float)o[a] * vs, w1 = (float)(o[a] + 8) * vs;
+        const int32_t v0 = (&R.q4.x)[a], v1 = v0 + (&R.q5.x)[a];
+        const float w0 = (float)v0 * vs, w1 = (float)v1 * vs;
         const float W = fmaxf(fabsf(w0), fabsf(w1)) * (1.f + 0x1p-20f);
         Cm[a] = fmaxf(fabsf(w0 - mu[a]), fabsf(w1 - mu[a])) * (1.f + 0x1p-20f);
-        Gr[a] = 0.5f * ulp_of(W) + 0.5f * ulp_of(Cm[a]) + 0x1p-21f * Cm[a];
-        const float E = (fabsf(d0[a]) + 8.f * vs) * (1.f + 0x1p-20f);
-        G[a] = Gr[a] + 0.5f * ulp_of(E) + 0x1p-20f * E;
+        const float E = (Cm[a] + vs) * (1.f + 0x1p-20f);
+        G[a] = 0.5f * ulp_of(W) + 0.5f * ulp_of(Cm[a]) + 0x1p-21f * Cm[a] + 0.5f * ulp_of(E) + 0x1.8p-20f * E;
     }
+    float hA[3][3], h[3], dab[3], k[3];
     float Dl = 0.f;
 #pragma unroll
     for (int r = 0; r < 3; r++)
     {
-        const float k = VOX_FMUL(il, is[r]);
-        const float base =
-            VOX_FMUL(VOX_FFMA(M.m[r][2], d0[2], VOX_FFMA(M.m[r][0], d0[0], VOX_FMUL(M.m[r][1], d0[1]))), k);
+        k[r] = VOX_FMUL(il, is[r]);
+        float A[3];
 #pragma unroll
         for (int a = 0; a < 3; a++)
-            c.A[r][a] = VOX_FMUL(VOX_FMUL(vs, M.m[r][a]), k);
-        c.lo0[r] = VOX_FADD(VOX_FADD(VOX_FADD(base, fminf(c.A[r][0], 0.f)), fminf(c.A[r][1], 0.f)),
-                            fminf(c.A[r][2], 0.f));
-        c.W[r] = VOX_FADD(VOX_FADD(fabsf(c.A[r][0]), fabsf(c.A[r][1])), fabsf(c.A[r][2]));
-        c.c[r] = 0.5f * base + 0.25f * ((c.A[r][0] + c.A[r][1]) + c.A[r][2]);
+        {
+            A[a] = VOX_FMUL(VOX_FMUL(vs, M.m[r][a]), k[r]);
+            hA[r][a] = 0.5f * A[a];
+        }
+        h[r] = 0.25f * VOX_FADD(VOX_FADD(fabsf(A[0]), fabsf(A[1])), fabsf(A[2]));
         const float s = (1.f + 0x1p-20f) * il * is[r];
         const float m0 = fabsf(M.m[r][0]), m1 = fabsf(M.m[r][1]), m2 = fabsf(M.m[r][2]);
         const float Bl = s * (m0 * Cm[0] + m1 * Cm[1] + m2 * Cm[2]);
-        // with the scalings' and lattice points' roundings, 2^-20 B_r <= 2^-20 2 Bl_r
-        c.dab[r] = s * (m0 * G[0] + m1 * G[1] + m2 * G[2]) + 0x1p-20f * 2.f * Bl;
-        Dl += c.dab[r];
+        dab[r] = s * (m0 * G[0] + m1 * G[1] + m2 * G[2]) + 0x1p-20f * 2.f * Bl;
+        Dl += dab[r];
     }
-    Dl *= 1.5f * (1.f + 0x1p-20f);
+    Dl *= 1.f + 0x1p-20f;
+    // a quarter of the squared distances below which a voxel surely passes / above which it surely fails
+    float lo_t = -1.f, hi_t = __int_as_float(0x7f800000); // every voxel takes the reference test
     if (Dl <= 0.0625f) // false for NaN
     {
-        c.lo_t = 0.25f * (1.f - (2.f * Dl + 0x1p-19f));
-        c.hi_t = 0.25f * (1.f + (2.f * Dl + Dl * Dl + 0x1p-18f));
+        lo_t = 0.25f * (1.f - (2.f * Dl + 0x1p-19f));
+        hi_t = 0.25f * (1.f + (2.f * Dl + Dl * Dl + 0x1p-18f));
     }
-    else
-    {
-        c.lo_t = -1.f; // every voxel takes the reference test
-        c.hi_t = __int_as_float(0x7f800000);
-    }
-    return c;
+    const uint32_t rgb24 = rgba8_byte(R.q7.x) | (rgba8_byte(R.q7.y) << 8) | (rgba8_byte(R.q7.z) << 16);
+    WalkRec o;
+    o.w0 = make_float4(hA[0][0], hA[1][0], hA[2][0], hi_t);
+    o.w1 = make_float4(hA[0][1], hA[1][1], hA[2][1], h[0]);
+    o.w2 = make_float4(hA[0][2], hA[1][2], hA[2][2], h[1]);
+    o.w3 = make_float4(dab[0], dab[1], dab[2], vs);
+    o.w4 = make_float4(k[0], k[1], k[2], h[2]);
+    o.w5 = make_float4(lo_t, __uint_as_float(rgb24), 0.f, 0.f);
+    return o;
 }
 
-// the float channels' local AABB of the voxel (fx, fy, fz) voxels from the anchor
-__device__ __forceinline__ Aabb stable_leaf_aabb(const float lo0[3], const float W[3], const float A[3][3], float fx,
+// per row of a (leaf, Gaussian): the anchor voxel's lower bound and half its centre
+struct LeafConst
+{
+    float lo0[3], c[3];
+};
+__device__ __forceinline__ LeafConst leaf_consts(const RInv& M, const float mu[3], const float4& w0, const float4& w1,
+                                                 const float4& w2, const float4& w4, float vs, const int32_t o[3],
+                                                 const int32_t r0[3])
+{
+    LeafConst L;
+    float d0[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+        d0[a] = VOX_FFMA((float)(o[a] + r0[a]), vs, -mu[a]);
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+    {
+        const float h0 = (&w0.x)[r], h1 = (&w1.x)[r], h2 = (&w2.x)[r];
+        const float base = VOX_FMUL(
+            VOX_FFMA(M.m[r][2], d0[2], VOX_FFMA(M.m[r][0], d0[0], VOX_FMUL(M.m[r][1], d0[1]))), (&w4.x)[r]);
+        L.lo0[r] = VOX_FADD(VOX_FADD(VOX_FADD(base, 2.f * fminf(h0, 0.f)), 2.f * fminf(h1, 0.f)), 2.f * fminf(h2, 0.f));
+        L.c[r] = 0.5f * base + 0.5f * ((h0 + h1) + h2);
+    }
+    return L;
+}
+
+// the float channels' local AABB of the voxel (fx, fy, fz) / 2 voxels from the
+// anchor; h: half steps [row][axis], W4: W / 4
+__device__ __forceinline__ Aabb stable_leaf_aabb(const float lo0[3], const float W4[3], const float h[3][3], float fx,
                                                  float fy, float fz)
 {
     Aabb b;
 #pragma unroll
     for (int r = 0; r < 3; r++)
     {
-        b.lo[r] = VOX_FFMA(fz, A[r][2], VOX_FFMA(fy, A[r][1], VOX_FFMA(fx, A[r][0], lo0[r])));
-        b.hi[r] = VOX_FADD(b.lo[r], W[r]);
+        b.lo[r] = VOX_FFMA(fz, h[r][2], VOX_FFMA(fy, h[r][1], VOX_FFMA(fx, h[r][0], lo0[r])));
+        b.hi[r] = VOX_FFMA(4.f, W4[r], b.lo[r]);
     }
     return b;
 }
@@ -675,7 +701,7 @@ __device__ __forceinline__ AlphaF pair_alpha_f_ex(const float4& q6, const Aabb& 
 // with b_ref = voxel_local_aabb(...), decided where possible from the float
 // channel's alpha f (same formula, evaluated from stable_leaf_aabb).
 // Per row the two AABBs' bounds, and so their four lattice points, differ by at
-// most D_r = dab_r (leaf_pair_consts: the scalings' and lattice points'
+// most D_r = dab_r (WalkRec: the scalings' and lattice points'
 // roundings included).  With p_r the float evaluation's lattice point nearest to
 // zero, either evaluation's minimizing point is within u_r = |p_r| + D_r of zero,
 // so the row minima differ by at most 2 |p_r| D_r + D_r^2 + 2^-22 u_r^2 (rounded

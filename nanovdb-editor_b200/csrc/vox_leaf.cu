@@ -325,18 +325,16 @@ struct RecSlot
 
 struct LeafChunk
 {
-    RecSlot rec[LQ_CHUNK]; // first member: 16-byte aligned for cp.async
-    // Constants of each (leaf, Gaussian) as 16-byte words, one load each:
-    // the test's (leaf_pair_consts, halved; c at the box origin's voxel)
-    //   [0] c 0..2, lo_t   [1] x steps 0..2, hi_t   [2] y steps 0..2, h 0   [3] z steps 0..2, h 1
-    //   [4] h 2, 65536 / ny rounded up (exact division below 64), ny | nz << 8, j << 9 | box origin's leaf_n
-    float4 tq[5][LQ_CHUNK];
-    // the float channels'
-    //   [r] lo0 r, W r, x step r, y step r   [3] z steps 0..2, colour bytes of the RGBA8 value
-    //   [4] dab 0..2, voxel size   [5] 2^23 + anchor x, y, z
-    float4 aq[6][LQ_CHUNK];
-    uint32_t cstart[16];    // first column of box j (boxes past the chunk's count: none left); [LQ_CHUNK]: all
-    uint8_t flag[LQ_CHUNK];
+    float4 rec[8][LQ_CHUNK];         // the records, word by word
+    float4 walk[WALK_WORDS][LQ_CHUNK]; // their walk constants
+    // per (leaf, Gaussian)
+    float4 tc[LQ_CHUNK]; // the test's c at the box origin's voxel, lo_t
+    float4 tb[LQ_CHUNK]; // 65536 / ny rounded up (exact division below 64), ny | nz << 8 | leaf test failed << 16 (check
+                         // mode), j << 9 | box origin's leaf_n, h_2
+    float4 al[LQ_CHUNK]; // lo0, the colour bytes of the RGBA8 value
+    float4 aa[LQ_CHUNK]; // 2^24 + 2 anchor x, y, z, h_2
+    uint32_t gid[LQ_CHUNK];
+    uint32_t cstart[16]; // first column of box j (boxes past the chunk's count: none left); [LQ_CHUNK]: all
     uint64_t wf0[LQ_CHUNK], wbase[LQ_CHUNK]; // reference windows: fragment offset in its batch, windows before
 };
 
@@ -355,15 +353,17 @@ struct LeafQSmem
     LeafAcc acc;
     uint32_t mask[3][16]; // value masks of the leaf being tested and of the two before it
     uint16_t queue[2][LQ_CHUNK * 512];
-    uint16_t defer[LP_THREADS / 32][64]; // per warp: queued pairs whose RGBA8 byte the bound left open
-    uint32_t dcount[LP_THREADS / 32];     // per warp: the open pairs left at the end of its alpha
-    uint32_t dfin;                        // warps done with this phase's alpha
+    uint32_t defer[LP_THREADS / 32][64]; // per warp: the leaf's pairs whose RGBA8 byte the bound left open
+    uint32_t dcount[LP_THREADS / 32];     // per warp: the open pairs left at the leaf's end
+    uint32_t dfin;                        // warps done with the leaf's alpha
     uint32_t qn[3];
     int32_t nxt_o[2][3]; // the next chunk (by phase parity): leaf origin and sorted pair range
     uint32_t nxt_q0[2], nxt_p1[2];
     uint32_t cand_next[2];
     uint32_t cand;
 };
+
+static_assert(sizeof(LeafQSmem) <= 56 * 1024, "four CTAs of the leaf walk fit an SM's 228 KB (1 KB of it reserved per CTA)");
 
 // One term of an exact fixed-point sum, (hi, lo) += (xh, xl) with the carry from
 // the low word's old value: the total is the same integer in any order.  A
@@ -466,12 +466,12 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
         uint32_t zmask = 0, ebase = 0;
         if (e < T)
         {
-            const float4 q0 = C.tq[0][j], q1 = C.tq[1][j], q2 = C.tq[2][j], q3 = C.tq[3][j], q4 = C.tq[4][j];
-            const uint32_t ext = __float_as_uint(q4.z), ny = ext & 255u, nz = ext >> 8;
+            const float4 q0 = C.tc[j], q1 = C.walk[0][j], q2 = C.walk[1][j], q3 = C.walk[2][j], q4 = C.tb[j];
+            const uint32_t ext = __float_as_uint(q4.y), ny = ext & 255u, nz = (ext >> 8) & 255u;
             const uint32_t local = e - sj;
-            const uint32_t dx = (local * __float_as_uint(q4.y)) >> 16;
+            const uint32_t dx = (local * __float_as_uint(q4.x)) >> 16;
             const uint32_t dy = local - dx * ny;
-            ebase = __float_as_uint(q4.w) + (dx << 6) + (dy << 3);
+            ebase = __float_as_uint(q4.z) + (dx << 6) + (dy << 3);
             const float fx = (float)dx, fy = (float)dy;
             const float b0 = VOX_FFMA(fy, q2.x, VOX_FFMA(fx, q1.x, q0.x)), b1 = VOX_FFMA(fy, q2.y, VOX_FFMA(fx, q1.y, q0.y)),
                         b2 = VOX_FFMA(fy, q2.z, VOX_FFMA(fx, q1.z, q0.z));
@@ -479,7 +479,7 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
             const F2 S0 = f2(q3.x, q3.x), S1 = f2(q3.y, q3.y), S2 = f2(q3.z, q3.z);
             const F2 nlo = f2(-q0.w, -q0.w), hi2 = f2(q1.w, q1.w), m1 = f2(-1.f, -1.f), m2 = f2(-2.f, -2.f),
                      zero = f2(0.f, 0.f);
-            const float h0 = q2.w, h1 = q3.w, h2 = q4.x;
+            const float h0 = q2.w, h1 = q3.w, h2 = q4.w;
             const uint32_t steps = (nz + 1u) >> 1; // voxels (2 k - 2, 2 k - 1) for k = steps .. 1
             const float ft = (float)(2u * steps);
             F2 K = f2(ft - 2.f, ft - 1.f);
@@ -503,9 +503,9 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
             zmask = pass & valid;
             // the reference test of one voxel, from the record (nothing of the column kept live)
             auto exact_voxel = [&](uint32_t k) -> uint32_t {
-                const GaussRec& R = C.rec[j].r;
+                const GaussRec R = P.recs[C.gid[j]];
                 const uint32_t n = (ebase & 511u) + k;
-                const Aabb b = voxel_local_aabb(R, rinv_of(R), C.aq[4][j].w, o[0] + (int32_t)(n >> 6),
+                const Aabb b = voxel_local_aabb(R, rinv_of(R), C.walk[3][j].w, o[0] + (int32_t)(n >> 6),
                                                 o[1] + (int32_t)((n >> 3) & 7u), o[2] + (int32_t)(n & 7u));
                 return aabb_hits_unit_sphere(b) ? 1u << k : 0u;
             };
@@ -518,7 +518,7 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
                     ex |= exact_voxel(k);
                 if (ex != zmask)
                     atomicOr(P.err, ERR_BOUNDS); // a classification differs from the reference test
-                if (zmask && C.flag[j])
+                if (zmask && ext >> 16)
                     atomicOr(P.err, ERR_BOUNDS); // the leaf test would have dropped a passing voxel
             }
             if (zmask)
@@ -538,8 +538,11 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
         if (lane == 31 && incl)
             qb = atomicAdd(qcount, incl);
         qb = __shfl_sync(0xffffffffu, qb, 31) + incl - np;
-        for (uint32_t m = zmask; m; m &= m - 1)
-            queue[qb++] = (uint16_t)(ebase + (uint32_t)(__ffs(m) - 1));
+        uint16_t* dst = queue + qb;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++)
+            if (zmask & (1u << k))
+                *dst++ = (uint16_t)(ebase + k);
     }
 }
 
@@ -713,36 +716,54 @@ __device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, Ga
     return g;
 }
 
+// the same for the forward walk: record and walk constants into slot j
+__device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, LeafChunk& C, int j, uint32_t q)
+{
+    const uint32_t g = P.pair_gid[q];
+    const float4* rec = reinterpret_cast<const float4*>(&P.recs[g]);
+    const float4* walk = reinterpret_cast<const float4*>(&P.walk[g]);
+#pragma unroll
+    for (int w = 0; w < 8; w++)
+        cp_async16(&C.rec[w][j], rec + w);
+#pragma unroll
+    for (int w = 0; w < WALK_WORDS; w++)
+        cp_async16(&C.walk[w][j], walk + w);
+    return g;
+}
+
 // once the record landed: the chunk's constants of Gaussian j; returns its box columns
 template <bool CHECK, bool WINDOW>
 __device__ __forceinline__ uint32_t leaf_stage_box(const LeafPassParams& P, LeafChunk& C, int j, uint32_t q, uint32_t g,
                                                    const int32_t o[3])
 {
-    const GaussRec& R = C.rec[j].r;
+    GaussRec R;
+    R.q4 = *reinterpret_cast<const int4*>(&C.rec[4][j]);
+    R.q5 = *reinterpret_cast<const int4*>(&C.rec[5][j]);
     const LeafBox b = leaf_box(R, o);
-    const float vs = rec_vs(R, P.voxel_size, P.cloud_vs);
-    const LeafPairConst K = leaf_pair_consts(R, vs, o);
-    const uint32_t rgb24 = rgba8_byte(R.q7.x) | (rgba8_byte(R.q7.y) << 8) | (rgba8_byte(R.q7.z) << 16);
-    const float bx = (float)(b.lo[0] - K.r0[0]), by = (float)(b.lo[1] - K.r0[1]), bz = (float)(b.lo[2] - K.r0[2]);
+    int32_t r0[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+        r0[a] = anchor_of((&R.q4.x)[a], (&R.q5.x)[a], o[a]);
+    R.q0 = C.rec[0][j];
+    R.q1 = C.rec[1][j];
+    R.q2 = C.rec[2][j];
+    R.q3.x = C.rec[3][j].x;
+    const float mu[3] = { R.q0.x, R.q0.y, R.q0.z };
+    const float4 w0 = C.walk[0][j], w1 = C.walk[1][j], w2 = C.walk[2][j], w4 = C.walk[4][j], w5 = C.walk[5][j];
+    const LeafConst K = leaf_consts(rinv_of(R), mu, w0, w1, w2, w4, C.walk[3][j].w, o, r0);
+    const float bx = (float)(b.lo[0] - r0[0]), by = (float)(b.lo[1] - r0[1]), bz = (float)(b.lo[2] - r0[2]);
     float c[3];
 #pragma unroll
     for (int r = 0; r < 3; r++)
-        c[r] = VOX_FFMA(bz, 0.5f * K.A[r][2], VOX_FFMA(by, 0.5f * K.A[r][1], VOX_FFMA(bx, 0.5f * K.A[r][0], K.c[r])));
-    C.tq[0][j] = make_float4(c[0], c[1], c[2], K.lo_t);
-    C.tq[1][j] = make_float4(0.5f * K.A[0][0], 0.5f * K.A[1][0], 0.5f * K.A[2][0], K.hi_t);
-    C.tq[2][j] = make_float4(0.5f * K.A[0][1], 0.5f * K.A[1][1], 0.5f * K.A[2][1], 0.25f * K.W[0]);
-    C.tq[3][j] = make_float4(0.5f * K.A[0][2], 0.5f * K.A[1][2], 0.5f * K.A[2][2], 0.25f * K.W[1]);
-    C.tq[4][j] = make_float4(0.25f * K.W[2], __uint_as_float((65536u + b.ny - 1u) / b.ny),
-                             __uint_as_float(b.ny | b.nz << 8),
-                             __uint_as_float((uint32_t)j << 9 | (uint32_t)(b.lo[0] << 6 | b.lo[1] << 3 | b.lo[2])));
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-        C.aq[r][j] = make_float4(K.lo0[r], K.W[r], K.A[r][0], K.A[r][1]);
-    C.aq[3][j] = make_float4(K.A[0][2], K.A[1][2], K.A[2][2], __uint_as_float(rgb24));
-    C.aq[4][j] = make_float4(K.dab[0], K.dab[1], K.dab[2], vs);
-    C.aq[5][j] = make_float4(8388608.f + (float)K.r0[0], 8388608.f + (float)K.r0[1], 8388608.f + (float)K.r0[2], 0.f);
-    if (CHECK)
-        C.flag[j] = P.emit_flag[P.vals[q]];
+        c[r] = VOX_FFMA(bz, (&w2.x)[r], VOX_FFMA(by, (&w1.x)[r], VOX_FFMA(bx, (&w0.x)[r], K.c[r])));
+    const uint32_t failed = CHECK ? (uint32_t)P.emit_flag[P.vals[q]] : 0u;
+    C.tc[j] = make_float4(c[0], c[1], c[2], w5.x);
+    C.tb[j] = make_float4(__uint_as_float((65536u + b.ny - 1u) / b.ny), __uint_as_float(b.ny | b.nz << 8 | failed << 16),
+                          __uint_as_float((uint32_t)j << 9 | (uint32_t)(b.lo[0] << 6 | b.lo[1] << 3 | b.lo[2])), w4.w);
+    C.al[j] = make_float4(K.lo0[0], K.lo0[1], K.lo0[2], w5.y);
+    C.aa[j] = make_float4(16777216.f + (float)(2 * r0[0]), 16777216.f + (float)(2 * r0[1]), 16777216.f + (float)(2 * r0[2]),
+                          w4.w);
+    C.gid[j] = g;
     if (WINDOW)
     {
         const int64_t batch = (int64_t)g / REF_PRIM_BATCH;
@@ -750,6 +771,16 @@ __device__ __forceinline__ uint32_t leaf_stage_box(const LeafPassParams& P, Leaf
         C.wbase[j] = P.win_before[batch];
     }
     return b.nx * b.ny;
+}
+
+// the record in slot j of a chunk
+__device__ __forceinline__ GaussRec chunk_rec(const LeafChunk& C, uint32_t j)
+{
+    GaussRec R;
+#pragma unroll
+    for (int w = 0; w < 8; w++)
+        reinterpret_cast<float4*>(&R)[w] = C.rec[w][j];
+    return R;
 }
 
 template <bool CHECK, bool WINDOW, int MINB = 4>
@@ -797,7 +828,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         uint32_t cols = 0;
         if (js < (int)min((uint32_t)LQ_CHUNK, tp1 - tq0))
         {
-            const uint32_t g = leaf_stage_issue(P, &S.ch[0].rec[js].r, tq0 + (uint32_t)js);
+            const uint32_t g = leaf_stage_issue(P, S.ch[0], js, tq0 + (uint32_t)js);
             cp_async_wait_all();
             cols = leaf_stage_box<CHECK, WINDOW>(P, S.ch[0], js, tq0 + (uint32_t)js, g, to);
         }
@@ -809,6 +840,8 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
     int64_t ac = 0, fc = 0;
     int32_t ao[3] = { 0, 0, 0 };
     unsigned long long leaf_pairs = 0, all_pairs = 0; // thread 0's
+    uint32_t tleaf0 = tq0, aleaf0 = 0, alocal = 0;    // first pair of the leaf; the alpha's chunk's place after it
+    uint32_t dn = 0;                                  // this warp's deferred pairs (warp-uniform)
     uint32_t i = 0; // phase
     while (t_valid || a_valid || f_valid)
     {
@@ -836,7 +869,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
             np1 = t_leaf_end ? pre_p1 : tp1;
             ncnt = min((uint32_t)LQ_CHUNK, np1 - nq0);
             if (js < (int)ncnt)
-                ng = leaf_stage_issue(P, &S.ch[nb].rec[js].r, nq0 + (uint32_t)js);
+                ng = leaf_stage_issue(P, S.ch[nb], js, nq0 + (uint32_t)js);
         }
         // ---- flush of the leaf whose last alpha ran in the previous phase
         if (f_valid)
@@ -888,9 +921,10 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         }
         const uint32_t a_rounds = a_valid ? (S.qn[ab] + 31u) / 32u : 0u; // the alpha's rounds of 32 pairs
         // ---- alpha of the previous chunk, one queued pair per thread.  A pair
-        // whose RGBA8 byte the bound leaves open (a few percent) is deferred to
-        // its warp's list and the reference's byte is evaluated 32 pairs at a
-        // time, so the rare branch costs one converged pass per 32 pairs.
+        // whose RGBA8 byte the bound leaves open (1 - 2%) is deferred to its
+        // warp's list, which lasts through the leaf, and the reference's byte is
+        // evaluated 32 pairs at a time (from the records in global memory), so the
+        // rare branch costs one converged pass per 32 pairs.
         if (a_valid)
         {
             const LeafChunk& C = S.ch[ab];
@@ -899,13 +933,14 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
             const uint32_t qn = S.qn[ab];
             if (t == 0)
                 leaf_pairs += qn;
-            uint16_t* dq = S.defer[warp];
-            uint32_t dn = 0; // this warp's deferred pairs (warp-uniform)
-            auto ref_byte = [&](uint32_t q) {
-                const uint32_t j = q >> 9, n = q & 511u;
-                const uint32_t a8 = ref_alpha_byte(C.rec[j].r, C.aq[4][j].w, ao[0] + (int32_t)(n >> 6),
+            uint32_t* dq = S.defer[warp];
+            // the reference's byte of voxel n and the leaf's Gaussian at position l of its pairs
+            auto ref_byte = [&](uint32_t l, uint32_t n) {
+                const uint32_t g = P.pair_gid[aleaf0 + l];
+                const GaussRec R = P.recs[g];
+                const uint32_t a8 = ref_alpha_byte(R, P.walk[g].w3.w, ao[0] + (int32_t)(n >> 6),
                                                    ao[1] + (int32_t)((n >> 3) & 7u), ao[2] + (int32_t)(n & 7u));
-                atomicMax(&A.rgba[n], (a8 << 24) | __float_as_uint(C.aq[3][j].w));
+                atomicMax(&A.rgba[n], (a8 << 24) | __float_as_uint(P.walk[g].w5.y));
             };
             for (uint32_t e0 = (uint32_t)(t & ~31); e0 < qn; e0 += LP_THREADS) // warp-uniform trip count
             {
@@ -916,42 +951,42 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 {
                     q = queue[e];
                     const uint32_t j = q >> 9, n = q & 511u;
-                    const GaussRec& R = C.rec[j].r;
-                    const float4 a3 = C.aq[3][j], q7 = R.q7;
+                    const float4 al = C.al[j], q7 = C.rec[7][j];
                     float a;
                     uint32_t a8;
                     if (P.smooth)
                     {
+                        const GaussRec R = chunk_rec(C, j);
                         const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
                                       zz = ao[2] + (int32_t)(n & 7);
-                        const float vsf = C.aq[4][j].w;
+                        const float vsf = C.walk[3][j].w;
                         SmoothTerms st;
                         a = smooth_kernel(R, rinv_of(R), vsf, x, yy, zz, st);
                         a8 = ref_alpha_byte(R, vsf, x, yy, zz) << 24;
                     }
                     else
                     {
-                        const float4 r0 = C.aq[0][j], r1 = C.aq[1][j], r2 = C.aq[2][j], anc = C.aq[5][j], q6 = R.q6;
-                        const float lo0[3] = { r0.x, r1.x, r2.x }, wid[3] = { r0.y, r1.y, r2.y };
-                        const float stp[3][3] = { { r0.z, r0.w, a3.x }, { r1.z, r1.w, a3.y }, { r2.z, r2.w, a3.z } };
-                        // voxels from the anchor, exactly (2^23 + n is a float's last place)
-                        const float fx = VOX_FSUB(__uint_as_float(0x4b000000u | (n >> 6)), anc.x),
-                                    fy = VOX_FSUB(__uint_as_float(0x4b000000u | ((n >> 3) & 7u)), anc.y),
-                                    fz = VOX_FSUB(__uint_as_float(0x4b000000u | (n & 7u)), anc.z);
-                        const AlphaF af = pair_alpha_f_ex(q6, stable_leaf_aabb(lo0, wid, stp, fx, fy, fz));
+                        const float4 w0 = C.walk[0][j], w1 = C.walk[1][j], w2 = C.walk[2][j], aa = C.aa[j], q6 = C.rec[6][j];
+                        const float lo0[3] = { al.x, al.y, al.z }, W4[3] = { w1.w, w2.w, aa.w };
+                        const float h[3][3] = { { w0.x, w1.x, w2.x }, { w0.y, w1.y, w2.y }, { w0.z, w1.z, w2.z } };
+                        // twice the voxels from the anchor, exactly (a last place is 2 from 2^24 on)
+                        const float fx = VOX_FSUB(__uint_as_float(0x4b800000u | (n >> 6)), aa.x),
+                                    fy = VOX_FSUB(__uint_as_float(0x4b800000u | ((n >> 3) & 7u)), aa.y),
+                                    fz = VOX_FSUB(__uint_as_float(0x4b800000u | (n & 7u)), aa.z);
+                        const AlphaF af = pair_alpha_f_ex(q6, stable_leaf_aabb(lo0, W4, h, fx, fy, fz));
                         a = q7.w != 0.f ? 0.f : af.a1;
                         bool decided;
-                        const float4 db = C.aq[4][j];
+                        const float4 db = C.walk[3][j];
                         const float dab[3] = { db.x, db.y, db.z };
                         a8 = alpha_byte_bound(q6, q7.w, af, dab, decided);
                         defer = !decided;
                         if (CHECK && decided &&
-                            a8 >> 24 != ref_alpha_byte(R, db.w, ao[0] + (int32_t)(n >> 6), ao[1] + (int32_t)((n >> 3) & 7),
-                                                       ao[2] + (int32_t)(n & 7)))
+                            a8 >> 24 != ref_alpha_byte(chunk_rec(C, j), db.w, ao[0] + (int32_t)(n >> 6),
+                                                       ao[1] + (int32_t)((n >> 3) & 7), ao[2] + (int32_t)(n & 7)))
                             atomicOr(P.err, ERR_BOUNDS); // the margin failed to cover the reference's byte
                     }
                     if (!defer)
-                        atomicMax(&A.rgba[n], a8 | __float_as_uint(a3.w));
+                        atomicMax(&A.rgba[n], a8 | __float_as_uint(al.w));
                     const float c0 = VOX_FMUL(a, q7.x), c1 = VOX_FMUL(a, q7.y), c2 = VOX_FMUL(a, q7.z);
                     if (a < 1.f && c0 >= 0.f && c0 < 1.f && c1 >= 0.f && c1 < 1.f && c2 >= 0.f && c2 < 1.f)
                     {
@@ -974,8 +1009,10 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         // (gaussian_frag_alloc.slang:55-58) after the Gaussian's batch offset
                         const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
                                       zz = ao[2] + (int32_t)(n & 7);
-                        const uint64_t r = (uint64_t)(x - R.q4.x) * (uint64_t)R.q5.y * (uint64_t)R.q5.z +
-                                           (uint64_t)(yy - R.q4.y) * (uint64_t)R.q5.z + (uint64_t)(zz - R.q4.z);
+                        const int4 b0 = *reinterpret_cast<const int4*>(&C.rec[4][j]),
+                                   ext = *reinterpret_cast<const int4*>(&C.rec[5][j]);
+                        const uint64_t r = (uint64_t)(x - b0.x) * (uint64_t)ext.y * (uint64_t)ext.z +
+                                           (uint64_t)(yy - b0.y) * (uint64_t)ext.z + (uint64_t)(zz - b0.z);
                         const unsigned long long wk = C.wbase[j] + (C.wf0[j] + r) / REF_WINDOW;
                         // read first: a 64-bit minimum in shared memory is a compare-and-swap loop,
                         // and nearly every pair's window is no earlier than the one there
@@ -983,18 +1020,27 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                             atomicMin(&A.wmin, wk);
                     }
                 }
+                // a list entry holds the pair's position among the leaf's pairs in 23 bits;
+                // a leaf of more pairs evaluates the rest at once
+                const uint32_t l = alocal + (q >> 9);
+                if (defer && l >= 1u << 23)
+                {
+                    ref_byte(l, q & 511u);
+                    defer = false;
+                }
                 const uint32_t bal = __ballot_sync(0xffffffffu, defer);
                 if (bal)
                 {
                     if (defer)
-                        dq[dn + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = (uint16_t)q;
+                        dq[dn + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = l << 9 | (q & 511u);
                     dn += (uint32_t)__popc(bal);
                     if (dn >= 32u) // dn <= 63: a batch of 32, the rest moved to the front
                     {
                         __syncwarp();
-                        ref_byte(dq[lane]);
+                        const uint32_t d = dq[lane];
+                        ref_byte(d >> 9, d & 511u);
                         const uint32_t rest = dn - 32u;
-                        const uint16_t mv = (uint32_t)lane < rest ? dq[32 + lane] : (uint16_t)0;
+                        const uint32_t mv = (uint32_t)lane < rest ? dq[32 + lane] : 0u;
                         __syncwarp();
                         if ((uint32_t)lane < rest)
                             dq[lane] = mv;
@@ -1003,48 +1049,54 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                     }
                 }
             }
-            // the open pairs left in every warp's list (fewer than 32 each): the last
-            // warp to finish this phase's alpha evaluates all of them, 32 at a time
-            // (the chunk's records stay in place until the next phase's staging)
-            uint32_t fin = 0;
-            if (lane == 0)
+            // at the leaf's end, the open pairs left in every warp's list (fewer than 32
+            // each): the last warp to finish evaluates all of them, 32 at a time
+            if (a_leaf_end)
             {
-                S.dcount[warp] = dn;
-                __threadfence_block();
-                fin = atomicAdd(&S.dfin, 1u);
-            }
-            fin = __shfl_sync(0xffffffffu, fin, 0);
-            if (fin == LP_THREADS / 32 - 1)
-            {
-                __threadfence_block();
-                const uint32_t c = (uint32_t)lane < LP_THREADS / 32 ? *(volatile uint32_t*)&S.dcount[lane] : 0u;
-                uint32_t incl = c;
-#pragma unroll
-                for (int off = 1; off < LP_THREADS / 32; off <<= 1)
-                {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-                    if (lane >= off)
-                        incl += y;
-                }
-                const uint32_t total = __shfl_sync(0xffffffffu, incl, LP_THREADS / 32 - 1);
-                for (uint32_t b = 0; b < total; b += 32)
-                {
-                    const uint32_t item = b + (uint32_t)lane;
-                    // the warp list holding item: the first w whose inclusive count exceeds it
-                    uint32_t w = 0, before = 0;
-#pragma unroll
-                    for (int v = 0; v < LP_THREADS / 32; v++)
-                    {
-                        const uint32_t iv = __shfl_sync(0xffffffffu, incl, v);
-                        const bool past = item >= iv;
-                        w += past ? 1u : 0u;
-                        before = past ? iv : before;
-                    }
-                    if (item < total)
-                        ref_byte(*(volatile uint16_t*)&S.defer[w][item - before]);
-                }
+                uint32_t fin = 0;
                 if (lane == 0)
-                    S.dfin = 0;
+                {
+                    S.dcount[warp] = dn;
+                    __threadfence_block();
+                    fin = atomicAdd(&S.dfin, 1u);
+                }
+                dn = 0;
+                fin = __shfl_sync(0xffffffffu, fin, 0);
+                if (fin == LP_THREADS / 32 - 1)
+                {
+                    __threadfence_block();
+                    const uint32_t c = (uint32_t)lane < LP_THREADS / 32 ? *(volatile uint32_t*)&S.dcount[lane] : 0u;
+                    uint32_t incl = c;
+#pragma unroll
+                    for (int off = 1; off < LP_THREADS / 32; off <<= 1)
+                    {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+                        if (lane >= off)
+                            incl += y;
+                    }
+                    const uint32_t total = __shfl_sync(0xffffffffu, incl, LP_THREADS / 32 - 1);
+                    for (uint32_t b = 0; b < total; b += 32)
+                    {
+                        const uint32_t item = b + (uint32_t)lane;
+                        // the warp list holding item: the first w whose inclusive count exceeds it
+                        uint32_t w = 0, before = 0;
+#pragma unroll
+                        for (int v = 0; v < LP_THREADS / 32; v++)
+                        {
+                            const uint32_t iv = __shfl_sync(0xffffffffu, incl, v);
+                            const bool past = item >= iv;
+                            w += past ? 1u : 0u;
+                            before = past ? iv : before;
+                        }
+                        if (item < total)
+                        {
+                            const uint32_t d = *(volatile uint32_t*)&S.defer[w][item - before];
+                            ref_byte(d >> 9, d & 511u);
+                        }
+                    }
+                    if (lane == 0)
+                        S.dfin = 0;
+                }
             }
         }
         // ---- test of this chunk
@@ -1091,6 +1143,8 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         a_leaf_end = t_leaf_end;
         ac = tc;
         am = tm;
+        aleaf0 = tleaf0;
+        alocal = tq0 - tleaf0;
         ao[0] = to[0];
         ao[1] = to[1];
         ao[2] = to[2];
@@ -1106,6 +1160,8 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
             tc = nc;
             tq0 = S.nxt_q0[pp];
             tp1 = S.nxt_p1[pp];
+            if (t_leaf_end)
+                tleaf0 = tq0;
             to[0] = S.nxt_o[pp][0];
             to[1] = S.nxt_o[pp][1];
             to[2] = S.nxt_o[pp][2];

@@ -38,8 +38,8 @@ __device__ __forceinline__ void mark_bit(unsigned long long* bits, uint64_t i)
 }
 
 // ------------------------------------------------------------------ prep ----
-__global__ void __launch_bounds__(256) k_prep(PrepParams P, GaussRec* recs, uint64_t* footprints,
-                                              unsigned long long* root_bits, int* err)
+__global__ void __launch_bounds__(256) k_prep(PrepParams P, GaussRec* recs, WalkRec* walk,
+                                              uint64_t* footprints, unsigned long long* root_bits, int* err)
 {
     const int64_t g = P.g0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= (P.g1 < 0 ? P.count : P.g1))
@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(256) k_prep(PrepParams P, GaussRec* recs, uint
     footprints[g] = fp;
     if (fp)
     {
+        walk[g] = walk_record(R, vs);
         // root tiles (4096^3 voxels) spanned by the bbox
         for (int32_t x = R.q4.x >> 12; x <= (bmax[0] >> 12); x++)
             for (int32_t y = R.q4.y >> 12; y <= (bmax[1] >> 12); y++)
@@ -651,13 +652,13 @@ __global__ void __launch_bounds__(NODE_THREADS) k_write_nodes(NodeParams N, uint
 static_assert(node_parts(2) == 1, "a lower node is one stretch");
 
 // =================================================================== launch
-void launch_prep(const PrepParams& P, GaussRec* recs, uint64_t* footprints, uint64_t* root_bits, int* err,
+void launch_prep(const PrepParams& P, GaussRec* recs, WalkRec* walk, uint64_t* footprints, uint64_t* root_bits, int* err,
                  cudaStream_t s)
 {
     const int64_t n = (P.g1 < 0 ? P.count : P.g1) - P.g0;
     if (n <= 0)
         return;
-    { k_prep<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, recs, footprints, (unsigned long long*)root_bits, err); count_launch(); }
+    { k_prep<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, recs, walk, footprints, (unsigned long long*)root_bits, err); count_launch(); }
 }
 
 void launch_mark_lower(const GaussRec* recs, int64_t G, const uint64_t* root_bits, const uint64_t* root_prefix,

@@ -125,6 +125,7 @@ struct LeafEmitParams
 struct LeafPassParams
 {
     const GaussRec* recs;
+    const WalkRec* walk;
     const uint32_t* vals;      // sorted leaf pairs' emission indices
     const uint32_t* emit_gid;
     const uint32_t* pair_gid;  // sorted leaf pairs' Gaussian ids
@@ -225,7 +226,7 @@ void launch_window_place(const WindowOrderParams& W, const NodeParams& N, cudaSt
 
 void launch_bwd_finalize(const BwdFinalParams& F, cudaStream_t s);
 
-void launch_prep(const PrepParams& P, GaussRec* recs, uint64_t* footprints, uint64_t* root_bits, int* err,
+void launch_prep(const PrepParams& P, GaussRec* recs, WalkRec* walk, uint64_t* footprints, uint64_t* root_bits, int* err,
                  cudaStream_t s);
 void launch_mark_lower(const GaussRec* recs, int64_t G, const uint64_t* root_bits, const uint64_t* root_prefix,
                        uint64_t* lower_bits, cudaStream_t s);
