@@ -500,9 +500,10 @@ struct __align__(16) WalkRec
     float4 w0; // half x steps A_00 A_10 A_20, hi_t
     float4 w1; // half y steps, h_0
     float4 w2; // half z steps, h_1
-    float4 w3; // dab_0..2, voxel size
+    float4 w3; // 2 dab_0..2 and sum_r dab_r^2, raised by 2^-19 (alpha_byte_bound); the sum negative
+               // (sign bit set) when a colour lies outside [0, 1]
     float4 w4; // k_0..2, h_2
-    float4 w5; // lo_t, the colour bytes of the RGBA8 value
+    float4 w5; // lo_t, the colour bytes of the RGBA8 value, voxel size
 };
 constexpr int WALK_WORDS = 6; // 16-byte words of a WalkRec
 
@@ -566,13 +567,15 @@ __device__ __forceinline__ WalkRec walk_record(const GaussRec& R, float vs)
         hi_t = 0.25f * (1.f + (2.f * Dl + Dl * Dl + 0x1p-18f));
     }
     const uint32_t rgb24 = rgba8_byte(R.q7.x) | (rgba8_byte(R.q7.y) << 8) | (rgba8_byte(R.q7.z) << 16);
+    const bool unit = R.q7.x >= 0.f && R.q7.x <= 1.f && R.q7.y >= 0.f && R.q7.y <= 1.f && R.q7.z >= 0.f && R.q7.z <= 1.f;
+    const float up = 1.f + 0x1p-19f, dd = (dab[0] * dab[0] + dab[1] * dab[1] + dab[2] * dab[2]) * up;
     WalkRec o;
     o.w0 = make_float4(hA[0][0], hA[1][0], hA[2][0], hi_t);
     o.w1 = make_float4(hA[0][1], hA[1][1], hA[2][1], h[0]);
     o.w2 = make_float4(hA[0][2], hA[1][2], hA[2][2], h[1]);
-    o.w3 = make_float4(dab[0], dab[1], dab[2], vs);
+    o.w3 = make_float4(2.f * dab[0] * up, 2.f * dab[1] * up, 2.f * dab[2] * up, unit ? dd : -dd);
     o.w4 = make_float4(k[0], k[1], k[2], h[2]);
-    o.w5 = make_float4(lo_t, __uint_as_float(rgb24), 0.f, 0.f);
+    o.w5 = make_float4(lo_t, __uint_as_float(rgb24), vs, 0.f);
     return o;
 }
 
@@ -705,8 +708,10 @@ __device__ __forceinline__ AlphaF pair_alpha_f_ex(const float4& q6, const Aabb& 
 // roundings included).  With p_r the float evaluation's lattice point nearest to
 // zero, either evaluation's minimizing point is within u_r = |p_r| + D_r of zero,
 // so the row minima differ by at most 2 |p_r| D_r + D_r^2 + 2^-22 u_r^2 (rounded
-// squares) and the lattice minima d by md = sum_r of that (times 1 + 2^-20) +
-// 2^-21 d (the two rounded sums); and the
+// squares) and the lattice minima d by sum_r of that + 2^-21 d (the two rounded
+// sums).  With u^2 <= 2 p^2 + 2 D^2 and sum p^2 <= d (1 + 2^-22) this is at most
+// md = sum_r 2 |p_r| D_r + (1 + 2^-21) sum_r D_r^2 + 2^-20 (1 + 2^-8) d, whose
+// own four roundings the record's terms, raised by 2^-19, cover; and the
 // alpha a' = 1 - (1 - op e^-ls d)^e, whose slope in d is at most
 // e ls a_hi (times 1 / (1 - a_hi) when e < 1) for a_hi >= op e^-ls (d - md),
 // by at most that slope times md, plus both evaluations' own error: the exps
@@ -728,30 +733,22 @@ __device__ __forceinline__ uint32_t alpha_byte_bits(float v)
     return __float_as_uint(__fadd_rd(VOX_FMUL(255.f, __saturatef(v)), 8388608.f));
 }
 
-// the byte in bits 24-31, the rest 0
-__device__ __forceinline__ uint32_t alpha_byte_bound(const float4& q6, float cull, const AlphaF& f, const float dab[3],
+// the byte in bits 24-31, the rest 0 (w3: the Gaussian's WalkRec::w3)
+__device__ __forceinline__ uint32_t alpha_byte_bound(const float4& q6, float cull, const AlphaF& f, const float4& w3,
                                                      bool& decided)
 {
-    // branch-free (the pairs of a warp take different cases): every quantity is
-    // computed and the cases are combined at the end
-    float md = 0.f;
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-    {
-        const float D = dab[r];
-        const float u = f.p[r] + D; // bounds both evaluations' minimizing lattice point
-        md += (2.f * u - D) * D + 0x1p-22f * u * u;
-    }
-    md = md * (1.f + 0x1p-20f) + 0x1p-21f * f.d;
+    const float md = VOX_FFMA(
+        f.p[0], w3.x, VOX_FFMA(f.p[1], w3.y, VOX_FFMA(f.p[2], w3.z, VOX_FFMA(0x1.02p-20f, f.d, fabsf(w3.w)))));
     const float ls = q6.y, e = q6.z;
     const float x = ls * md;
-    const float a_hi = f.a * (1.f + 2.f * x) * (1.f + 1e-6f); // e^x <= 1 + 2x for x <= 1
-    // 1 / (1 - a_hi) from the fast reciprocal (within 2 ulp for 1 - a_hi >= 2^-24,
-    // as it is when a_hi < 1), raised by 2^-20 so it stays an upper bound
-    const float inv = __fdividef(1.f, 1.f - a_hi) * (1.f + 0x1p-20f);
-    const float slope_e = e < 1.f ? e * inv : e; // the pow's slope bound
-    const float slope = slope_e * ls * a_hi;
-    const float delta = 1.25f * slope * md + slope_e * (1.1e-6f * a_hi + 1.8e-7f) + 9.3e-7f;
+    const float a_hi = VOX_FFMA(2.f * x, f.a, f.a) * (1.f + 1e-6f); // e^x <= 1 + 2x for x <= 1
+    float slope_e = e; // the pow's slope bound
+    if (e < 1.f)       // (a Gaussian of more than 10 voxels: few warps have one)
+        // 1 / (1 - a_hi) from the fast reciprocal (within 2 ulp for 1 - a_hi >= 2^-24,
+        // as it is when a_hi < 1), raised by 2^-20 so it stays an upper bound
+        slope_e = e * (__fdividef(1.f, 1.f - a_hi) * (1.f + 0x1p-20f));
+    // slope_e (ls a_hi 1.25 md + 1.1e-6 a_hi + 1.8e-7) + 9.3e-7
+    const float delta = VOX_FFMA(slope_e, VOX_FFMA(a_hi, VOX_FFMA(1.25f, x, 1.1e-6f), 1.8e-7f), 9.3e-7f);
     const uint32_t lo = alpha_byte_bits(f.a1 - delta), hi = alpha_byte_bits(f.a1 + delta);
     const bool culled = cull != 0.f; // culled by scale: both alphas are 0
     decided = culled || (x < 0.25f && a_hi < 1.f && lo == hi);

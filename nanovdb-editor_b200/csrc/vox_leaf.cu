@@ -295,25 +295,31 @@ __device__ __forceinline__ void stage_chunk(const LeafPassParams& P, LeafSmem& S
 }
 
 // ------------------------------------------------------ forward leaf walk
-// A CTA walks a stream of candidate leaves in chunks of LQ_CHUNK Gaussians
-// (a leaf's Gaussians in ascending id).  Per chunk:
+// A CTA walks a stream of candidate leaves in chunks of Gaussians (a leaf's
+// Gaussians in ascending id): as many of the next LF_CHUNK as have boxes of
+// LF_CAP voxels together, since every voxel may pass and take a queue entry.
+// Per chunk:
 //   test   the part of each Gaussian's bbox inside the leaf, one (Gaussian,
-//          column) per thread: the column's x / y share once, then its z run,
-//          each z's corner products shared with the next; passing (Gaussian,
-//          voxel) pairs go to a shared queue;
+//          column) per thread: the column's x / y share once, then its z run;
+//          passing (Gaussian, voxel) pairs go to a shared queue;
 //   alpha  one queued pair per thread: the reference's RGBA8 alpha and the
 //          float channels' stable alpha, accumulated per voxel with shared
-//          atomics - RGBA8 maximum, pair count, 64-bit fixed-point density /
-//          colour sums (exact, so independent of order);
+//          atomics - RGBA8 maximum, fixed-point density / colour sums (exact,
+//          so independent of order);
 //   flush  once a leaf's last alpha is done: its staged values, value mask
 //          and pair count.
 // One barrier per chunk: phase i runs the flush of the leaf that ended with
 // chunk i - 2, the alpha of chunk i - 1, the test of chunk i, and the staging
 // of chunk i + 1 (lanes of the last warp copy its records with cp.async and
-// place its boxes).  Chunk data is triple-buffered, queues double-buffered,
-// the per-voxel accumulators double-buffered by leaf parity.
-constexpr int LQ_CHUNK = 12;
-constexpr int LQ_STAGE_T0 = LP_THREADS - 32; // lanes 0..LQ_CHUNK-1 of the last warp stage the next chunk
+// place its boxes).  Chunk data is triple-buffered, queues double-buffered.
+// The barrier, the staging and the partly filled rounds cost the same for any
+// chunk, so the larger it is the better; 56 KB of shared memory (4 CTAs per SM)
+// bound it.  Against chunks of 12 Gaussians (with their whole records in each
+// buffer), the walk of 200k Gaussians 3.52 -> 3.05 ms, a call on 2M 37.1 -> 32.5.
+constexpr int LF_CHUNK = 24;
+constexpr uint32_t LF_CAP = 5120;
+constexpr int LQ_CHUNK = 12;                 // the adjoint walk's chunk
+constexpr int LQ_STAGE_T0 = LP_THREADS - 32; // the last warp's lanes stage the next chunk
 
 // A record slot padded to 144 B: the same field of a chunk's 8 records falls in
 // 8 different shared-memory banks (a 128 B stride puts them all in one).
@@ -323,19 +329,41 @@ struct RecSlot
     float4 pad;
 };
 
-struct LeafChunk
+// what the stagers read of the next chunk, each its own column (overwritten by
+// its own next copies)
+struct LeafStage
 {
-    float4 rec[8][LQ_CHUNK];         // the records, word by word
-    float4 walk[WALK_WORDS][LQ_CHUNK]; // their walk constants
+    float4 rec[6][LF_CHUNK];  // record words 0 - 5
+    float4 walk[2][LF_CHUNK]; // walk constants 4, 5
+};
+
+// record words 0 - 3, for the differentiable channels' kernel
+template <bool SMOOTH>
+struct LeafSmooth
+{
+};
+template <>
+struct LeafSmooth<true>
+{
+    float4 rec[4][LF_CHUNK];
+};
+
+template <bool SMOOTH>
+struct LeafChunk : LeafSmooth<SMOOTH>
+{
+    float4 q6[LF_CHUNK], q7[LF_CHUNK]; // record words 6, 7
+    float4 walk[4][LF_CHUNK];          // walk constants 0 - 3
     // per (leaf, Gaussian)
-    float4 tc[LQ_CHUNK]; // the test's c at the box origin's voxel, lo_t
-    float4 tb[LQ_CHUNK]; // 65536 / ny rounded up (exact division below 64), ny | nz << 8 | leaf test failed << 16 (check
+    float4 tc[LF_CHUNK]; // the test's c at the box origin's voxel, lo_t
+    float4 tb[LF_CHUNK]; // 65536 / ny rounded up (exact division below 64), ny | nz << 8 | leaf test failed << 16 (check
                          // mode), j << 9 | box origin's leaf_n, h_2
-    float4 al[LQ_CHUNK]; // lo0, the colour bytes of the RGBA8 value
-    float4 aa[LQ_CHUNK]; // 2^24 + 2 anchor x, y, z, h_2
-    uint32_t gid[LQ_CHUNK];
-    uint32_t cstart[16]; // first column of box j (boxes past the chunk's count: none left); [LQ_CHUNK]: all
-    uint64_t wf0[LQ_CHUNK], wbase[LQ_CHUNK]; // reference windows: fragment offset in its batch, windows before
+    float4 al[LF_CHUNK]; // lo0, the colour bytes of the RGBA8 value
+    float4 aa[LF_CHUNK]; // 2^24 + 2 anchor x, y, z, h_2
+    uint64_t win[LF_CHUNK]; // reference windows: of the box's fragments, ~0 if they lie in several
+    uint32_t gid[LF_CHUNK];
+    uint32_t cstart[LF_CHUNK]; // first column of box j (boxes past the chunk's count: the end)
+    uint32_t cols;             // all columns
+    uint32_t pad;
 };
 
 // Per-voxel sums as two 32-bit words (acc_add)
@@ -347,23 +375,25 @@ struct LeafAcc
     unsigned long long wmin;  // creation window (reference node order)
 };
 
+template <bool SMOOTH>
 struct LeafQSmem
 {
-    LeafChunk ch[3];
+    LeafStage st;
+    LeafChunk<SMOOTH> ch[3];
     LeafAcc acc;
     uint32_t mask[3][16]; // value masks of the leaf being tested and of the two before it
-    uint16_t queue[2][LQ_CHUNK * 512];
+    uint16_t queue[2][LF_CAP];
     uint32_t defer[LP_THREADS / 32][64]; // per warp: the leaf's pairs whose RGBA8 byte the bound left open
     uint32_t dcount[LP_THREADS / 32];     // per warp: the open pairs left at the leaf's end
     uint32_t dfin;                        // warps done with the leaf's alpha
     uint32_t qn[3];
-    int32_t nxt_o[2][3]; // the next chunk (by phase parity): leaf origin and sorted pair range
-    uint32_t nxt_q0[2], nxt_p1[2];
+    int32_t nxt_o[2][3]; // the next chunk (by phase parity): leaf origin, sorted pair range and count
+    uint32_t nxt_q0[2], nxt_p1[2], nxt_cnt[2];
     uint32_t cand_next[2];
     uint32_t cand;
 };
 
-static_assert(sizeof(LeafQSmem) <= 56 * 1024, "four CTAs of the leaf walk fit an SM's 228 KB (1 KB of it reserved per CTA)");
+static_assert(sizeof(LeafQSmem<false>) <= 56 * 1024, "four CTAs of the leaf walk fit an SM's 228 KB (1 KB of it reserved per CTA)");
 
 // One term of an exact fixed-point sum, (hi, lo) += (xh, xl) with the carry from
 // the low word's old value: the total is the same integer in any order.  A
@@ -442,13 +472,13 @@ __device__ __forceinline__ F2 f2_add(F2 a, F2 b)
 // first): 11 instructions per voxel for 24.  With acc_add, the constants as
 // 16-byte words and the value masks set here instead of counted per pair, the
 // walk of 2M Gaussians (1.6e9 pairs) 42.9 -> 34.1 ms.
-template <bool CHECK>
-__device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const LeafChunk& C, const int32_t o[3],
+template <bool CHECK, class Chunk>
+__device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const Chunk& C, const int32_t o[3],
                                                   uint16_t* queue, uint32_t* qcount, uint32_t* mask, int t, int lane,
                                                   uint32_t rot)
 {
-    const uint32_t T = C.cstart[LQ_CHUNK];
-    const uint32_t cs = lane < LQ_CHUNK ? C.cstart[lane] : 0x7fffffffu;
+    const uint32_t T = C.cols;
+    const uint32_t cs = lane < LF_CHUNK ? C.cstart[lane] : 0x7fffffffu;
     const uint32_t le = 0xffffffffu >> (31 - lane);
     // rounds of 32 columns dealt to the warps in turn, starting at warp rot (mod 8):
     // the deal continues where the alpha's rounds of 32 pairs stopped, so the warps'
@@ -460,7 +490,7 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
         // emitted leaf meets its Gaussian's bbox); sj its first column
         const uint32_t rel = cs - e0;
         const uint32_t heads = __reduce_or_sync(0xffffffffu, rel - 1u < 31u ? 1u << rel : 0u);
-        const uint32_t j = (uint32_t)(__popc(__ballot_sync(0xffffffffu, cs <= e0)) - 1 + __popc(heads & le)) & 15u;
+        const uint32_t j = (uint32_t)(__popc(__ballot_sync(0xffffffffu, cs <= e0)) - 1 + __popc(heads & le)) & 31u;
         const uint32_t sj = __shfl_sync(0xffffffffu, cs, (int)j);
         const uint32_t e = e0 + (uint32_t)lane;
         uint32_t zmask = 0, ebase = 0;
@@ -505,7 +535,7 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
             auto exact_voxel = [&](uint32_t k) -> uint32_t {
                 const GaussRec R = P.recs[C.gid[j]];
                 const uint32_t n = (ebase & 511u) + k;
-                const Aabb b = voxel_local_aabb(R, rinv_of(R), C.walk[3][j].w, o[0] + (int32_t)(n >> 6),
+                const Aabb b = voxel_local_aabb(R, rinv_of(R), P.walk[C.gid[j]].w5.z, o[0] + (int32_t)(n >> 6),
                                                 o[1] + (int32_t)((n >> 3) & 7u), o[2] + (int32_t)(n & 7u));
                 return aabb_hits_unit_sphere(b) ? 1u << k : 0u;
             };
@@ -678,20 +708,35 @@ __device__ __forceinline__ LeafBox leaf_box(const GaussRec& R, const int32_t o[3
     return b;
 }
 
-// all stagers (lanes 0 .. LQ_CHUNK - 1 of the last warp): the chunk's column
-// prefix from each stager's own box columns (0 past the chunk's count)
-__device__ __forceinline__ void leaf_stage_prefix(LeafChunk& C, int js, uint32_t b)
+// the last warp, each lane with its own box's columns and voxels (0 past the
+// Gaussians at hand): the chunk takes the first boxes of LF_CAP voxels together;
+// its column prefix, and how many Gaussians it has
+template <class Chunk>
+__device__ __forceinline__ uint32_t leaf_stage_prefix(Chunk& C, int lane, uint32_t avail, uint32_t cols, uint32_t voxels)
 {
+    uint32_t v = voxels;
 #pragma unroll
-    for (int off = 1; off < LQ_CHUNK; off <<= 1)
+    for (int off = 1; off < 32; off <<= 1)
     {
-        const uint32_t y = __shfl_up_sync((1u << LQ_CHUNK) - 1u, b, off);
-        if (js >= off)
-            b += y;
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, off);
+        if (lane >= off)
+            v += y;
     }
-    C.cstart[js + 1] = b;
-    if (js == 0)
-        C.cstart[0] = 0;
+    const uint32_t cnt = (uint32_t)__popc(__ballot_sync(0xffffffffu, (uint32_t)lane < avail && v <= LF_CAP));
+    const uint32_t mine = (uint32_t)lane < cnt ? cols : 0u;
+    uint32_t c = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, c, off);
+        if (lane >= off)
+            c += y;
+    }
+    if (lane < LF_CHUNK)
+        C.cstart[lane] = c - mine;
+    if (lane == 31)
+        C.cols = c;
+    return cnt;
 }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src)
@@ -717,40 +762,61 @@ __device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, Ga
 }
 
 // the same for the forward walk: record and walk constants into slot j
-__device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, LeafChunk& C, int j, uint32_t q)
+template <bool SMOOTH>
+__device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, LeafStage& T, LeafChunk<SMOOTH>& C, int j,
+                                                     uint32_t q)
 {
     const uint32_t g = P.pair_gid[q];
     const float4* rec = reinterpret_cast<const float4*>(&P.recs[g]);
     const float4* walk = reinterpret_cast<const float4*>(&P.walk[g]);
 #pragma unroll
-    for (int w = 0; w < 8; w++)
-        cp_async16(&C.rec[w][j], rec + w);
+    for (int w = 0; w < 6; w++)
+        cp_async16(&T.rec[w][j], rec + w);
+    cp_async16(&C.q6[j], rec + 6);
+    cp_async16(&C.q7[j], rec + 7);
 #pragma unroll
-    for (int w = 0; w < WALK_WORDS; w++)
+    for (int w = 0; w < 4; w++)
         cp_async16(&C.walk[w][j], walk + w);
+    cp_async16(&T.walk[0][j], walk + 4);
+    cp_async16(&T.walk[1][j], walk + 5);
+    if constexpr (SMOOTH)
+#pragma unroll
+        for (int w = 0; w < 4; w++)
+            cp_async16(&C.rec[w][j], rec + w);
     return g;
 }
 
-// once the record landed: the chunk's constants of Gaussian j; returns its box columns
-template <bool CHECK, bool WINDOW>
-__device__ __forceinline__ uint32_t leaf_stage_box(const LeafPassParams& P, LeafChunk& C, int j, uint32_t q, uint32_t g,
-                                                   const int32_t o[3])
+// the reference's window of voxel (x, y, z)'s fragment of Gaussian g: its x-major
+// index in the bbox (gaussian_frag_alloc.slang:55-58) after the Gaussian's batch offset
+__device__ __forceinline__ uint64_t frag_window(const LeafPassParams& P, uint32_t g, const int4& b0, const int4& ext,
+                                                int32_t x, int32_t y, int32_t z)
+{
+    const int64_t batch = (int64_t)g / REF_PRIM_BATCH;
+    const uint64_t r = (uint64_t)(x - b0.x) * (uint64_t)ext.y * (uint64_t)ext.z + (uint64_t)(y - b0.y) * (uint64_t)ext.z +
+                       (uint64_t)(z - b0.z);
+    return P.win_before[batch] + (P.frag_off[g] - P.frag_off[batch * REF_PRIM_BATCH] + r) / REF_WINDOW;
+}
+
+// once the record landed: the chunk's constants of Gaussian j, and its box's columns and voxels
+template <bool CHECK, bool WINDOW, class Chunk>
+__device__ __forceinline__ void leaf_stage_box(const LeafPassParams& P, const LeafStage& T, Chunk& C, int j, uint32_t q,
+                                               uint32_t g, const int32_t o[3], uint32_t& cols, uint32_t& voxels)
 {
     GaussRec R;
-    R.q4 = *reinterpret_cast<const int4*>(&C.rec[4][j]);
-    R.q5 = *reinterpret_cast<const int4*>(&C.rec[5][j]);
+    R.q4 = *reinterpret_cast<const int4*>(&T.rec[4][j]);
+    R.q5 = *reinterpret_cast<const int4*>(&T.rec[5][j]);
     const LeafBox b = leaf_box(R, o);
     int32_t r0[3];
 #pragma unroll
     for (int a = 0; a < 3; a++)
         r0[a] = anchor_of((&R.q4.x)[a], (&R.q5.x)[a], o[a]);
-    R.q0 = C.rec[0][j];
-    R.q1 = C.rec[1][j];
-    R.q2 = C.rec[2][j];
-    R.q3.x = C.rec[3][j].x;
+    R.q0 = T.rec[0][j];
+    R.q1 = T.rec[1][j];
+    R.q2 = T.rec[2][j];
+    R.q3.x = T.rec[3][j].x;
     const float mu[3] = { R.q0.x, R.q0.y, R.q0.z };
-    const float4 w0 = C.walk[0][j], w1 = C.walk[1][j], w2 = C.walk[2][j], w4 = C.walk[4][j], w5 = C.walk[5][j];
-    const LeafConst K = leaf_consts(rinv_of(R), mu, w0, w1, w2, w4, C.walk[3][j].w, o, r0);
+    const float4 w0 = C.walk[0][j], w1 = C.walk[1][j], w2 = C.walk[2][j], w4 = T.walk[0][j], w5 = T.walk[1][j];
+    const LeafConst K = leaf_consts(rinv_of(R), mu, w0, w1, w2, w4, w5.z, o, r0);
     const float bx = (float)(b.lo[0] - r0[0]), by = (float)(b.lo[1] - r0[1]), bz = (float)(b.lo[2] - r0[2]);
     float c[3];
 #pragma unroll
@@ -766,31 +832,23 @@ __device__ __forceinline__ uint32_t leaf_stage_box(const LeafPassParams& P, Leaf
     C.gid[j] = g;
     if (WINDOW)
     {
-        const int64_t batch = (int64_t)g / REF_PRIM_BATCH;
-        C.wf0[j] = P.frag_off[g] - P.frag_off[batch * REF_PRIM_BATCH];
-        C.wbase[j] = P.win_before[batch];
+        // fragments are numbered x-major, so the box's lie between its two corners'
+        const int32_t x = o[0] + b.lo[0], y = o[1] + b.lo[1], z = o[2] + b.lo[2];
+        const uint64_t first = frag_window(P, g, R.q4, R.q5, x, y, z);
+        const uint64_t last = frag_window(P, g, R.q4, R.q5, x + (int32_t)b.nx - 1, y + (int32_t)b.ny - 1, z + (int32_t)b.nz - 1);
+        C.win[j] = first == last ? first : ~0ull;
     }
-    return b.nx * b.ny;
+    cols = b.nx * b.ny;
+    voxels = cols * b.nz;
 }
 
-// the record in slot j of a chunk
-__device__ __forceinline__ GaussRec chunk_rec(const LeafChunk& C, uint32_t j)
-{
-    GaussRec R;
-#pragma unroll
-    for (int w = 0; w < 8; w++)
-        reinterpret_cast<float4*>(&R)[w] = C.rec[w][j];
-    return R;
-}
-
-template <bool CHECK, bool WINDOW, int MINB = 4>
+template <bool CHECK, bool WINDOW, bool SMOOTH, int MINB>
 __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P, uint32_t* counter)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    LeafQSmem& S = *reinterpret_cast<LeafQSmem*>(smem_raw);
+    LeafQSmem<SMOOTH>& S = *reinterpret_cast<LeafQSmem<SMOOTH>*>(smem_raw);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int js = t - LQ_STAGE_T0; // staging slot (0 .. LQ_CHUNK - 1 on the stagers)
-    const bool stager = js >= 0 && js < LQ_CHUNK;
+    const bool stager = warp == LP_THREADS / 32 - 1; // lane j < LF_CHUNK stages Gaussian j of the next chunk
     if (t == 0)
     {
         S.cand = atomicAdd(counter, 1u);
@@ -825,16 +883,20 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
     uint32_t tq0 = P.cand_start[tc], tp1 = P.cand_start[tc + 1];
     if (stager)
     {
-        uint32_t cols = 0;
-        if (js < (int)min((uint32_t)LQ_CHUNK, tp1 - tq0))
+        uint32_t cols = 0, voxels = 0;
+        const uint32_t avail = min((uint32_t)LF_CHUNK, tp1 - tq0);
+        if ((uint32_t)lane < avail)
         {
-            const uint32_t g = leaf_stage_issue(P, S.ch[0], js, tq0 + (uint32_t)js);
+            const uint32_t g = leaf_stage_issue<SMOOTH>(P, S.st, S.ch[0], lane, tq0 + (uint32_t)lane);
             cp_async_wait_all();
-            cols = leaf_stage_box<CHECK, WINDOW>(P, S.ch[0], js, tq0 + (uint32_t)js, g, to);
+            leaf_stage_box<CHECK, WINDOW>(P, S.st, S.ch[0], lane, tq0 + (uint32_t)lane, g, to, cols, voxels);
         }
-        leaf_stage_prefix(S.ch[0], js, cols);
+        const uint32_t cnt = leaf_stage_prefix(S.ch[0], lane, avail, cols, voxels);
+        if (lane == 0)
+            S.nxt_cnt[1] = cnt;
     }
     __syncthreads();
+    uint32_t tcnt = S.nxt_cnt[1]; // (phase 0 fills the other)
     bool t_valid = true, a_valid = false, f_valid = false, a_leaf_end = false;
     int tm = 0, am = 0, fm = 0; // value mask buffers, one per leaf in turn
     int64_t ac = 0, fc = 0;
@@ -846,7 +908,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
     while (t_valid || a_valid || f_valid)
     {
         const int tb = (int)(i % 3u), ab = (int)((i + 2u) % 3u), nb = (int)((i + 1u) % 3u);
-        const bool t_leaf_end = t_valid && tq0 + LQ_CHUNK >= tp1;
+        const bool t_leaf_end = t_valid && tq0 + tcnt >= tp1;
         const int64_t nc = t_leaf_end ? cn : tc;
         const bool n_valid = t_valid && nc < P.NCL;
         if (stager && cn_fresh)
@@ -856,20 +918,20 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 pre_org = P.cand_org[cn];
                 pre_q0 = P.cand_start[cn];
                 pre_p1 = P.cand_start[cn + 1];
-                if (js == 0)
+                if (lane == 0)
                     cn2 = atomicAdd(counter, 1u);
             }
         }
         cn_fresh = false;
         // ---- stagers: the next chunk's pair range, its record copies
-        uint32_t nq0 = 0, np1 = 0, ncnt = 0, ng = 0;
+        uint32_t nq0 = 0, np1 = 0, avail = 0, ng = 0;
         if (stager && n_valid)
         {
-            nq0 = t_leaf_end ? pre_q0 : tq0 + LQ_CHUNK;
+            nq0 = t_leaf_end ? pre_q0 : tq0 + tcnt;
             np1 = t_leaf_end ? pre_p1 : tp1;
-            ncnt = min((uint32_t)LQ_CHUNK, np1 - nq0);
-            if (js < (int)ncnt)
-                ng = leaf_stage_issue(P, S.ch[nb], js, nq0 + (uint32_t)js);
+            avail = min((uint32_t)LF_CHUNK, np1 - nq0);
+            if ((uint32_t)lane < avail)
+                ng = leaf_stage_issue<SMOOTH>(P, S.st, S.ch[nb], lane, nq0 + (uint32_t)lane);
         }
         // ---- flush of the leaf whose last alpha ran in the previous phase
         if (f_valid)
@@ -889,7 +951,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                     for (int k = 0; k < 3; k++)
                     {
                         col[k] = fx_to_float((unsigned long long)A.col[k][1][n] << 32 | A.col[k][0][n]);
-                        if (!P.smooth)
+                        if (!SMOOTH)
                             col[k] = ds > 0.f ? VOX_FDIV(col[k], ds) : 0.f;
                     }
                     P.s_rgba[slot] = A.rgba[n];
@@ -927,7 +989,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         // rare branch costs one converged pass per 32 pairs.
         if (a_valid)
         {
-            const LeafChunk& C = S.ch[ab];
+            const LeafChunk<SMOOTH>& C = S.ch[ab];
             LeafAcc& A = S.acc;
             const uint16_t* queue = S.queue[(i + 1u) & 1u];
             const uint32_t qn = S.qn[ab];
@@ -938,7 +1000,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
             auto ref_byte = [&](uint32_t l, uint32_t n) {
                 const uint32_t g = P.pair_gid[aleaf0 + l];
                 const GaussRec R = P.recs[g];
-                const uint32_t a8 = ref_alpha_byte(R, P.walk[g].w3.w, ao[0] + (int32_t)(n >> 6),
+                const uint32_t a8 = ref_alpha_byte(R, P.walk[g].w5.z, ao[0] + (int32_t)(n >> 6),
                                                    ao[1] + (int32_t)((n >> 3) & 7u), ao[2] + (int32_t)(n & 7u));
                 atomicMax(&A.rgba[n], (a8 << 24) | __float_as_uint(P.walk[g].w5.y));
             };
@@ -951,22 +1013,28 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 {
                     q = queue[e];
                     const uint32_t j = q >> 9, n = q & 511u;
-                    const float4 al = C.al[j], q7 = C.rec[7][j];
+                    const float4 al = C.al[j], q7 = C.q7[j], w3 = C.walk[3][j];
                     float a;
                     uint32_t a8;
-                    if (P.smooth)
+                    if constexpr (SMOOTH)
                     {
-                        const GaussRec R = chunk_rec(C, j);
                         const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
                                       zz = ao[2] + (int32_t)(n & 7);
-                        const float vsf = C.walk[3][j].w;
+                        GaussRec R;
+                        R.q0 = C.rec[0][j];
+                        R.q1 = C.rec[1][j];
+                        R.q2 = C.rec[2][j];
+                        R.q3 = C.rec[3][j];
+                        R.q6 = C.q6[j];
+                        R.q7 = q7;
+                        const float vsf = P.cloud_vs ? P.walk[C.gid[j]].w5.z : P.voxel_size;
                         SmoothTerms st;
                         a = smooth_kernel(R, rinv_of(R), vsf, x, yy, zz, st);
                         a8 = ref_alpha_byte(R, vsf, x, yy, zz) << 24;
                     }
                     else
                     {
-                        const float4 w0 = C.walk[0][j], w1 = C.walk[1][j], w2 = C.walk[2][j], aa = C.aa[j], q6 = C.rec[6][j];
+                        const float4 w0 = C.walk[0][j], w1 = C.walk[1][j], w2 = C.walk[2][j], aa = C.aa[j], q6 = C.q6[j];
                         const float lo0[3] = { al.x, al.y, al.z }, W4[3] = { w1.w, w2.w, aa.w };
                         const float h[3][3] = { { w0.x, w1.x, w2.x }, { w0.y, w1.y, w2.y }, { w0.z, w1.z, w2.z } };
                         // twice the voxels from the anchor, exactly (a last place is 2 from 2^24 on)
@@ -976,21 +1044,19 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         const AlphaF af = pair_alpha_f_ex(q6, stable_leaf_aabb(lo0, W4, h, fx, fy, fz));
                         a = q7.w != 0.f ? 0.f : af.a1;
                         bool decided;
-                        const float4 db = C.walk[3][j];
-                        const float dab[3] = { db.x, db.y, db.z };
-                        a8 = alpha_byte_bound(q6, q7.w, af, dab, decided);
+                        a8 = alpha_byte_bound(q6, q7.w, af, w3, decided);
                         defer = !decided;
                         if (CHECK && decided &&
-                            a8 >> 24 != ref_alpha_byte(chunk_rec(C, j), db.w, ao[0] + (int32_t)(n >> 6),
+                            a8 >> 24 != ref_alpha_byte(P.recs[C.gid[j]], P.walk[C.gid[j]].w5.z, ao[0] + (int32_t)(n >> 6),
                                                        ao[1] + (int32_t)((n >> 3) & 7), ao[2] + (int32_t)(n & 7)))
                             atomicOr(P.err, ERR_BOUNDS); // the margin failed to cover the reference's byte
                     }
                     if (!defer)
                         atomicMax(&A.rgba[n], a8 | __float_as_uint(al.w));
                     const float c0 = VOX_FMUL(a, q7.x), c1 = VOX_FMUL(a, q7.y), c2 = VOX_FMUL(a, q7.z);
-                    if (a < 1.f && c0 >= 0.f && c0 < 1.f && c1 >= 0.f && c1 < 1.f && c2 >= 0.f && c2 < 1.f)
+                    if (a < 1.f && (int32_t)__float_as_uint(w3.w) >= 0)
                     {
-                        // terms in [0, 1): below 2^32 units (a is never negative)
+                        // colours in [0, 1], so terms in [0, 1): below 2^32 units (a is never negative)
                         acc_add(&A.dens[0][n], &A.dens[1][n], __float2uint_rn(VOX_FMUL(a, FX_SCALE)), 0u);
                         acc_add(&A.col[0][0][n], &A.col[0][1][n], __float2uint_rn(VOX_FMUL(c0, FX_SCALE)), 0u);
                         acc_add(&A.col[1][0][n], &A.col[1][1][n], __float2uint_rn(VOX_FMUL(c1, FX_SCALE)), 0u);
@@ -1005,15 +1071,13 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                     }
                     if (WINDOW)
                     {
-                        // the reference's window of this fragment: x-major index in the bbox
-                        // (gaussian_frag_alloc.slang:55-58) after the Gaussian's batch offset
-                        const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
-                                      zz = ao[2] + (int32_t)(n & 7);
-                        const int4 b0 = *reinterpret_cast<const int4*>(&C.rec[4][j]),
-                                   ext = *reinterpret_cast<const int4*>(&C.rec[5][j]);
-                        const uint64_t r = (uint64_t)(x - b0.x) * (uint64_t)ext.y * (uint64_t)ext.z +
-                                           (uint64_t)(yy - b0.y) * (uint64_t)ext.z + (uint64_t)(zz - b0.z);
-                        const unsigned long long wk = C.wbase[j] + (C.wf0[j] + r) / REF_WINDOW;
+                        unsigned long long wk = C.win[j];
+                        if (wk == ~0ull)
+                        {
+                            const GaussRec& R = P.recs[C.gid[j]];
+                            wk = frag_window(P, C.gid[j], R.q4, R.q5, ao[0] + (int32_t)(n >> 6),
+                                             ao[1] + (int32_t)((n >> 3) & 7), ao[2] + (int32_t)(n & 7));
+                        }
                         // read first: a 64-bit minimum in shared memory is a compare-and-swap loop,
                         // and nearly every pair's window is no earlier than the one there
                         if (wk < *(volatile unsigned long long*)&A.wmin)
@@ -1115,14 +1179,14 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 no[1] = pre_org.y;
                 no[2] = pre_org.z;
             }
-            uint32_t cols = 0;
-            if (js < (int)ncnt)
+            uint32_t cols = 0, voxels = 0;
+            if ((uint32_t)lane < avail)
             {
                 cp_async_wait_all();
-                cols = leaf_stage_box<CHECK, WINDOW>(P, S.ch[nb], js, nq0 + (uint32_t)js, ng, no);
+                leaf_stage_box<CHECK, WINDOW>(P, S.st, S.ch[nb], lane, nq0 + (uint32_t)lane, ng, no, cols, voxels);
             }
-            leaf_stage_prefix(S.ch[nb], js, cols);
-            if (js == 0)
+            const uint32_t ncnt = leaf_stage_prefix(S.ch[nb], lane, avail, cols, voxels);
+            if (lane == 0)
             {
                 const int pp = (int)(i & 1u);
                 S.nxt_o[pp][0] = no[0];
@@ -1130,6 +1194,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 S.nxt_o[pp][2] = no[2];
                 S.nxt_q0[pp] = nq0;
                 S.nxt_p1[pp] = np1;
+                S.nxt_cnt[pp] = ncnt;
                 if (t_leaf_end)
                     S.cand_next[pp] = cn2;
             }
@@ -1160,6 +1225,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
             tc = nc;
             tq0 = S.nxt_q0[pp];
             tp1 = S.nxt_p1[pp];
+            tcnt = S.nxt_cnt[pp];
             if (t_leaf_end)
                 tleaf0 = tq0;
             to[0] = S.nxt_o[pp][0];
@@ -1758,15 +1824,11 @@ static unsigned walk_grid(int64_t NCL, int num_sms)
     return (unsigned)(g < NCL ? g : (NCL > 0 ? NCL : 1));
 }
 
-int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant)
+template <bool CHECK, bool WINDOW, bool SMOOTH, int MINB>
+static int launch_walk(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s)
 {
-    if (P.NCL <= 0)
-        return 0;
-    cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    const size_t smem = sizeof(LeafQSmem);
-    auto kern = P.emit_flag ? (P.window ? k_leaf_pass<true, true> : k_leaf_pass<true, false>)
-                : variant == 1 ? (P.window ? k_leaf_pass<false, true, 3> : k_leaf_pass<false, false, 3>)
-                               : (P.window ? k_leaf_pass<false, true> : k_leaf_pass<false, false>);
+    auto kern = k_leaf_pass<CHECK, WINDOW, SMOOTH, MINB>;
+    const size_t smem = sizeof(LeafQSmem<SMOOTH>);
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, LP_THREADS, smem);
@@ -1775,6 +1837,26 @@ int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cu
         grid = P.NCL;
     { kern<<<(unsigned)grid, LP_THREADS, smem, s>>>(P, counter); count_launch(); }
     return per_sm;
+}
+
+int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant)
+{
+    if (P.NCL <= 0)
+        return 0;
+    cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
+    if (P.smooth) // its chunks carry record words: 3 CTAs per SM either way
+        return P.emit_flag ? (P.window ? launch_walk<true, true, true, 3>(P, counter, num_sms, s)
+                                       : launch_walk<true, false, true, 3>(P, counter, num_sms, s))
+                           : (P.window ? launch_walk<false, true, true, 3>(P, counter, num_sms, s)
+                                       : launch_walk<false, false, true, 3>(P, counter, num_sms, s));
+    if (P.emit_flag)
+        return P.window ? launch_walk<true, true, false, 4>(P, counter, num_sms, s)
+                        : launch_walk<true, false, false, 4>(P, counter, num_sms, s);
+    if (variant == 1)
+        return P.window ? launch_walk<false, true, false, 3>(P, counter, num_sms, s)
+                        : launch_walk<false, false, false, 3>(P, counter, num_sms, s);
+    return P.window ? launch_walk<false, true, false, 4>(P, counter, num_sms, s)
+                    : launch_walk<false, false, false, 4>(P, counter, num_sms, s);
 }
 
 void launch_leaf_backward(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s)
