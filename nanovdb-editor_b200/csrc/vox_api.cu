@@ -892,7 +892,7 @@ static int run_backward(vox_context_t* ctx, const vox_gaussians_t* gs, const flo
     cudaStream_t s = ctx->stream;
     const int64_t launches0 = launch_count();
     const uint64_t Q = ctx->last_Q;
-    if (!ensure(ctx, ctx->partials, sizeof(float) * BWD_NACC * (size_t)(Q + 1)))
+    if (!ensure(ctx, ctx->partials, sizeof(float) * BWD_STRIDE * (size_t)(Q + 1)))
         return VOX_ERR_MEMORY;
     cudaEventRecord(ctx->timers.ev[0], s);
     cudaMemsetAsync((uint64_t*)ctx->scal.p + SC_ERR, 0, sizeof(uint64_t), s);
@@ -904,10 +904,10 @@ static int run_backward(vox_context_t* ctx, const vox_gaussians_t* gs, const flo
         LP.grad_density = grad_density;
         LP.grad_color = grad_color;
         LP.partials = partials;
-        launch_leaf_backward(LP, (uint32_t*)((uint64_t*)ctx->scal.p + SC_SCRATCH), ctx->num_sms, s);
+        launch_leaf_backward(LP, (int64_t)Q, s);
     }
     else
-        cudaMemsetAsync(partials, 0, sizeof(float) * BWD_NACC * (size_t)Q, s);
+        cudaMemsetAsync(partials, 0, sizeof(float) * BWD_STRIDE * (size_t)Q, s);
     BwdFinalParams F;
     memset(&F, 0, sizeof(F));
     F.partials = partials;

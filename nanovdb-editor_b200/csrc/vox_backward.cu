@@ -7,20 +7,23 @@
 //   e = op E,  K = max(e - 0.01, 0),
 //   density[v] += K,  colour[v] += K rgb.
 // Given dL/d density and dL/d colour (value-indexed), with
-// GK = dL/d density[v] + dL/d colour[v] . rgb, a pair with e > 0.01 adds
-//   dL/d op  += GK E
-//   dL/d z_r  = -GK e z_r,   dL/d u_r = dL/d z_r / s_r
+// GK = dL/d density[v] + dL/d colour[v] . rgb, a pair with e > 0.01 adds, with
+// f = -GK e,
+//   dL/d op  += GK E = -f / op
+//   dL/d z_r  = f z_r, dL/d u_r = f z_r / s_r
 //   U_r += dL/d u_r,  W_r += dL/d z_r z_r,  Q[r][a] += dL/d u_r d_a
 //   dL/d rgb += K dL/d colour[v]
 // and per Gaussian dL/d mu = -R U, dL/d s_r = -W_r / s_r, dL/d R[a][r] = Q[r][a],
 // chained through the rotation of gaussian_prim.slang:83-90, the quaternion
 // normalisation, exp, the sigmoid and SH0 of raster/RasterUtils.cpp:59-117.
+// Since d_a = sum_b R_ab s_b z_b, all of these follow from 13 sums: f, f z_r,
+// f z_r z_b and K dL/d colour (in the Gaussian's own axes, where the products of
+// a thin and a long one keep their relative precision).
 //
-// k_leaf_backward (vox_leaf.cu) replays the forward leaf walk: per candidate
-// leaf and Gaussian, the terms above summed over the leaf's voxels (a block
-// reduction) are stored by the pair's emission index; k_bwd_finalize sums a
-// Gaussian's partials (its emission indices are contiguous) in FP64 and
-// chains them.  No atomics, nothing stored per voxel pair.
+// k_leaf_backward (vox_leaf.cu) sums them per (leaf, Gaussian), stored by the
+// pair's emission index; k_bwd_finalize sums a Gaussian's rows (its emission
+// indices are contiguous) in FP64 and chains them.  No atomics, nothing stored
+// per voxel pair.
 #include <cstdio>
 #include <cuda_runtime.h>
 
@@ -46,8 +49,15 @@ __global__ void __launch_bounds__(256) k_bwd_finalize(BwdFinalParams F)
         for (int i = 0; i < BWD_NACC; i++)
             a[i] = 0.0;
         for (uint64_t e = e0; e < e1; e++)
+        {
+            const float4* row = reinterpret_cast<const float4*>(F.partials + e * BWD_STRIDE);
+            const float4 r0 = row[0], r1 = row[1], r2 = row[2];
+            const float v[BWD_NACC] = { r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w,
+                                        F.partials[e * BWD_STRIDE + 12] };
+#pragma unroll
             for (int i = 0; i < BWD_NACC; i++)
-                a[i] += (double)F.partials[e * BWD_NACC + i];
+                a[i] += (double)v[i];
+        }
         for (int i = 0; i < BWD_NACC; i++)
             any = any || a[i] != 0.0;
     }
@@ -74,8 +84,11 @@ __global__ void __launch_bounds__(256) k_bwd_finalize(BwdFinalParams F)
         R[2][0] = 2 * (x * z - y * w);
         R[2][1] = 2 * (y * z + x * w);
         R[2][2] = 1 - 2 * (x * x + y * y);
-        const double* U = &a[1];
+        const GaussRec& rec = F.recs[g];
+        const double is[3] = { rec.q3.y, rec.q3.z, rec.q3.w }; // the forward's 1 / s
+        const double U[3] = { is[0] * a[1], is[1] * a[2], is[2] * a[3] };
         const double* W = &a[4];
+        const double zz[3][3] = { { a[4], a[7], a[8] }, { a[7], a[5], a[9] }, { a[8], a[9], a[6] } };
         for (int k = 0; k < 3; k++)
             dmu[k] = (float)(-(R[k][0] * U[0] + R[k][1] * U[1] + R[k][2] * U[2]));
         const float min_scale = VOX_FMUL(0.125f, vsf);
@@ -92,7 +105,7 @@ __global__ void __launch_bounds__(256) k_bwd_finalize(BwdFinalParams F)
         double G[3][3];
         for (int k = 0; k < 3; k++)
             for (int r = 0; r < 3; r++)
-                G[k][r] = a[7 + 3 * r + k];
+                G[k][r] = is[r] * (R[k][0] / is[0] * zz[r][0] + R[k][1] / is[1] * zz[r][1] + R[k][2] / is[2] * zz[r][2]);
         double dx = 2 * y * (G[0][1] + G[1][0]) + 2 * z * (G[0][2] + G[2][0]) + 2 * w * (G[2][1] - G[1][2]) -
                     4 * x * (G[1][1] + G[2][2]);
         double dy = 2 * x * (G[0][1] + G[1][0]) + 2 * w * (G[0][2] - G[2][0]) + 2 * z * (G[1][2] + G[2][1]) -
@@ -115,15 +128,15 @@ __global__ void __launch_bounds__(256) k_bwd_finalize(BwdFinalParams F)
         if (F.raw)
         {
             const double op = 1.0 / (1.0 + exp(-(double)ld_attr(F.opacities, g, F.bf16)));
-            dop = (float)(a[0] * op * (1.0 - op));
+            dop = (float)(-a[0] / (double)rec.q6.x * op * (1.0 - op));
             for (int c = 0; c < 3; c++)
-                dc[c] = (float)(0.28209479177387814 * a[16 + c]);
+                dc[c] = (float)(0.28209479177387814 * a[10 + c]);
         }
         else
         {
-            dop = (float)a[0];
+            dop = (float)(-a[0] / (double)rec.q6.x);
             for (int c = 0; c < 3; c++)
-                dc[c] = (float)a[16 + c];
+                dc[c] = (float)a[10 + c];
         }
     }
     if (F.d_means)

@@ -503,7 +503,8 @@ struct __align__(16) WalkRec
     float4 w3; // 2 dab_0..2 and sum_r dab_r^2, raised by 2^-19 (alpha_byte_bound); the sum negative
                // (sign bit set) when a colour lies outside [0, 1]
     float4 w4; // k_0..2, h_2
-    float4 w5; // lo_t, the colour bytes of the RGBA8 value, voxel size
+    float4 w5; // lo_t, the colour bytes of the RGBA8 value, voxel size, 1 where a voxel centre's offset from mu
+               // is exact in double (smooth_kernel)
 };
 constexpr int WALK_WORDS = 6; // 16-byte words of a WalkRec
 
@@ -528,12 +529,15 @@ __device__ __forceinline__ WalkRec walk_record(const GaussRec& R, float vs)
     const float is[3] = { R.q3.y, R.q3.z, R.q3.w };
     const RInv M = rinv_of(R);
     float G[3], Cm[3];
+    bool exact_d = true;
 #pragma unroll
     for (int a = 0; a < 3; a++)
     {
         const int32_t v0 = (&R.q4.x)[a], v1 = v0 + (&R.q5.x)[a];
         const float w0 = (float)v0 * vs, w1 = (float)v1 * vs;
         const float W = fmaxf(fabsf(w0), fabsf(w1)) * (1.f + 0x1p-20f);
+        // (c + 1/2) vs has at most 42 bits; with mu's last place no lower than 2^-52 W the difference fits 53
+        exact_d = exact_d && (mu[a] == 0.f || fabsf(mu[a]) >= 0x1p-28f * W);
         Cm[a] = fmaxf(fabsf(w0 - mu[a]), fabsf(w1 - mu[a])) * (1.f + 0x1p-20f);
         const float E = (Cm[a] + vs) * (1.f + 0x1p-20f);
         G[a] = 0.5f * ulp_of(W) + 0.5f * ulp_of(Cm[a]) + 0x1p-21f * Cm[a] + 0.5f * ulp_of(E) + 0x1.8p-20f * E;
@@ -575,7 +579,7 @@ __device__ __forceinline__ WalkRec walk_record(const GaussRec& R, float vs)
     o.w2 = make_float4(hA[0][2], hA[1][2], hA[2][2], h[1]);
     o.w3 = make_float4(2.f * dab[0] * up, 2.f * dab[1] * up, 2.f * dab[2] * up, unit ? dd : -dd);
     o.w4 = make_float4(k[0], k[1], k[2], h[2]);
-    o.w5 = make_float4(lo_t, __uint_as_float(rgb24), vs, 0.f);
+    o.w5 = make_float4(lo_t, __uint_as_float(rgb24), vs, exact_d ? 1.f : 0.f);
     return o;
 }
 
@@ -768,27 +772,31 @@ __device__ __forceinline__ uint32_t ref_alpha_byte(const GaussRec& R, float vs, 
 // x the voxel centre, over the same pairs.  K vanishes on the 0.01-opacity
 // ellipsoid the pair test is built on (radius ls = sqrt(2 log(op / 0.01)),
 // gaussian_prim.slang:65), so the channels are continuous in every parameter.
-// Centre offsets are rounded once from double (stable far from the origin).
+// Centre offsets are rounded once from double (stable far from the origin);
+// where the double difference is exact (exact_d, WalkRec) one FP32 fma rounds the
+// same value.
 constexpr float SMOOTH_TAU = 0.01f;
 struct SmoothTerms
 {
     float d[3], z[3], E, e;
 };
-__device__ __forceinline__ float smooth_kernel(const GaussRec& R, const RInv& M, float vs, int32_t x, int32_t y,
-                                               int32_t z, SmoothTerms& t)
+__device__ __forceinline__ float smooth_kernel(const float mu[3], const float inv_s[3], float op, const RInv& M, float vs,
+                                               bool exact_d, int32_t x, int32_t y, int32_t z, SmoothTerms& t)
 {
     const int32_t c[3] = { x, y, z };
-    const float mu[3] = { R.q0.x, R.q0.y, R.q0.z };
-    const float inv_s[3] = { R.q3.y, R.q3.z, R.q3.w };
 #pragma unroll
     for (int a = 0; a < 3; a++)
-        t.d[a] = (float)VOX_DSUB(VOX_DMUL(VOX_DADD((double)c[a], 0.5), (double)vs), (double)mu[a]);
+        t.d[a] = VOX_FFMA((float)c[a] + 0.5f, vs, -mu[a]);
+    if (!exact_d)
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            t.d[a] = (float)VOX_DSUB(VOX_DMUL(VOX_DADD((double)c[a], 0.5), (double)vs), (double)mu[a]);
 #pragma unroll
     for (int r = 0; r < 3; r++)
         t.z[r] = VOX_FMUL(dot3_rn(t.d[0], t.d[1], t.d[2], M.m[r][0], M.m[r][1], M.m[r][2]), inv_s[r]);
     const float q = dot3_rn(t.z[0], t.z[1], t.z[2], t.z[0], t.z[1], t.z[2]);
     t.E = vox_expf_cr(VOX_FMUL(-0.5f, q));
-    t.e = VOX_FMUL(R.q6.x, t.E);
+    t.e = VOX_FMUL(op, t.E);
     return t.e > SMOOTH_TAU ? VOX_FSUB(t.e, SMOOTH_TAU) : 0.f;
 }
 

@@ -21,7 +21,7 @@
 //   k_write_leaves   once the tree's tables stand (k_tree): staged values to
 //       their value index, leaf nodes, bbox.
 // The adjoint (k_leaf_backward) and the sorted pair list (k_leaf_export)
-// replay the same walk.
+// go through the same (leaf, Gaussian) pairs.
 #include <cstdio>
 #include <cuda_runtime.h>
 
@@ -259,7 +259,6 @@ struct LeafSmem
     uint32_t eidx[LP_CHUNK];
     uint8_t flag[LP_CHUNK];
     uint64_t mask[8];
-    float red[LP_THREADS / 32][BWD_NACC];
     uint32_t pairs;
     uint32_t cand;
 };
@@ -318,16 +317,6 @@ __device__ __forceinline__ void stage_chunk(const LeafPassParams& P, LeafSmem& S
 // buffer), the walk of 200k Gaussians 3.52 -> 3.05 ms, a call on 2M 37.1 -> 32.5.
 constexpr int LF_CHUNK = 24;
 constexpr uint32_t LF_CAP = 5120;
-constexpr int LQ_CHUNK = 12;                 // the adjoint walk's chunk
-constexpr int LQ_STAGE_T0 = LP_THREADS - 32; // the last warp's lanes stage the next chunk
-
-// A record slot padded to 144 B: the same field of a chunk's 8 records falls in
-// 8 different shared-memory banks (a 128 B stride puts them all in one).
-struct RecSlot
-{
-    GaussRec r;
-    float4 pad;
-};
 
 // what the stagers read of the next chunk, each its own column (overwritten by
 // its own next copies)
@@ -337,7 +326,7 @@ struct LeafStage
     float4 walk[2][LF_CHUNK]; // walk constants 4, 5
 };
 
-// record words 0 - 3, for the differentiable channels' kernel
+// for the differentiable channels' kernel: record words 0 - 3, voxel size, WalkRec::w5.w
 template <bool SMOOTH>
 struct LeafSmooth
 {
@@ -346,6 +335,8 @@ template <>
 struct LeafSmooth<true>
 {
     float4 rec[4][LF_CHUNK];
+    float vs[LF_CHUNK];
+    uint32_t exact_d[LF_CHUNK];
 };
 
 template <bool SMOOTH>
@@ -444,6 +435,42 @@ __device__ __forceinline__ F2 f2_add(F2 a, F2 b)
     return o;
 }
 
+// The z run of one column (fx, fy voxels from the box's origin): which of its nz
+// voxels surely pass, and which need the reference test (leaf_test_columns has
+// the bounds).  q0 .. q3, h2: the test's constants (LeafChunk::tc, walk, tb).
+__device__ __forceinline__ uint32_t column_test(const float4& q0, const float4& q1, const float4& q2, const float4& q3,
+                                                float h2, float fx, float fy, uint32_t nz, uint32_t& unsure)
+{
+    const float b0 = VOX_FFMA(fy, q2.x, VOX_FFMA(fx, q1.x, q0.x)), b1 = VOX_FFMA(fy, q2.y, VOX_FFMA(fx, q1.y, q0.y)),
+                b2 = VOX_FFMA(fy, q2.z, VOX_FFMA(fx, q1.z, q0.z));
+    const F2 B0 = f2(b0, b0), B1 = f2(b1, b1), B2 = f2(b2, b2);
+    const F2 S0 = f2(q3.x, q3.x), S1 = f2(q3.y, q3.y), S2 = f2(q3.z, q3.z);
+    const F2 nlo = f2(-q0.w, -q0.w), hi2 = f2(q1.w, q1.w), m1 = f2(-1.f, -1.f), m2 = f2(-2.f, -2.f), zero = f2(0.f, 0.f);
+    const float h0 = q2.w, h1 = q3.w;
+    const uint32_t steps = (nz + 1u) >> 1; // voxels (2 k - 2, 2 k - 1) for k = steps .. 1
+    const float ft = (float)(2u * steps);
+    F2 K = f2(ft - 2.f, ft - 1.f);
+    uint32_t pass = 0, fail = 0;
+#pragma unroll 1
+    for (uint32_t k = steps; k; k--)
+    {
+        const float2 c0 = f2_get(f2_fma(K, S0, B0)), c1 = f2_get(f2_fma(K, S1, B1)), c2 = f2_get(f2_fma(K, S2, B2));
+        const F2 x0 = f2(__saturatef(VOX_FSUB(fabsf(c0.x), h0)), __saturatef(VOX_FSUB(fabsf(c0.y), h0)));
+        const F2 x1 = f2(__saturatef(VOX_FSUB(fabsf(c1.x), h1)), __saturatef(VOX_FSUB(fabsf(c1.y), h1)));
+        const F2 x2 = f2(__saturatef(VOX_FSUB(fabsf(c2.x), h2)), __saturatef(VOX_FSUB(fabsf(c2.y), h2)));
+        const F2 D = f2_fma(x2, x2, f2_fma(x1, x1, f2_fma(x0, x0, zero)));
+        const float2 dl = f2_get(f2_add(D, nlo)), dh = f2_get(f2_fma(D, m1, hi2));
+        pass = __funnelshift_l(__float_as_uint(dl.y), pass, 1);
+        pass = __funnelshift_l(__float_as_uint(dl.x), pass, 1);
+        fail = __funnelshift_l(__float_as_uint(dh.y), fail, 1);
+        fail = __funnelshift_l(__float_as_uint(dh.x), fail, 1);
+        K = f2_add(K, m2);
+    }
+    const uint32_t valid = (1u << nz) - 1u;
+    unsure = ~(pass | fail) & valid;
+    return pass & valid;
+}
+
 // The forward walk's test: the boxes of a chunk, one box column per lane; the
 // passing (Gaussian, voxel) pairs are appended to queue (entry j << 9 | leaf_n)
 // and their voxels set in mask (the leaf's value mask as 32-bit words).  The
@@ -502,35 +529,8 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
             const uint32_t dx = (local * __float_as_uint(q4.x)) >> 16;
             const uint32_t dy = local - dx * ny;
             ebase = __float_as_uint(q4.z) + (dx << 6) + (dy << 3);
-            const float fx = (float)dx, fy = (float)dy;
-            const float b0 = VOX_FFMA(fy, q2.x, VOX_FFMA(fx, q1.x, q0.x)), b1 = VOX_FFMA(fy, q2.y, VOX_FFMA(fx, q1.y, q0.y)),
-                        b2 = VOX_FFMA(fy, q2.z, VOX_FFMA(fx, q1.z, q0.z));
-            const F2 B0 = f2(b0, b0), B1 = f2(b1, b1), B2 = f2(b2, b2);
-            const F2 S0 = f2(q3.x, q3.x), S1 = f2(q3.y, q3.y), S2 = f2(q3.z, q3.z);
-            const F2 nlo = f2(-q0.w, -q0.w), hi2 = f2(q1.w, q1.w), m1 = f2(-1.f, -1.f), m2 = f2(-2.f, -2.f),
-                     zero = f2(0.f, 0.f);
-            const float h0 = q2.w, h1 = q3.w, h2 = q4.w;
-            const uint32_t steps = (nz + 1u) >> 1; // voxels (2 k - 2, 2 k - 1) for k = steps .. 1
-            const float ft = (float)(2u * steps);
-            F2 K = f2(ft - 2.f, ft - 1.f);
-            uint32_t pass = 0, fail = 0;
-#pragma unroll 1
-            for (uint32_t k = steps; k; k--)
-            {
-                const float2 c0 = f2_get(f2_fma(K, S0, B0)), c1 = f2_get(f2_fma(K, S1, B1)), c2 = f2_get(f2_fma(K, S2, B2));
-                const F2 x0 = f2(__saturatef(VOX_FSUB(fabsf(c0.x), h0)), __saturatef(VOX_FSUB(fabsf(c0.y), h0)));
-                const F2 x1 = f2(__saturatef(VOX_FSUB(fabsf(c1.x), h1)), __saturatef(VOX_FSUB(fabsf(c1.y), h1)));
-                const F2 x2 = f2(__saturatef(VOX_FSUB(fabsf(c2.x), h2)), __saturatef(VOX_FSUB(fabsf(c2.y), h2)));
-                const F2 D = f2_fma(x2, x2, f2_fma(x1, x1, f2_fma(x0, x0, zero)));
-                const float2 dl = f2_get(f2_add(D, nlo)), dh = f2_get(f2_fma(D, m1, hi2));
-                pass = __funnelshift_l(__float_as_uint(dl.y), pass, 1);
-                pass = __funnelshift_l(__float_as_uint(dl.x), pass, 1);
-                fail = __funnelshift_l(__float_as_uint(dh.y), fail, 1);
-                fail = __funnelshift_l(__float_as_uint(dh.x), fail, 1);
-                K = f2_add(K, m2);
-            }
-            const uint32_t valid = (1u << nz) - 1u;
-            zmask = pass & valid;
+            uint32_t unsure;
+            zmask = column_test(q0, q1, q2, q3, q4.w, (float)dx, (float)dy, nz, unsure);
             // the reference test of one voxel, from the record (nothing of the column kept live)
             auto exact_voxel = [&](uint32_t k) -> uint32_t {
                 const GaussRec R = P.recs[C.gid[j]];
@@ -539,7 +539,7 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
                                                 o[1] + (int32_t)((n >> 3) & 7u), o[2] + (int32_t)(n & 7u));
                 return aabb_hits_unit_sphere(b) ? 1u << k : 0u;
             };
-            for (uint32_t m = ~(pass | fail) & valid; m; m &= m - 1u)
+            for (uint32_t m = unsure; m; m &= m - 1u)
                 zmask |= exact_voxel((uint32_t)(__ffs(m) - 1));
             if (CHECK)
             {
@@ -574,116 +574,6 @@ __device__ __forceinline__ void leaf_test_columns(const LeafPassParams& P, const
             if (zmask & (1u << k))
                 *dst++ = (uint16_t)(ebase + k);
     }
-}
-
-// The adjoint walk's test, the reference's own on every voxel: one box column
-// per thread, the passing (Gaussian, voxel) pairs appended to queue (entry j <<
-// 9 | leaf_n), warp w to its own region queue[w * 512, ...) at warp-local
-// positions, its count in qcount[w] - a deterministic order (a warp tests at
-// most 2 x 32 columns of 8 voxels).
-// Bit-identical to voxel_local_aabb + aabb_hits_unit_sphere per voxel: the z
-// corner c1 of voxel z is c0 of voxel z + 1 (integer-valued floats), and "lo >
-// 0: subtract lo^2, else hi < 0: subtract hi^2" selects the pre-scale bound
-// with the same sign (inv_ls, inv_s > 0; an underflow to zero subtracts zero).
-// Every thread of the CTA calls it (warp-synchronous queue slots).
-template <class Chunk>
-__device__ __forceinline__ void leaf_test_chunk(const Chunk& C, uint32_t cnt, const int32_t o[3], uint16_t* queue,
-                                                uint32_t* qcount, int t, int lane)
-{
-    uint32_t wbase = 0; // entries this warp has written
-    queue += (t >> 5) * (LQ_CHUNK * 64);
-    uint32_t start[LQ_CHUNK + 1];
-    start[0] = 0;
-#pragma unroll
-    for (int j = 0; j < LQ_CHUNK; j++)
-        start[j + 1] = start[j] + (j < (int)cnt ? C.bcol[j] : 0u);
-    const uint32_t T = start[LQ_CHUNK];
-    for (uint32_t tu = (uint32_t)(t >> 5); tu * 32u < T; tu += LP_THREADS / 32)
-    {
-        const uint32_t e = tu * 32u + (uint32_t)lane;
-        uint32_t zmask = 0, ebase = 0;
-        if (e < T)
-        {
-            // j: the last box whose first column is <= e (empty boxes skipped); sj its first column
-            int j = 0;
-            uint32_t sj = 0;
-#pragma unroll
-            for (int q = 1; q < LQ_CHUNK; q++) // without a dynamically indexed (local memory) array
-            {
-                const bool ge = e >= start[q];
-                j += ge ? 1 : 0;
-                sj = ge ? start[q] : sj;
-            }
-            const uint32_t local = e - sj;
-            const uint32_t dx = (local * C.bdiv_y[j]) >> 16;
-            const uint32_t dy = local - dx * C.bny[j];
-            const int32_t rx = C.bx0[j] + (int32_t)dx, ry = C.by0[j] + (int32_t)dy, rz0 = C.bz0[j];
-            const GaussRec& R = C.rec[j].r;
-            const float vsf = C.vs[j];
-            const uint32_t nz = C.bnz[j];
-            const RInv M = rinv_of(R);
-            const float il = R.q0.w, pz = R.q0.z;
-            const float is[3] = { R.q3.y, R.q3.z, R.q3.w };
-            float cx0, cx1, cy0, cy1;
-            axis_corners(vsf, R.q0.x, o[0] + rx, cx0, cx1);
-            axis_corners(vsf, R.q0.y, o[1] + ry, cy0, cy1);
-            float slo[3], shi[3], pa[3];
-            float v = (float)(o[2] + rz0);
-            float cz = VOX_FSUB(VOX_FMUL(v, vsf), pz);
-#pragma unroll
-            for (int r = 0; r < 3; r++)
-            {
-                float xn, xx, yn, yx;
-                minmax_prod(cx0, cx1, M.m[r][0], xn, xx);
-                minmax_prod(cy0, cy1, M.m[r][1], yn, yx);
-                slo[r] = VOX_FADD(xn, yn);
-                shi[r] = VOX_FADD(xx, yx);
-                pa[r] = VOX_FMUL(cz, M.m[r][2]);
-            }
-            // the reference test along the z run
-#pragma unroll 2
-            for (uint32_t k = 0; k < nz; k++)
-            {
-                v = VOX_FADD(v, 1.f);
-                cz = VOX_FSUB(VOX_FMUL(v, vsf), pz);
-                float d2 = 1.f;
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-                {
-                    // the corner offsets grow with z: per row the smaller product is the
-                    // lower corner's when the matrix entry is >= 0 (fl(c m) is monotone
-                    // in c; a tie differs at most in the sign of a zero, which is squared)
-                    const float pb = VOX_FMUL(cz, M.m[r][2]);
-                    const bool up = M.m[r][2] >= 0.f;
-                    const float zn = up ? pa[r] : pb, zx = up ? pb : pa[r];
-                    pa[r] = pb;
-                    const float xl = VOX_FADD(slo[r], zn), xh = VOX_FADD(shi[r], zx);
-                    // xl <= xh: the bound of the row's interval nearest to zero, or zero
-                    const float xs = VOX_FADD(fmaxf(xl, 0.f), fminf(xh, 0.f));
-                    const float sv = VOX_FMUL(VOX_FMUL(xs, il), is[r]);
-                    d2 = VOX_FSUB(d2, VOX_FMUL(sv, sv));
-                }
-                zmask |= (d2 > 0.f ? 1u : 0u) << k;
-            }
-            ebase = ((uint32_t)j << 9) | (uint32_t)((rx << 6) | (ry << 3) | rz0);
-        }
-        // queue slots: warp inclusive scan of the pass counts
-        const uint32_t np = (uint32_t)__popc(zmask);
-        uint32_t incl = np;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1)
-        {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off)
-                incl += y;
-        }
-        uint32_t qb = wbase + incl - np;
-        wbase += __shfl_sync(0xffffffffu, incl, 31);
-        for (uint32_t m = zmask; m; m &= m - 1)
-            queue[qb++] = (uint16_t)(ebase + (uint32_t)(__ffs(m) - 1));
-    }
-    if (lane == 0)
-        qcount[t >> 5] = wbase;
 }
 
 // the part of a Gaussian's bbox inside the leaf at o, leaf-relative
@@ -750,18 +640,7 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-// the record of sorted leaf pair q into shared memory (asynchronous); returns its Gaussian id
-__device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, GaussRec* dst, uint32_t q)
-{
-    const uint32_t g = P.pair_gid[q];
-    const float4* src = reinterpret_cast<const float4*>(&P.recs[g]);
-#pragma unroll
-    for (int w = 0; w < 8; w++)
-        cp_async16(reinterpret_cast<float4*>(dst) + w, src + w);
-    return g;
-}
-
-// the same for the forward walk: record and walk constants into slot j
+// record and walk constants of sorted leaf pair q into slot j (asynchronous); returns its Gaussian id
 template <bool SMOOTH>
 __device__ __forceinline__ uint32_t leaf_stage_issue(const LeafPassParams& P, LeafStage& T, LeafChunk<SMOOTH>& C, int j,
                                                      uint32_t q)
@@ -798,8 +677,8 @@ __device__ __forceinline__ uint64_t frag_window(const LeafPassParams& P, uint32_
 }
 
 // once the record landed: the chunk's constants of Gaussian j, and its box's columns and voxels
-template <bool CHECK, bool WINDOW, class Chunk>
-__device__ __forceinline__ void leaf_stage_box(const LeafPassParams& P, const LeafStage& T, Chunk& C, int j, uint32_t q,
+template <bool CHECK, bool WINDOW, bool SMOOTH>
+__device__ __forceinline__ void leaf_stage_box(const LeafPassParams& P, const LeafStage& T, LeafChunk<SMOOTH>& C, int j, uint32_t q,
                                                uint32_t g, const int32_t o[3], uint32_t& cols, uint32_t& voxels)
 {
     GaussRec R;
@@ -830,6 +709,11 @@ __device__ __forceinline__ void leaf_stage_box(const LeafPassParams& P, const Le
     C.aa[j] = make_float4(16777216.f + (float)(2 * r0[0]), 16777216.f + (float)(2 * r0[1]), 16777216.f + (float)(2 * r0[2]),
                           w4.w);
     C.gid[j] = g;
+    if constexpr (SMOOTH)
+    {
+        C.vs[j] = w5.z;
+        C.exact_d[j] = w5.w != 0.f ? 1u : 0u;
+    }
     if (WINDOW)
     {
         // fragments are numbered x-major, so the box's lie between its two corners'
@@ -1027,10 +911,10 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         R.q3 = C.rec[3][j];
                         R.q6 = C.q6[j];
                         R.q7 = q7;
-                        const float vsf = P.cloud_vs ? P.walk[C.gid[j]].w5.z : P.voxel_size;
+                        const float mu[3] = { R.q0.x, R.q0.y, R.q0.z }, inv_s[3] = { R.q3.y, R.q3.z, R.q3.w };
                         SmoothTerms st;
-                        a = smooth_kernel(R, rinv_of(R), vsf, x, yy, zz, st);
-                        a8 = ref_alpha_byte(R, vsf, x, yy, zz) << 24;
+                        a = smooth_kernel(mu, inv_s, R.q6.x, rinv_of(R), C.vs[j], C.exact_d[j] != 0u, x, yy, zz, st);
+                        a8 = ref_alpha_byte(R, C.vs[j], x, yy, zz) << 24;
                     }
                     else
                     {
@@ -1247,279 +1131,233 @@ __device__ __forceinline__ uint32_t mask_rank(const uint64_t* m, uint32_t n)
     return r + __popcll(m[n >> 6] & ((1ull << (n & 63)) - 1ull));
 }
 
-// adjoint: per (leaf, Gaussian) pair, the sum of its voxel pairs' terms,
-// stored by the leaf pair's emission index.  The forward walk's pipeline: phase
-// p flushes the sums of chunk p - 2, runs the adjoint terms of chunk p - 1's
-// queued pairs, tests chunk p's columns (the same test) and stages chunk p + 1.
-// The queue has one region per warp at warp-local positions, so its order is
-// fixed; a pair's terms are summed per Gaussian across each warp (shuffles)
-// into that warp's slots, and the flush adds the warps' slots in warp order:
-// deterministic, no atomics.
-struct LeafBChunk
+// The adjoint: per (leaf, Gaussian) pair, the sums of its voxel pairs' terms
+// (vox_backward.cu), stored by the pair's emission index.  A warp takes 32
+// consecutive sorted pairs: their constants once, a pair per lane, then one after
+// the other - the forward's column test (the same pairs pass), the passing
+// voxels' terms a voxel per lane, and the BWD_NACC sums across the warp.  Every
+// sum has a fixed order (deterministic, no atomics), and no warp waits for
+// another.  Bound by instruction issue (79% of the slots): 0.78 ms for 200k
+// Gaussians (1.17M pairs, 33M voxel pairs).  A walk of whole leaves by CTAs, whose
+// warps mixed Gaussians and so summed 19 values per Gaussian and round, took 2.12.
+constexpr int BW_WARPS = 4;
+
+struct BwdWarp
 {
-    RecSlot rec[LQ_CHUNK]; // first member: 16-byte aligned for cp.async
-    int32_t bx0[LQ_CHUNK], by0[LQ_CHUNK], bz0[LQ_CHUNK];
-    uint32_t bny[LQ_CHUNK], bnz[LQ_CHUNK], bdiv_y[LQ_CHUNK], bcol[LQ_CHUNK];
-    float vs[LQ_CHUNK];
-    uint32_t eidx[LQ_CHUNK]; // emission index of each leaf pair
-    uint64_t mask[8];        // the leaf's value mask
-    uint64_t vbase;          // value index of the leaf's first voxel
+    // constants of the 32 pairs
+    float4 tc[32], tb[32], w0[32], w1[32], w2[32]; // the test's (LeafChunk)
+    float4 m0[32], m1[32], m2[32], m3[32];         // mu, opacity; rows of the inverse rotation, each with its 1 / s
+    float4 rgb[32];                                // colour, voxel size
+    uint32_t eidx[32], gid[32], cand[32];
+    uint32_t mask[16], before[16]; // the leaf's value mask and the voxels before each word
+    uint16_t queue[512];           // the pair's passing voxels
 };
 
-struct LeafGradSum
+// v[0 .. N) summed across the warp's lanes: at each step lanes that differ in one
+// bit of their number split the values, so N + N / 2 + ... shuffles do for N.
+// Afterwards lane l holds the sum of value k(l) in v[0]; returns k(l) (>= N: none).
+template <int N>
+__device__ __forceinline__ int warp_sum_split(float* v, int lane)
 {
-    float part[LP_THREADS / 32][LQ_CHUNK][BWD_NACC]; // per warp: a fixed set of rounds, summed in order
-    uint32_t eidx[LQ_CHUNK];
-    uint32_t cnt;
-};
-
-// a warp tests at most ceil(LQ_CHUNK * 64 / LP_THREADS) rounds of 32 columns of
-// up to 8 voxels; its queue region (LQ_CHUNK * 64 entries) must hold them all
-static_assert(((LQ_CHUNK * 64 + LP_THREADS - 1) / LP_THREADS) * 32 * 8 <= LQ_CHUNK * 64,
-              "per-warp queue regions too small for this chunk size");
-
-struct LeafBSmem
-{
-    LeafBChunk ch[3];
-    LeafGradSum gs[2];
-    uint16_t queue[2][LQ_CHUNK * 512]; // per warp regions of LQ_CHUNK * 64 entries
-    uint32_t wqn[2][LP_THREADS / 32];   // entries per warp region
-    int32_t nxt_o[2][3];
-    uint32_t nxt_q0[2], nxt_p1[2];
-    uint32_t cand_next[2];
-    uint32_t cand;
-};
-
-// stager js of the chunk at sorted pair q0 of candidate c (origin o): the leaf's
-// mask word js, and for js < cnt its record's box once the copy has landed
-__device__ __forceinline__ void leaf_bstage(const LeafPassParams& P, LeafBChunk& C, int js, uint32_t cnt, uint32_t q0,
-                                            int64_t c, const int32_t o[3])
-{
-    if (js < 8)
-        C.mask[js] = P.cand_mask[8 * (uint64_t)c + js];
-    if (js == 0)
-        C.vbase = P.cand_vbase[c];
-    if (js < (int)cnt)
+    int first = 0; // first value of this lane's share
+    int width = N;
+#pragma unroll
+    for (int bit = 16, n = N; bit; bit >>= 1)
     {
-        cp_async_wait_all();
-        const LeafBox b = leaf_box(C.rec[js].r, o);
-        C.bx0[js] = b.lo[0];
-        C.by0[js] = b.lo[1];
-        C.bz0[js] = b.lo[2];
-        C.bny[js] = b.ny;
-        C.bnz[js] = b.nz;
-        C.bdiv_y[js] = (65536u + b.ny - 1u) / b.ny;
-        C.bcol[js] = b.nx * b.ny;
-        C.vs[js] = rec_vs(C.rec[js].r, P.voxel_size, P.cloud_vs);
-        C.eidx[js] = P.vals[q0 + (uint32_t)js];
+        const int half = (n + 1) / 2;
+        const bool up = (lane & bit) != 0;
+#pragma unroll
+        for (int i = 0; i < half; i++)
+        {
+            const float hi = half + i < n ? v[half + i] : 0.f;
+            const float give = up ? v[i] : hi;
+            v[i] = (up ? hi : v[i]) + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+        first += up ? half : 0;
+        width = up ? width - half : min(width, half);
+        n = half;
     }
+    return width > 0 ? first : N;
 }
 
-__global__ void __launch_bounds__(LP_THREADS, 3) k_leaf_backward(LeafPassParams P, uint32_t* counter)
+__global__ void __launch_bounds__(BW_WARPS * 32) k_leaf_backward(LeafPassParams P, int64_t Q)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    LeafBSmem& S = *reinterpret_cast<LeafBSmem*>(smem_raw);
-    const int t = threadIdx.x, lane = t & 31;
-    const int js = t - LQ_STAGE_T0;
-    const bool stager = js >= 0 && js < LQ_CHUNK;
-    if (t == 0)
-    {
-        S.cand = atomicAdd(counter, 1u);
-        S.cand_next[0] = atomicAdd(counter, 1u);
-    }
-    for (int i = t; i < (LP_THREADS / 32) * LQ_CHUNK * BWD_NACC; i += LP_THREADS)
-    {
-        (&S.gs[0].part[0][0][0])[i] = 0.f;
-        (&S.gs[1].part[0][0][0])[i] = 0.f;
-    }
-    __syncthreads();
-    int64_t tc = S.cand;
-    if (tc >= P.NCL)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    BwdWarp& S = reinterpret_cast<BwdWarp*>(smem_raw)[warp];
+    const int64_t base = ((int64_t)blockIdx.x * BW_WARPS + warp) * 32;
+    if (base >= Q)
         return;
-    int64_t cn = S.cand_next[0];
-    int32_t to[3];
-    cand_origin(P, P.cand_key[tc], to);
-    uint32_t tq0 = P.cand_start[tc], tp1 = P.cand_start[tc + 1];
-    if (stager)
+    const int items = (int)min((int64_t)32, Q - base);
+    if (lane < items)
     {
-        const uint32_t cnt = min((uint32_t)LQ_CHUNK, tp1 - tq0);
-        if (js < (int)cnt)
-            leaf_stage_issue(P, &S.ch[0].rec[js].r, tq0 + (uint32_t)js);
-        leaf_bstage(P, S.ch[0], js, cnt, tq0, tc, to);
+        const uint32_t q = (uint32_t)(base + lane);
+        // its leaf: the last candidate whose first pair is <= q
+        int64_t lo = 0, hi = P.NCL;
+        while (lo < hi)
+        {
+            const int64_t mid = (lo + hi) >> 1;
+            if (P.cand_start[mid] <= q)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        const int4 o4 = P.cand_org[lo - 1];
+        const int32_t o[3] = { o4.x, o4.y, o4.z };
+        const uint32_t g = P.pair_gid[q];
+        const GaussRec R = P.recs[g];
+        const WalkRec W = P.walk[g];
+        const LeafBox b = leaf_box(R, o);
+        int32_t r0[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            r0[a] = anchor_of((&R.q4.x)[a], (&R.q5.x)[a], o[a]);
+        const float mu[3] = { R.q0.x, R.q0.y, R.q0.z };
+        const LeafConst K = leaf_consts(rinv_of(R), mu, W.w0, W.w1, W.w2, W.w4, W.w5.z, o, r0);
+        const float bx = (float)(b.lo[0] - r0[0]), by = (float)(b.lo[1] - r0[1]), bz = (float)(b.lo[2] - r0[2]);
+        float c[3];
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            c[r] = VOX_FFMA(bz, (&W.w2.x)[r], VOX_FFMA(by, (&W.w1.x)[r], VOX_FFMA(bx, (&W.w0.x)[r], K.c[r])));
+        S.tc[lane] = make_float4(c[0], c[1], c[2], W.w5.x);
+        S.tb[lane] = make_float4(__uint_as_float((65536u + b.ny - 1u) / b.ny),
+                                 __uint_as_float(b.ny | b.nz << 8 | (W.w5.w != 0.f ? 1u : 0u) << 16 | (b.nx * b.ny) << 17),
+                                 __uint_as_float((uint32_t)(b.lo[0] << 6 | b.lo[1] << 3 | b.lo[2])), W.w4.w);
+        S.w0[lane] = W.w0;
+        S.w1[lane] = W.w1;
+        S.w2[lane] = W.w2;
+        S.m0[lane] = make_float4(mu[0], mu[1], mu[2], R.q6.x);
+        S.m1[lane] = make_float4(R.q1.x, R.q1.y, R.q1.z, R.q3.y);
+        S.m2[lane] = make_float4(R.q1.w, R.q2.x, R.q2.y, R.q3.z);
+        S.m3[lane] = make_float4(R.q2.z, R.q2.w, R.q3.x, R.q3.w);
+        S.rgb[lane] = make_float4(R.q7.x, R.q7.y, R.q7.z, W.w5.z);
+        S.gid[lane] = g;
+        S.cand[lane] = (uint32_t)(lo - 1);
+        S.eidx[lane] = P.vals[q];
     }
-    __syncthreads();
-    bool t_valid = true, a_valid = false, f_valid = false;
-    uint32_t acnt = 0;
-    int32_t ao[3] = { 0, 0, 0 };
-    uint32_t p = 0;
-    while (t_valid || a_valid || f_valid)
+    __syncwarp();
+    uint32_t cur = ~0u;
+    uint64_t vbase = 0;
+    int32_t o[3] = { 0, 0, 0 };
+    for (int it = 0; it < items; it++)
     {
-        const int tb = (int)(p % 3u), ab = (int)((p + 2u) % 3u), nb = (int)((p + 1u) % 3u);
-        const bool t_end = t_valid && tq0 + LQ_CHUNK >= tp1;
-        const int64_t nc = t_end ? cn : tc;
-        const bool n_valid = t_valid && nc < P.NCL;
-        uint32_t nq0 = 0, np1 = 0, ncnt = 0;
-        if (stager && n_valid)
+        const uint32_t c = S.cand[it];
+        if (c != cur)
         {
-            nq0 = t_end ? P.cand_start[nc] : tq0 + LQ_CHUNK;
-            np1 = t_end ? P.cand_start[nc + 1] : tp1;
-            ncnt = min((uint32_t)LQ_CHUNK, np1 - nq0);
-            if (js < (int)ncnt)
-                leaf_stage_issue(P, &S.ch[nb].rec[js].r, nq0 + (uint32_t)js);
-        }
-        // ---- flush: chunk p - 2's sums to its leaf pairs' partials
-        if (f_valid)
-        {
-            LeafGradSum& Gs = S.gs[p & 1u];
-            const uint32_t n = Gs.cnt * BWD_NACC;
-            for (uint32_t i = (uint32_t)t; i < n; i += LP_THREADS)
+            cur = c;
+            const int4 o4 = P.cand_org[c];
+            o[0] = o4.x;
+            o[1] = o4.y;
+            o[2] = o4.z;
+            vbase = P.cand_vbase[c];
+            const uint32_t m = lane < 16 ? reinterpret_cast<const uint32_t*>(P.cand_mask + 8 * (uint64_t)c)[lane] : 0u;
+            uint32_t incl = __popc(m);
+#pragma unroll
+            for (int off = 1; off < 16; off <<= 1)
             {
-                const uint32_t j = i / BWD_NACC, k = i - j * BWD_NACC;
-                float v = 0.f;
-                for (int w = 0; w < LP_THREADS / 32; w++)
-                {
-                    v += Gs.part[w][j][k];
-                    Gs.part[w][j][k] = 0.f;
-                }
-                P.partials[(uint64_t)Gs.eidx[j] * BWD_NACC + k] = v;
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off)
+                    incl += y;
+            }
+            if (lane < 16)
+            {
+                S.mask[lane] = m;
+                S.before[lane] = incl - __popc(m);
             }
         }
-        // ---- adjoint terms of chunk p - 1's queued pairs
-        if (a_valid)
+        // ---- the pair's passing voxels
+        const float4 tb = S.tb[it];
+        const uint32_t ext = __float_as_uint(tb.y), ny = ext & 255u, nz = (ext >> 8) & 255u, cols = ext >> 17;
+        uint32_t qn = 0;
+        for (uint32_t e0 = 0; e0 < cols; e0 += 32)
         {
-            const LeafBChunk& C = S.ch[ab];
-            LeafGradSum& Gs = S.gs[(p + 1u) & 1u];
-            if (t < LQ_CHUNK)
-                Gs.eidx[t] = C.eidx[t];
-            if (t == 0)
-                Gs.cnt = acnt;
-            const uint16_t* queue = S.queue[(p + 1u) & 1u];
-            const uint32_t* wqn = S.wqn[(p + 1u) & 1u];
-            uint32_t wstart[LP_THREADS / 32 + 1];
-            wstart[0] = 0;
-#pragma unroll
-            for (int w = 0; w < LP_THREADS / 32; w++)
-                wstart[w + 1] = wstart[w] + wqn[w];
-            const uint32_t qn = wstart[LP_THREADS / 32];
-            const int warp = t >> 5;
-            for (uint32_t b0 = 0; b0 < qn; b0 += LP_THREADS)
+            const uint32_t e = e0 + (uint32_t)lane;
+            uint32_t zmask = 0, n0 = 0;
+            if (e < cols)
             {
-                const uint32_t e = b0 + (uint32_t)t;
-                int j = -1;
-                float cc[BWD_NACC];
-#pragma unroll
-                for (int k = 0; k < BWD_NACC; k++)
-                    cc[k] = 0.f;
-                if (e < qn)
+                const uint32_t dx = (e * __float_as_uint(tb.x)) >> 16, dy = e - dx * ny;
+                n0 = __float_as_uint(tb.z) + (dx << 6) + (dy << 3);
+                uint32_t unsure;
+                zmask = column_test(S.tc[it], S.w0[it], S.w1[it], S.w2[it], tb.w, (float)dx, (float)dy, nz, unsure);
+                for (uint32_t m = unsure; m; m &= m - 1u)
                 {
-                    // entry e of the concatenated warp regions
-                    uint32_t wr = 0, ws = 0;
-#pragma unroll
-                    for (int w = 1; w < LP_THREADS / 32; w++)
-                    {
-                        const bool ge = e >= wstart[w];
-                        wr = ge ? (uint32_t)w : wr;
-                        ws = ge ? wstart[w] : ws;
-                    }
-                    const uint32_t q = queue[wr * (LQ_CHUNK * 64) + (e - ws)];
-                    j = (int)(q >> 9);
-                    const uint32_t n = q & 511u;
-                    const GaussRec& R = C.rec[j].r;
-                    const RInv M = rinv_of(R);
-                    const float vsf = C.vs[j];
-                    const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7), zz = ao[2] + (int32_t)(n & 7);
-                    SmoothTerms st;
-                    const float Kw = smooth_kernel(R, M, vsf, x, yy, zz, st);
-                    if (st.e > SMOOTH_TAU)
-                    {
-                        const uint64_t vi = C.vbase + mask_rank(C.mask, n);
-                        const float gd = P.grad_density ? P.grad_density[vi] : 0.f;
-                        float gc[3] = { 0.f, 0.f, 0.f };
-                        if (P.grad_color)
-                            for (int k = 0; k < 3; k++)
-                                gc[k] = P.grad_color[3 * vi + k];
-                        const float GK = gd + gc[0] * R.q7.x + gc[1] * R.q7.y + gc[2] * R.q7.z;
-                        cc[0] = GK * st.E;
-#pragma unroll
-                        for (int r = 0; r < 3; r++)
-                        {
-                            const float dzr = -GK * st.e * st.z[r];
-                            const float du = dzr * (r == 0 ? R.q3.y : (r == 1 ? R.q3.z : R.q3.w));
-                            cc[1 + r] = du;
-                            cc[4 + r] = dzr * st.z[r];
-#pragma unroll
-                            for (int a = 0; a < 3; a++)
-                                cc[7 + 3 * r + a] = du * st.d[a];
-                        }
-                        cc[16] = Kw * gc[0];
-                        cc[17] = Kw * gc[1];
-                        cc[18] = Kw * gc[2];
-                    }
-                }
-                // per Gaussian present in this warp: its terms summed across the warp
-                // (fixed shuffle tree) into this warp's slots
-                uint32_t todo = __ballot_sync(0xffffffffu, j >= 0);
-                while (todo)
-                {
-                    const int jx = __shfl_sync(0xffffffffu, j, __ffs(todo) - 1);
-                    const bool mine = j == jx;
-#pragma unroll
-                    for (int k = 0; k < BWD_NACC; k++)
-                    {
-                        float v = mine ? cc[k] : 0.f;
-#pragma unroll
-                        for (int off = 16; off; off >>= 1)
-                            v += __shfl_xor_sync(0xffffffffu, v, off);
-                        if (lane == 0)
-                            Gs.part[warp][jx][k] += v;
-                    }
-                    todo &= ~__ballot_sync(0xffffffffu, mine);
+                    const uint32_t k = (uint32_t)(__ffs(m) - 1), n = n0 + k;
+                    const GaussRec R = P.recs[S.gid[it]];
+                    const Aabb b = voxel_local_aabb(R, rinv_of(R), S.rgb[it].w, o[0] + (int32_t)(n >> 6),
+                                                    o[1] + (int32_t)((n >> 3) & 7u), o[2] + (int32_t)(n & 7u));
+                    zmask |= aabb_hits_unit_sphere(b) ? 1u << k : 0u;
                 }
             }
-        }
-        // ---- test of chunk p
-        if (t_valid)
-            leaf_test_chunk(S.ch[tb], min((uint32_t)LQ_CHUNK, tp1 - tq0), to, S.queue[p & 1u], S.wqn[p & 1u], t, lane);
-        // ---- stagers: chunk p + 1's mask words and boxes
-        if (stager && n_valid)
-        {
-            int32_t no[3] = { to[0], to[1], to[2] };
-            if (t_end)
-                cand_origin(P, P.cand_key[nc], no);
-            leaf_bstage(P, S.ch[nb], js, ncnt, nq0, nc, no);
-            if (js == 0)
+            const uint32_t np = (uint32_t)__popc(zmask);
+            uint32_t incl = np;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1)
             {
-                const int pp = (int)(p & 1u);
-                S.nxt_o[pp][0] = no[0];
-                S.nxt_o[pp][1] = no[1];
-                S.nxt_o[pp][2] = no[2];
-                S.nxt_q0[pp] = nq0;
-                S.nxt_p1[pp] = np1;
-                if (t_end)
-                    S.cand_next[pp] = atomicAdd(counter, 1u);
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= off)
+                    incl += y;
+            }
+            uint16_t* dst = S.queue + qn + incl - np;
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++)
+                if (zmask & (1u << k))
+                    *dst++ = (uint16_t)(n0 + k);
+            qn += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        __syncwarp();
+        // ---- their terms
+        float acc[BWD_NACC];
+#pragma unroll
+        for (int k = 0; k < BWD_NACC; k++)
+            acc[k] = 0.f;
+        for (uint32_t p = (uint32_t)lane; p < qn; p += 32)
+        {
+            const uint32_t n = S.queue[p];
+            const float4 m0 = S.m0[it], m1 = S.m1[it], m2 = S.m2[it], m3 = S.m3[it], col = S.rgb[it];
+            const float mu[3] = { m0.x, m0.y, m0.z }, inv_s[3] = { m1.w, m2.w, m3.w };
+            RInv M;
+            M.m[0][0] = m1.x;
+            M.m[0][1] = m1.y;
+            M.m[0][2] = m1.z;
+            M.m[1][0] = m2.x;
+            M.m[1][1] = m2.y;
+            M.m[1][2] = m2.z;
+            M.m[2][0] = m3.x;
+            M.m[2][1] = m3.y;
+            M.m[2][2] = m3.z;
+            SmoothTerms st;
+            const float Kw = smooth_kernel(mu, inv_s, m0.w, M, col.w, (ext >> 16) & 1u, o[0] + (int32_t)(n >> 6),
+                                           o[1] + (int32_t)((n >> 3) & 7), o[2] + (int32_t)(n & 7), st);
+            if (st.e > SMOOTH_TAU)
+            {
+                const uint64_t vi = vbase + S.before[n >> 5] + __popc(S.mask[n >> 5] & ((1u << (n & 31u)) - 1u));
+                const float gd = P.grad_density ? P.grad_density[vi] : 0.f;
+                float gc[3] = { 0.f, 0.f, 0.f };
+                if (P.grad_color)
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        gc[k] = P.grad_color[3 * vi + k];
+                const float f = -(gd + gc[0] * col.x + gc[1] * col.y + gc[2] * col.z) * st.e;
+                const float f0 = f * st.z[0], f1 = f * st.z[1], f2 = f * st.z[2];
+                acc[0] += f;
+                acc[1] += f0;
+                acc[2] += f1;
+                acc[3] += f2;
+                acc[4] += f0 * st.z[0];
+                acc[5] += f1 * st.z[1];
+                acc[6] += f2 * st.z[2];
+                acc[7] += f0 * st.z[1];
+                acc[8] += f0 * st.z[2];
+                acc[9] += f1 * st.z[2];
+                acc[10] += Kw * gc[0];
+                acc[11] += Kw * gc[1];
+                acc[12] += Kw * gc[2];
             }
         }
-        __syncthreads();
-        f_valid = a_valid;
-        a_valid = t_valid;
-        acnt = t_valid ? min((uint32_t)LQ_CHUNK, tp1 - tq0) : 0u;
-        ao[0] = to[0];
-        ao[1] = to[1];
-        ao[2] = to[2];
-        if (n_valid)
-        {
-            const int pp = (int)(p & 1u);
-            if (t_end)
-                cn = S.cand_next[pp];
-            tc = nc;
-            tq0 = S.nxt_q0[pp];
-            tp1 = S.nxt_p1[pp];
-            to[0] = S.nxt_o[pp][0];
-            to[1] = S.nxt_o[pp][1];
-            to[2] = S.nxt_o[pp][2];
-        }
-        t_valid = n_valid;
-        p++;
+        const int k = warp_sum_split<BWD_NACC>(acc, lane);
+        if (k < BWD_NACC)
+            P.partials[(uint64_t)S.eidx[it] * BWD_STRIDE + k] = acc[0];
+        __syncwarp(); // the queue and the leaf's mask are filled again
     }
 }
 
@@ -1859,19 +1697,14 @@ int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cu
                     : launch_walk<false, false, false, 4>(P, counter, num_sms, s);
 }
 
-void launch_leaf_backward(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s)
+void launch_leaf_backward(const LeafPassParams& P, int64_t Q, cudaStream_t s)
 {
-    if (P.NCL <= 0)
+    if (Q <= 0)
         return;
-    cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    const size_t smem = sizeof(LeafBSmem);
+    const size_t smem = sizeof(BwdWarp) * BW_WARPS;
     cudaFuncSetAttribute(k_leaf_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_leaf_backward, LP_THREADS, smem);
-    int64_t grid = (int64_t)num_sms * (per_sm > 0 ? per_sm : 1);
-    if (grid > P.NCL)
-        grid = P.NCL;
-    { k_leaf_backward<<<(unsigned)grid, LP_THREADS, smem, s>>>(P, counter); count_launch(); }
+    const int64_t per = 32 * BW_WARPS;
+    { k_leaf_backward<<<(unsigned)((Q + per - 1) / per), BW_WARPS * 32, smem, s>>>(P, Q); count_launch(); }
 }
 
 void launch_leaf_export(const LeafPassParams& P, uint64_t* vpairs, uint32_t* counter, int num_sms, cudaStream_t s)

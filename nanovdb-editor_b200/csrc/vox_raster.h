@@ -79,8 +79,10 @@ struct NodeParams
     uint64_t *leaf_idx, *leaf_addr, *leaf_vidx;
 };
 
-// per-Gaussian adjoint sums: [0] dL/d op, [1..3] U, [4..6] W, [7..15] Q[r][a], [16..18] dL/d rgb
-constexpr int BWD_NACC = 19;
+// adjoint sums of a (leaf, Gaussian) pair (vox_backward.cu): [0] f, [1..3] f z_r, [4..6] f z_r^2,
+// [7..9] f z_0 z_1, f z_0 z_2, f z_1 z_2, [10..12] dL/d rgb, in rows of BWD_STRIDE floats
+constexpr int BWD_NACC = 13;
+constexpr int BWD_STRIDE = 16;
 
 struct BwdFinalParams
 {
@@ -150,7 +152,7 @@ struct LeafPassParams
     const uint64_t* cand_vbase; // [NCL] value index of each candidate's first voxel
     const float* grad_density;
     const float* grad_color;
-    float* partials;            // [emission index][BWD_NACC]
+    float* partials;            // [emission index][BWD_STRIDE]
     // reference node order: creation window of each candidate leaf
     int window;
     const uint64_t* frag_off;   // exclusive scan of footprints
@@ -175,7 +177,7 @@ void launch_leaf_compact(const uint32_t* keys, const uint32_t* vals, const uint3
 // variant 0: 4 resident CTAs per SM (64 registers per thread), 1: 3 CTAs per SM;
 // returns the CTAs per SM it ran with
 int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant = 0);
-void launch_leaf_backward(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s);
+void launch_leaf_backward(const LeafPassParams& P, int64_t Q, cudaStream_t s);
 // vpairs non-null: only the pairs per voxel (canonical order), into it
 void launch_leaf_export(const LeafPassParams& P, uint64_t* vpairs, uint32_t* counter, int num_sms, cudaStream_t s);
 
