@@ -296,7 +296,7 @@ __device__ __forceinline__ void stage_chunk(const LeafPassParams& P, LeafSmem& S
 // ------------------------------------------------------ forward leaf walk
 // A CTA walks a stream of candidate leaves in chunks of Gaussians (a leaf's
 // Gaussians in ascending id): as many of the next LF_CHUNK as have boxes of
-// LF_CAP voxels together, since every voxel may pass and take a queue entry.
+// lf_cap voxels together, since every voxel may pass and take a queue entry.
 // Per chunk:
 //   test   the part of each Gaussian's bbox inside the leaf, one (Gaussian,
 //          column) per thread: the column's x / y share once, then its z run;
@@ -316,7 +316,10 @@ __device__ __forceinline__ void stage_chunk(const LeafPassParams& P, LeafSmem& S
 // bound it.  Against chunks of 12 Gaussians (with their whole records in each
 // buffer), the walk of 200k Gaussians 3.52 -> 3.05 ms, a call on 2M 37.1 -> 32.5.
 constexpr int LF_CHUNK = 24;
-constexpr uint32_t LF_CAP = 5120;
+// the differentiable walk's chunks carry more per Gaussian and take fewer voxels
+// to fit 4 CTAs as well (5120 and 3 CTAs: 2.37 instead of 2.27 ms for 500k Gaussians)
+template <bool SMOOTH>
+constexpr uint32_t lf_cap = SMOOTH ? 3840 : 5120;
 
 // what the stagers read of the next chunk, each its own column (overwritten by
 // its own next copies)
@@ -373,7 +376,7 @@ struct LeafQSmem
     LeafChunk<SMOOTH> ch[3];
     LeafAcc acc;
     uint32_t mask[3][16]; // value masks of the leaf being tested and of the two before it
-    uint16_t queue[2][LF_CAP];
+    uint16_t queue[2][lf_cap<SMOOTH>];
     uint32_t defer[LP_THREADS / 32][64]; // per warp: the leaf's pairs whose RGBA8 byte the bound left open
     uint32_t dcount[LP_THREADS / 32];     // per warp: the open pairs left at the leaf's end
     uint32_t dfin;                        // warps done with the leaf's alpha
@@ -384,7 +387,7 @@ struct LeafQSmem
     uint32_t cand;
 };
 
-static_assert(sizeof(LeafQSmem<false>) <= 56 * 1024, "four CTAs of the leaf walk fit an SM's 228 KB (1 KB of it reserved per CTA)");
+static_assert(sizeof(LeafQSmem<false>) <= 56 * 1024 && sizeof(LeafQSmem<true>) <= 56 * 1024, "four CTAs of the leaf walk fit an SM's 228 KB (1 KB of it reserved per CTA)");
 
 // One term of an exact fixed-point sum, (hi, lo) += (xh, xl) with the carry from
 // the low word's old value: the total is the same integer in any order.  A
@@ -599,10 +602,10 @@ __device__ __forceinline__ LeafBox leaf_box(const GaussRec& R, const int32_t o[3
 }
 
 // the last warp, each lane with its own box's columns and voxels (0 past the
-// Gaussians at hand): the chunk takes the first boxes of LF_CAP voxels together;
+// Gaussians at hand): the chunk takes the first boxes of lf_cap voxels together;
 // its column prefix, and how many Gaussians it has
-template <class Chunk>
-__device__ __forceinline__ uint32_t leaf_stage_prefix(Chunk& C, int lane, uint32_t avail, uint32_t cols, uint32_t voxels)
+template <bool SMOOTH>
+__device__ __forceinline__ uint32_t leaf_stage_prefix(LeafChunk<SMOOTH>& C, int lane, uint32_t avail, uint32_t cols, uint32_t voxels)
 {
     uint32_t v = voxels;
 #pragma unroll
@@ -612,7 +615,7 @@ __device__ __forceinline__ uint32_t leaf_stage_prefix(Chunk& C, int lane, uint32
         if (lane >= off)
             v += y;
     }
-    const uint32_t cnt = (uint32_t)__popc(__ballot_sync(0xffffffffu, (uint32_t)lane < avail && v <= LF_CAP));
+    const uint32_t cnt = (uint32_t)__popc(__ballot_sync(0xffffffffu, (uint32_t)lane < avail && v <= lf_cap<SMOOTH>));
     const uint32_t mine = (uint32_t)lane < cnt ? cols : 0u;
     uint32_t c = mine;
 #pragma unroll
@@ -1682,11 +1685,11 @@ int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cu
     if (P.NCL <= 0)
         return 0;
     cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    if (P.smooth) // its chunks carry record words: 3 CTAs per SM either way
-        return P.emit_flag ? (P.window ? launch_walk<true, true, true, 3>(P, counter, num_sms, s)
-                                       : launch_walk<true, false, true, 3>(P, counter, num_sms, s))
-                           : (P.window ? launch_walk<false, true, true, 3>(P, counter, num_sms, s)
-                                       : launch_walk<false, false, true, 3>(P, counter, num_sms, s));
+    if (P.smooth)
+        return P.emit_flag ? (P.window ? launch_walk<true, true, true, 4>(P, counter, num_sms, s)
+                                       : launch_walk<true, false, true, 4>(P, counter, num_sms, s))
+                           : (P.window ? launch_walk<false, true, true, 4>(P, counter, num_sms, s)
+                                       : launch_walk<false, false, true, 4>(P, counter, num_sms, s));
     if (P.emit_flag)
         return P.window ? launch_walk<true, true, false, 4>(P, counter, num_sms, s)
                         : launch_walk<true, false, false, 4>(P, counter, num_sms, s);
