@@ -72,7 +72,7 @@ struct vox_context_t
     DevBuf lower_upper_n, lower_parent, upper_root_n, upper_lostart;
     DevBuf leaf_cand, leaf_lower, leaf_lower_n, leaf_origin;
     // leaf-granular pipeline
-    DevBuf cand_org, tile_g0, lcols, lcol_off, lc_count, lc_mask, lc_off, emit_gid, emit_flag, lflags, lpos, cand_key, cand_start, cand_mask, pair_gid;
+    DevBuf cand_org, tile_g0, lcols, lcol_off, lc_count, lc_mask, lc_off, emit_gid, emit_flag, cand_key, cand_start, cand_mask, pair_gid;
     DevBuf s_rgba, s_dens, s_col, cand_pairs, cand_voff, vpairs, pair_off, cand_vbase, cloud_pairs;
     DevBuf partials, exp_keys, exp_ids;
     // reference node order
@@ -561,6 +561,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     if (rc)
         return rc;
     const uint64_t Q = ctx->hscal[SC_Q];
+    const bool by_emission = diff || ctx->check_emit; // the sort's values are emission indices
     if (Q >= 0xFFFFFFF0ull)
     {
         set_error(ctx, "voxelize: %llu (leaf, Gaussian) pairs exceed the 32-bit pair index range", (unsigned long long)Q);
@@ -568,20 +569,17 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     }
     if (!ensure(ctx, ctx->keys, 4 * (size_t)(Q + 1)) || !ensure(ctx, ctx->ids, 4 * (size_t)(Q + 1)) ||
         !ensure(ctx, ctx->keys_alt, 4 * (size_t)(Q + 1)) || !ensure(ctx, ctx->ids_alt, 4 * (size_t)(Q + 1)) ||
-        !ensure(ctx, ctx->emit_gid, 4 * (size_t)(Q + 1)) || !ensure(ctx, ctx->pair_gid, 4 * (size_t)(Q + 1)) ||
+        (by_emission && (!ensure(ctx, ctx->emit_gid, 4 * (size_t)(Q + 1)) || !ensure(ctx, ctx->pair_gid, 4 * (size_t)(Q + 1)))) ||
         (ctx->check_emit && !ensure(ctx, ctx->emit_flag, (size_t)(Q + 1))) ||
-        !ensure(ctx, ctx->sort_ws, sort_workspace_bytes((int64_t)Q, 4)) || !ensure(ctx, ctx->lflags, 8 * (size_t)(Q + 1)) ||
-        !ensure(ctx, ctx->lpos, 8 * (size_t)(Q + 1)) || !ensure(ctx, ctx->cand_key, 4 * (size_t)(Q + 1)) ||
+        !ensure(ctx, ctx->sort_ws, sort_workspace_bytes((int64_t)Q, 4)) || !ensure(ctx, ctx->cand_key, 4 * (size_t)(Q + 1)) ||
         !ensure(ctx, ctx->cand_org, 16 * (size_t)(Q + 1)) ||
         !ensure(ctx, ctx->cand_start, 4 * (size_t)(Q + 2)) ||
-        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * scan_status_words((int64_t)Q + 1) * 2))
+        !ensure(ctx, ctx->run_status, sizeof(uint64_t) * (cand_status_words((int64_t)Q) + 16)))
         return VOX_ERR_MEMORY;
-    scan_status = (uint64_t*)ctx->scan_status.p;
-    scan_words = ctx->scan_status.cap / sizeof(uint64_t);
     LE.lc_off = lc_off;
     LE.keys = (uint32_t*)ctx->keys.p;
     LE.vals = (uint32_t*)ctx->ids.p;
-    LE.emit_gid = (uint32_t*)ctx->emit_gid.p;
+    LE.emit_gid = by_emission ? (uint32_t*)ctx->emit_gid.p : nullptr;
     LE.emit_flag = ctx->check_emit ? (uint8_t*)ctx->emit_flag.p : nullptr;
     launch_leaf_emit(LE, T, true, s);
     cudaEventRecord(ctx->timers.ev[2], s);
@@ -608,17 +606,20 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
             return VOX_ERR_CUDA;
         }
     }
-    uint64_t* lflags = (uint64_t*)ctx->lflags.p;
-    uint64_t* lpos = (uint64_t*)ctx->lpos.p;
-    launch_leaf_heads(lkeys, (int64_t)Q, lflags, s);
-    scan_exclusive_u64(lflags, lpos, (int64_t)Q, 0, sc + SC_NCL, scan_status,
-                       ctx->scan_epochs.next(scan_status, scan_words, s), d_counter, d_err, ctx->num_sms, s);
     if (Q == 0)
         cudaMemsetAsync(ctx->cand_start.p, 0, 4, s);
-    launch_leaf_compact(lkeys, lvals, (const uint32_t*)ctx->emit_gid.p, (int64_t)Q, lflags, lpos,
-                        (const uint32_t*)ctx->lower_cell.p, (const uint32_t*)ctx->root_of_rank.p,
-                        (uint32_t*)ctx->cand_key.p, (int4*)ctx->cand_org.p, (uint32_t*)ctx->cand_start.p,
-                        (uint32_t*)ctx->pair_gid.p, s);
+    CandParams CP;
+    CP.cand_key = (uint32_t*)ctx->cand_key.p;
+    CP.cand_org = (int4*)ctx->cand_org.p;
+    CP.cand_start = (uint32_t*)ctx->cand_start.p;
+    CP.pair_gid = (uint32_t*)ctx->pair_gid.p;
+    CP.total = sc + SC_NCL;
+    CP.status = (uint64_t*)ctx->run_status.p;
+    CP.epoch = ctx->run_epochs.next(CP.status, ctx->run_status.cap / sizeof(uint64_t), s);
+    CP.counter = d_counter;
+    CP.err = d_err;
+    launch_leaf_cands(lkeys, lvals, LE.emit_gid, (int64_t)Q, (const uint32_t*)ctx->lower_cell.p,
+                      (const uint32_t*)ctx->root_of_rank.p, CP, s);
     rc = sync_scalars(ctx, "candidate leaves");
     if (rc)
         return rc;
@@ -660,8 +661,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LP.recs = recs;
     LP.walk = walk;
     LP.vals = lvals;
-    LP.emit_gid = (const uint32_t*)ctx->emit_gid.p;
-    LP.pair_gid = (const uint32_t*)ctx->pair_gid.p;
+    LP.pair_gid = by_emission ? (const uint32_t*)ctx->pair_gid.p : lvals;
     LP.emit_flag = ctx->check_emit ? (const uint8_t*)ctx->emit_flag.p : nullptr;
     LP.cand_key = (const uint32_t*)ctx->cand_key.p;
     LP.cand_org = (const int4*)ctx->cand_org.p;
@@ -1015,7 +1015,7 @@ void vox_context_destroy(vox_context_t* ctx)
                       &ctx->leaf_lower_n, &ctx->leaf_origin, &ctx->order, &ctx->grid, &ctx->scal,
                       &ctx->hier_keys, &ctx->prim_keys_alt, &ctx->prim_vals_alt, &ctx->vb_work, &ctx->vb_keys, &ctx->vb_ids_c, &ctx->vb_used, &ctx->dual_idx, &ctx->vb_rec, &ctx->cloud_start,
                       &ctx->cloud_vs, &ctx->clouds, &ctx->lcols, &ctx->lcol_off, &ctx->lc_count, &ctx->lc_mask, &ctx->lc_off,
-                      &ctx->cand_org, &ctx->tile_g0, &ctx->emit_gid, &ctx->emit_flag, &ctx->lflags, &ctx->lpos, &ctx->cand_key, &ctx->cand_start,
+                      &ctx->cand_org, &ctx->tile_g0, &ctx->emit_gid, &ctx->emit_flag, &ctx->cand_key, &ctx->cand_start,
                       &ctx->cand_mask, &ctx->pair_gid, &ctx->s_rgba, &ctx->s_dens, &ctx->s_col, &ctx->cand_pairs,
                       &ctx->cand_voff, &ctx->vpairs, &ctx->pair_off, &ctx->cand_vbase, &ctx->cloud_pairs,
                       &ctx->partials, &ctx->exp_keys, &ctx->exp_ids, &ctx->nwin, &ctx->win_before,

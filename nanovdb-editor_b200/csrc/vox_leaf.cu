@@ -190,8 +190,11 @@ __global__ void __launch_bounds__(256) k_leaf_emit(LeafEmitParams P, RankTables 
                 if (WRITE)
                 {
                     P.keys[e] = leaf_key_of(R, ox, oy, oz, T.root_bits, T.root_prefix, T.lower_bits, T.lower_prefix);
-                    P.vals[e] = (uint32_t)e;
-                    P.emit_gid[e] = (uint32_t)g;
+                    // the sort's value: the Gaussian itself, or the emission index where
+                    // something is kept by it (the adjoint's rows, check mode's flags)
+                    P.vals[e] = P.emit_gid ? (uint32_t)e : (uint32_t)g;
+                    if (P.emit_gid)
+                        P.emit_gid[e] = (uint32_t)g;
                     if (P.check)
                         P.emit_flag[e] = hit ? 0 : 1;
                     e++;
@@ -209,13 +212,6 @@ __global__ void __launch_bounds__(256) k_leaf_emit(LeafEmitParams P, RankTables 
     }
 }
 
-__global__ void k_leaf_heads(const uint32_t* keys, int64_t Q, uint64_t* flags)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < Q)
-        flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1ull : 0ull;
-}
-
 // origin of the leaf with compact key lower_rank << 12 | lower_n
 __device__ __forceinline__ void leaf_origin_of_key(uint32_t key, const uint32_t* lower_cell,
                                                    const uint32_t* root_of_rank, int32_t o[3])
@@ -229,26 +225,88 @@ __device__ __forceinline__ void leaf_origin_of_key(uint32_t key, const uint32_t*
     o[2] += (int32_t)(un & 31) * 128 + (int32_t)(ln & 15) * 8;
 }
 
-// candidate leaves (key, origin, first pair) from the run heads; each sorted pair's Gaussian id
-__global__ void k_leaf_compact(const uint32_t* keys, const uint32_t* vals, const uint32_t* emit_gid, int64_t Q,
-                               const uint64_t* flags, const uint64_t* pos, const uint32_t* lower_cell,
-                               const uint32_t* root_of_rank, uint32_t* cand_key, int4* cand_org,
-                               uint32_t* cand_start, uint32_t* pair_gid)
+// Candidate leaves (key, origin, first pair) from the runs of the sorted keys,
+// and each sorted pair's Gaussian where the sort's values are emission indices
+// (emit_gid non-null): one pass, run heads against the key before (a shuffle
+// inside a warp), their count before the tile by look-back.  HBM-bound: 4 B per
+// pair (flags, their scan and a compaction pass moved 40).  Sort and candidates of
+// 29.6M pairs, with the sort carrying the Gaussians themselves: 1.65 -> 1.27 ms.
+constexpr int LC_BLOCK = 256;
+constexpr int LC_ITEMS = 8;
+constexpr int LC_TILE = LC_BLOCK * LC_ITEMS;
+
+__global__ void __launch_bounds__(LC_BLOCK) k_leaf_cands(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+                                                         const uint32_t* __restrict__ emit_gid, int64_t Q,
+                                                         const uint32_t* lower_cell, const uint32_t* root_of_rank,
+                                                         CandParams C)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Q)
-        return;
-    pair_gid[i] = emit_gid[vals[i]];
-    if (flags[i])
+    __shared__ uint32_t s_cnt[LC_BLOCK / 32];
+    __shared__ uint64_t s_ex;
+    __shared__ uint32_t s_tile;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0)
+        s_tile = atomicAdd(C.counter, 1u);
+    __syncthreads();
+    const uint64_t tile = s_tile;
+    const int64_t wbase = (int64_t)tile * LC_TILE + (int64_t)warp * (32 * LC_ITEMS);
+    uint32_t k[LC_ITEMS], heads[LC_ITEMS];
+    uint32_t carry = wbase > 0 && wbase - 1 < Q ? keys[wbase - 1] : 0u, count = 0;
+#pragma unroll
+    for (int i = 0; i < LC_ITEMS; i++)
     {
-        int32_t o[3];
-        leaf_origin_of_key(keys[i], lower_cell, root_of_rank, o);
-        cand_org[pos[i]] = make_int4(o[0], o[1], o[2], 0);
-        cand_key[pos[i]] = keys[i];
-        cand_start[pos[i]] = (uint32_t)i;
+        const int64_t q = wbase + i * 32 + lane;
+        k[i] = q < Q ? keys[q] : 0u;
+        if (emit_gid && q < Q)
+            C.pair_gid[q] = emit_gid[vals[q]];
     }
-    if (i == Q - 1)
-        cand_start[pos[i] + flags[i]] = (uint32_t)Q;
+#pragma unroll
+    for (int i = 0; i < LC_ITEMS; i++)
+    {
+        const int64_t q = wbase + i * 32 + lane;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, k[i], 1);
+        if (lane == 0)
+            prev = carry;
+        carry = __shfl_sync(0xffffffffu, k[i], 31);
+        heads[i] = __ballot_sync(0xffffffffu, q < Q && (q == 0 || k[i] != prev));
+        count += __popc(heads[i]);
+    }
+    if (lane == 0)
+        s_cnt[warp] = count;
+    __syncthreads();
+    if (warp == 0)
+    {
+        uint64_t agg = 0;
+        for (int w = 0; w < LC_BLOCK / 32; w++)
+            agg += s_cnt[w];
+        const uint64_t e = lookback_exclusive_warp(C.status, tile, agg, C.epoch, C.err);
+        if (lane == 0)
+            s_ex = e;
+    }
+    __syncthreads();
+    uint64_t at = s_ex;
+    for (int w = 0; w < warp; w++)
+        at += s_cnt[w];
+#pragma unroll
+    for (int i = 0; i < LC_ITEMS; i++)
+    {
+        const int64_t q = wbase + i * 32 + lane;
+        const bool head = (heads[i] >> lane) & 1u;
+        const uint64_t c = at + __popc(heads[i] & ((1u << lane) - 1u)); // candidates before this pair's own
+        if (head)
+        {
+            int32_t o[3];
+            leaf_origin_of_key(k[i], lower_cell, root_of_rank, o);
+            C.cand_org[c] = make_int4(o[0], o[1], o[2], 0);
+            C.cand_key[c] = k[i];
+            C.cand_start[c] = (uint32_t)q;
+        }
+        if (q == Q - 1)
+        {
+            C.cand_start[c + (head ? 1u : 0u)] = (uint32_t)Q;
+            *C.total = c + (head ? 1u : 0u);
+        }
+        at += __popc(heads[i]);
+    }
 }
 
 // ------------------------------------------------------------ leaf walk ----
@@ -256,10 +314,7 @@ struct LeafSmem
 {
     GaussRec rec[LP_CHUNK];
     uint32_t gid[LP_CHUNK];
-    uint32_t eidx[LP_CHUNK];
-    uint8_t flag[LP_CHUNK];
     uint64_t mask[8];
-    uint32_t pairs;
     uint32_t cand;
 };
 
@@ -281,15 +336,10 @@ __device__ __forceinline__ void stage_chunk(const LeafPassParams& P, LeafSmem& S
     if (t < (int)cnt * 8)
     {
         const uint32_t j = (uint32_t)t >> 3, w = (uint32_t)t & 7u;
-        const uint32_t e = P.vals[q0 + j];
-        const uint32_t g = P.emit_gid[e];
+        const uint32_t g = P.pair_gid[q0 + j];
         reinterpret_cast<float4*>(&S.rec[j])[w] = reinterpret_cast<const float4*>(&P.recs[g])[w];
         if (w == 0)
-        {
             S.gid[j] = g;
-            S.eidx[j] = e;
-            S.flag[j] = P.emit_flag ? P.emit_flag[e] : 0;
-        }
     }
 }
 
@@ -1642,21 +1692,18 @@ void launch_leaf_emit(const LeafEmitParams& P, const RankTables& T, bool write, 
         { k_leaf_emit<false><<<(unsigned)blocks, 256, 0, s>>>(P, T); count_launch(); }
 }
 
-void launch_leaf_heads(const uint32_t* keys, int64_t Q, uint64_t* flags, cudaStream_t s)
+size_t cand_status_words(int64_t Q)
 {
-    if (Q <= 0)
-        return;
-    { k_leaf_heads<<<(unsigned)((Q + 255) / 256), 256, 0, s>>>(keys, Q, flags); count_launch(); }
+    return 4 * (size_t)((Q + LC_TILE - 1) / LC_TILE);
 }
 
-void launch_leaf_compact(const uint32_t* keys, const uint32_t* vals, const uint32_t* emit_gid, int64_t Q,
-                         const uint64_t* flags, const uint64_t* pos, const uint32_t* lower_cell,
-                         const uint32_t* root_of_rank, uint32_t* cand_key, int4* cand_org, uint32_t* cand_start,
-                         uint32_t* pair_gid, cudaStream_t s)
+void launch_leaf_cands(const uint32_t* keys, const uint32_t* vals, const uint32_t* emit_gid, int64_t Q,
+                       const uint32_t* lower_cell, const uint32_t* root_of_rank, const CandParams& C, cudaStream_t s)
 {
     if (Q <= 0)
         return;
-    { k_leaf_compact<<<(unsigned)((Q + 255) / 256), 256, 0, s>>>(keys, vals, emit_gid, Q, flags, pos, lower_cell, root_of_rank, cand_key, cand_org, cand_start, pair_gid); count_launch(); }
+    cudaMemsetAsync(C.counter, 0, sizeof(uint32_t), s);
+    { k_leaf_cands<<<(unsigned)((Q + LC_TILE - 1) / LC_TILE), LC_BLOCK, 0, s>>>(keys, vals, emit_gid, Q, lower_cell, root_of_rank, C); count_launch(); }
 }
 
 static unsigned walk_grid(int64_t NCL, int num_sms)

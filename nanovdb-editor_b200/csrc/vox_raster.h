@@ -116,8 +116,8 @@ struct LeafEmitParams
                               // column's first 32 leaves (bit lz - lz0)
     const uint64_t* lc_off;   // write pass: exclusive scan of lc_count
     uint32_t* keys;           // leaf key: lower rank << 12 | lower_n
-    uint32_t* vals;           // emission index (the sort's value)
-    uint32_t* emit_gid;       // Gaussian of each emission index
+    uint32_t* vals;           // the sort's value: the Gaussian, or the emission index
+    uint32_t* emit_gid;       // Gaussian of each emission index (null: vals are Gaussians)
     uint8_t* emit_flag;       // check mode: 1 = the leaf test culls this pair
     float voxel_size;
     const float* cloud_vs;
@@ -128,8 +128,7 @@ struct LeafPassParams
 {
     const GaussRec* recs;
     const WalkRec* walk;
-    const uint32_t* vals;      // sorted leaf pairs' emission indices
-    const uint32_t* emit_gid;
+    const uint32_t* vals;      // sorted leaf pairs' emission indices (differentiable calls and check mode)
     const uint32_t* pair_gid;  // sorted leaf pairs' Gaussian ids
     const uint8_t* emit_flag;  // check mode or null
     const uint32_t* cand_key;  // [NCL] candidate leaf keys
@@ -169,11 +168,22 @@ struct LeafPassParams
 void launch_leaf_cols(const GaussRec* recs, int64_t G, uint64_t* lcols, cudaStream_t s);
 void launch_leaf_emit(const LeafEmitParams& P, const RankTables& T, bool write, cudaStream_t s);
 void launch_tile_gauss(const uint64_t* lcol_off, int64_t G, uint64_t NLC, int64_t* tile_g0, cudaStream_t s);
-void launch_leaf_heads(const uint32_t* keys, int64_t Q, uint64_t* flags, cudaStream_t s);
-void launch_leaf_compact(const uint32_t* keys, const uint32_t* vals, const uint32_t* emit_gid, int64_t Q,
-                         const uint64_t* flags, const uint64_t* pos, const uint32_t* lower_cell,
-                         const uint32_t* root_of_rank, uint32_t* cand_key, int4* cand_org, uint32_t* cand_start,
-                         uint32_t* pair_gid, cudaStream_t s);
+// candidate leaves from the sorted pairs (k_leaf_cands)
+struct CandParams
+{
+    uint32_t* cand_key;
+    int4* cand_org;
+    uint32_t* cand_start; // [candidates + 1]
+    uint32_t* pair_gid;   // Gaussian of each sorted pair (written where the values are emission indices)
+    uint64_t* total;
+    uint64_t* status;     // cand_status_words(Q)
+    uint32_t epoch;
+    uint32_t* counter;
+    int* err;
+};
+size_t cand_status_words(int64_t Q);
+void launch_leaf_cands(const uint32_t* keys, const uint32_t* vals, const uint32_t* emit_gid, int64_t Q,
+                       const uint32_t* lower_cell, const uint32_t* root_of_rank, const CandParams& C, cudaStream_t s);
 // variant 0: 4 resident CTAs per SM (64 registers per thread), 1: 3 CTAs per SM;
 // returns the CTAs per SM it ran with
 int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant = 0);
