@@ -9,6 +9,7 @@
 // counts) that size the buffers; buffers persist in the context and only
 // grow, so repeated calls allocate nothing.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -16,6 +17,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -88,7 +90,9 @@ struct vox_context_t
     DevBuf vb_keys, vb_ids_c, vb_used; // VoxelBVH ingestion: compressed sort keys (also the dual-key sort's keys)
     DevBuf dual_idx; // dual-key sort: original indices
     DevBuf vb_rec;   // VoxelBVH ingestion: per-Gaussian search records
-    uint64_t* hscal = nullptr; // pinned mirror
+    uint64_t* hscal = nullptr; // pinned, mapped mirror
+    uint64_t* hscal_dev = nullptr; // its device address
+    uint64_t publications = 0;     // of the scalars, by this context
     Epochs scan_epochs, run_epochs, sort_epochs;
     int check_sort = 0; // VOX_CHECK_SORT=1: validate key order after every sort
     int check_emit = 0; // VOX_CHECK_EMIT=1: also walk the leaves the leaf test culls; a pass there is an error
@@ -139,7 +143,19 @@ enum
     SC_VBU,  // VoxelBVH: used key slots
     SC_BBOX, // 3 words (6 int32)
     SC_COUNT = SC_BBOX + 3,
-    SC_SCRATCH = 24
+    // tile / queue counters of one call's kernels (u32 in the low half of a word
+    // each), zeroed with the scalars
+    SC_CTR = SC_COUNT,
+    CTR_FOOT = SC_CTR,
+    CTR_COLS,
+    CTR_ROOT,
+    CTR_LOWER,
+    CTR_PAIRS,
+    CTR_CANDS,
+    CTR_WALK,
+    CTR_TREE,
+    SC_CLEAR, // words cleared at the start of a call
+    SC_SCRATCH = 32
 };
 
 static void set_error(vox_context_t* ctx, const char* fmt, ...)
@@ -165,7 +181,7 @@ static void arm_wait(vox_context_t* ctx, uint64_t* sc, cudaStream_t s)
 // zeroes the per-call device scalars (counts, error word) and re-arms the wait control
 static void clear_scalars(vox_context_t* ctx, uint64_t* sc, cudaStream_t s)
 {
-    cudaMemsetAsync(sc, 0, sizeof(uint64_t) * SC_COUNT, s);
+    cudaMemsetAsync(sc, 0, sizeof(uint64_t) * SC_CLEAR, s);
     arm_wait(ctx, sc, s);
 }
 
@@ -203,12 +219,51 @@ static int check_cuda(vox_context_t* ctx, const char* where)
     return VOX_OK;
 }
 
+// The scalars of a call, copied by a kernel to page-locked host memory the host
+// can watch; the last word is the publication's number.
+__global__ void k_publish(const uint64_t* sc, volatile uint64_t* host, uint64_t number)
+{
+    if (threadIdx.x < SC_COUNT)
+        host[threadIdx.x] = sc[threadIdx.x];
+    __threadfence_system();
+    __syncwarp();
+    if (threadIdx.x == 0)
+        host[SC_COUNT] = number;
+}
+
 static int sync_scalars(vox_context_t* ctx, const char* where)
 {
-    cudaMemcpyAsync(ctx->hscal, ctx->scal.p, sizeof(uint64_t) * SC_COUNT, cudaMemcpyDeviceToHost, ctx->stream);
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    // A kernel's own write and the host's poll instead of a copy and a stream
+    // synchronisation: with 5 of these per call instead of 7 and fewer launches, a
+    // call of 32 Gaussians 404 -> 318 us.  The poll asks the stream now and then, so a
+    // failed launch or a device error ends it.
+    volatile uint64_t* h = ctx->hscal;
+    const uint64_t number = ++ctx->publications;
+    k_publish<<<1, 32, 0, ctx->stream>>>(((const uint64_t*)ctx->scal.p), ctx->hscal_dev, number);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    for (uint32_t spins = 1; e == cudaSuccess && h[SC_COUNT] != number; spins++)
+        if ((spins & 1023u) == 0)
+        {
+            e = cudaStreamQuery(ctx->stream);
+            if (e == cudaSuccess)
+            {
+                e = cudaStreamSynchronize(ctx->stream); // done: the word is there, or something is wrong
+                if (e == cudaSuccess && h[SC_COUNT] != number)
+                    e = cudaErrorUnknown;
+                break;
+            }
+            if (e == cudaErrorNotReady)
+            {
+                e = cudaSuccess;
+                if (spins >= 1u << 16)
+                    std::this_thread::yield(); // a long call: let other threads have the core
+            }
+        }
+    std::atomic_thread_fence(std::memory_order_acquire);
     if (e != cudaSuccess)
     {
+        cudaGetLastError();
         set_error(ctx, "CUDA error at %s: %s", where, cudaGetErrorString(e));
         return VOX_ERR_CUDA;
     }
@@ -402,7 +457,9 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         !ensure(ctx, ctx->footprints, sizeof(uint64_t) * (size_t)(G + 1)) ||
         !ensure(ctx, ctx->frag_off, sizeof(uint64_t) * (size_t)(G + 1)) ||
         !ensure(ctx, ctx->root_bits, sizeof(uint64_t) * 512 * B) || !ensure(ctx, ctx->root_prefix, sizeof(uint64_t) * 512 * B) ||
-        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * scan_status_words(G > 512 * B ? G : 512 * B) * 2))
+        !ensure(ctx, ctx->lcols, 8 * (size_t)(G + 1)) || !ensure(ctx, ctx->lcol_off, 8 * (size_t)(G + 1)) ||
+        !ensure(ctx, ctx->root_of_rank, sizeof(uint32_t) * 32768 * (size_t)B) || // every root tile of every cloud
+        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * (2 * scan_status_words(G) + scan_status_words(512 * B))))
         return VOX_ERR_MEMORY;
     const int64_t* d_cloud_start = nullptr;
     const float* d_cloud_vs = nullptr;
@@ -421,6 +478,8 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     uint64_t* frag_off = (uint64_t*)ctx->frag_off.p;
     uint64_t* root_bits = (uint64_t*)ctx->root_bits.p;
     uint64_t* root_prefix = (uint64_t*)ctx->root_prefix.p;
+    uint64_t* lcols = (uint64_t*)ctx->lcols.p;
+    uint64_t* lcol_off = (uint64_t*)ctx->lcol_off.p;
     cudaMemsetAsync(root_bits, 0, sizeof(uint64_t) * 512 * B, s);
     PrepParams P;
     P.means = gs->means;
@@ -455,7 +514,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
             cudaStreamWaitEvent(s, ctx->up_ev[1 + c], 0);
             P.g0 = g0;
             P.g1 = g1;
-            launch_prep(P, recs, walk, footprints, root_bits, d_err, s);
+            launch_prep(P, recs, walk, footprints, lcols, root_bits, d_err, s);
         }
     }
     else
@@ -464,82 +523,51 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
             for (int a = 0; a < 5; a++)
                 cudaMemcpyAsync(ctx->upload.dev[a], ctx->upload.host[a],
                                 (size_t)ctx->upload.width[a] * ctx->upload.es * (size_t)G, cudaMemcpyHostToDevice, s);
-        launch_prep(P, recs, walk, footprints, root_bits, d_err, s);
+        launch_prep(P, recs, walk, footprints, lcols, root_bits, d_err, s);
     }
     ctx->upload.active = false;
+    // fragments, leaf columns and touched root tiles (with their inverse) in one launch
     uint64_t* scan_status = (uint64_t*)ctx->scan_status.p;
     size_t scan_words = ctx->scan_status.cap / sizeof(uint64_t);
-    scan_exclusive_u64(footprints, frag_off, G, 0, sc + SC_F, scan_status, ctx->scan_epochs.next(scan_status, scan_words, s),
-                       d_counter, d_err, ctx->num_sms, s);
-    scan_exclusive_u64(root_bits, root_prefix, 512 * B, 1, sc + SC_NROOT, scan_status,
-                       ctx->scan_epochs.next(scan_status, scan_words, s), d_counter, d_err, ctx->num_sms, s);
+    auto ctr = [&](int slot) { return (uint32_t*)(sc + slot); };
+    {
+        uint64_t* st1 = scan_status + scan_status_words(G);
+        ScanJobs J;
+        J.count = 3;
+        J.job[0] = { footprints, frag_off, G, 0, sc + SC_F, scan_status, ctr(CTR_FOOT), nullptr, 0 };
+        J.job[1] = { lcols, lcol_off, G, 0, sc + SC_NLC, st1, ctr(CTR_COLS), nullptr, 0 };
+        J.job[2] = { root_bits, root_prefix, 512 * B, 1, sc + SC_NROOT, st1 + scan_status_words(G), ctr(CTR_ROOT),
+                     (uint32_t*)ctx->root_of_rank.p, 0 };
+        scan_jobs(J, ctx->scan_epochs.next(scan_status, scan_words, s), d_err, s);
+    }
     int rc = sync_scalars(ctx, "prep");
     if (rc)
         return rc;
     const uint64_t F = ctx->hscal[SC_F];
     const uint64_t NR = ctx->hscal[SC_NROOT];
-    if (!ensure(ctx, ctx->root_of_rank, sizeof(uint32_t) * (NR + 1)))
-        return VOX_ERR_MEMORY;
-    launch_invert_bits(root_bits, root_prefix, 512 * B, (uint32_t*)ctx->root_of_rank.p, s);
+    const uint64_t NLC = ctx->hscal[SC_NLC];
     ctx->stats.candidates = (int64_t)F;
     // one batch and at most one window: every node is created in window 0, and
     // the order by (window, parent rank, n) is the canonical one
     if (G <= REF_PRIM_BATCH && F <= REF_WINDOW)
         window = false;
 
-    // ------------------------------------------------------- lower ranks
+    // ------------------------------ lower ranks, leaf pairs per leaf column
     const int64_t lwords = (int64_t)(NR > 0 ? NR : 1) * 512;
     if (!ensure(ctx, ctx->lower_bits, sizeof(uint64_t) * lwords) ||
         !ensure(ctx, ctx->lower_prefix, sizeof(uint64_t) * lwords) ||
-        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * scan_status_words(lwords > G ? lwords : G) * 2))
+        !ensure(ctx, ctx->lc_count, 8 * (size_t)(NLC + 1)) || !ensure(ctx, ctx->lc_off, 8 * (size_t)(NLC + 1)) ||
+        !ensure(ctx, ctx->lc_mask, 4 * (size_t)(NLC + 1)) || !ensure(ctx, ctx->tile_g0, 8 * (size_t)(NLC / 256 + 2)) ||
+        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * (scan_status_words(lwords) + scan_status_words((int64_t)NLC + 1))))
         return VOX_ERR_MEMORY;
     scan_status = (uint64_t*)ctx->scan_status.p;
     scan_words = ctx->scan_status.cap / sizeof(uint64_t);
     uint64_t* lower_bits = (uint64_t*)ctx->lower_bits.p;
     uint64_t* lower_prefix = (uint64_t*)ctx->lower_prefix.p;
+    RankTables T{ root_bits, root_prefix, lower_bits, lower_prefix };
     cudaMemsetAsync(lower_bits, 0, sizeof(uint64_t) * lwords, s);
     launch_mark_lower(recs, G, root_bits, root_prefix, lower_bits, s);
-    scan_exclusive_u64(lower_bits, lower_prefix, lwords, 1, sc + SC_NLOWER, scan_status,
-                       ctx->scan_epochs.next(scan_status, scan_words, s), d_counter, d_err, ctx->num_sms, s);
-    rc = sync_scalars(ctx, "lower ranks");
-    if (rc)
-        return rc;
-    const uint64_t NL = ctx->hscal[SC_NLOWER];
-    if (!ensure(ctx, ctx->lower_cell, sizeof(uint32_t) * (NL + 1)))
-        return VOX_ERR_MEMORY;
-    launch_invert_bits(lower_bits, lower_prefix, lwords, (uint32_t*)ctx->lower_cell.p, s);
-    const int key_bits = 21 + bits_for(NL > 1 ? NL : 2);
-    const int key64 = key_bits > 32 ? 1 : 0;
-    ctx->key64 = key64;
-    ctx->stats.key_bits = key_bits;
     cudaEventRecord(ctx->timers.ev[1], s);
-
-    // ---------------------------------------------------------- leaf pairs
-    RankTables T{ root_bits, root_prefix, lower_bits, lower_prefix };
-    const int leaf_key_bits = 12 + bits_for(NL > 1 ? NL : 2);
-    if (leaf_key_bits > 32)
-    {
-        set_error(ctx, "voxelize: %llu touched lower-node cells (128^3 voxels) exceed the 2^20 leaf keys hold",
-                  (unsigned long long)NL);
-        return VOX_ERR_SIZE;
-    }
-    if (!ensure(ctx, ctx->lcols, 8 * (size_t)(G + 1)) || !ensure(ctx, ctx->lcol_off, 8 * (size_t)(G + 1)))
-        return VOX_ERR_MEMORY;
-    uint64_t* lcols = (uint64_t*)ctx->lcols.p;
-    uint64_t* lcol_off = (uint64_t*)ctx->lcol_off.p;
-    launch_leaf_cols(recs, G, lcols, s);
-    scan_exclusive_u64(lcols, lcol_off, G, 0, sc + SC_NLC, scan_status, ctx->scan_epochs.next(scan_status, scan_words, s),
-                       d_counter, d_err, ctx->num_sms, s);
-    rc = sync_scalars(ctx, "leaf columns");
-    if (rc)
-        return rc;
-    const uint64_t NLC = ctx->hscal[SC_NLC];
-    if (!ensure(ctx, ctx->lc_count, 8 * (size_t)(NLC + 1)) || !ensure(ctx, ctx->lc_off, 8 * (size_t)(NLC + 1)) ||
-        !ensure(ctx, ctx->lc_mask, 4 * (size_t)(NLC + 1)) || !ensure(ctx, ctx->tile_g0, 8 * (size_t)(NLC / 256 + 2)) ||
-        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * scan_status_words((int64_t)NLC + 1) * 2))
-        return VOX_ERR_MEMORY;
-    scan_status = (uint64_t*)ctx->scan_status.p;
-    scan_words = ctx->scan_status.cap / sizeof(uint64_t);
     LeafEmitParams LE;
     memset(&LE, 0, sizeof(LE));
     LE.recs = recs;
@@ -555,11 +583,32 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LE.check = ctx->check_emit;
     launch_leaf_emit(LE, T, false, s);
     uint64_t* lc_off = (uint64_t*)ctx->lc_off.p;
-    scan_exclusive_u64(LE.lc_count, lc_off, (int64_t)NLC, 0, sc + SC_Q, scan_status,
-                       ctx->scan_epochs.next(scan_status, scan_words, s), d_counter, d_err, ctx->num_sms, s);
+    {
+        ScanJobs J;
+        J.count = 2;
+        J.job[0] = { lower_bits, lower_prefix, lwords, 1, sc + SC_NLOWER, scan_status, ctr(CTR_LOWER), nullptr, 0 };
+        J.job[1] = { LE.lc_count, lc_off, (int64_t)NLC, 0, sc + SC_Q, scan_status + scan_status_words(lwords),
+                     ctr(CTR_PAIRS), nullptr, 0 };
+        scan_jobs(J, ctx->scan_epochs.next(scan_status, scan_words, s), d_err, s);
+    }
     rc = sync_scalars(ctx, "leaf pairs");
     if (rc)
         return rc;
+    const uint64_t NL = ctx->hscal[SC_NLOWER];
+    if (!ensure(ctx, ctx->lower_cell, sizeof(uint32_t) * (NL + 1)))
+        return VOX_ERR_MEMORY;
+    launch_invert_bits(lower_bits, lower_prefix, lwords, (uint32_t*)ctx->lower_cell.p, s);
+    const int key_bits = 21 + bits_for(NL > 1 ? NL : 2);
+    const int key64 = key_bits > 32 ? 1 : 0;
+    ctx->key64 = key64;
+    ctx->stats.key_bits = key_bits;
+    const int leaf_key_bits = 12 + bits_for(NL > 1 ? NL : 2);
+    if (leaf_key_bits > 32)
+    {
+        set_error(ctx, "voxelize: %llu touched lower-node cells (128^3 voxels) exceed the 2^20 leaf keys hold",
+                  (unsigned long long)NL);
+        return VOX_ERR_SIZE;
+    }
     const uint64_t Q = ctx->hscal[SC_Q];
     const bool by_emission = diff || ctx->check_emit; // the sort's values are emission indices
     if (Q >= 0xFFFFFFF0ull)
@@ -616,7 +665,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     CP.total = sc + SC_NCL;
     CP.status = (uint64_t*)ctx->run_status.p;
     CP.epoch = ctx->run_epochs.next(CP.status, ctx->run_status.cap / sizeof(uint64_t), s);
-    CP.counter = d_counter;
+    CP.counter = ctr(CTR_CANDS);
     CP.err = d_err;
     launch_leaf_cands(lkeys, lvals, LE.emit_gid, (int64_t)Q, (const uint32_t*)ctx->lower_cell.p,
                       (const uint32_t*)ctx->root_of_rank.p, CP, s);
@@ -684,7 +733,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LP.key64 = key64;
     ctx->walk_mode = (LP.window ? 1 : 0) | (LP.smooth ? 2 : 0); // the modes differ in cost per pair
     ctx->walk_variant = ctx->walk_choice[ctx->walk_mode].pick((int64_t)Q);
-    ctx->stats.walk_ctas_per_sm = launch_leaf_pass(LP, d_counter, ctx->num_sms, s, ctx->walk_variant);
+    ctx->stats.walk_ctas_per_sm = launch_leaf_pass(LP, ctr(CTR_WALK), ctx->num_sms, s, ctx->walk_variant);
     cudaEventRecord(ctx->timers.ev[4], s);
 
     // ------------------------------------------------ tree: tables and layout
@@ -754,7 +803,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     TP.counts = sc + SC_V;
     TP.status = (uint64_t*)ctx->run_status.p;
     TP.epoch = ctx->run_epochs.next(TP.status, ctx->run_status.cap / sizeof(uint64_t), s);
-    TP.counter = d_counter;
+    TP.counter = ctr(CTR_TREE);
     TP.err = d_err;
     TP.lower_cap = lcap;
     launch_tree(TP, N, s);
@@ -978,7 +1027,8 @@ vox_context_t* vox_context_create(int device)
     cudaSetDevice(device);
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMallocHost((void**)&ctx->hscal, sizeof(uint64_t) * SC_SCRATCH * 8) != cudaSuccess)
+        cudaHostAlloc((void**)&ctx->hscal, sizeof(uint64_t) * SC_SCRATCH * 8, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&ctx->hscal_dev, ctx->hscal, 0) != cudaSuccess)
     {
         set_error(nullptr, "vox_context_create: stream / pinned allocation failed");
         delete ctx;

@@ -66,6 +66,28 @@ size_t scan_status_words(int64_t n);
 void scan_exclusive_u64(const uint64_t* in, uint64_t* out, int64_t n, int mode, uint64_t* total, uint64_t* status,
                         uint32_t epoch, uint32_t* counter, int* err, int num_sms, cudaStream_t s);
 
+// up to three such scans in one launch: each with its own status words and its
+// own counter, which the caller has zeroed; invert: also the positions of the
+// set bits of a popcount scan, in order
+struct ScanJob
+{
+    const uint64_t* in;
+    uint64_t* out;
+    int64_t n;
+    int mode;
+    uint64_t* total;
+    uint64_t* status;
+    uint32_t* counter;
+    uint32_t* invert;
+    uint32_t tiles; // set by scan_jobs
+};
+struct ScanJobs
+{
+    int count;
+    ScanJob job[3];
+};
+void scan_jobs(ScanJobs S, uint32_t epoch, int* err, cudaStream_t s);
+
 // u32 scan (sum mod 2^32, or running maximum with max_op), inclusive or
 // exclusive; *total (u64) receives the sum / maximum
 void scan_u32(const uint32_t* in, uint32_t* out, int64_t n, int inclusive, int max_op, uint64_t* total,

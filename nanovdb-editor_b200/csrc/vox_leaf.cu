@@ -6,12 +6,11 @@
 // (raster/Raster.cpp:420-558, gaussian_frag_alloc.slang, grid_build_*.slang,
 // gaussian_frag_color.slang).  Here the unit of sorting is the leaf (8^3
 // voxels, the node2 leaf of PNanoVDBExt.h:72-81):
-//   k_leaf_cols / k_leaf_emit   per Gaussian, the leaf cells of its bbox whose
-//       box may reach its 0.01-opacity ellipsoid (a conservative test in
-//       double), written as (leaf key, emission index) in Gaussian-major
-//       order; a stable sort by leaf key keeps each leaf's Gaussians in
-//       ascending id;
-//   k_leaf_heads / k_leaf_compact   runs of equal leaf keys -> candidate leaves;
+//   k_leaf_emit   per Gaussian, the leaf cells of its bbox whose box may reach
+//       its 0.01-opacity ellipsoid (a conservative test in double), written as
+//       (leaf key, Gaussian) in Gaussian-major order; a stable sort by leaf key
+//       keeps each leaf's Gaussians in ascending id;
+//   k_leaf_cands  runs of equal leaf keys -> candidate leaves;
 //   k_leaf_pass   one CTA per candidate leaf, one thread per voxel (two per
 //       thread): the CTA walks the leaf's Gaussians in ascending id and every
 //       thread runs the reference test (gaussian_frag_alloc.slang:84-162) on
@@ -49,22 +48,6 @@ __device__ __forceinline__ int64_t upper_bound_u64_l(const uint64_t* a, int64_t 
 }
 
 // ------------------------------------------------------------ emission ----
-__global__ void k_leaf_cols(const GaussRec* recs, int64_t G, uint64_t* lcols)
-{
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G)
-        return;
-    const GaussRec R = recs[g];
-    if (!R.q4.w)
-    {
-        lcols[g] = 0;
-        return;
-    }
-    const int32_t lx0 = R.q4.x >> 3, lx1 = (R.q4.x + R.q5.x - 1) >> 3;
-    const int32_t ly0 = R.q4.y >> 3, ly1 = (R.q4.y + R.q5.y - 1) >> 3;
-    lcols[g] = (uint64_t)(lx1 - lx0 + 1) * (uint64_t)(ly1 - ly0 + 1);
-}
-
 // May a voxel of the leaf at origin o pass the reference test?  The local AABB
 // of the leaf box (monotone-corner identity, in double) contains every voxel's
 // local AABB; the float test's rounding is bounded by delta = 1e-5 (1 + B), B
@@ -1664,13 +1647,6 @@ __global__ void k_voxel_coords(NodeParams N, int32_t* out)
 }
 
 // ---------------------------------------------------------------- launch ----
-void launch_leaf_cols(const GaussRec* recs, int64_t G, uint64_t* lcols, cudaStream_t s)
-{
-    if (G <= 0)
-        return;
-    { k_leaf_cols<<<(unsigned)((G + 255) / 256), 256, 0, s>>>(recs, G, lcols); count_launch(); }
-}
-
 void launch_tile_gauss(const uint64_t* lcol_off, int64_t G, uint64_t NLC, int64_t* tile_g0, cudaStream_t s)
 {
     if (NLC == 0)
@@ -1702,7 +1678,6 @@ void launch_leaf_cands(const uint32_t* keys, const uint32_t* vals, const uint32_
 {
     if (Q <= 0)
         return;
-    cudaMemsetAsync(C.counter, 0, sizeof(uint32_t), s);
     { k_leaf_cands<<<(unsigned)((Q + LC_TILE - 1) / LC_TILE), LC_BLOCK, 0, s>>>(keys, vals, emit_gid, Q, lower_cell, root_of_rank, C); count_launch(); }
 }
 
@@ -1731,7 +1706,6 @@ int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cu
 {
     if (P.NCL <= 0)
         return 0;
-    cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
     if (P.smooth)
         return P.emit_flag ? (P.window ? launch_walk<true, true, true, 4>(P, counter, num_sms, s)
                                        : launch_walk<true, false, true, 4>(P, counter, num_sms, s))

@@ -39,7 +39,8 @@ __device__ __forceinline__ void mark_bit(unsigned long long* bits, uint64_t i)
 
 // ------------------------------------------------------------------ prep ----
 __global__ void __launch_bounds__(256) k_prep(PrepParams P, GaussRec* recs, WalkRec* walk,
-                                              uint64_t* footprints, unsigned long long* root_bits, int* err)
+                                              uint64_t* footprints, uint64_t* lcols, unsigned long long* root_bits,
+                                              int* err)
 {
     const int64_t g = P.g0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= (P.g1 < 0 ? P.count : P.g1))
@@ -84,6 +85,8 @@ __global__ void __launch_bounds__(256) k_prep(PrepParams P, GaussRec* recs, Walk
     }
     recs[g] = R;
     footprints[g] = fp;
+    // leaf columns (lx, ly) of the bbox
+    lcols[g] = fp ? (uint64_t)((bmax[0] >> 3) - (R.q4.x >> 3) + 1) * (uint64_t)((bmax[1] >> 3) - (R.q4.y >> 3) + 1) : 0ull;
     if (fp)
     {
         walk[g] = walk_record(R, vs);
@@ -652,13 +655,13 @@ __global__ void __launch_bounds__(NODE_THREADS) k_write_nodes(NodeParams N, uint
 static_assert(node_parts(2) == 1, "a lower node is one stretch");
 
 // =================================================================== launch
-void launch_prep(const PrepParams& P, GaussRec* recs, WalkRec* walk, uint64_t* footprints, uint64_t* root_bits, int* err,
-                 cudaStream_t s)
+void launch_prep(const PrepParams& P, GaussRec* recs, WalkRec* walk, uint64_t* footprints, uint64_t* lcols,
+                 uint64_t* root_bits, int* err, cudaStream_t s)
 {
     const int64_t n = (P.g1 < 0 ? P.count : P.g1) - P.g0;
     if (n <= 0)
         return;
-    { k_prep<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, recs, walk, footprints, (unsigned long long*)root_bits, err); count_launch(); }
+    { k_prep<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, recs, walk, footprints, lcols, (unsigned long long*)root_bits, err); count_launch(); }
 }
 
 void launch_mark_lower(const GaussRec* recs, int64_t G, const uint64_t* root_bits, const uint64_t* root_prefix,
@@ -687,7 +690,6 @@ void launch_tree(const TreeParams& T, const NodeParams& N, cudaStream_t s)
 {
     if (T.NCL <= 0)
         return;
-    cudaMemsetAsync(T.counter, 0, sizeof(uint32_t), s);
     { k_tree<<<(unsigned)((T.NCL + TREE_TILE - 1) / TREE_TILE), TREE_BLOCK, 0, s>>>(T, N); count_launch(); }
 }
 void launch_canonical_order(const NodeParams& N, uint64_t U, cudaStream_t s)

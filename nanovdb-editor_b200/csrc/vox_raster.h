@@ -165,7 +165,6 @@ struct LeafPassParams
     int key64;
 };
 
-void launch_leaf_cols(const GaussRec* recs, int64_t G, uint64_t* lcols, cudaStream_t s);
 void launch_leaf_emit(const LeafEmitParams& P, const RankTables& T, bool write, cudaStream_t s);
 void launch_tile_gauss(const uint64_t* lcol_off, int64_t G, uint64_t NLC, int64_t* tile_g0, cudaStream_t s);
 // candidate leaves from the sorted pairs (k_leaf_cands)
@@ -186,6 +185,7 @@ void launch_leaf_cands(const uint32_t* keys, const uint32_t* vals, const uint32_
                        const uint32_t* lower_cell, const uint32_t* root_of_rank, const CandParams& C, cudaStream_t s);
 // variant 0: 4 resident CTAs per SM (64 registers per thread), 1: 3 CTAs per SM;
 // returns the CTAs per SM it ran with
+// (counter: zeroed by the caller)
 int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant = 0);
 void launch_leaf_backward(const LeafPassParams& P, int64_t Q, cudaStream_t s);
 // vpairs non-null: only the pairs per voxel (canonical order), into it
@@ -238,8 +238,8 @@ void launch_window_place(const WindowOrderParams& W, const NodeParams& N, cudaSt
 
 void launch_bwd_finalize(const BwdFinalParams& F, cudaStream_t s);
 
-void launch_prep(const PrepParams& P, GaussRec* recs, WalkRec* walk, uint64_t* footprints, uint64_t* root_bits, int* err,
-                 cudaStream_t s);
+void launch_prep(const PrepParams& P, GaussRec* recs, WalkRec* walk, uint64_t* footprints, uint64_t* lcols,
+                 uint64_t* root_bits, int* err, cudaStream_t s);
 void launch_mark_lower(const GaussRec* recs, int64_t G, const uint64_t* root_bits, const uint64_t* root_prefix,
                        uint64_t* lower_bits, cudaStream_t s);
 void launch_invert_bits(const uint64_t* bits, const uint64_t* prefix, int64_t words, uint32_t* out, cudaStream_t s);

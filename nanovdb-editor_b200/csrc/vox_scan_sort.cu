@@ -38,25 +38,18 @@ size_t scan_status_words(int64_t n)
     return 4 * ((size_t)((n + SCAN_TILE - 1) / SCAN_TILE) + 1);
 }
 
-// VEC: in and out are 16-byte aligned (full tiles move as 16-byte words)
-template <bool VEC>
-__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_excl(const uint64_t* in, uint64_t* out, int64_t n, int mode,
-                                                            uint64_t* total, uint64_t* status, uint32_t epoch,
-                                                            uint32_t* counter, int* err)
+// One tile of a scan; vec: in and out are 16-byte aligned (full tiles move as
+// 16-byte words).  invert: also the positions of the set bits of a popcount scan
+// (mode bit 0), in order.
+__device__ __forceinline__ void scan_tile(const ScanJob& J, uint64_t tile, bool vec, uint32_t epoch, int* err,
+                                          uint64_t* s_warp, uint64_t& s_excl)
 {
-    __shared__ uint64_t s_warp[33];
-    __shared__ uint64_t s_excl;
-    __shared__ uint32_t s_tile;
-    if (threadIdx.x == 0)
-        s_tile = counter ? atomicAdd(counter, 1u) : 0u; // no counter: a single tile
-    __syncthreads();
-    const uint64_t tile = s_tile;
     const int64_t base = (int64_t)tile * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    const bool full = VEC && ((int64_t)tile + 1) * SCAN_TILE <= n;
-    uint64_t v[SCAN_ITEMS];
+    const bool full = vec && ((int64_t)tile + 1) * SCAN_TILE <= J.n;
+    uint64_t v[SCAN_ITEMS], bits[SCAN_ITEMS];
     if (full)
     {
-        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(in + base);
+        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(J.in + base);
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS / 2; i++)
         {
@@ -68,12 +61,13 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_excl(const uint64_t* in, ui
     else
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS; i++)
-            v[i] = base + i < n ? in[base + i] : 0ull;
+            v[i] = base + i < J.n ? J.in[base + i] : 0ull;
     uint64_t sum = 0;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++)
     {
-        if (mode & 1)
+        bits[i] = v[i];
+        if (J.mode & 1)
             v[i] = (uint64_t)__popcll(v[i]);
         sum += v[i];
     }
@@ -81,24 +75,32 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_excl(const uint64_t* in, ui
     const uint64_t texcl = block_excl_scan_u64(sum, s_warp, block_total);
     if (threadIdx.x < 32)
     {
-        const uint64_t e = lookback_exclusive_warp(status, tile, block_total, epoch, err);
+        const uint64_t e = lookback_exclusive_warp(J.status, tile, block_total, epoch, err);
         if (threadIdx.x == 0)
             s_excl = e;
     }
     __syncthreads();
     uint64_t run = s_excl + texcl;
+    if (J.invert)
+    {
+        uint64_t at = run;
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; i++)
+            for (uint64_t m = bits[i]; m; m &= m - 1)
+                J.invert[at++] = (uint32_t)((base + i) * 64 + __ffsll((long long)m) - 1);
+    }
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++)
     {
         const uint64_t next = run + v[i];
-        if (base + i == n - 1)
-            *total = next;
-        v[i] = (mode & 2) ? next : run;
+        if (base + i == J.n - 1)
+            *J.total = next;
+        v[i] = (J.mode & 2) ? next : run;
         run = next;
     }
     if (full)
     {
-        ulonglong2* dst = reinterpret_cast<ulonglong2*>(out + base);
+        ulonglong2* dst = reinterpret_cast<ulonglong2*>(J.out + base);
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS / 2; i++)
             dst[i] = make_ulonglong2(v[2 * i], v[2 * i + 1]);
@@ -106,28 +108,63 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_excl(const uint64_t* in, ui
     else
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS; i++)
-            if (base + i < n)
-                out[base + i] = v[i];
+            if (base + i < J.n)
+                J.out[base + i] = v[i];
+}
+
+// CTAs [tiles of the jobs before, + its own tiles) work on a job; within it they
+// take tiles in the order of its counter (no counter: a single tile)
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_excl(ScanJobs S, uint32_t epoch, int* err)
+{
+    __shared__ uint64_t s_warp[33];
+    __shared__ uint64_t s_excl;
+    __shared__ uint32_t s_tile;
+    uint32_t b = blockIdx.x;
+    int j = 0;
+    while (j + 1 < S.count && b >= S.job[j].tiles)
+        b -= S.job[j++].tiles;
+    const ScanJob& J = S.job[j];
+    if (threadIdx.x == 0)
+        s_tile = J.counter ? atomicAdd(J.counter, 1u) : 0u;
+    __syncthreads();
+    scan_tile(J, s_tile, (((uintptr_t)J.in | (uintptr_t)J.out) & 15u) == 0, epoch, err, s_warp, s_excl);
+}
+
+// jobs of no elements write their total by a memset
+void scan_jobs(ScanJobs S, uint32_t epoch, int* err, cudaStream_t s)
+{
+    ScanJobs R;
+    R.count = 0;
+    uint64_t grid = 0;
+    for (int j = 0; j < S.count; j++)
+    {
+        ScanJob J = S.job[j];
+        if (J.n <= 0)
+        {
+            cudaMemsetAsync(J.total, 0, sizeof(uint64_t), s);
+            continue;
+        }
+        J.tiles = (uint32_t)((J.n + SCAN_TILE - 1) / SCAN_TILE);
+        if (J.tiles == 1)
+            J.counter = nullptr;
+        grid += J.tiles;
+        R.job[R.count++] = J;
+    }
+    if (grid == 0)
+        return;
+    { k_scan_excl<<<(unsigned)grid, SCAN_BLOCK, 0, s>>>(R, epoch, err); count_launch(); }
 }
 
 void scan_exclusive_u64(const uint64_t* in, uint64_t* out, int64_t n, int mode, uint64_t* total, uint64_t* status,
                         uint32_t epoch, uint32_t* counter, int* err, int num_sms, cudaStream_t s)
 {
     (void)num_sms;
-    if (n <= 0)
-    {
-        cudaMemsetAsync(total, 0, sizeof(uint64_t), s);
-        return;
-    }
-    const int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    if (tiles == 1)
-        counter = nullptr;
-    else
+    if (n > SCAN_TILE)
         cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    const bool vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0;
-    auto kern = vec ? k_scan_excl<true> : k_scan_excl<false>;
-    kern<<<(unsigned)tiles, SCAN_BLOCK, 0, s>>>(in, out, n, mode, total, status, epoch, counter, err);
-    count_launch();
+    ScanJobs S;
+    S.count = 1;
+    S.job[0] = { in, out, n, mode, total, status, counter, nullptr, 0u };
+    scan_jobs(S, epoch, err, s);
 }
 
 // u32 scans: the reference's global_scan (sum, wrapping mod 2^32) and
