@@ -849,14 +849,17 @@ constexpr uint64_t LB_VALUE_MASK = (1ull << 55) - 1ull;
 constexpr uint64_t LB_INCL = 1ull << 55;
 constexpr uint32_t LB_SPIN_LIMIT = 1u << 22;
 
-__device__ __forceinline__ void st_release_u64(uint64_t* p, uint64_t v)
+// Status words carry their own tag and value and stand for nothing else in
+// memory, so their accesses need no order (acquire and release forms: the sort of
+// 29.6M pairs 1.27 instead of 1.19 ms).
+__device__ __forceinline__ void st_relaxed_u64(uint64_t* p, uint64_t v)
 {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p)
+__device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p)
 {
     uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -886,7 +889,6 @@ __device__ __forceinline__ LbControl lb_control(const int* err)
 // other tile work) lets the predecessors' inclusive prefixes land meanwhile.
 // Every wait is bounded; on timeout *err is set and the partial prefix (never
 // larger than the true one) is returned, and the host treats the call as failed.
-// max_op: combine predecessors by maximum instead of sum (a running-max scan)
 __device__ __forceinline__ void lookback_publish(uint64_t* status, uint64_t tile, uint64_t aggregate, uint32_t epoch,
                                                  int* err, size_t stride = 1)
 {
@@ -894,11 +896,11 @@ __device__ __forceinline__ void lookback_publish(uint64_t* status, uint64_t tile
     if (ctl.withhold)
         return;
     const uint64_t tag = (uint64_t)epoch << 56;
-    st_release_u64(&status[tile * stride], tag | (tile == 0 ? LB_INCL : 0ull) | (aggregate & LB_VALUE_MASK));
+    st_relaxed_u64(&status[tile * stride], tag | (tile == 0 ? LB_INCL : 0ull) | (aggregate & LB_VALUE_MASK));
 }
 
 __device__ __forceinline__ uint64_t lookback_walk(uint64_t* status, uint64_t tile, uint64_t aggregate, uint32_t epoch,
-                                                  int* err, size_t stride = 1, bool max_op = false)
+                                                  int* err, size_t stride = 1)
 {
     if (tile == 0)
         return 0;
@@ -909,7 +911,7 @@ __device__ __forceinline__ uint64_t lookback_walk(uint64_t* status, uint64_t til
     uint32_t spins = 0;
     while (p >= 0)
     {
-        uint64_t s = ld_acquire_u64(&status[(uint64_t)p * stride]);
+        uint64_t s = ld_relaxed_u64(&status[(uint64_t)p * stride]);
         if ((s >> 56) != epoch)
         {
             if (++spins > ctl.limit)
@@ -921,48 +923,89 @@ __device__ __forceinline__ uint64_t lookback_walk(uint64_t* status, uint64_t til
             continue;
         }
         const uint64_t v = s & LB_VALUE_MASK;
-        excl = max_op ? (v > excl ? v : excl) : excl + v;
+        excl += v;
         if (s & LB_INCL)
             break;
         p--;
     }
-    const uint64_t incl = max_op ? (aggregate > excl ? aggregate : excl) : excl + aggregate;
+    const uint64_t incl = excl + aggregate;
     if (!ctl.withhold)
-        st_release_u64(&status[tile * stride], tag | LB_INCL | (incl & LB_VALUE_MASK));
+        st_relaxed_u64(&status[tile * stride], tag | LB_INCL | (incl & LB_VALUE_MASK));
     return excl;
 }
 
 // publish and walk at once
 __device__ __forceinline__ uint64_t lookback_exclusive(uint64_t* status, uint64_t tile, uint64_t aggregate,
-                                                       uint32_t epoch, int* err, size_t stride = 1,
-                                                       bool max_op = false)
+                                                       uint32_t epoch, int* err, size_t stride = 1)
 {
     lookback_publish(status, tile, aggregate, epoch, err, stride);
-    return lookback_walk(status, tile, aggregate, epoch, err, stride, max_op);
+    return lookback_walk(status, tile, aggregate, epoch, err, stride);
 }
 
-// The same for sums that may use all 64 bits (the prefix is exact mod 2^64, as
-// uint64 addition is), walked by a whole warp: every lane of it must call, and
-// gets the exclusive prefix.  Per tile four words: the aggregate's low and high
-// halves, then the inclusive prefix's, each word (epoch << 32) | half.  Every
-// word is written once per use and carries its own tag, so two halves that both
-// carry the current epoch belong to the same value, and no order among the
-// words matters (relaxed accesses).
-// A launch's tiles start together, so a tile's nearest inclusive prefix may be
-// hundreds of tiles back, and a walk of one thread is a chain of that many L2
-// round trips; here a round trip covers 32 tiles (lane i reads the predecessor
-// p - i): the scans of a 2M-Gaussian call 1.31 -> 0.30 ms.
-__device__ __forceinline__ void st_relaxed_u64(uint64_t* p, uint64_t v)
+// Look-backs walked by a whole warp: every lane of it must call, and gets the
+// exclusive prefix.  A launch's tiles start together, so a tile's nearest
+// inclusive prefix may be hundreds of tiles back, and a walk of one thread is a
+// chain of that many L2 round trips; here a round trip covers 32 tiles (lane i
+// reads the predecessor p - i): the scans of a 2M-Gaussian call 1.31 -> 0.30 ms.
+
+// One word per tile (values mod 2^55, as lookback_publish stores them), summed or
+// combined by maximum.
+template <bool MAX>
+__device__ __forceinline__ uint64_t lookback_narrow_warp(uint64_t* status, uint64_t tile, uint64_t aggregate,
+                                                         uint32_t epoch, int* err)
 {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p)
-{
-    uint64_t v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
+    const int lane = threadIdx.x & 31;
+    const LbControl ctl = lb_control(err);
+    const uint64_t tag = (uint64_t)epoch << 56;
+    if (!ctl.withhold && lane == 0)
+        st_relaxed_u64(&status[tile], tag | (tile == 0 ? LB_INCL : 0ull) | (aggregate & LB_VALUE_MASK));
+    if (tile == 0)
+        return 0;
+    uint64_t excl = 0;
+    int64_t p = (int64_t)tile - 1;
+    uint32_t spins = 0;
+    while (p >= 0)
+    {
+        const int64_t q = p - lane;
+        const uint64_t w = q >= 0 ? ld_relaxed_u64(&status[q]) : tag | LB_INCL;
+        const bool ready = (w >> 56) == epoch;
+        const uint32_t mi = __ballot_sync(0xffffffffu, ready && (w & LB_INCL)), mr = __ballot_sync(0xffffffffu, ready);
+        const int first_incl = mi ? __ffs(mi) - 1 : 32, first_gap = ~mr ? __ffs(~mr) - 1 : 32;
+        const int take = first_incl < first_gap ? first_incl + 1 : first_gap; // lanes [0, take) are added
+        if (take == 0)
+        {
+            if (++spins > ctl.limit)
+            {
+                if (lane == 0)
+                    atomicOr(err, 1); // ERR_LOOKBACK
+                break;
+            }
+            __nanosleep(32);
+            continue;
+        }
+        uint64_t c = lane < take ? w & LB_VALUE_MASK : 0;
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+        {
+            const uint64_t y = __shfl_xor_sync(0xffffffffu, c, o);
+            c = MAX ? (y > c ? y : c) : c + y;
+        }
+        excl = MAX ? (c > excl ? c : excl) : excl + c;
+        if (first_incl < first_gap)
+            break;
+        p -= take;
+    }
+    const uint64_t incl = MAX ? (aggregate > excl ? aggregate : excl) : excl + aggregate;
+    if (!ctl.withhold && lane == 0)
+        st_relaxed_u64(&status[tile], tag | LB_INCL | (incl & LB_VALUE_MASK));
+    return excl;
 }
 
+// For sums that may use all 64 bits (the prefix is exact mod 2^64, as uint64
+// addition is).  Per tile four words: the aggregate's low and high halves, then
+// the inclusive prefix's, each word (epoch << 32) | half.  Every word is written
+// once per use and carries its own tag, so two halves that both carry the current
+// epoch belong to the same value, and no order among the words matters.
 __device__ __forceinline__ uint64_t lookback_exclusive_warp(uint64_t* status, uint64_t tile, uint64_t aggregate,
                                                             uint32_t epoch, int* err)
 {

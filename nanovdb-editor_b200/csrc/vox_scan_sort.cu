@@ -241,8 +241,12 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_u32(const uint32_t* in, uin
     }
     uint64_t block_total;
     const uint64_t texcl = block_excl_scan_op<MAX>(agg, s_warp, block_total);
-    if (threadIdx.x == 0)
-        s_excl = lookback_exclusive(status, tile, block_total, epoch, err, 1, MAX);
+    if (threadIdx.x < 32)
+    {
+        const uint64_t e = lookback_narrow_warp<MAX>(status, tile, block_total, epoch, err);
+        if (threadIdx.x == 0)
+            s_excl = e;
+    }
     __syncthreads();
     uint64_t run = scan_op<MAX>(s_excl, texcl);
 #pragma unroll
