@@ -345,7 +345,7 @@ typedef struct vox_stats_t
     int64_t vb_launches;  /* kernels launched by that call */
     /* the online tuner's choices (variants give identical results) */
     int32_t walk_ctas_per_sm; /* leaf walk: resident CTAs per SM it ran with */
-    int32_t vb_search;        /* VoxelBVH level search: 0 lane-balanced, 1 thread per Gaussian */
+    int32_t vb_search;        /* VoxelBVH level search: 0, the only variant */
 } vox_stats_t;
 
 /* One context per caller thread; it owns a CUDA stream on `device` and a

@@ -86,10 +86,9 @@ struct vox_context_t
     DevBuf scal; // device scalars
     DevBuf hier_keys;
     DevBuf prim_keys_alt, prim_vals_alt; // ping-pong buffers of vox_radix_sort_key64
-    DevBuf vb_work; // VoxelBVH ingestion: world-box keys, range tile counts
+    DevBuf vb_work; // VoxelBVH ingestion: world-box keys
     DevBuf vb_keys, vb_ids_c, vb_used; // VoxelBVH ingestion: compressed sort keys (also the dual-key sort's keys)
     DevBuf dual_idx; // dual-key sort: original indices
-    DevBuf vb_rec;   // VoxelBVH ingestion: per-Gaussian search records
     uint64_t* hscal = nullptr; // pinned, mapped mirror
     uint64_t* hscal_dev = nullptr; // its device address
     uint64_t publications = 0;     // of the scalars, by this context
@@ -103,8 +102,7 @@ struct vox_context_t
     SortTuning tuning;
     OnlineChoice walk_choice[4] = { OnlineChoice(2), OnlineChoice(2), OnlineChoice(2), OnlineChoice(2) }; // leaf walk: 4 or 3 CTAs per SM, per mode (window | smooth << 1)
     int walk_mode = 0;
-    OnlineChoice vb_search_choice{ 2 }; // VoxelBVH level search: lane-balanced or thread per Gaussian
-    int walk_variant = 0, vb_variant = 0;
+    int walk_variant = 0;
     // last result
     int64_t last_P = 0;
     uint64_t last_grid_bytes = 0;
@@ -1063,7 +1061,7 @@ void vox_context_destroy(vox_context_t* ctx)
                       &ctx->sort_ws, &ctx->leaf_vstart, &ctx->lower_lstart, &ctx->lower_upper_n,
                       &ctx->lower_parent, &ctx->upper_root_n, &ctx->upper_lostart, &ctx->leaf_cand, &ctx->leaf_lower,
                       &ctx->leaf_lower_n, &ctx->leaf_origin, &ctx->order, &ctx->grid, &ctx->scal,
-                      &ctx->hier_keys, &ctx->prim_keys_alt, &ctx->prim_vals_alt, &ctx->vb_work, &ctx->vb_keys, &ctx->vb_ids_c, &ctx->vb_used, &ctx->dual_idx, &ctx->vb_rec, &ctx->cloud_start,
+                      &ctx->hier_keys, &ctx->prim_keys_alt, &ctx->prim_vals_alt, &ctx->vb_work, &ctx->vb_keys, &ctx->vb_ids_c, &ctx->vb_used, &ctx->dual_idx, &ctx->cloud_start,
                       &ctx->cloud_vs, &ctx->clouds, &ctx->lcols, &ctx->lcol_off, &ctx->lc_count, &ctx->lc_mask, &ctx->lc_off,
                       &ctx->cand_org, &ctx->tile_g0, &ctx->emit_gid, &ctx->emit_flag, &ctx->cand_key, &ctx->cand_start,
                       &ctx->cand_mask, &ctx->pair_gid, &ctx->s_rgba, &ctx->s_dens, &ctx->s_col, &ctx->cand_pairs,
@@ -1575,10 +1573,10 @@ int vox_voxelbvh_ijkl_from_gaussians(vox_context_t* ctx, const float* d_means, c
     cudaStream_t s = ctx->stream;
     const int64_t launches0 = launch_count();
     const int64_t N = 8 * count;
-    const int64_t tiles = vb_range_tiles(N);
     if (!ensure(ctx, ctx->scal, sizeof(uint64_t) * SC_SCRATCH * 4) ||
-        !ensure(ctx, ctx->vb_work, 256 + sizeof(uint64_t) * (size_t)(2 * tiles + 2)) ||
-        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * scan_status_words(tiles > 512 ? tiles : 512) * 2))
+        !ensure(ctx, ctx->vb_work, 256) ||
+        !ensure(ctx, ctx->vb_used, 8 * (size_t)(count + 1)) ||
+        !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * std::max(scan_status_words(count > 512 ? count : 512), vb_range_status_words(N))))
         return VOX_ERR_MEMORY;
     if (N > 1 && (!ensure(ctx, ctx->vb_keys, 8 * (size_t)N) || !ensure(ctx, ctx->prim_keys_alt, 8 * (size_t)N) ||
                   !ensure(ctx, ctx->prim_vals_alt, 4 * (size_t)N) || !ensure(ctx, ctx->sort_ws, sort_workspace_bytes(N, 8))))
@@ -1592,26 +1590,19 @@ int vox_voxelbvh_ijkl_from_gaussians(vox_context_t* ctx, const float* d_means, c
     P.keys = d_ijkl;
     P.ids = d_prim_id;
     P.err = err;
-    uint64_t* tile_cnt = (uint64_t*)((char*)ctx->vb_work.p + 256);
-    uint64_t* tile_off = tile_cnt + tiles;
-    uint64_t* d_total = tile_off + tiles;
+    P.used = (uint32_t*)ctx->vb_used.p;
+    uint32_t* uoff = P.used + count + 1;
     cudaEventRecord(ctx->timers.ev[0], s);
     launch_vb_init(P.box_keys, P.cell_minmax, s);
     launch_vb_box(P, ctx->num_sms, s);
-    // the level search variant: the tuner's choice, or VOX_VB_SEARCH=thread / lane
-    const char* search = getenv("VOX_VB_SEARCH");
-    ctx->vb_variant = search && search[0] == 't' ? 1 : search && search[0] == 'l' ? 0 : ctx->vb_search_choice.pick(count);
-    ctx->stats.vb_search = ctx->vb_variant;
-    if (ctx->vb_variant == 1)
-        launch_vb_ijkl(P, s);
-    else
-    {
-        if (!ensure(ctx, ctx->vb_rec, sizeof(float) * 24 * (size_t)(count > 0 ? count : 1)))
-            return VOX_ERR_MEMORY;
-        P.rec = (float*)ctx->vb_rec.p;
-        launch_vb_search(P, ctx->num_sms, s);
-    }
+    launch_vb_keys(P, s);
     cudaEventRecord(ctx->timers.ev[1], s);
+    {
+        // the used slots before each Gaussian's, and (read back with the cells' range) all of them
+        uint64_t* status = (uint64_t*)ctx->scan_status.p;
+        scan_u32(P.used, uoff, count, 0, 0, sc + SC_VBU, status,
+                 ctx->scan_epochs.next(status, ctx->scan_status.cap / sizeof(uint64_t), s), (uint32_t*)(sc + CTR_FOOT), err, s);
+    }
     int rc = check_cuda(ctx, "vox_voxelbvh_ijkl_from_gaussians");
     if (rc == VOX_OK)
         rc = sync_scalars(ctx, "vox_voxelbvh_ijkl_from_gaussians");
@@ -1654,23 +1645,12 @@ int vox_voxelbvh_ijkl_from_gaussians(vox_context_t* ctx, const float* d_means, c
             key32 = sort_bits <= 32;
             R.sentinel = sort_bits >= 64 ? ~0ull : (1ull << sort_bits) - 1;
             R.expand = 1;
-            // only the used slots are sorted: per-Gaussian counts, their scan (the total U
-            // read back to size the sort), then the compressed keys and ids compacted
-            if (!ensure(ctx, ctx->vb_ids_c, 4 * (size_t)N) || !ensure(ctx, ctx->vb_used, 8 * (size_t)(count + 1)))
+            // only the used slots are sorted
+            if (!ensure(ctx, ctx->vb_ids_c, 4 * (size_t)N))
                 return VOX_ERR_MEMORY;
-            uint32_t* used = (uint32_t*)ctx->vb_used.p;
-            uint32_t* uoff = used + count + 1;
             uint32_t* ids_c = (uint32_t*)ctx->vb_ids_c.p;
-            launch_vb_used(d_prim_id, count, used, s);
-            uint64_t* status = (uint64_t*)ctx->scan_status.p;
-            scan_u32(used, uoff, count, 0, 0, sc + SC_VBU, status,
-                     ctx->scan_epochs.next(status, ctx->scan_status.cap / sizeof(uint64_t), s),
-                     (uint32_t*)(sc + SC_SCRATCH), err, s);
-            rc = sync_scalars(ctx, "vox_voxelbvh_ijkl_from_gaussians");
-            if (rc != VOX_OK)
-                return rc;
             n_sorted = (int64_t)ctx->hscal[SC_VBU];
-            launch_vb_compress_used(d_ijkl, d_prim_id, count, used, uoff, R, ctx->vb_keys.p, ids_c, key32, ctx->num_sms,
+            launch_vb_compress_used(d_ijkl, d_prim_id, count, P.used, uoff, R, ctx->vb_keys.p, ids_c, key32, ctx->num_sms,
                                     s);
             if (key32)
                 in_alt = sort_pairs_u32((uint32_t*)ctx->vb_keys.p, ids_c, (uint32_t*)alt_k, alt_v, n_sorted, sort_bits,
@@ -1693,19 +1673,14 @@ int vox_voxelbvh_ijkl_from_gaussians(vox_context_t* ctx, const float* d_means, c
             R.ids_src = alt_v;
     }
     cudaEventRecord(ctx->timers.ev[3], s);
-    if (n_sorted > 0)
     {
-        const int64_t rtiles = vb_range_tiles(n_sorted);
-        launch_vb_range_count(sorted_keys, key32, n_sorted, tile_cnt, s);
         uint64_t* status = (uint64_t*)ctx->scan_status.p;
-        scan_exclusive_u64(tile_cnt, tile_off, rtiles, 0, d_total, status,
-                           ctx->scan_epochs.next(status, ctx->scan_status.cap / sizeof(uint64_t), s),
-                           (uint32_t*)(sc + SC_SCRATCH), err, ctx->num_sms, s);
-        launch_vb_range_scatter(sorted_keys, key32, n_sorted, tile_off, d_total, R, s);
-        if (n_sorted < N) // compacted: the unused run [U, N) is the last range
-            launch_vb_tail(n_sorted, N, d_total, sc + SC_F, R, ctx->num_sms, s);
-        else
-            cudaMemcpyAsync(sc + SC_F, d_total, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
+        R.total = sc + SC_F;
+        R.status = status;
+        R.epoch = ctx->scan_epochs.next(status, ctx->scan_status.cap / sizeof(uint64_t), s);
+        R.counter = (uint32_t*)(sc + CTR_CANDS);
+        R.err = err;
+        launch_vb_ranges(sorted_keys, key32, n_sorted, N, R, s);
     }
     cudaEventRecord(ctx->timers.ev[4], s);
     rc = check_cuda(ctx, "vox_voxelbvh_ijkl_from_gaussians");
@@ -1723,8 +1698,6 @@ int vox_voxelbvh_ijkl_from_gaussians(vox_context_t* ctx, const float* d_means, c
     };
     vox_stats_t& st = ctx->stats;
     st.ms_vb_keys = elapsed(ctx->timers.ev[0], ctx->timers.ev[1]);
-    if (!search)
-        ctx->vb_search_choice.report(count, ctx->vb_variant, st.ms_vb_keys);
     st.ms_vb_sort = elapsed(ctx->timers.ev[2], ctx->timers.ev[3]);
     st.ms_vb_ranges = elapsed(ctx->timers.ev[3], ctx->timers.ev[4]);
     st.vb_sort_bits = sort_bits;

@@ -266,7 +266,7 @@ struct VoxelBvhParams
     float* world_bbox;   // [6] output
     uint64_t* keys;      // [8 n], 16-byte aligned
     uint32_t* ids;       // [8 n], 16-byte aligned
-    float* rec;          // [n][24] per-Gaussian search records (lane-balanced search)
+    uint32_t* used;      // [n] used slots of each Gaussian
     int* err;
 };
 // sorted-key pass: compressed key layout, range headers, 64-bit key write-back
@@ -279,20 +279,20 @@ struct VbRangeParams
     uint64_t* keys_out;  // [N] 64-bit keys (expand)
     const uint32_t* ids_src; // sorted ids to copy into ids_out, or null
     uint32_t* ids_out;
+    uint64_t* total;     // ranges
+    uint64_t* status;    // vb_range_status_words(N)
+    uint32_t epoch;
+    uint32_t* counter;   // zeroed by the caller
+    int* err;
 };
 void launch_vb_init(uint32_t* box_keys, int* cell_minmax, cudaStream_t s);
 void launch_vb_box(const VoxelBvhParams& P, int num_sms, cudaStream_t s);
-void launch_vb_ijkl(const VoxelBvhParams& P, cudaStream_t s);
-void launch_vb_search(const VoxelBvhParams& P, int num_sms, cudaStream_t s);
-int64_t vb_range_tiles(int64_t N);
-void launch_vb_used(const uint32_t* ids, int64_t count, uint32_t* used, cudaStream_t s);
+void launch_vb_keys(const VoxelBvhParams& P, cudaStream_t s);
 void launch_vb_compress_used(const uint64_t* keys, const uint32_t* ids, int64_t count, const uint32_t* used,
                              const uint32_t* off, const VbRangeParams& R, void* out_keys, uint32_t* out_ids, int key32,
                              int num_sms, cudaStream_t s);
-void launch_vb_tail(int64_t U, int64_t N, const uint64_t* nr_used, uint64_t* ranges_out, const VbRangeParams& R,
-                    int num_sms, cudaStream_t s);
-void launch_vb_range_count(const void* keys, int key32, int64_t N, uint64_t* counts, cudaStream_t s);
-void launch_vb_range_scatter(const void* keys, int key32, int64_t N, const uint64_t* offs, const uint64_t* total,
-                             const VbRangeParams& R, cudaStream_t s);
+size_t vb_range_status_words(int64_t N);
+// the first U of N sorted keys are used ones
+void launch_vb_ranges(const void* keys, int key32, int64_t U, int64_t N, const VbRangeParams& R, cudaStream_t s);
 
 } // namespace vox
