@@ -737,9 +737,10 @@ __device__ __forceinline__ uint32_t alpha_byte_bits(float v)
     return __float_as_uint(__fadd_rd(VOX_FMUL(255.f, __saturatef(v)), 8388608.f));
 }
 
-// the byte in bits 24-31, the rest 0 (w3: the Gaussian's WalkRec::w3)
+// the byte in bits 24-31, the rest 0 (w3: the Gaussian's WalkRec::w3); most: the
+// largest byte it can be, likewise (also where it is not decided)
 __device__ __forceinline__ uint32_t alpha_byte_bound(const float4& q6, float cull, const AlphaF& f, const float4& w3,
-                                                     bool& decided)
+                                                     bool& decided, uint32_t& most)
 {
     const float md = VOX_FFMA(
         f.p[0], w3.x, VOX_FFMA(f.p[1], w3.y, VOX_FFMA(f.p[2], w3.z, VOX_FFMA(0x1.02p-20f, f.d, fabsf(w3.w)))));
@@ -755,7 +756,9 @@ __device__ __forceinline__ uint32_t alpha_byte_bound(const float4& q6, float cul
     const float delta = VOX_FFMA(slope_e, VOX_FFMA(a_hi, VOX_FFMA(1.25f, x, 1.1e-6f), 1.8e-7f), 9.3e-7f);
     const uint32_t lo = alpha_byte_bits(f.a1 - delta), hi = alpha_byte_bits(f.a1 + delta);
     const bool culled = cull != 0.f; // culled by scale: both alphas are 0
-    decided = culled || (x < 0.25f && a_hi < 1.f && lo == hi);
+    const bool bounded = x < 0.25f && a_hi < 1.f;
+    decided = culled || (bounded && lo == hi);
+    most = bounded ? hi << 24 : 0xff000000u;
     return culled ? 0u : lo << 24;
 }
 

@@ -964,8 +964,12 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         const AlphaF af = pair_alpha_f_ex(q6, stable_leaf_aabb(lo0, W4, h, fx, fy, fz));
                         a = q7.w != 0.f ? 0.f : af.a1;
                         bool decided;
-                        a8 = alpha_byte_bound(q6, q7.w, af, w3, decided);
-                        defer = !decided;
+                        uint32_t most;
+                        a8 = alpha_byte_bound(q6, q7.w, af, w3, decided, most);
+                        // an open pair that cannot exceed the voxel's maximum so far needs no byte
+                        // (a8 <= most: the maximum below changes nothing).  Of a voxel's k-th pair
+                        // that holds but for about one in k: the walk of 2M Gaussians 26.8 -> 26.1 ms
+                        defer = !decided && *(volatile uint32_t*)&A.rgba[n] < (most | __float_as_uint(al.w));
                         if (CHECK && decided &&
                             a8 >> 24 != ref_alpha_byte(P.recs[C.gid[j]], P.walk[C.gid[j]].w5.z, ao[0] + (int32_t)(n >> 6),
                                                        ao[1] + (int32_t)((n >> 3) & 7), ao[2] + (int32_t)(n & 7)))
