@@ -89,6 +89,7 @@ def voxel_coords(vox: VoxContext, value_count: int, device) -> torch.Tensor:
     """(i, j, k) of the active voxels of the context's last (single-cloud) grid, row r = value index r + 2."""
     out = torch.full((max(int(value_count), 2), 3), -(1 << 31), dtype=torch.int32, device=device)
     if value_count > 2:
+        torch.cuda.current_stream(out.device).synchronize()  # the fill: the library writes on its own stream
         vox.voxel_coords(out)
     return out[2:]
 
@@ -144,6 +145,7 @@ def batch_voxel_keys(vox: VoxContext, value_offsets, device):
     total = int(voff[-1])
     ijk = torch.full((max(total, 1), 3), -(1 << 31), dtype=torch.int32, device=device)
     if total:
+        torch.cuda.current_stream(ijk.device).synchronize()  # the fill: the library writes on its own stream
         vox.voxel_coords(ijk)
     ijk = ijk[:total]
     counts = voff[1:] - voff[:-1]
