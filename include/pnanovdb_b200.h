@@ -556,6 +556,17 @@ PNANOVDB_API int vox_voxelbvh_transform_inverse(const float* m, float* inv);
 PNANOVDB_API int vox_adam_bf16(float* master, float* m, float* v, const float* grad, uint16_t* out_bf16, int64_t n,
                                float lr, float beta1, float beta2, float eps, int64_t step, void* stream);
 
+/* A target grid's density at n voxels, one pass over device arrays, ordered on
+ * `stream` (cudaStream_t, may be 0), asynchronous.  `keys` (ascending) and
+ * `density` are the target's `count` voxels.  The voxels are given either as
+ * int32 (i, j, k) rows in `ijk`, whose keys are
+ * (i + 2^20) << 42 | (j + 2^20) << 21 | (k + 2^20) in 64-bit arithmetic, or as
+ * keys in `query`; the other is NULL.  value[r] = the density of the first equal
+ * key, 0 where there is none; hit[r] (may be NULL) = 1 or 0.  No counterpart in
+ * the reference (it has no training loop). */
+PNANOVDB_API int vox_target_lookup(const int64_t* keys, const float* density, int64_t count, const int32_t* ijk,
+                                   const int64_t* query, int64_t n, float* value, uint8_t* hit, void* stream);
+
 /* Scan that allocates nothing.  No counterpart in the reference.
  *
  * Same result as vox_global_scan_u64 (exact mod 2^64), for callers that cannot

@@ -16,7 +16,7 @@ import torch
 
 from .exceptions import PipelineError
 from .grid import HEADER_DTYPE
-from .vox import FLAG_BF16_INPUTS, FLAG_DIFFERENTIABLE, FLAG_RAW_INPUTS, VoxContext
+from .vox import FLAG_BF16_INPUTS, FLAG_DIFFERENTIABLE, FLAG_RAW_INPUTS, STATUS, VoxContext, _lib, _ptr
 
 _NAMES = ("means", "quats", "scales", "opacities", "colors")
 
@@ -100,6 +100,37 @@ def pack_coords(ijk: torch.Tensor) -> torch.Tensor:
     return (b[:, 0] << 42) | (b[:, 1] << 21) | b[:, 2]
 
 
+def _plain(t: torch.Tensor, dtype: torch.dtype, device) -> bool:
+    return (type(t) is torch.Tensor and t.dtype == dtype and t.device == device and t.is_contiguous()
+            and not t.requires_grad and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and torch.autograd.forward_ad.unpack_dual(t).tangent is None)
+
+
+def _fused_lookup(keys: torch.Tensor, density: torch.Tensor, ijk, query, want_hit: bool):
+    """The library's one-pass lookup, on torch's current stream, or None where torch's operators
+    have to be seen or do what the kernel does not: other devices, types and strides than the
+    grids' own, a density that is differentiated, vmap and tracing.  10.8M voxels:
+    0.90 ms by the operators' twelve launches, 0.18 ms by the kernel; 1.5M: 139 and 28 us."""
+    src = query if ijk is None else ijk
+    if not src.is_cuda or torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack():
+        return None
+    dev = src.device
+    if not (_plain(keys, torch.int64, dev) and _plain(density, torch.float32, dev)
+            and _plain(src, torch.int32 if query is None else torch.int64, dev)):
+        return None
+    if keys.dim() != 1 or density.shape != keys.shape or (src.dim() != 1 if ijk is None else src.dim() != 2 or src.shape[1] != 3):
+        return None
+    n = int(src.shape[0])
+    value = torch.empty(n, dtype=torch.float32, device=dev)
+    hit = torch.empty(n, dtype=torch.bool, device=dev) if want_hit else None
+    with torch.cuda.device(dev):
+        rc = _lib().vox_target_lookup(_ptr(keys), _ptr(density), int(keys.shape[0]), _ptr(ijk), _ptr(query), n, _ptr(value),
+                                      _ptr(hit), torch.cuda.current_stream(dev).cuda_stream)
+    if rc != 0:
+        raise PipelineError(f"vox_target_lookup: {STATUS.get(rc, rc)}")
+    return value, hit
+
+
 class TargetGrid:
     """Density of a fixed grid, looked up by voxel coordinate (0 where inactive)."""
 
@@ -117,6 +148,9 @@ class TargetGrid:
         return cls(coords, density[2:].detach())
 
     def lookup(self, coords: torch.Tensor):
+        fused = _fused_lookup(self.keys, self.density, coords, None, True)
+        if fused is not None:
+            return fused
         k = pack_coords(coords)
         if self.keys.numel() == 0:
             return torch.zeros(k.shape, dtype=torch.float32, device=k.device), torch.zeros(k.shape, dtype=torch.bool, device=k.device)
@@ -169,6 +203,9 @@ class BatchTargetGrid:
         self.total_sq = float((self.density.double() ** 2).sum())
 
     def lookup(self, keys: torch.Tensor):
+        fused = _fused_lookup(self.keys, self.density, None, keys, False)
+        if fused is not None:
+            return fused[0]
         if self.keys.numel() == 0:
             return torch.zeros(keys.shape, dtype=torch.float32, device=keys.device)
         pos = torch.searchsorted(self.keys, keys).clamp(max=self.keys.numel() - 1)

@@ -129,6 +129,8 @@ def _lib():
         lib.vox_context_set_wait_limit.argtypes = [c_void_p, c_uint32, c_int]
         lib.vox_adam_bf16.restype = c_int
         lib.vox_adam_bf16.argtypes = [c_void_p] * 5 + [c_int64, c_float, c_float, c_float, c_float, c_int64, c_void_p]
+        lib.vox_target_lookup.restype = c_int
+        lib.vox_target_lookup.argtypes = [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p]
         lib._vox_bound = True
     return lib
 
