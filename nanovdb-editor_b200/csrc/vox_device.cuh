@@ -683,9 +683,8 @@ struct AlphaF
     float a;    // op exp(-ls d), before the opacity transform
     float p[3]; // the smallest lattice |p| per axis
 };
-__device__ __forceinline__ AlphaF pair_alpha_f_ex(const float4& q6, const Aabb& b)
+__device__ __forceinline__ void pair_alpha_lattice(const Aabb& b, AlphaF& f)
 {
-    AlphaF f;
     float m[3];
 #pragma unroll
     for (int a = 0; a < 3; a++)
@@ -696,10 +695,37 @@ __device__ __forceinline__ AlphaF pair_alpha_f_ex(const float4& q6, const Aabb& 
         m[a] = VOX_FMUL(f.p[a], f.p[a]);
     }
     f.d = VOX_FADD(VOX_FADD(m[0], m[1]), m[2]);
+}
+__device__ __forceinline__ AlphaF pair_alpha_f_ex(const float4& q6, const Aabb& b)
+{
+    AlphaF f;
+    pair_alpha_lattice(b, f);
     float a = VOX_FMUL(q6.x, expf_ch_dev(-VOX_FMUL(q6.y, f.d)));
     a = fmaxf(a, 0.f);
     f.a = a;
     f.a1 = VOX_FSUB(1.f, powf_ch_dev(VOX_FSUB(1.f, a), q6.z));
+    return f;
+}
+// the same from the approximate base-2 exponential and logarithm, where only the
+// byte is wanted (alpha_byte_bound<true>)
+__device__ __forceinline__ float ex2_approx(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float lg2_approx(float x)
+{
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ AlphaF pair_alpha_approx(const float4& q6, const Aabb& b)
+{
+    AlphaF f;
+    pair_alpha_lattice(b, f);
+    f.a = q6.x * ex2_approx(-1.44269504f * (q6.y * f.d));
+    f.a1 = 1.f - ex2_approx(q6.z * lg2_approx(1.f - f.a));
     return f;
 }
 
@@ -729,6 +755,16 @@ __device__ __forceinline__ AlphaF pair_alpha_f_ex(const float4& q6, const Aabb& 
 // decided is set; otherwise the caller runs the reference's evaluation
 // (ref_alpha_byte).  VOX_CHECK_EMIT=1 compares every decided byte with the
 // reference's evaluation.
+//
+// APPROX: f from pair_alpha_approx.  ex2.approx is within 2^-22 relative, lg2.approx
+// within 2^-22 absolute in (0.5, 2) and relative elsewhere.  With u = ls d, whose
+// product with log2 e is rounded three times, a is within a (3.0e-7 + 1.8e-7 u), and
+// a u <= 0.37: at most 4e-7 a + 1.1e-7 more than before (1 + 4e-6 keeps a_hi an upper
+// bound up to u = 18, past which a < 2e-8).  The power 2^(e L), L = lg2(1 - a): for
+// |L| >= 1 its exponent's relative error 3e-7 gives 0.37 3e-7 = 1.1e-7, for |L| < 1 the
+// absolute error gives e 2^-22 ln 2 (1 - a)^e <= slope_e 1.65e-7, and the ex2 2.4e-7
+// with the last rounding 6e-8.  A base of 0 gives a1 = 1, a negative one (a > 1) a NaN:
+// both have a_hi >= 1.
 
 // the byte as the low bits of a float in [2^23, 2^23 + 256): clamped to [0, 1]
 // (a NaN to 0: its pair is never decided), the truncation an addition rounded down
@@ -739,6 +775,7 @@ __device__ __forceinline__ uint32_t alpha_byte_bits(float v)
 
 // the byte in bits 24-31, the rest 0 (w3: the Gaussian's WalkRec::w3); most: the
 // largest byte it can be, likewise (also where it is not decided)
+template <bool APPROX>
 __device__ __forceinline__ uint32_t alpha_byte_bound(const float4& q6, float cull, const AlphaF& f, const float4& w3,
                                                      bool& decided, uint32_t& most)
 {
@@ -746,14 +783,15 @@ __device__ __forceinline__ uint32_t alpha_byte_bound(const float4& q6, float cul
         f.p[0], w3.x, VOX_FFMA(f.p[1], w3.y, VOX_FFMA(f.p[2], w3.z, VOX_FFMA(0x1.02p-20f, f.d, fabsf(w3.w)))));
     const float ls = q6.y, e = q6.z;
     const float x = ls * md;
-    const float a_hi = VOX_FFMA(2.f * x, f.a, f.a) * (1.f + 1e-6f); // e^x <= 1 + 2x for x <= 1
+    const float a_hi = VOX_FFMA(2.f * x, f.a, f.a) * (APPROX ? 1.f + 4e-6f : 1.f + 1e-6f); // e^x <= 1 + 2x for x <= 1
     float slope_e = e; // the pow's slope bound
     if (e < 1.f)       // (a Gaussian of more than 10 voxels: few warps have one)
         // 1 / (1 - a_hi) from the fast reciprocal (within 2 ulp for 1 - a_hi >= 2^-24,
         // as it is when a_hi < 1), raised by 2^-20 so it stays an upper bound
         slope_e = e * (__fdividef(1.f, 1.f - a_hi) * (1.f + 0x1p-20f));
     // slope_e (ls a_hi 1.25 md + 1.1e-6 a_hi + 1.8e-7) + 9.3e-7
-    const float delta = VOX_FFMA(slope_e, VOX_FFMA(a_hi, VOX_FFMA(1.25f, x, 1.1e-6f), 1.8e-7f), 9.3e-7f);
+    const float delta = APPROX ? VOX_FFMA(slope_e, VOX_FFMA(a_hi, VOX_FFMA(1.25f, x, 1.6e-6f), 4.6e-7f), 1.4e-6f)
+                               : VOX_FFMA(slope_e, VOX_FFMA(a_hi, VOX_FFMA(1.25f, x, 1.1e-6f), 1.8e-7f), 9.3e-7f);
     const uint32_t lo = alpha_byte_bits(f.a1 - delta), hi = alpha_byte_bits(f.a1 + delta);
     const bool culled = cull != 0.f; // culled by scale: both alphas are 0
     const bool bounded = x < 0.25f && a_hi < 1.f;

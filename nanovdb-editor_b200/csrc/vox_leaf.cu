@@ -410,9 +410,7 @@ struct LeafQSmem
     LeafAcc acc;
     uint32_t mask[3][16]; // value masks of the leaf being tested and of the two before it
     uint16_t queue[2][lf_cap<SMOOTH>];
-    uint32_t defer[LP_THREADS / 32][64]; // per warp: the leaf's pairs whose RGBA8 byte the bound left open
-    uint32_t dcount[LP_THREADS / 32];     // per warp: the open pairs left at the leaf's end
-    uint32_t dfin;                        // warps done with the leaf's alpha
+    uint32_t defer[SMOOTH ? 1 : LP_THREADS / 32][64]; // per warp: the leaf's pairs whose RGBA8 byte is open
     uint32_t qn[3];
     int32_t nxt_o[2][3]; // the next chunk (by phase parity): leaf origin, sorted pair range and count
     uint32_t nxt_q0[2], nxt_p1[2], nxt_cnt[2];
@@ -774,7 +772,6 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
         S.cand = atomicAdd(counter, 1u);
         S.cand_next[0] = atomicAdd(counter, 1u);
         S.qn[0] = S.qn[1] = S.qn[2] = 0;
-        S.dfin = 0;
         S.acc.wmin = ~0ull;
     }
     for (int i = t; i < 9 * 512; i += LP_THREADS) // the sums and the RGBA8 maxima
@@ -902,11 +899,15 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 S.mask[fm][t] = 0; // filled again by the leaf after next, from the next phase on
         }
         const uint32_t a_rounds = a_valid ? (S.qn[ab] + 31u) / 32u : 0u; // the alpha's rounds of 32 pairs
-        // ---- alpha of the previous chunk, one queued pair per thread.  A pair
-        // whose RGBA8 byte the bound leaves open (1 - 2%) is deferred to its
-        // warp's list, which lasts through the leaf, and the reference's byte is
-        // evaluated 32 pairs at a time (from the records in global memory), so the
-        // rare branch costs one converged pass per 32 pairs.
+        // ---- alpha of the previous chunk, one queued pair per thread.  A pair whose
+        // RGBA8 byte the bound leaves open (1 - 2%) and that may be its voxel's
+        // maximum goes to its warp's list, which lasts through the leaf, and the
+        // reference's byte is evaluated 32 pairs at a time (from the records in global
+        // memory) or at the leaf's end, each warp its own: one warp taking all that
+        // were left held the others up at the barrier (walk of 4999 Gaussians 120 us,
+        // now 111; of 64 clouds 8.11 ms, now 7.88; with each pair evaluated on the spot
+        // 102 us and 8.00 ms, but 100k 600 us for 565).  The smooth mode, whose records
+        // are in shared memory, evaluates on the spot (500k 2.14 -> 2.05 ms).
         if (a_valid)
         {
             const LeafChunk<SMOOTH>& C = S.ch[ab];
@@ -915,7 +916,7 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
             const uint32_t qn = S.qn[ab];
             if (t == 0)
                 leaf_pairs += qn;
-            uint32_t* dq = S.defer[warp];
+            uint32_t* dq = S.defer[SMOOTH ? 0 : warp];
             // the reference's byte of voxel n and the leaf's Gaussian at position l of its pairs
             auto ref_byte = [&](uint32_t l, uint32_t n) {
                 const uint32_t g = P.pair_gid[aleaf0 + l];
@@ -933,9 +934,34 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                 {
                     q = queue[e];
                     const uint32_t j = q >> 9, n = q & 511u;
-                    const float4 al = C.al[j], q7 = C.q7[j], w3 = C.walk[3][j];
+                    const float4 al = C.al[j], q7 = C.q7[j], w3 = C.walk[3][j], w0 = C.walk[0][j], w1 = C.walk[1][j],
+                                 w2 = C.walk[2][j], aa = C.aa[j], q6 = C.q6[j];
                     float a;
-                    uint32_t a8;
+                    AlphaF af;
+                    {
+                        const float lo0[3] = { al.x, al.y, al.z }, W4[3] = { w1.w, w2.w, aa.w };
+                        const float h[3][3] = { { w0.x, w1.x, w2.x }, { w0.y, w1.y, w2.y }, { w0.z, w1.z, w2.z } };
+                        // twice the voxels from the anchor, exactly (a last place is 2 from 2^24 on)
+                        const float fx = VOX_FSUB(__uint_as_float(0x4b800000u | (n >> 6)), aa.x),
+                                    fy = VOX_FSUB(__uint_as_float(0x4b800000u | ((n >> 3) & 7u)), aa.y),
+                                    fz = VOX_FSUB(__uint_as_float(0x4b800000u | (n & 7u)), aa.z);
+                        const Aabb box = stable_leaf_aabb(lo0, W4, h, fx, fy, fz);
+                        if constexpr (SMOOTH)
+                            af = pair_alpha_approx(q6, box);
+                        else
+                            af = pair_alpha_f_ex(q6, box);
+                    }
+                    bool decided;
+                    uint32_t most;
+                    uint32_t a8 = alpha_byte_bound<SMOOTH>(q6, q7.w, af, w3, decided, most);
+                    // an open pair that cannot exceed the voxel's maximum so far needs no byte
+                    // (a8 <= most: the maximum below changes nothing).  Of a voxel's k-th pair
+                    // that holds but for about one in k: the walk of 2M Gaussians 26.8 -> 26.1 ms
+                    defer = !decided && *(volatile uint32_t*)&A.rgba[n] < (most | __float_as_uint(al.w));
+                    if (CHECK && decided &&
+                        a8 >> 24 != ref_alpha_byte(P.recs[C.gid[j]], P.walk[C.gid[j]].w5.z, ao[0] + (int32_t)(n >> 6),
+                                                   ao[1] + (int32_t)((n >> 3) & 7), ao[2] + (int32_t)(n & 7)))
+                        atomicOr(P.err, ERR_BOUNDS); // the margin failed to cover the reference's byte
                     if constexpr (SMOOTH)
                     {
                         const int32_t x = ao[0] + (int32_t)(n >> 6), yy = ao[1] + (int32_t)((n >> 3) & 7),
@@ -945,36 +971,19 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         R.q1 = C.rec[1][j];
                         R.q2 = C.rec[2][j];
                         R.q3 = C.rec[3][j];
-                        R.q6 = C.q6[j];
-                        R.q7 = q7;
                         const float mu[3] = { R.q0.x, R.q0.y, R.q0.z }, inv_s[3] = { R.q3.y, R.q3.z, R.q3.w };
                         SmoothTerms st;
-                        a = smooth_kernel(mu, inv_s, R.q6.x, rinv_of(R), C.vs[j], C.exact_d[j] != 0u, x, yy, zz, st);
-                        a8 = ref_alpha_byte(R, C.vs[j], x, yy, zz) << 24;
+                        a = smooth_kernel(mu, inv_s, q6.x, rinv_of(R), C.vs[j], C.exact_d[j] != 0u, x, yy, zz, st);
+                        if (defer) // the records are at hand
+                        {
+                            R.q6 = q6;
+                            R.q7 = q7;
+                            a8 = ref_alpha_byte(R, C.vs[j], x, yy, zz) << 24;
+                            defer = false;
+                        }
                     }
                     else
-                    {
-                        const float4 w0 = C.walk[0][j], w1 = C.walk[1][j], w2 = C.walk[2][j], aa = C.aa[j], q6 = C.q6[j];
-                        const float lo0[3] = { al.x, al.y, al.z }, W4[3] = { w1.w, w2.w, aa.w };
-                        const float h[3][3] = { { w0.x, w1.x, w2.x }, { w0.y, w1.y, w2.y }, { w0.z, w1.z, w2.z } };
-                        // twice the voxels from the anchor, exactly (a last place is 2 from 2^24 on)
-                        const float fx = VOX_FSUB(__uint_as_float(0x4b800000u | (n >> 6)), aa.x),
-                                    fy = VOX_FSUB(__uint_as_float(0x4b800000u | ((n >> 3) & 7u)), aa.y),
-                                    fz = VOX_FSUB(__uint_as_float(0x4b800000u | (n & 7u)), aa.z);
-                        const AlphaF af = pair_alpha_f_ex(q6, stable_leaf_aabb(lo0, W4, h, fx, fy, fz));
                         a = q7.w != 0.f ? 0.f : af.a1;
-                        bool decided;
-                        uint32_t most;
-                        a8 = alpha_byte_bound(q6, q7.w, af, w3, decided, most);
-                        // an open pair that cannot exceed the voxel's maximum so far needs no byte
-                        // (a8 <= most: the maximum below changes nothing).  Of a voxel's k-th pair
-                        // that holds but for about one in k: the walk of 2M Gaussians 26.8 -> 26.1 ms
-                        defer = !decided && *(volatile uint32_t*)&A.rgba[n] < (most | __float_as_uint(al.w));
-                        if (CHECK && decided &&
-                            a8 >> 24 != ref_alpha_byte(P.recs[C.gid[j]], P.walk[C.gid[j]].w5.z, ao[0] + (int32_t)(n >> 6),
-                                                       ao[1] + (int32_t)((n >> 3) & 7), ao[2] + (int32_t)(n & 7)))
-                            atomicOr(P.err, ERR_BOUNDS); // the margin failed to cover the reference's byte
-                    }
                     if (!defer)
                         atomicMax(&A.rgba[n], a8 | __float_as_uint(al.w));
                     const float c0 = VOX_FMUL(a, q7.x), c1 = VOX_FMUL(a, q7.y), c2 = VOX_FMUL(a, q7.z);
@@ -1008,83 +1017,49 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                             atomicMin(&A.wmin, wk);
                     }
                 }
-                // a list entry holds the pair's position among the leaf's pairs in 23 bits;
-                // a leaf of more pairs evaluates the rest at once
-                const uint32_t l = alocal + (q >> 9);
-                if (defer && l >= 1u << 23)
+                if constexpr (!SMOOTH)
                 {
-                    ref_byte(l, q & 511u);
-                    defer = false;
-                }
-                const uint32_t bal = __ballot_sync(0xffffffffu, defer);
-                if (bal)
-                {
-                    if (defer)
-                        dq[dn + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = l << 9 | (q & 511u);
-                    dn += (uint32_t)__popc(bal);
-                    if (dn >= 32u) // dn <= 63: a batch of 32, the rest moved to the front
+                    // a list entry holds the pair's position among the leaf's pairs in 23 bits;
+                    // a leaf of more pairs evaluates the rest at once
+                    const uint32_t l = alocal + (q >> 9);
+                    if (defer && l >= 1u << 23)
                     {
-                        __syncwarp();
-                        const uint32_t d = dq[lane];
-                        ref_byte(d >> 9, d & 511u);
-                        const uint32_t rest = dn - 32u;
-                        const uint32_t mv = (uint32_t)lane < rest ? dq[32 + lane] : 0u;
-                        __syncwarp();
-                        if ((uint32_t)lane < rest)
-                            dq[lane] = mv;
-                        __syncwarp();
-                        dn = rest;
+                        ref_byte(l, q & 511u);
+                        defer = false;
+                    }
+                    const uint32_t bal = __ballot_sync(0xffffffffu, defer);
+                    if (bal)
+                    {
+                        if (defer)
+                            dq[dn + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = l << 9 | (q & 511u);
+                        dn += (uint32_t)__popc(bal);
+                        if (dn >= 32u) // dn <= 63: a batch of 32, the rest moved to the front
+                        {
+                            __syncwarp();
+                            const uint32_t d = dq[lane];
+                            ref_byte(d >> 9, d & 511u);
+                            const uint32_t rest = dn - 32u;
+                            const uint32_t mv = (uint32_t)lane < rest ? dq[32 + lane] : 0u;
+                            __syncwarp();
+                            if ((uint32_t)lane < rest)
+                                dq[lane] = mv;
+                            __syncwarp();
+                            dn = rest;
+                        }
                     }
                 }
             }
-            // at the leaf's end, the open pairs left in every warp's list (fewer than 32
-            // each): the last warp to finish evaluates all of them, 32 at a time
-            if (a_leaf_end)
+            // at the leaf's end, the open pairs left in the warp's list (fewer than 32)
+            if (a_leaf_end && dn)
             {
-                uint32_t fin = 0;
-                if (lane == 0)
+                __syncwarp();
+                if ((uint32_t)lane < dn)
                 {
-                    S.dcount[warp] = dn;
-                    __threadfence_block();
-                    fin = atomicAdd(&S.dfin, 1u);
+                    const uint32_t d = dq[lane];
+                    ref_byte(d >> 9, d & 511u);
                 }
                 dn = 0;
-                fin = __shfl_sync(0xffffffffu, fin, 0);
-                if (fin == LP_THREADS / 32 - 1)
-                {
-                    __threadfence_block();
-                    const uint32_t c = (uint32_t)lane < LP_THREADS / 32 ? *(volatile uint32_t*)&S.dcount[lane] : 0u;
-                    uint32_t incl = c;
-#pragma unroll
-                    for (int off = 1; off < LP_THREADS / 32; off <<= 1)
-                    {
-                        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-                        if (lane >= off)
-                            incl += y;
-                    }
-                    const uint32_t total = __shfl_sync(0xffffffffu, incl, LP_THREADS / 32 - 1);
-                    for (uint32_t b = 0; b < total; b += 32)
-                    {
-                        const uint32_t item = b + (uint32_t)lane;
-                        // the warp list holding item: the first w whose inclusive count exceeds it
-                        uint32_t w = 0, before = 0;
-#pragma unroll
-                        for (int v = 0; v < LP_THREADS / 32; v++)
-                        {
-                            const uint32_t iv = __shfl_sync(0xffffffffu, incl, v);
-                            const bool past = item >= iv;
-                            w += past ? 1u : 0u;
-                            before = past ? iv : before;
-                        }
-                        if (item < total)
-                        {
-                            const uint32_t d = *(volatile uint32_t*)&S.defer[w][item - before];
-                            ref_byte(d >> 9, d & 511u);
-                        }
-                    }
-                    if (lane == 0)
-                        S.dfin = 0;
-                }
+                __syncwarp();
             }
         }
         // ---- test of this chunk

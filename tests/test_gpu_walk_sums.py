@@ -53,3 +53,23 @@ def test_walk_matches_oracle(vox_ctx, oracle_mod, kind, n, vs):
     np.testing.assert_array_equal(k_got, k_ref)
     np.testing.assert_array_equal(i_got, i_ref)
     ref.close()
+
+
+@pytest.mark.parametrize("check", [False, True])
+@pytest.mark.parametrize("kind", ["colors", "opaque", "stack", "thin", "far"])
+def test_differentiable_walk_keeps_the_bytes(oracle_mod, monkeypatch, kind, check):
+    """The differentiable channels' walk decides the RGBA8 alpha from its own, approximate
+    evaluation; the bytes are the oracle's.  check: every decided byte against the
+    reference's evaluation on the device."""
+    from nanovdb_editor.vox import FLAG_DIFFERENTIABLE, VoxContext
+
+    if check:
+        monkeypatch.setenv("VOX_CHECK_EMIT", "1")
+    ctx = VoxContext(0)
+    for n, vs in ((13, 0.01), (700, 0.004)):
+        c = _cloud(kind, n, vs, n + 1)
+        g = ctx.voxelize_host(*[c[k] for k in NAMES], vs, 100.0, FLAG_DIFFERENTIABLE)
+        ref = oracle_mod.OracleResult(c, vs, 100.0, window_mode=0)
+        np.testing.assert_array_equal(g.rgba8, ref.values()["rgba8"])
+        ref.close()
+    ctx.close()
