@@ -112,6 +112,7 @@ struct vox_context_t
     int64_t last_V = -1; // -1: no successful call yet
     uint64_t last_value_count = 0;
     uint32_t last_flags = 0;
+    bool rgba8_only = false; // context_rgba8_only
     float last_voxel_size = 0.f;
     NodeParams last_N{};
     LeafPassParams last_LP{};
@@ -435,6 +436,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     ctx->diff_ready = false;
     ctx->last_V = -1;
     const bool diff = (flags & VOX_FLAG_DIFFERENTIABLE) != 0;
+    const bool bytes = ctx->rgba8_only && !diff; // no float channels
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
     const int64_t G = gs->count;
@@ -683,7 +685,8 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     // ------------------------------------------------------------ leaf walk
     const size_t slots = 512 * (size_t)(NCL + 1);
     if (!ensure(ctx, ctx->cand_mask, 64 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->s_rgba, 4 * slots) ||
-        !ensure(ctx, ctx->s_dens, 4 * slots) || !ensure(ctx, ctx->s_col, 12 * slots) || !ensure(ctx, ctx->cand_pairs, 8 * (size_t)(NCL + 1)) ||
+        (!bytes && (!ensure(ctx, ctx->s_dens, 4 * slots) || !ensure(ctx, ctx->s_col, 12 * slots))) ||
+        !ensure(ctx, ctx->cand_pairs, 8 * (size_t)(NCL + 1)) ||
         !ensure(ctx, ctx->cand_voff, 8 * (size_t)(NCL + 1)) || !ensure(ctx, ctx->cand_vbase, 8 * (size_t)(NCL + 1)))
         return VOX_ERR_MEMORY;
     uint64_t* win_before = nullptr;
@@ -719,10 +722,11 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LP.voxel_size = voxel_size;
     LP.cloud_vs = d_cloud_vs;
     LP.smooth = diff ? 1 : 0;
+    LP.bytes = bytes ? 1 : 0;
     LP.cand_mask = (uint64_t*)ctx->cand_mask.p;
     LP.s_rgba = (uint32_t*)ctx->s_rgba.p;
-    LP.s_dens = (float*)ctx->s_dens.p;
-    LP.s_col = (float*)ctx->s_col.p;
+    LP.s_dens = bytes ? nullptr : (float*)ctx->s_dens.p;
+    LP.s_col = bytes ? nullptr : (float*)ctx->s_col.p;
     LP.cand_pairs = (uint64_t*)ctx->cand_pairs.p;
     LP.total_pairs = sc + SC_P;
     LP.err = d_err;
@@ -730,7 +734,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LP.cand_voff = (const uint64_t*)ctx->cand_voff.p;
     LP.key64 = key64;
     ctx->walk_mode = (LP.window ? 1 : 0) | (LP.smooth ? 2 : 0); // the modes differ in cost per pair
-    ctx->walk_variant = ctx->walk_choice[ctx->walk_mode].pick((int64_t)Q);
+    ctx->walk_variant = bytes ? 0 : ctx->walk_choice[ctx->walk_mode].pick((int64_t)Q);
     ctx->stats.walk_ctas_per_sm = launch_leaf_pass(LP, ctr(CTR_WALK), ctx->num_sms, s, ctx->walk_variant);
     cudaEventRecord(ctx->timers.ev[4], s);
 
@@ -786,6 +790,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         C.F_total = sc + SC_F;
         C.G = G;
         C.node_order = (flags & VOX_FLAG_WINDOW_ORDER) ? 1u : 0u;
+        C.floats = bytes ? 0 : 1;
         if (NCL == 0) // no candidate, no tables: every cloud starts (and ends) at 0
         {
             cudaMemsetAsync(C.vstart, 0, 8 * (size_t)(B + 1), s);
@@ -891,7 +896,8 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     st.ms_emit = elapsed(ctx->timers.ev[1], ctx->timers.ev[2]);       // (leaf, Gaussian) pairs
     st.ms_sort = elapsed(ctx->timers.ev[2], ctx->timers.ev[3]);       // sort + candidate leaves
     st.ms_accumulate = elapsed(ctx->timers.ev[3], ctx->timers.ev[4]); // leaf walk: test, RGBA8, float sums
-    ctx->walk_choice[ctx->walk_mode].report((int64_t)Q, ctx->walk_variant, st.ms_accumulate);
+    if (!bytes)
+        ctx->walk_choice[ctx->walk_mode].report((int64_t)Q, ctx->walk_variant, st.ms_accumulate);
     st.ms_build = elapsed(ctx->timers.ev[4], ctx->timers.ev[6]);      // topology, values, node2
     st.ms_total = elapsed(ctx->timers.ev[0], ctx->timers.ev[6]);
     st.kernel_launches = launch_count() - launches0;
@@ -1007,6 +1013,11 @@ __global__ void k_export_keys(const void* keys, int key64, const uint32_t* lower
 // ---------------------------------------------------------------------------
 // vox_* C ABI
 // ---------------------------------------------------------------------------
+void vox::context_rgba8_only(vox_context_t* ctx)
+{
+    ctx->rgba8_only = true;
+}
+
 extern "C" {
 
 vox_context_t* vox_context_create(int device)

@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include "pnanovdb_b200.h"
+#include "vox_internal.h"
 
 // ------------------------------------------------------------- queue / device
 // A queue is a CUDA device plus its own voxelization context (one stream and
@@ -102,7 +103,11 @@ static pnanovdb_compute_queue_t* resolve_queue(pnanovdb_compute_queue_t* q)
 static vox_context_t* queue_context(pnanovdb_compute_queue_t* q)
 {
     if (!q->vox)
+    {
         q->vox = vox_context_create(q->device);
+        if (q->vox)
+            vox::context_rgba8_only(q->vox); // run_host copies no more
+    }
     return q->vox;
 }
 
@@ -373,6 +378,7 @@ static pnanovdb_raster_context_t* PNANOVDB_ABI r_create_context(const pnanovdb_c
         vox_context_t* v = vox_context_create(queue_device(queue));
         if (!v)
             return nullptr;
+        vox::context_rgba8_only(v); // raster_gaussian_3d copies no more
         pnanovdb_raster_context_t* c = new pnanovdb_raster_context_t();
         c->vox = v;
         return c;

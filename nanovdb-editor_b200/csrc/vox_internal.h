@@ -6,8 +6,14 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+struct vox_context_t;
+
 namespace vox
 {
+
+// The context's grids get no float channels (offsets 0 in the header): for callers that
+// copy them out with vox_copy_grid_rgba8 only.
+void context_rgba8_only(vox_context_t* ctx);
 
 // number of kernels this library has launched (all contexts, all threads)
 int64_t launch_count();

@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(1024) k_cloud_layout(NodeParams N)
             o_rgba = al256(o_bbox + 32);
             o_dens = al256(o_rgba + 4 * vc);
             o_col = al256(o_dens + 4 * vc);
-            size = al256(o_col + 12 * vc);
+            size = C.floats ? al256(o_col + 12 * vc) : o_dens;
             for (int a = 0; a < 6; a++)
                 C.bbox[6 * b + a] = a < 3 ? 0x7FFFFFFF : (int32_t)0x80000000;
         }
@@ -578,8 +578,8 @@ __device__ __forceinline__ void write_grid_header(const NodeParams& N, uint64_t 
         h.value_count = vc;
         h.bbox_offset = C.bbox_off[b] - g;
         h.rgba8_offset = C.rgba_off[b] - g;
-        h.density_offset = C.dens_off[b] - g;
-        h.color_offset = C.col_off[b] - g;
+        h.density_offset = C.floats ? C.dens_off[b] - g : 0;
+        h.color_offset = C.floats ? C.col_off[b] - g : 0;
         h.voxel_size = C.cloud_vs ? C.cloud_vs[b] : C.voxel_size;
         if (vc > 2)
             for (int a = 0; a < 6; a++)
@@ -596,6 +596,11 @@ __device__ __forceinline__ void write_grid_header(const NodeParams& N, uint64_t 
         ((int32_t*)(out + C.bbox_off[b]))[threadIdx.x] = h.bbox[threadIdx.x];
     zero_words(out, g + VOX_GRID_HEADER_BYTES + C.node2_bytes[b], C.bbox_off[b]);
     zero_words(out, C.bbox_off[b] + 24, C.rgba_off[b] + 8);
+    if (!C.floats)
+    {
+        zero_words(out, C.rgba_off[b] + 4 * vc, C.grid_off[b + 1]);
+        return;
+    }
     zero_words(out, C.rgba_off[b] + 4 * vc, C.dens_off[b] + 8);
     zero_words(out, C.dens_off[b] + 4 * vc, C.col_off[b] + 24);
     zero_words(out, C.col_off[b] + 12 * vc, C.grid_off[b + 1]);

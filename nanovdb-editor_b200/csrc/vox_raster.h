@@ -55,6 +55,7 @@ struct CloudParams
     const uint64_t* cloud_pairs; // [B] passing pairs per cloud (null: one cloud, P)
     int64_t G, P, V;
     uint32_t node_order;
+    int floats;                  // the grid has the float density / colour channels
 };
 
 struct NodeParams
@@ -140,9 +141,10 @@ struct LeafPassParams
     float voxel_size;
     const float* cloud_vs;
     int smooth;
+    int bytes;                 // the RGBA8 values alone
     uint64_t* cand_mask;       // [NCL][8]
     uint32_t* s_rgba;          // staging [NCL * 512]
-    float* s_dens;
+    float* s_dens;             // (null with bytes, as s_col)
     float* s_col;              // [NCL * 512][3]
     uint64_t* cand_pairs;      // [NCL] passing pairs
     uint64_t* total_pairs;
