@@ -930,11 +930,11 @@ def main():
     A = 56
     # algorithmic bytes per stage: what each stage must read and write once
     stage_bytes = {
-        "prep": G * (A + 128 + 8),  # raw attributes in, record + footprint out
-        "leaf_pairs": 2 * G * 128 + 12 * Q,  # records read by the count and write passes, (key, index, id) out
+        "prep": G * (A + 224 + 16),  # raw attributes in, record + walk record + footprint + columns out
+        "leaf_pairs": 2 * G * 128 + 8 * Q,  # records read by the count and write passes, (key, id) out
         "sort": Q * (4 + 16 * passes),  # histogram read + per pass read/write (key, value)
-        "leaf_walk": 8 * Q + 128 * Q + 72 * NCL + 24 * V,  # pair lists, record gathers, masks, staged values
-        "tree_values": 60 * V,  # voxel keys, runs, node tables, values
+        "leaf_walk": 4 * Q + 224 * Q + 72 * NCL + 20 * V,  # pair lists, record gathers, masks, staged values
+        "tree_values": 40 * V + 64 * NCL,  # staged values to the grid, masks
     }
     stage_ms = {
         "prep": float(np.mean([s["ms_prep"] for s in stats])),

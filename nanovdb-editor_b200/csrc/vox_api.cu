@@ -5,9 +5,9 @@
 // 256K-prim x 8M-fragment windows with a per-window queue flush and a
 // frame-lagged readback of the fragment total (raster/Raster.cpp:420-558,
 // raster/GridBuild.cpp:830-942).  Here one call runs the whole chain on one
-// CUDA stream with three small read-backs (candidate count, pair count, node
-// counts) that size the buffers; buffers persist in the context and only
-// grow, so repeated calls allocate nothing.
+// CUDA stream; five times the host waits for counts that size the next buffers
+// (sync_scalars).  Buffers persist in the context and only grow, so repeated
+// calls allocate nothing.
 #include <algorithm>
 #include <atomic>
 #include <cmath>

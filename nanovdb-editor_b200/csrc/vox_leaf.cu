@@ -11,12 +11,11 @@
 //       (leaf key, Gaussian) in Gaussian-major order; a stable sort by leaf key
 //       keeps each leaf's Gaussians in ascending id;
 //   k_leaf_cands  runs of equal leaf keys -> candidate leaves;
-//   k_leaf_pass   one CTA per candidate leaf, one thread per voxel (two per
-//       thread): the CTA walks the leaf's Gaussians in ascending id and every
-//       thread runs the reference test (gaussian_frag_alloc.slang:84-162) on
-//       its voxels, keeps the RGBA8 maximum (gaussian_frag_color.slang:239-246)
-//       and sums the float channels in (voxel key, Gaussian id) order; the
-//       leaf's value mask comes from ballots;
+//   k_leaf_pass   persistent CTAs over the candidate leaves, a leaf's Gaussians
+//       in chunks: the test (gaussian_frag_alloc.slang:84-162) one (Gaussian, box
+//       column) per thread, which sets the leaf's value mask, then the passing
+//       pairs' RGBA8 maximum (gaussian_frag_color.slang:239-246) and float sums,
+//       one pair per thread, in any order;
 //   k_write_leaves   once the tree's tables stand (k_tree): staged values to
 //       their value index, leaf nodes, bbox.
 // The adjoint (k_leaf_backward) and the sorted pair list (k_leaf_export)
@@ -510,7 +509,7 @@ __device__ __forceinline__ uint32_t column_test(const float4& q0, const float4& 
 // and their voxels set in mask (the leaf's value mask as 32-bit words).  The
 // results are voxel_local_aabb + aabb_hits_unit_sphere per voxel, decided where
 // possible from the float channels' local AABB as centre and half width
-// (leaf_pair_consts; per row x = max(|c| - h, 0) is the AABB's point nearest to
+// (leaf_consts; per row x = max(|c| - h, 0) is the AABB's point nearest to
 // zero, 1-Lipschitz in c and h).  Per row that is within delta_r = 1.5 dab_r of
 // the reference's, so the vectors of the three differ by eta <= Delta = sum
 // delta_r in norm.  The reference passes a voxel when its fl-evaluated 1 - S >

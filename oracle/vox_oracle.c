@@ -317,7 +317,7 @@ static float fx_to_float(int64_t s)
  *   lattice points lo + w (hi - lo), w = 0, 1/3, 2/3, 1; the maximum of the
  *     decreasing exp is at the per-axis smallest square;
  *   float exp / pow (vox_expf_ch, vox_powf_ch).
- * The device evaluates the same operations in the same order (leaf_pair_consts,
+ * The device evaluates the same operations in the same order (leaf_consts,
  * stable_leaf_aabb); the signs of zero sums may differ, which the squares hide. */
 static float frag_alpha_f(const prim_t* P, const float rinv[3][3], float vs, const int32_t* ijk, float cull_scale)
 {
