@@ -93,17 +93,22 @@ __device__ __forceinline__ bool leaf_may_hit(const GaussRec& R, const RInv& M, f
     return sum < bound * bound;
 }
 
-__device__ __forceinline__ uint32_t leaf_key_of(const GaussRec& R, int32_t x, int32_t y, int32_t z,
-                                                const uint64_t* root_bits, const uint64_t* root_prefix,
-                                                const uint64_t* lower_bits, const uint64_t* lower_prefix)
+// the same from the record in global memory, out of line: for the write pass, which
+// needs it in columns of more than 32 leaves alone
+__device__ __noinline__ bool leaf_may_hit_at(const GaussRec* rec, float vsf, int32_t ox, int32_t oy, int32_t oz)
 {
-    const uint64_t rr = bit_rank(root_bits, root_prefix, root_index(rec_cloud(R), x, y, z));
-    const uint64_t cell = rr * 32768ull + upper_n_of(x, y, z);
-    const uint64_t lr = bit_rank(lower_bits, lower_prefix, cell);
-    return (uint32_t)((lr << 12) | lower_n_of(x, y, z));
+    const GaussRec R = *rec;
+    return leaf_may_hit(R, rinv_of(R), vsf, ox, oy, oz);
 }
 
-// one thread per leaf column (lx, ly) of a Gaussian's bbox, looping over lz
+// rank of the lower node of voxel (x, y, z) of a cloud, at its place in the leaf's key
+__device__ __forceinline__ uint32_t lower_key_of(uint32_t cloud, int32_t x, int32_t y, int32_t z, const RankTables& T)
+{
+    const uint64_t rr = bit_rank(T.root_bits, T.root_prefix, root_index(cloud, x, y, z));
+    const uint64_t cell = rr * 32768ull + upper_n_of(x, y, z);
+    return (uint32_t)(bit_rank(T.lower_bits, T.lower_prefix, cell) << 12);
+}
+
 // the Gaussian of each 256-column tile's first column
 __global__ void k_tile_gauss(const uint64_t* lcol_off, int64_t G, uint64_t NLC, int64_t* tile_g0)
 {
@@ -112,11 +117,16 @@ __global__ void k_tile_gauss(const uint64_t* lcol_off, int64_t G, uint64_t NLC, 
         tile_g0[tile] = upper_bound_u64_l(lcol_off, 0, G, tile * 256) - 1;
 }
 
+// One thread per leaf column (lx, ly) of a Gaussian's bbox, looping over lz.  Bound by
+// the latency of the records' loads and of the double-precision chains, so by the CTAs an
+// SM holds: the count pass 4 (64 registers), the write pass, which reads the box alone, 6.
+// Both passes of 2M Gaussians' 29.6M pairs with their scan 1.34 -> 1.14 ms, 64 clouds 0.576
+// -> 0.493 (3 CTAs each before; count 5: 1.18 ms, 6: 1.23; write 4: 1.21 with count 5).
 // Blocks walk 256-column tiles; a tile's Gaussians [g0, g1] (g1 = the next
 // tile's first) have their column offsets copied to shared memory, where each
 // thread finds its column's Gaussian.
 template <bool WRITE>
-__global__ void __launch_bounds__(256) k_leaf_emit(LeafEmitParams P, RankTables T)
+__global__ void __launch_bounds__(256, WRITE ? 6 : 4) k_leaf_emit(LeafEmitParams P, RankTables T)
 {
     __shared__ uint64_t s_off[257];
     const uint64_t ntiles = (P.NLC + 255) / 256;
@@ -147,8 +157,14 @@ __global__ void __launch_bounds__(256) k_leaf_emit(LeafEmitParams P, RankTables 
         }
         else
             g = upper_bound_u64_l(P.lcol_off, g0, g1 + 1, t) - 1;
-        const GaussRec R = P.recs[g];
-        const RInv M = rinv_of(R);
+        GaussRec R;
+        if (WRITE) // the box and the cloud
+        {
+            R.q4 = P.recs[g].q4;
+            R.q5 = P.recs[g].q5;
+        }
+        else
+            R = P.recs[g];
         const float vsf = rec_vs(R, P.voxel_size, P.cloud_vs);
         const int32_t lx0 = R.q4.x >> 3, ly0 = R.q4.y >> 3, ly1 = (R.q4.y + R.q5.y - 1) >> 3;
         const int32_t lz0 = R.q4.z >> 3, lz1 = (R.q4.z + R.q5.z - 1) >> 3;
@@ -159,19 +175,27 @@ __global__ void __launch_bounds__(256) k_leaf_emit(LeafEmitParams P, RankTables 
         uint64_t npairs = 0;
         // the write pass reuses the count pass's test results (first 32 leaves)
         const uint32_t known = WRITE ? P.lc_mask[t] : 0u;
-        uint32_t mask = 0;
+        uint32_t mask = 0, lower = 0;
+        int32_t lower_z = INT32_MIN;
         for (int32_t lz = lz0; lz <= lz1; lz++)
         {
             const int32_t oz = lz * 8;
             const int32_t i = lz - lz0;
-            const bool hit = (WRITE && i < 32) ? ((known >> i) & 1u) != 0u : leaf_may_hit(R, M, vsf, ox, oy, oz);
+            const bool hit = !WRITE    ? leaf_may_hit(R, rinv_of(R), vsf, ox, oy, oz)
+                             : i < 32 ? ((known >> i) & 1u) != 0u
+                                      : leaf_may_hit_at(&P.recs[g], vsf, ox, oy, oz);
             if (!WRITE && hit && i < 32)
                 mask |= 1u << i;
             if (hit || P.check)
             {
                 if (WRITE)
                 {
-                    P.keys[e] = leaf_key_of(R, ox, oy, oz, T.root_bits, T.root_prefix, T.lower_bits, T.lower_prefix);
+                    if (oz >> 7 != lower_z) // a lower node is 16 leaves of the column
+                    {
+                        lower_z = oz >> 7;
+                        lower = lower_key_of(rec_cloud(R), ox, oy, oz, T);
+                    }
+                    P.keys[e] = lower | lower_n_of(ox, oy, oz);
                     // the sort's value: the Gaussian itself, or the emission index where
                     // something is kept by it (the adjoint's rows, check mode's flags)
                     P.vals[e] = P.emit_gid ? (uint32_t)e : (uint32_t)g;
