@@ -1043,6 +1043,9 @@ vox_context_t* vox_context_create(int device)
         delete ctx;
         return nullptr;
     }
+    // Page-locked memory comes with any contents, another context's last publication
+    // among them; this context's numbers start at 1, so no word of 0 is one of them.
+    memset(ctx->hscal, 0, sizeof(uint64_t) * SC_SCRATCH * 8);
     for (auto& e : ctx->timers.ev)
         cudaEventCreate(&e);
     cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
