@@ -640,14 +640,21 @@ __global__ void __launch_bounds__(VB_THREADS) k_vb_ranges(const K* __restrict__ 
             }
             if (q == U - 1)
             {
+                // key 0 starts a run, so there is one, unless the look-back gave up and the
+                // prefix lacks it: nothing is written then (the call reports the wait)
                 const uint64_t runs = r + (head ? 1u : 0u);
-                R.range[2 * runs - 1] = (uint32_t)U;
-                if (U < N)
+                if (runs == 0)
+                    atomicOr(R.err, ERR_BOUNDS);
+                else
                 {
-                    R.range[2 * runs] = (uint32_t)U;
-                    R.range[2 * runs + 1] = (uint32_t)N;
+                    R.range[2 * runs - 1] = (uint32_t)U;
+                    if (U < N)
+                    {
+                        R.range[2 * runs] = (uint32_t)U;
+                        R.range[2 * runs + 1] = (uint32_t)N;
+                    }
+                    *R.total = runs + (U < N ? 1u : 0u);
                 }
-                *R.total = runs + (U < N ? 1u : 0u);
             }
             if (R.expand)
                 R.keys_out[q] = vb_expand(k[i], R);
