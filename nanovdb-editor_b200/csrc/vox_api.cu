@@ -945,7 +945,9 @@ static int run_backward(vox_context_t* ctx, const vox_gaussians_t* gs, const flo
     cudaStream_t s = ctx->stream;
     const int64_t launches0 = launch_count();
     const uint64_t Q = ctx->last_Q;
-    if (!ensure(ctx, ctx->partials, sizeof(float) * BWD_STRIDE * (size_t)(Q + 1)))
+    const bool raw = (ctx->last_flags & VOX_FLAG_RAW_INPUTS) != 0;
+    const size_t row = sizeof(float) * (raw ? bwd_stride<true> : bwd_stride<false>);
+    if (!ensure(ctx, ctx->partials, row * (size_t)(Q + 1)))
         return VOX_ERR_MEMORY;
     cudaEventRecord(ctx->timers.ev[0], s);
     cudaMemsetAsync((uint64_t*)ctx->scal.p + SC_ERR, 0, sizeof(uint64_t), s);
@@ -957,10 +959,10 @@ static int run_backward(vox_context_t* ctx, const vox_gaussians_t* gs, const flo
         LP.grad_density = grad_density;
         LP.grad_color = grad_color;
         LP.partials = partials;
-        launch_leaf_backward(LP, (int64_t)Q, s);
+        launch_leaf_backward(LP, (int64_t)Q, raw, s);
     }
     else
-        cudaMemsetAsync(partials, 0, sizeof(float) * BWD_STRIDE * (size_t)Q, s);
+        cudaMemsetAsync(partials, 0, row * (size_t)Q, s);
     BwdFinalParams F;
     memset(&F, 0, sizeof(F));
     F.partials = partials;
@@ -974,7 +976,7 @@ static int run_backward(vox_context_t* ctx, const vox_gaussians_t* gs, const flo
     F.scales = gs->scales;
     F.opacities = gs->opacities;
     F.colors = gs->colors;
-    F.raw = (ctx->last_flags & VOX_FLAG_RAW_INPUTS) ? 1 : 0;
+    F.raw = raw ? 1 : 0;
     F.bf16 = (ctx->last_flags & VOX_FLAG_BF16_INPUTS) ? 1 : 0;
     F.voxel_size = ctx->last_voxel_size;
     F.cloud_vs = ctx->last_cloud_vs;

@@ -1184,8 +1184,8 @@ __device__ __forceinline__ uint32_t mask_rank(const uint64_t* m, uint32_t n)
 // consecutive sorted pairs: their constants once, a pair per lane; then, in batches
 // of as many pairs as have boxes of BW_CAP voxels together, the forward's column
 // test (the same pairs pass) with the batch's columns packed into the lanes, and
-// pair by pair the passing voxels' terms a voxel per lane and the BWD_NACC sums
-// across the warp.  Every sum has a fixed order (deterministic, no atomics), and no
+// pair by pair the passing voxels' terms a voxel per lane and the pair's sums
+// across the warp.  RAW: 13 sums; without it, 19 (bwd_nacc).  Every sum has a fixed order (deterministic, no atomics), and no
 // warp waits for another.  Bound by instruction issue (70% of the slots; gathers of
 // the upstream gradients behind them): 0.78 ms for 200k Gaussians (1.17M pairs, 33M
 // voxel pairs).  With the columns tested pair by pair 16 clouds took 1.20 ms for
@@ -1209,30 +1209,36 @@ struct BwdWarp
 // v[0 .. N) summed across the warp's lanes: at each step lanes that differ in one
 // bit of their number split the values, so N + N / 2 + ... shuffles do for N.
 // Afterwards lane l holds the sum of value k(l) in v[0]; returns k(l) (>= N: none).
-template <int N>
-__device__ __forceinline__ int warp_sum_split(float* v, int lane)
+// (One instance per step, so that every index is a constant: as a loop over the
+// steps 19 values were selected by comparisons, 2,000 instructions per sum.)
+template <int N, int BIT = 16>
+__device__ __forceinline__ void warp_sum_steps(float* v, int lane, int& first, int& width)
 {
-    int first = 0; // first value of this lane's share
-    int width = N;
-#pragma unroll
-    for (int bit = 16, n = N; bit; bit >>= 1)
+    if constexpr (BIT > 0)
     {
-        const int half = (n + 1) / 2;
-        const bool up = (lane & bit) != 0;
+        constexpr int half = (N + 1) / 2;
+        const bool up = (lane & BIT) != 0;
 #pragma unroll
         for (int i = 0; i < half; i++)
         {
-            const float hi = half + i < n ? v[half + i] : 0.f;
+            const float hi = half + i < N ? v[half + i] : 0.f;
             const float give = up ? v[i] : hi;
-            v[i] = (up ? hi : v[i]) + __shfl_xor_sync(0xffffffffu, give, bit);
+            v[i] = (up ? hi : v[i]) + __shfl_xor_sync(0xffffffffu, give, BIT);
         }
         first += up ? half : 0;
         width = up ? width - half : min(width, half);
-        n = half;
+        warp_sum_steps<half, BIT / 2>(v, lane, first, width);
     }
+}
+template <int N>
+__device__ __forceinline__ int warp_sum_split(float* v, int lane)
+{
+    int first = 0, width = N; // this lane's share
+    warp_sum_steps<N>(v, lane, first, width);
     return width > 0 ? first : N;
 }
 
+template <bool RAW>
 __global__ void __launch_bounds__(BW_WARPS * 32) k_leaf_backward(LeafPassParams P, int64_t Q)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1397,9 +1403,10 @@ __global__ void __launch_bounds__(BW_WARPS * 32) k_leaf_backward(LeafPassParams 
             }
             const uint32_t end = S.qs[it + 1];
             const bool exact_d = (__float_as_uint(S.tb[it].y) >> 16) & 1u;
-            float acc[BWD_NACC];
+            constexpr int NACC = bwd_nacc<RAW>;
+            float acc[NACC];
 #pragma unroll
-            for (int k = 0; k < BWD_NACC; k++)
+            for (int k = 0; k < NACC; k++)
                 acc[k] = 0.f;
             for (uint32_t p = S.qs[it] + (uint32_t)lane; p < end; p += 32)
             {
@@ -1437,17 +1444,28 @@ __global__ void __launch_bounds__(BW_WARPS * 32) k_leaf_backward(LeafPassParams 
                     acc[4] += f0 * st.z[0];
                     acc[5] += f1 * st.z[1];
                     acc[6] += f2 * st.z[2];
-                    acc[7] += f0 * st.z[1];
-                    acc[8] += f0 * st.z[2];
-                    acc[9] += f1 * st.z[2];
-                    acc[10] += Kw * gc[0];
-                    acc[11] += Kw * gc[1];
-                    acc[12] += Kw * gc[2];
+                    if constexpr (RAW)
+                    {
+                        acc[7] += f0 * st.z[1];
+                        acc[8] += f0 * st.z[2];
+                        acc[9] += f1 * st.z[2];
+                    }
+                    else
+#pragma unroll
+                        for (int a = 0; a < 3; a++)
+                        {
+                            acc[7 + a] += f0 * st.d[a];
+                            acc[10 + a] += f1 * st.d[a];
+                            acc[13 + a] += f2 * st.d[a];
+                        }
+                    acc[NACC - 3] += Kw * gc[0];
+                    acc[NACC - 2] += Kw * gc[1];
+                    acc[NACC - 1] += Kw * gc[2];
                 }
             }
-            const int k = warp_sum_split<BWD_NACC>(acc, lane);
-            if (k < BWD_NACC)
-                P.partials[(uint64_t)S.eidx[it] * BWD_STRIDE + k] = acc[0];
+            const int k = warp_sum_split<NACC>(acc, lane);
+            if (k < NACC)
+                P.partials[(uint64_t)S.eidx[it] * bwd_stride<RAW> + k] = acc[0];
             __syncwarp(); // the leaf's mask and, at the end, the queue are filled again
         }
     }
@@ -1789,14 +1807,15 @@ int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cu
                     : launch_walk<false, false, false, 4>(P, counter, num_sms, s);
 }
 
-void launch_leaf_backward(const LeafPassParams& P, int64_t Q, cudaStream_t s)
+void launch_leaf_backward(const LeafPassParams& P, int64_t Q, bool raw, cudaStream_t s)
 {
     if (Q <= 0)
         return;
     const size_t smem = sizeof(BwdWarp) * BW_WARPS;
-    cudaFuncSetAttribute(k_leaf_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto kern = raw ? k_leaf_backward<true> : k_leaf_backward<false>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int64_t per = 32 * BW_WARPS;
-    { k_leaf_backward<<<(unsigned)((Q + per - 1) / per), BW_WARPS * 32, smem, s>>>(P, Q); count_launch(); }
+    { kern<<<(unsigned)((Q + per - 1) / per), BW_WARPS * 32, smem, s>>>(P, Q); count_launch(); }
 }
 
 void launch_leaf_export(const LeafPassParams& P, uint64_t* vpairs, uint32_t* counter, int num_sms, cudaStream_t s)

@@ -80,10 +80,14 @@ struct NodeParams
     uint64_t *leaf_idx, *leaf_addr, *leaf_vidx;
 };
 
-// adjoint sums of a (leaf, Gaussian) pair (vox_backward.cu): [0] f, [1..3] f z_r, [4..6] f z_r^2,
-// [7..9] f z_0 z_1, f z_0 z_2, f z_1 z_2, [10..12] dL/d rgb, in rows of BWD_STRIDE floats
-constexpr int BWD_NACC = 13;
-constexpr int BWD_STRIDE = 16;
+// adjoint sums of a (leaf, Gaussian) pair (vox_backward.cu): [0] f, [1..3] f z_r, [4..6] f z_r^2, then
+// normalised quaternions (RAW): [7..9] f z_0 z_1, f z_0 z_2, f z_1 z_2
+// quaternions as given:         [7 + 3 r + a] f z_r d_a
+// and the last three dL/d rgb, in rows of bwd_stride floats (16-byte rows)
+template <bool RAW>
+constexpr int bwd_nacc = RAW ? 13 : 19;
+template <bool RAW>
+constexpr int bwd_stride = RAW ? 16 : 20;
 
 struct BwdFinalParams
 {
@@ -153,7 +157,7 @@ struct LeafPassParams
     const uint64_t* cand_vbase; // [NCL] value index of each candidate's first voxel
     const float* grad_density;
     const float* grad_color;
-    float* partials;            // [emission index][BWD_STRIDE]
+    float* partials;            // [emission index][bwd_stride]
     // reference node order: creation window of each candidate leaf
     int window;
     const uint64_t* frag_off;   // exclusive scan of footprints
@@ -189,7 +193,7 @@ void launch_leaf_cands(const uint32_t* keys, const uint32_t* vals, const uint32_
 // returns the CTAs per SM it ran with
 // (counter: zeroed by the caller)
 int launch_leaf_pass(const LeafPassParams& P, uint32_t* counter, int num_sms, cudaStream_t s, int variant = 0);
-void launch_leaf_backward(const LeafPassParams& P, int64_t Q, cudaStream_t s);
+void launch_leaf_backward(const LeafPassParams& P, int64_t Q, bool raw, cudaStream_t s);
 // vpairs non-null: only the pairs per voxel (canonical order), into it
 void launch_leaf_export(const LeafPassParams& P, uint64_t* vpairs, uint32_t* counter, int num_sms, cudaStream_t s);
 
