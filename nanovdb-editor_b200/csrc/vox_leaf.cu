@@ -1018,10 +1018,11 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         atomicMax(&A.rgba[n], a8 | __float_as_uint(al.w));
                     if constexpr (!BYTES)
                     {
-                        const float c0 = VOX_FMUL(a, q7.x), c1 = VOX_FMUL(a, q7.y), c2 = VOX_FMUL(a, q7.z);
                         if (a < 1.f && (int32_t)__float_as_uint(w3.w) >= 0)
                         {
-                            // colours in [0, 1], so terms in [0, 1): below 2^32 units (a is never negative)
+                            // the colours and the opacity in [0, 1], so alpha and terms in [0, 1):
+                            // below 2^32 units
+                            const float c0 = VOX_FMUL(a, q7.x), c1 = VOX_FMUL(a, q7.y), c2 = VOX_FMUL(a, q7.z);
                             acc_add(&A.dens[0][n], &A.dens[1][n], __float2uint_rn(VOX_FMUL(a, FX_SCALE)), 0u);
                             acc_add(&A.col[0][0][n], &A.col[0][1][n], __float2uint_rn(VOX_FMUL(c0, FX_SCALE)), 0u);
                             acc_add(&A.col[1][0][n], &A.col[1][1][n], __float2uint_rn(VOX_FMUL(c1, FX_SCALE)), 0u);
@@ -1029,10 +1030,14 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         }
                         else
                         {
+                            // near the centre of an opacity above 1 the power's base in
+                            // pair_alpha_f_ex is negative: the alpha is 0 there, as the oracle's
+                            if (!SMOOTH && af.a > 1.f)
+                                a = 0.f;
                             acc_add(&A.dens[0][n], &A.dens[1][n], fx_of_unit(a));
-                            acc_add(&A.col[0][0][n], &A.col[0][1][n], fx_of(c0));
-                            acc_add(&A.col[1][0][n], &A.col[1][1][n], fx_of(c1));
-                            acc_add(&A.col[2][0][n], &A.col[2][1][n], fx_of(c2));
+                            acc_add(&A.col[0][0][n], &A.col[0][1][n], fx_of(VOX_FMUL(a, q7.x)));
+                            acc_add(&A.col[1][0][n], &A.col[1][1][n], fx_of(VOX_FMUL(a, q7.y)));
+                            acc_add(&A.col[2][0][n], &A.col[2][1][n], fx_of(VOX_FMUL(a, q7.z)));
                         }
                     }
                     if (WINDOW)
