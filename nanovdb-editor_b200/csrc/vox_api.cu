@@ -451,6 +451,11 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     uint32_t* d_counter = (uint32_t*)(sc + SC_SCRATCH);
     cudaEventRecord(ctx->timers.ev[0], s);
 
+    // The ranks' inverse comes with the scan of the root bits, in the same launch, where
+    // a table of every root tile of every cloud stays small (128 KB per cloud, 8 MB for
+    // 64); a larger batch reads the count of touched tiles first and spends a launch.
+    const bool every_root = B <= 64;
+
     // ---------------------------------------------------------------- prep
     const float cull = cull_scale > 0.f ? cull_scale : 0.05f;
     if (!ensure(ctx, ctx->recs, sizeof(GaussRec) * (size_t)(G + 1)) || !ensure(ctx, ctx->walk, sizeof(WalkRec) * (size_t)(G + 1)) ||
@@ -458,7 +463,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         !ensure(ctx, ctx->frag_off, sizeof(uint64_t) * (size_t)(G + 1)) ||
         !ensure(ctx, ctx->root_bits, sizeof(uint64_t) * 512 * B) || !ensure(ctx, ctx->root_prefix, sizeof(uint64_t) * 512 * B) ||
         !ensure(ctx, ctx->lcols, 8 * (size_t)(G + 1)) || !ensure(ctx, ctx->lcol_off, 8 * (size_t)(G + 1)) ||
-        !ensure(ctx, ctx->root_of_rank, sizeof(uint32_t) * 32768 * (size_t)B) || // every root tile of every cloud
+        (every_root && !ensure(ctx, ctx->root_of_rank, sizeof(uint32_t) * 32768 * (size_t)B)) ||
         !ensure(ctx, ctx->scan_status, sizeof(uint64_t) * (2 * scan_status_words(G) + scan_status_words(512 * B))))
         return VOX_ERR_MEMORY;
     const int64_t* d_cloud_start = nullptr;
@@ -537,7 +542,7 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
         J.job[0] = { footprints, frag_off, G, 0, sc + SC_F, scan_status, ctr(CTR_FOOT), nullptr, 0 };
         J.job[1] = { lcols, lcol_off, G, 0, sc + SC_NLC, st1, ctr(CTR_COLS), nullptr, 0 };
         J.job[2] = { root_bits, root_prefix, 512 * B, 1, sc + SC_NROOT, st1 + scan_status_words(G), ctr(CTR_ROOT),
-                     (uint32_t*)ctx->root_of_rank.p, 0 };
+                     every_root ? (uint32_t*)ctx->root_of_rank.p : nullptr, 0 };
         scan_jobs(J, ctx->scan_epochs.next(scan_status, scan_words, s), d_err, s);
     }
     int rc = sync_scalars(ctx, "prep");
@@ -546,6 +551,12 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     const uint64_t F = ctx->hscal[SC_F];
     const uint64_t NR = ctx->hscal[SC_NROOT];
     const uint64_t NLC = ctx->hscal[SC_NLC];
+    if (!every_root)
+    {
+        if (!ensure(ctx, ctx->root_of_rank, sizeof(uint32_t) * (NR + 1)))
+            return VOX_ERR_MEMORY;
+        launch_invert_bits(root_bits, root_prefix, 512 * B, (uint32_t*)ctx->root_of_rank.p, s);
+    }
     ctx->stats.candidates = (int64_t)F;
     // one batch and at most one window: every node is created in window 0, and
     // the order by (window, parent rank, n) is the canonical one
