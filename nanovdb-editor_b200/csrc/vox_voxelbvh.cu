@@ -309,11 +309,14 @@ __device__ __forceinline__ int64_t vb_level_cells(const int lo[3], const int hi[
 // d their offsets from the mean, X the box's extent there (with a transform: M
 // = sum |lp t| + |t_3|, X through |t|), the shader's row values are within inv_r
 // sum |R| (2 |lp| + 5 |d|) (transform: 6 M + 5 |d|) of exact; this form's base
-// within the same, its B within 3 X (6 X), the sums 3 (|d| + X), the half width
-// 6 X (9 X), the difference |d| + 2 X.  delta_r = inv_r sum |R| (5 |lp| + 16 |d| +
-// 16 X), or (14 M + 16 |d| + 24 X), covers both; Delta = sum_r delta_r gives the
-// thresholds on D exactly as in the leaf test (vox_leaf.cu), and what lies
-// between them, or a Gaussian with Delta > 1/16, takes the shader's arithmetic.
+// within the same, its B (two products and 1 / sc, each rounded once) within 3 X
+// (6 X), the sums 3 (|d| + X), the half width 6 X (9 X), the difference |d| + 2 X.
+// delta_r = inv_r sum |R| (5 |lp| + 16 |d| + 16 X), or (14 M + 16 |d| + 24 X), covers
+// both; Delta = sum_r delta_r gives the thresholds on D exactly as in the leaf test
+// (vox_leaf.cu), and what lies between them, or a Gaussian with Delta > 1/16, takes
+// the shader's arithmetic.  So does one whose cells or ellipsoid are below 2^-100:
+// products that leave the normal range have roundings that are not relative (1 / sc
+// itself does from 2^126 on).
 // Everything is held halved (D quartered), so that a saturating difference is
 // max(|c| - h, 0) up to far above the threshold.
 //
@@ -414,7 +417,8 @@ __global__ void __launch_bounds__(VB_THREADS, 3) k_vb_keys(const __grid_constant
                 M[c] = XF ? 14.f * M[c] + 16.f * (fabsf(w[c]) + X[c]) + 24.f * X[c]
                           : 5.f * M[c] + 16.f * (fabsf(w[c]) + X[c]) + 16.f * X[c];
             }
-            const float rs = __fdividef(1.f, sc);
+            const float rs = __fdiv_rn(1.f, sc);
+            float big = sc;
 #pragma unroll
             for (int r = 0; r < 3; r++)
             {
@@ -426,10 +430,11 @@ __global__ void __launch_bounds__(VB_THREADS, 3) k_vb_keys(const __grid_constant
                                        : G.R[a][r];
                     B[r][a] = 0.5f * G.inv[r] * m * rs;
                 }
+                big = fmaxf(big, G.inv[r]);
                 Dl += G.inv[r] * (fabsf(G.R[0][r]) * M[0] + fabsf(G.R[1][r]) * M[1] + fabsf(G.R[2][r]) * M[2]);
             }
             Dl *= 0x1.02p-24f;
-            if (Dl <= 0.0625f) // false for NaN
+            if (Dl <= 0.0625f && big < 0x1p100f) // false for NaN
             {
                 lo_t = 0.25f * (1.f - (2.f * Dl + 0x1p-19f));
                 hi_t = 0.25f * (1.f + (2.f * Dl + Dl * Dl + 0x1p-18f));
