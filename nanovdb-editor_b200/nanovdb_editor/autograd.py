@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import numpy as np
 import torch
+from torch.utils._device import DeviceContext
 
 from .exceptions import PipelineError
 from .grid import HEADER_DTYPE
@@ -102,17 +103,25 @@ def pack_coords(ijk: torch.Tensor) -> torch.Tensor:
 
 def _plain(t: torch.Tensor, dtype: torch.dtype, device) -> bool:
     return (type(t) is torch.Tensor and t.dtype == dtype and t.device == device and t.is_contiguous()
-            and not t.requires_grad and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and not t.requires_grad and not t.is_neg() and not t._is_zerotensor()
+            and not torch._C._functorch.is_functorch_wrapped_tensor(t)
             and torch.autograd.forward_ad.unpack_dual(t).tangent is None)
+
+
+def _function_modes() -> bool:
+    # (a default device changes nothing of a call that names its devices)
+    return any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(torch._C._len_torch_function_stack()))
 
 
 def _fused_lookup(keys: torch.Tensor, density: torch.Tensor, ijk, query, want_hit: bool):
     """The library's one-pass lookup, on torch's current stream, or None where torch's operators
     have to be seen or do what the kernel does not: other devices, types and strides than the
-    grids' own, a density that is differentiated, vmap and tracing.  10.8M voxels:
+    grids' own, lazily negated or zero tensors, a density that is differentiated, vmap, tracing
+    and the function and dispatch modes.  10.8M voxels:
     0.90 ms by the operators' twelve launches, 0.18 ms by the kernel; 1.5M: 139 and 28 us."""
     src = query if ijk is None else ijk
-    if not src.is_cuda or torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack():
+    if (not src.is_cuda or torch.compiler.is_compiling() or torch.jit.is_tracing()
+            or torch._C._len_torch_dispatch_stack() or _function_modes()):
         return None
     dev = src.device
     if not (_plain(keys, torch.int64, dev) and _plain(density, torch.float32, dev)
