@@ -100,9 +100,7 @@ struct vox_context_t
     vox_stats_t stats{};
     Timers timers;
     SortTuning tuning;
-    OnlineChoice walk_choice[4] = { OnlineChoice(2), OnlineChoice(2), OnlineChoice(2), OnlineChoice(2) }; // leaf walk: 4 or 3 CTAs per SM, per mode (window | smooth << 1)
-    int walk_mode = 0;
-    int walk_variant = 0;
+    OnlineChoice walk_choice[2] = { OnlineChoice(2), OnlineChoice(2) }; // leaf walk: 4 or 3 CTAs per SM, without and with windows
     // last result
     int64_t last_P = 0;
     uint64_t last_grid_bytes = 0;
@@ -744,9 +742,11 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     LP.cand_vbase = (const uint64_t*)ctx->cand_vbase.p;
     LP.cand_voff = (const uint64_t*)ctx->cand_voff.p;
     LP.key64 = key64;
-    ctx->walk_mode = (LP.window ? 1 : 0) | (LP.smooth ? 2 : 0); // the modes differ in cost per pair
-    ctx->walk_variant = bytes ? 0 : ctx->walk_choice[ctx->walk_mode].pick((int64_t)Q);
-    ctx->stats.walk_ctas_per_sm = launch_leaf_pass(LP, ctr(CTR_WALK), ctx->num_sms, s, ctx->walk_variant);
+    // the walk of all channels has two variants, which the tuner times per size class
+    // (with windows a pair costs more); the others have one
+    OnlineChoice* walk_choice = bytes || diff || ctx->check_emit ? nullptr : &ctx->walk_choice[LP.window ? 1 : 0];
+    const int walk_variant = walk_choice ? walk_choice->pick((int64_t)Q) : 0;
+    ctx->stats.walk_ctas_per_sm = launch_leaf_pass(LP, ctr(CTR_WALK), ctx->num_sms, s, walk_variant);
     cudaEventRecord(ctx->timers.ev[4], s);
 
     // ------------------------------------------------ tree: tables and layout
@@ -907,8 +907,8 @@ static int run_voxelize(vox_context_t* ctx, const vox_gaussians_t* gs, float vox
     st.ms_emit = elapsed(ctx->timers.ev[1], ctx->timers.ev[2]);       // (leaf, Gaussian) pairs
     st.ms_sort = elapsed(ctx->timers.ev[2], ctx->timers.ev[3]);       // sort + candidate leaves
     st.ms_accumulate = elapsed(ctx->timers.ev[3], ctx->timers.ev[4]); // leaf walk: test, RGBA8, float sums
-    if (!bytes)
-        ctx->walk_choice[ctx->walk_mode].report((int64_t)Q, ctx->walk_variant, st.ms_accumulate);
+    if (walk_choice)
+        walk_choice->report((int64_t)Q, walk_variant, st.ms_accumulate);
     st.ms_build = elapsed(ctx->timers.ev[4], ctx->timers.ev[6]);      // topology, values, node2
     st.ms_total = elapsed(ctx->timers.ev[0], ctx->timers.ev[6]);
     st.kernel_launches = launch_count() - launches0;
