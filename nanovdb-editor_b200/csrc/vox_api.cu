@@ -5,9 +5,10 @@
 // 256K-prim x 8M-fragment windows with a per-window queue flush and a
 // frame-lagged readback of the fragment total (raster/Raster.cpp:420-558,
 // raster/GridBuild.cpp:830-942).  Here one call runs the whole chain on one
-// CUDA stream; five times the host waits for counts that size the next buffers
-// (sync_scalars).  Buffers persist in the context and only grow, so repeated
-// calls allocate nothing.
+// CUDA stream.  Four times the host waits for counts that size the next buffers
+// (sync_scalars), and once at the end, after two copies of the grids' offsets to
+// pageable memory, which return when they are done.  Buffers persist in the
+// context and only grow, so repeated calls allocate nothing.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -96,7 +97,6 @@ struct vox_context_t
     int check_sort = 0; // VOX_CHECK_SORT=1: validate key order after every sort
     int check_emit = 0; // VOX_CHECK_EMIT=1: also walk the leaves the leaf test culls; a pass there is an error
     int key64 = 0;
-    int sorted_in_alt = 0;
     vox_stats_t stats{};
     Timers timers;
     SortTuning tuning;
@@ -135,7 +135,6 @@ enum
     SC_NLC,  // leaf columns
     SC_Q,    // (leaf, Gaussian) pairs
     SC_NCL,  // candidate leaves
-    SC_NVOX, // active voxels from the leaf masks
     SC_NWIN, // reference fragment windows (window order)
     SC_VBU,  // VoxelBVH: used key slots
     SC_BBOX, // 3 words (6 int32)

@@ -78,10 +78,6 @@ __device__ __forceinline__ uint32_t lower_n_of(int32_t x, int32_t y, int32_t z)
 {
     return ((((uint32_t)x & 0x7Fu) >> 3) << 8) | ((((uint32_t)y & 0x7Fu) >> 3) << 4) | (((uint32_t)z & 0x7Fu) >> 3);
 }
-__device__ __forceinline__ uint32_t leaf_n_of(int32_t x, int32_t y, int32_t z)
-{
-    return (((uint32_t)x & 7u) << 6) | (((uint32_t)y & 7u) << 3) | ((uint32_t)z & 7u);
-}
 
 // rank of bit idx among the set bits of a bitmap with per-word exclusive
 // popcount prefixes
@@ -506,7 +502,6 @@ struct __align__(16) WalkRec
     float4 w5; // lo_t, the colour bytes of the RGBA8 value, voxel size, 1 where a voxel centre's offset from mu
                // is exact in double (smooth_kernel)
 };
-constexpr int WALK_WORDS = 6; // 16-byte words of a WalkRec
 
 // the anchor of the float channels' AABB along one axis (leaf origin o)
 // (bbox minimum bmin, extent range = max + 1 - min)
@@ -865,21 +860,6 @@ __device__ __forceinline__ float fx_to_float(unsigned long long s)
     return VOX_FMUL(__ll2float_rn((long long)s), FX_INV);
 }
 
-
-__device__ __forceinline__ uint32_t pack_rgba8(const GaussRec& R, float a)
-{
-    float ch[4] = { R.q7.x, R.q7.y, R.q7.z, a };
-    uint32_t out = 0;
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-    {
-        float v = ch[c] < 1.f ? ch[c] : 1.f;
-        v = 0.f > v ? 0.f : v;
-        out |= ((uint32_t)VOX_FMUL(255.f, v)) << (8 * c);
-    }
-    return out;
-}
-
 // ------------------------------------------------------------------------
 // decoupled look-back status words: [63:56] epoch, [55] inclusive flag,
 // [54:0] value.  Epoch 0 means "not yet written in this use".  Values are
@@ -1148,7 +1128,6 @@ __device__ __forceinline__ uint64_t block_excl_scan_u64(uint64_t v, uint64_t* s_
 constexpr int ERR_LOOKBACK = 1;
 constexpr int ERR_RANGE = 2;      // voxel coordinate outside [-65536, 65535]
 constexpr int ERR_FOOTPRINT = 4;  // one Gaussian's bbox above 2^31 fragments
-constexpr int ERR_CAPACITY = 8;   // pair buffer too small (host retries)
 constexpr int ERR_ORDER = 16;     // keys found out of order after the sort
 constexpr int ERR_BOUNDS = 32;    // an index check failed; the access was skipped
 

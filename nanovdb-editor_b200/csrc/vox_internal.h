@@ -19,28 +19,6 @@ void context_rgba8_only(vox_context_t* ctx);
 int64_t launch_count();
 void count_launch();
 
-// Bump allocator over one device arena; grows (re-allocates) between calls only.
-struct Arena
-{
-    char* base = nullptr;
-    size_t cap = 0;
-    size_t used = 0;
-    void reset()
-    {
-        used = 0;
-    }
-    template <class T>
-    T* take(size_t count, size_t align = 256)
-    {
-        size_t off = (used + align - 1) / align * align;
-        size_t bytes = count * sizeof(T);
-        if (off + bytes > cap)
-            return nullptr;
-        used = off + bytes;
-        return reinterpret_cast<T*>(base + off);
-    }
-};
-
 // Look-back bookkeeping: each user owns a status region and an epoch counter
 // so that regions need no clearing between uses (epoch wraps every 255 uses,
 // at which point the region is cleared once).

@@ -453,7 +453,6 @@ __global__ void k_canonical_order(NodeParams N, uint64_t U)
     }
 }
 
-// per cloud: the grid header (vox_grid_header_t) and the bbox blind data
 // ------------------------------------------------------------ node2 write ----
 // Node2 roots, uppers and lowers, headers and the gaps between a grid's parts,
 // in one launch.  A CTA writes a stretch of NODE_PART words of one node (a root

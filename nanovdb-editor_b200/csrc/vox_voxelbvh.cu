@@ -20,7 +20,7 @@
 //                       order in fewer radix passes, and compacted (the
 //                       unused slots, all-ones key and id, are the sorted tail)
 //   (sort)              stable LSD sort of the used compressed keys (of all
-//                       64-bit keys when a cell lies outside [0, 2^15))
+//                       64-bit keys when a cell lies outside [0, 2^16))
 //   k_vb_ranges         headers [2r] = start, [2r + 1] = end (the others are
 //                       zero), the sorted keys as 64-bit keys, the unused
 //                       tail's keys and ids all ones, its run the last range
