@@ -497,7 +497,8 @@ struct __align__(16) WalkRec
     float4 w1; // half y steps, h_0
     float4 w2; // half z steps, h_1
     float4 w3; // 2 dab_0..2 and sum_r dab_r^2, raised by 2^-19 (alpha_byte_bound); the sum negative
-               // (sign bit set) when a colour lies outside [0, 1] or the opacity above 1
+               // (sign bit set) when a colour lies outside [0, 1], the opacity above 1 or the
+               // opacity transform's exponent is infinite
     float4 w4; // k_0..2, h_2
     float4 w5; // lo_t, the colour bytes of the RGBA8 value, voxel size, 1 where a voxel centre's offset from mu
                // is exact in double (smooth_kernel)
@@ -566,9 +567,13 @@ __device__ __forceinline__ WalkRec walk_record(const GaussRec& R, float vs)
         hi_t = 0.25f * (1.f + (2.f * Dl + Dl * Dl + 0x1p-18f));
     }
     const uint32_t rgb24 = rgba8_byte(R.q7.x) | (rgba8_byte(R.q7.y) << 8) | (rgba8_byte(R.q7.z) << 16);
+    // voxels below 1e-22: the squared scales underflow and the transform's exponent is infinite.  No byte is
+    // bounded then (an infinite md)
+    const bool finite_e = finite_f(R.q6.z);
     const bool unit = R.q7.x >= 0.f && R.q7.x <= 1.f && R.q7.y >= 0.f && R.q7.y <= 1.f && R.q7.z >= 0.f &&
-                      R.q7.z <= 1.f && R.q6.x <= 1.f;
-    const float up = 1.f + 0x1p-19f, dd = (dab[0] * dab[0] + dab[1] * dab[1] + dab[2] * dab[2]) * up;
+                      R.q7.z <= 1.f && R.q6.x <= 1.f && finite_e;
+    const float up = 1.f + 0x1p-19f;
+    const float dd = finite_e ? (dab[0] * dab[0] + dab[1] * dab[1] + dab[2] * dab[2]) * up : __int_as_float(0x7f800000);
     WalkRec o;
     o.w0 = make_float4(hA[0][0], hA[1][0], hA[2][0], hi_t);
     o.w1 = make_float4(hA[0][1], hA[1][1], hA[2][1], h[0]);
@@ -620,12 +625,12 @@ __device__ __forceinline__ Aabb stable_leaf_aabb(const float lo0[3], const float
     return b;
 }
 
-// vox_expf_ch and vox_powf_ch (x <= 0; b in [0, 1], e >= 0), the same results from
-// cheaper instructions: floor as an addition rounded down to the integers'
-// binade (|x / ln2| < 2^22) instead of the conversion unit's floor and
-// float-to-int, 2^k from that sum's low bits, the exponent split with one
-// integer add (mantissas above sqrt(2)'s carry into the exponent).  The cases
-// b = 0 and b = 1 fold: log(1) = 0 and exp(0) = 1 come out exactly.
+// vox_expf_ch and vox_powf_ch (x <= 0; b in [0, 1], e >= 0, and not b = 1 with e
+// infinite), the same results from cheaper instructions: floor as an addition
+// rounded down to the integers' binade (|x / ln2| < 2^22) instead of the conversion
+// unit's floor and float-to-int, 2^k from that sum's low bits, the exponent split
+// with one integer add (mantissas above sqrt(2)'s carry into the exponent).  The
+// cases b = 0 and b = 1 fold: log(1) = 0 and exp(0) = 1 come out exactly.
 __device__ __forceinline__ float expf_ch_dev(float x)
 {
     const float xc = fmaxf(x, -87.3f);

@@ -1030,9 +1030,11 @@ __global__ void __launch_bounds__(LP_THREADS, MINB) k_leaf_pass(LeafPassParams P
                         }
                         else
                         {
-                            // near the centre of an opacity above 1 the power's base in
-                            // pair_alpha_f_ex is negative: the alpha is 0 there, as the oracle's
-                            if (!SMOOTH && af.a > 1.f)
+                            // where the power's base b in pair_alpha_f_ex is negative (near the
+                            // centre of an opacity above 1), or 1 with an infinite exponent, the
+                            // alpha is 0, as the oracle's (a base of 1 and a finite one give 0 too)
+                            const float b = VOX_FSUB(1.f, af.a);
+                            if (!SMOOTH && (b < 0.f || b == 1.f))
                                 a = 0.f;
                             acc_add(&A.dens[0][n], &A.dens[1][n], fx_of_unit(a));
                             acc_add(&A.col[0][0][n], &A.col[0][1][n], fx_of(VOX_FMUL(a, q7.x)));
